@@ -34,8 +34,10 @@ __device__ __forceinline__ int quantize_code(T x, T zero, T scale) {
 // Two gathered values travel in one 32-bit register.  Every step reproduces, per 16-bit half, exactly
 // what the scalar chain hsub -> hdiv -> half2int_rn -> clamp of the reference kernel produces:
 //   * __hsub2 rounds each half like __hsub;
-//   * __hdiv(a, b) is half(rcp.approx.ftz(b) * float(a)) plus a refinement that only touches quotients
-//     of magnitude below 2^-17, which become code 0 with or without it -- so the refinement is skipped;
+//   * the quotient of two fp16 numbers, rounded to fp16, is the fp16 rounding of the fp32 product with the correctly rounded
+//     fp32 reciprocal: a quotient of 11-bit significands never lies close enough to a rounding boundary for the product's
+//     error to matter (all 2^20 pairs of significands are checked in tests/test_host_logic.py), so one reciprocal per row
+//     replaces a division per value;
 //   * clamping the quotient to [0, 2^b - 1] before rounding equals clamping after (the bounds are
 //     integers and rounding is monotone; NaN turns into 0 either way);
 //   * adding 1024 in fp16 leaves round-to-nearest-even(q) in the low mantissa bits (ulp is 1 there).
@@ -259,8 +261,7 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
 
   // ---- pass 2: quantize + pack
   uint8_t *drow = dst + (size_t)r * (kPacked ? (size_t)(num_int >> 1) : (size_t)num_int);
-  float rcp_scale;
-  asm("{rcp.approx.ftz.f32 %0, %1;\n}" : "=f"(rcp_scale) : "f"(Traits<T>::to_float(scale)));
+  const float rcp_scale = __frcp_rn(Traits<T>::to_float(scale));
   auto emit = [&](int c, const uint32_t (&p)[4]) {
     uint32_t w0, w1;
     if (Traits<T>::kIsHalf) {

@@ -2,6 +2,7 @@
 import os
 
 import pytest
+import numpy as np
 import torch
 
 from oracle import fakequant, kernel_path as kp
@@ -163,3 +164,14 @@ def test_diagnostics_and_bench_import_without_a_gpu():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, os.path.join(root, "bench.py"), "--help"], capture_output=True, text=True)
     assert r.returncode == 0 and "--tp-copy" in r.stdout and "--stream-ring" in r.stdout
+
+
+def test_reciprocal_product_rounds_like_the_fp16_quotient():
+    """The quantizer multiplies by the fp32 reciprocal of the scale instead of dividing: for every pair of fp16 significands
+    and every exponent difference that gives a quotient between 2^-11 and 2^10 the product rounds to the same fp16 value as the
+    quotient (which fp32 division followed by rounding to fp16 gives exactly: 24 >= 2 * 11 + 2 bits)."""
+    sig = ((1024 + np.arange(1024)) / 1024).astype(np.float32)
+    rcp = np.float32(1) / sig
+    for e in range(-11, 10):
+        d = sig * np.float32(2.0 ** e)
+        assert np.array_equal((d[:, None] / sig[None, :]).astype(np.float16), (d[:, None] * rcp[None, :]).astype(np.float16))
