@@ -63,11 +63,8 @@ extern "C" {
  * it waits for the predecessor's completion before its first global load or store, so results are those of
  * plain stream order; 0 launches in plain stream order. */
 #define QUIK_CFG_PDL           5
-/* Threads that issue the integer products of a tile in the tcgen05 engine with both operands in shared memory: 1
- * (default) a single thread issues everything; 2 two threads share the k-slices of every block of a long sum
- * (K_int >= 2048) and accumulate into the same tensor-memory accumulator (integer sums do not depend on the order of
- * their terms; the outlier product stays on one thread).  One thread cannot issue these instructions as fast as the
- * tensor pipe could execute them, but under the board's power limit the second thread was measured to gain 1-2 %. */
+/* Accepted (1 or 2) for callers that set it and without effect: one warp issues every product of the tcgen05 engine, which
+ * keeps the tensor pipe busy (512 to 545 cycles per 256 x 256 x 128 block of a CTA pair, 512 being the pipe's own time). */
 #define QUIK_CFG_MMA_ISSUERS   6
 /* 1: the tiled tcgen05 engine loads its token operand (re-read by every column tile, small enough for L2) with an L2
  * evict-last hint, so that data streaming through L2 meanwhile does not push it out; 0 (default): plain loads. */

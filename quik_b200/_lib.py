@@ -147,7 +147,7 @@ def set_small_m(mode) -> None:
 
 
 def set_mma_issuers(n: int) -> None:
-    """1 or 2 threads issue the integer products of a tile (tcgen05 engine with both operands in shared memory)."""
+    """Accepted (1 or 2) and without effect: one warp issues all products of the tcgen05 engine at the tensor pipe's rate."""
     check(load().quik_config_set(CFG_MMA_ISSUERS, int(n)), "quik_config_set")
 
 

@@ -39,14 +39,13 @@ __device__ unsigned int g_device_status = 0;
 
 namespace {
 
-constexpr int NUM_THREADS = 352;              // TMA warp + MMA warp + 8 epilogue warps + second MMA warp
-constexpr int SECOND_ISSUER_WARP = 10;
+constexpr int NUM_THREADS = 320;              // TMA warp + MMA warp + 8 epilogue warps
 // Process-wide tuning knobs (quik_config_set): plain words, meant to be set once before the layers run; a
 // launch reads each of them once.
 std::atomic<int> g_tile_n{0};                                 // 0 = choose by shape, else a multiple of 16 in [32, 256]
 std::atomic<int> g_cta_pair{0};                               // 0 = by shape, 1 = never, 2 = always
 std::atomic<int> g_l2_hint{0};                                // 1 = token-operand loads carry an L2 evict-last hint
-std::atomic<int> g_issuers{1};                                // threads that issue the integer products of a tile (1 or 2)
+std::atomic<int> g_issuers{1};                                // kept for callers of QUIK_CFG_MMA_ISSUERS; no effect
 std::atomic<unsigned long long *> g_dbg{nullptr};             // diagnostic counters (device memory), off by default
 
 // Shared-memory plan after the 1024-byte aligned ring of stages: 256 bytes of barriers etc. and the
@@ -103,8 +102,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   uint64_t *acc_empty = acc_full + 2;                                  // [2] region free again
   uint64_t *fp_full = acc_empty + 2;                                   // [2] outlier product complete
   uint64_t *fp_drained = fp_full + 2;                                  // [2] outlier product parked
-  uint64_t *int_started = fp_drained + 2;                              // [2] first integer k-block of the tile complete
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(int_started + 2);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fp_drained + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // per-column epilogue vectors, one private copy per epilogue warp (no cross-warp barrier needed)
   float *s_vec = reinterpret_cast<float *>(aux + 256);                 // [8][3][HALF_CAP], 16-byte aligned
@@ -117,11 +115,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(full_bar + s), 1);
-      mbar_init(smem_u32(empty_bar + s), p.issuers);                 // every issuing thread commits the stage
+      mbar_init(smem_u32(empty_bar + s), 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(smem_u32(int_started + s), 1);
-      mbar_init(smem_u32(acc_full + s), p.issuers);
+      mbar_init(smem_u32(acc_full + s), 1);
       mbar_init(smem_u32(acc_empty + s), NUM_EPI_THREADS * CTAS);    // epilogue threads of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
       mbar_init(smem_u32(fp_drained + s), NUM_EPI_THREADS * CTAS);
@@ -154,22 +151,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
   if (warp == 0) {
     // ================= TMA producer =================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      // The token operand A is read again by every column tile of the launch and fits in L2: its lines are marked to
-      // be evicted last, so that data streaming through L2 meanwhile (the weights, the outputs, a tensor-parallel
-      // rank's peer copies) does not push it out.
-      const uint64_t keep = l2_policy_evict_last();
-      const bool hint = p.l2_hint != 0;
-      // one k-block range of one product of tile j into the ring
-      auto feed = [&](int j, bool fp, int kb0, int kb1) {
-        const int tile = unit + j * num_units;
-        const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M;      // this CTA's rows of A
-        const int n0 = (tile / p.num_m_tiles) * bn + rank * b_rows;           // this CTA's rows of B
-        for (int kb = kb0; kb < kb1 && ok; ++kb) {
-          if (!mbar_wait(smem_u32(empty_bar + stage), phase ^ 1, abort_flag, p.status)) { ok = false; break; }
+    const bool elected = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    // The token operand A is read again by every column tile of the launch and fits in L2: its lines are marked to
+    // be evicted last, so that data streaming through L2 meanwhile (the weights, the outputs, a tensor-parallel
+    // rank's peer copies) does not push it out.
+    const uint64_t keep = l2_policy_evict_last();
+    const bool hint = p.l2_hint != 0;
+    // one k-block range of one product of tile j into the ring
+    auto feed = [&](int j, bool fp, int kb0, int kb1) {
+      const int tile = unit + j * num_units;
+      const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M;      // this CTA's rows of A
+      const int n0 = (tile / p.num_m_tiles) * bn + rank * b_rows;           // this CTA's rows of B
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(smem_u32(empty_bar + stage), phase ^ 1, abort_flag, p.status);
+        if (!ok) return;
+        if (elected) {
           const uint32_t fb = smem_u32(full_bar + stage);
           const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
           if (rank == 0) mbar_expect_tx(fb, stage_tx);
@@ -181,89 +180,85 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             else tma_load_2d<CTAS>(sa, &tmap_a, fb, kb * STAGE_K_BYTES, m0);
             tma_load_2d<CTAS>(sa + A_BYTES, &tmap_b, fb, kb * STAGE_K_BYTES, n0);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-      };
-      if (HAS_FP && n_local > 0) feed(0, true, 0, p.fp_kb);
-      for (int j = 0; j < n_local && ok; ++j) {
-        feed(j, false, 0, int_half);
-        if (HAS_FP && j + 1 < n_local) feed(j + 1, true, 0, p.fp_kb);
-        feed(j, false, int_half, p.int_kb);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+    };
+    if (HAS_FP && n_local > 0) feed(0, true, 0, p.fp_kb);
+    for (int j = 0; j < n_local && ok; ++j) {
+      feed(j, false, 0, int_half);
+      if (HAS_FP && ok && j + 1 < n_local) feed(j + 1, true, 0, p.fp_kb);
+      if (ok) feed(j, false, int_half, p.int_kb);
     }
-  } else if (warp == 1 || warp == SECOND_ISSUER_WARP) {
-    // ================= MMA issuers (pair leader only) =================
-    // One thread issues tcgen05.mma with both operands in shared memory no faster than every ~217 cycles (measured,
-    // whatever the instruction's size), the tensor pipe needs 128 for the largest one; two threads together reach
-    // ~153 in isolation.  Inside this kernel the second thread gains 1-2 % only (the GPU runs into its power limit and
-    // lowers the clock instead), so one thread is the default and two are an option (QUIK_CFG_MMA_ISSUERS).
-    // With p.issuers == 2 the threads share the integer k-blocks of a tile: thread 0 takes the 32-byte slices
-    // 0 and 2 of each block, thread 1 the slices 1 and 3, both into the tile's accumulator.  Integer sums do not
-    // depend on the order of their terms, and the tensor pipe applies the multiply-accumulates of one accumulator one
-    // after the other whoever issued them (no update is lost: tests/test_gpu_b_matmul.py holds exact products of
-    // long sums against the oracle for this mode).  What does need an order is kept on thread 0: the first block of a
-    // tile (its first instruction overwrites the accumulator; thread 1 waits until that block is complete before its
-    // first instruction of the tile) and the outlier product (floating point: one fixed order).
-    const int me = warp == 1 ? 0 : 1;
-    if (lane == 0 && rank == 0 && me < p.issuers) {
-      const bool shared_work = p.issuers == 2;
+    __syncwarp();
+  } else if (warp == 1) {
+    // ================= MMA issuer (pair leader only) =================
+    // The whole warp walks the loop and one elected lane issues.  Loop exits are warp votes, so stage, phase and the
+    // descriptors made from them are uniform over the warp.  (With the loop inside a `lane == 0` branch whose exits
+    // depended on that lane's waits, one instruction left every ~217 cycles: a 256 x 256 x 128 block took 850 to 970
+    // cycles, now 512 to 545, the tensor pipe itself needing 512.  Llama-2-70B gate+up at 4096 tokens: 1845 -> 1440 us
+    // sustained, 7B qkv at 2048 tokens: 122 -> 102 us.)
+    if (rank == 0) {
+      const bool elected = elect_one();
+      const bool dbg = p.dbg != nullptr;
+      const uint64_t da0 = make_smem_desc(smem_u32(tiles)), db0 = make_smem_desc(smem_u32(tiles) + A_BYTES);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       long long w_region = 0, w_full = 0;
       const long long t_begin = clock64();
-      auto issue = [&](int j, bool fp, int kb0, int kb1) {
-        const int r = j & 1;
-        const uint32_t use_parity = (uint32_t)(j >> 1) & 1u;
-        const uint32_t d = tmem_base + r * CAP_N;
-        for (int kb = kb0; kb < kb1 && ok; ++kb) {
-          if (kb == 0 && me == 0) {
-            // the region must be free: after the previous tile's epilogue (outlier product, or
-            // integer product of an outlier-free layer), or after this tile's drain
-            const bool after_drain = HAS_FP && !fp;
-            const uint32_t bar = smem_u32((after_drain ? fp_drained : acc_empty) + r);
-            const long long t0 = clock64();
-            if (!mbar_wait(bar, after_drain ? use_parity : (use_parity ^ 1u), abort_flag, p.status)) { ok = false; break; }
-            w_region += clock64() - t0;
-            tc_fence_after();
-          }
-          if (!fp && kb == 1 && me == 1) {
-            if (!mbar_wait(smem_u32(int_started + r), use_parity, abort_flag, p.status)) { ok = false; break; }
-            tc_fence_after();
-          }
-          const long long t1 = clock64();
-          if (!mbar_wait(smem_u32(full_bar + stage), phase, abort_flag, p.status)) { ok = false; break; }
-          w_full += clock64() - t1;
-          tc_fence_after();
-          const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
-          const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + A_BYTES);
-          const bool alone = !shared_work || fp || kb == 0;       // thread 0 issues the whole block
-          if (!alone || me == 0) {
+      // one k-block of one product into the accumulator at `d`
+      auto block = [&](bool fp, uint32_t d, uint32_t idesc, bool first) {
+        const long long t1 = dbg ? clock64() : 0;
+        ok = mbar_wait_warp(smem_u32(full_bar + stage), phase, abort_flag, p.status);
+        if (dbg) w_full += clock64() - t1;
+        if (!ok) return;
+        tc_fence_after();
+        if (elected) {
+          // stage bases and 32-byte K steps inside the swizzled row are offsets of the 16-byte start-address field
+          const uint64_t da = da0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
-            for (int k = 0; k < STAGE_K_BYTES / 32; ++k) {
-              if (!alone && (k & 1) != me) continue;
-              // +32 bytes of K inside the swizzled row = +2 in the 16-byte start-address field
-              const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
-              if (fp) mma_f16<CTAS>(d, da + 2 * k, db + 2 * k, p.idesc_fp, accumulate);
-              else mma_i8<CTAS>(d, da + 2 * k, db + 2 * k, p.idesc_int, accumulate);
-            }
+          for (int k = 0; k < STAGE_K_BYTES / 32; ++k) {
+            if (fp) mma_f16<CTAS>(d, da + 2 * k, db + 2 * k, idesc, (k > 0 || !first) ? 1u : 0u);
+            else mma_i8<CTAS>(d, da + 2 * k, db + 2 * k, idesc, (k > 0 || !first) ? 1u : 0u);
           }
-          if (shared_work && me == 0 && !fp && kb == 0) mma_commit<CTAS>(smem_u32(int_started + r));
-          mma_commit<CTAS>(smem_u32(empty_bar + stage));    // stage reusable once these MMAs retire (every issuer arrives)
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          if (fp && kb == p.fp_kb - 1 && me == 0) mma_commit<CTAS>(smem_u32(fp_full + r));
-          if (!fp && kb == p.int_kb - 1) mma_commit<CTAS>(smem_u32(acc_full + r));
+          mma_commit<CTAS>(smem_u32(empty_bar + stage));    // stage reusable once these MMAs retire
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       };
-      if (HAS_FP && n_local > 0) issue(0, true, 0, p.fp_kb);
+      // waits until the accumulator region may be overwritten: after the previous tile's epilogue (outlier product, or
+      // integer product of an outlier-free layer), or after this tile's drain
+      auto region_free = [&](uint64_t *bar, uint32_t parity) {
+        const long long t0 = dbg ? clock64() : 0;
+        ok = mbar_wait_warp(smem_u32(bar), parity, abort_flag, p.status);
+        if (dbg) w_region += clock64() - t0;
+        tc_fence_after();
+      };
+      auto issue_fp = [&](int j) {
+        const int r = j & 1;
+        region_free(acc_empty + r, ((uint32_t)(j >> 1) & 1u) ^ 1u);
+        for (int kb = 0; kb < p.fp_kb && ok; ++kb) block(true, tmem_base + r * CAP_N, p.idesc_fp, kb == 0);
+        if (ok && elected) mma_commit<CTAS>(smem_u32(fp_full + r));
+      };
+      auto issue_int = [&](int j, int kb0, int kb1) {
+        const int r = j & 1;
+        for (int kb = kb0; kb < kb1 && ok; ++kb) block(false, tmem_base + r * CAP_N, p.idesc_int, kb == 0);
+      };
+      if (HAS_FP && n_local > 0) issue_fp(0);
       for (int j = 0; j < n_local && ok; ++j) {
-        issue(j, false, 0, int_half);
-        if (HAS_FP && j + 1 < n_local) issue(j + 1, true, 0, p.fp_kb);
-        issue(j, false, int_half, p.int_kb);
+        const uint32_t use_parity = (uint32_t)(j >> 1) & 1u;
+        if (HAS_FP) region_free(fp_drained + (j & 1), use_parity);
+        else region_free(acc_empty + (j & 1), use_parity ^ 1u);
+        if (!ok) break;
+        issue_int(j, 0, int_half);
+        if (HAS_FP && j + 1 < n_local && ok) issue_fp(j + 1);
+        if (!ok) break;
+        issue_int(j, int_half, p.int_kb);
+        if (ok && elected) mma_commit<CTAS>(smem_u32(acc_full + (j & 1)));
       }
-      if (p.dbg && me == 0) {
+      if (dbg && lane == 0) {
         unsigned long long *d = p.dbg + (size_t)blockIdx.x * 16;
-        d[0] = (unsigned long long)(clock64() - t_begin);   // MMA thread: issue loop
+        d[0] = (unsigned long long)(clock64() - t_begin);   // MMA warp: issue loop
         d[1] = (unsigned long long)w_region;                // ... waiting for a free accumulator region
         d[2] = (unsigned long long)w_full;                  // ... waiting for operands
         d[3] = (unsigned long long)n_local;
@@ -516,9 +511,6 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   p.idesc_int = make_idesc(2, 1, tile_m, block_n);                              // S32 accumulate, signed 8-bit operands
   p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, tile_m, block_n);   // F32 accumulate, F16 / BF16 operands
   p.acc_shift = 0;
-  // two issuing threads only for long sums: a thread can run at most one ring of stages ahead of the other, which must
-  // stay well inside one tile for the per-tile barriers that both arrive on
-  p.issuers = (g_issuers.load() >= 2 && p.int_kb >= 16) ? 2 : 1;
   p.l2_hint = g_l2_hint.load();
 
   CUtensorMap ta, tb, tfa, tfb;

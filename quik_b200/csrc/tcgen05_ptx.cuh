@@ -76,6 +76,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
+// The same wait by a whole warp, with one answer for all lanes.  A loop whose exits depend on such votes keeps its counters
+// uniform over the warp, so descriptors and barrier addresses derived from them stay in uniform registers.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                               unsigned int *status_word) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status_word));
+}
+// true in exactly one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // In a CTA pair the shared::cluster address of CTA 1 differs from CTA 0's in bit 24; clearing it
 // turns the address of a local barrier into the address of the leader's barrier at the same offset.
 constexpr uint32_t LEADER_ADDR_MASK = 0xFEFFFFFFu;
