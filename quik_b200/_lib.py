@@ -5,6 +5,7 @@ The library must be present: there is no CPU or eager fallback.  Build it with
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 
@@ -77,6 +78,26 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (quik_b200._host, csrc/host_ext.cpp), connected to the library's functions once."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError(f"quik_b200._host is missing or does not load ({e}): build it with "
+                               "`python -m quik_b200.build`") from e
+        mod.init(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
+            "quik_asym_quantize_u16", "quik_rmsnorm_quantize_u16", "quik_silu_mul_quantize_u16", "quik_mixed_linear_ld",
+            "quik_strerror", "quik_last_cuda_error", "quik_config_get")))
+        _host = mod
+    return _host
+
+
 def check(status: int, what: str) -> None:
     """Turn a status code into the RuntimeError the reference would raise (TORCH_CHECK)."""
     if status != QUIK_OK:
@@ -99,7 +120,15 @@ def ptr(t) -> int | None:
 
 
 def stream_of(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+_HERE_ALREADY = contextlib.nullcontext()
+
+
+def on_device(t: torch.Tensor):
+    """Context in which the device of ``t`` is current; costs nothing where it is already."""
+    return _HERE_ALREADY if torch.cuda.current_device() == t.get_device() else torch.cuda.device(t.device)
 
 
 def require_cuda_contiguous(op: str, **tensors) -> None:

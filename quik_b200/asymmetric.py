@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._lib import check, dtype_code, load, ptr, require_cuda_contiguous, stream_of
+from ._lib import check, dtype_code, host, load, on_device, ptr, require_cuda_contiguous, stream_of
 
 __all__ = ["quantize", "quantizeOld", "dequantize", "find_meta", "int4FusedDequantize",
            "int8FusedDequantize", "int4SpFusedDequantize", "int8SpFusedDequantize", "quantize_u16"]
@@ -32,7 +32,7 @@ def quantize(src, int_indices, fp_indices, bits):
         raise RuntimeError("Quantize: number of fp and int columns is not equal to total number of columns")
     if num_int % 2 != 0:
         raise RuntimeError("Quantize: number of int columns has to be even (implementation detail)")
-    with torch.cuda.device(src.device):
+    with on_device(src):
         if bits == 4:
             dst = torch.empty((rows, num_int // 2), dtype=torch.uint8, device=src.device)
         else:
@@ -48,68 +48,18 @@ def quantize(src, int_indices, fp_indices, bits):
 def quantize_u16(src, int_indices_u16, fp_indices_u16, bits, wide):
     """Layer-internal form of :func:`quantize`: 16-bit column ids (stored in int16 tensors) and an
     optional one-code-per-byte layout for 4-bit codes (the tensor-core GEMM operand)."""
-    require_cuda_contiguous("quantize", src=src, int_indices=int_indices_u16, fp_indices=fp_indices_u16)
-    _check_bits(bits)
-    rows, cols = src.shape
-    num_int, num_fp = int_indices_u16.numel(), fp_indices_u16.numel()
-    with torch.cuda.device(src.device):
-        if bits == 4 and not wide:
-            dst = torch.empty((rows, num_int // 2), dtype=torch.uint8, device=src.device)
-        else:
-            dst = torch.empty((rows, num_int), dtype=torch.int8, device=src.device)
-        meta = torch.empty((2 * rows,), dtype=src.dtype, device=src.device)
-        fp_x = torch.empty((rows, num_fp), dtype=src.dtype, device=src.device)
-        check(load().quik_asym_quantize_u16(ptr(src), dtype_code(src.dtype), rows, cols, ptr(int_indices_u16), num_int,
-                                            ptr(fp_indices_u16), num_fp, bits, int(bool(wide)), ptr(dst), ptr(meta),
-                                            ptr(fp_x), stream_of(src)), "quantize")
-    return dst, meta, fp_x
-
-
-def _alloc_quantized(src, num_int, num_fp, bits, wide):
-    rows = src.shape[0]
-    if bits == 4 and not wide:
-        dst = torch.empty((rows, num_int // 2), dtype=torch.uint8, device=src.device)
-    else:
-        dst = torch.empty((rows, num_int), dtype=torch.int8, device=src.device)
-    meta = torch.empty((2 * rows,), dtype=src.dtype, device=src.device)
-    fp_x = torch.empty((rows, num_fp), dtype=src.dtype, device=src.device)
-    return dst, meta, fp_x
+    return host().quantize(0, src, None, 0.0, int_indices_u16, fp_indices_u16, bits, wide)
 
 
 def rmsnorm_quantize_u16(x, norm_weight, eps, int_indices_u16, fp_indices_u16, bits, wide):
     """quantize_u16(rmsnorm(x) * norm_weight) in one pass over ``x``: the normalised matrix is never written
     (LlamaRMSNorm arithmetic: fp32 statistics, rounded to x.dtype, times the weight in x.dtype)."""
-    require_cuda_contiguous("rmsnorm_quantize", x=x, norm_weight=norm_weight, int_indices=int_indices_u16,
-                            fp_indices=fp_indices_u16)
-    _check_bits(bits)
-    rows, cols = x.shape
-    if norm_weight.numel() != cols or norm_weight.dtype != x.dtype:
-        raise RuntimeError("rmsnorm_quantize: norm_weight must have one entry per column, of x's dtype")
-    num_int, num_fp = int_indices_u16.numel(), fp_indices_u16.numel()
-    with torch.cuda.device(x.device):
-        dst, meta, fp_x = _alloc_quantized(x, num_int, num_fp, bits, wide)
-        check(load().quik_rmsnorm_quantize_u16(ptr(x), ptr(norm_weight), float(eps), dtype_code(x.dtype), rows, cols,
-                                               ptr(int_indices_u16), num_int, ptr(fp_indices_u16), num_fp, bits,
-                                               int(bool(wide)), ptr(dst), ptr(meta), ptr(fp_x), stream_of(x)),
-              "rmsnorm_quantize")
-    return dst, meta, fp_x
+    return host().quantize(1, x, norm_weight, eps, int_indices_u16, fp_indices_u16, bits, wide)
 
 
 def silu_mul_quantize_u16(gate, up, int_indices_u16, fp_indices_u16, bits, wide):
     """quantize_u16(silu(gate) * up) in one pass over ``gate`` and ``up``: the activated matrix is never written."""
-    require_cuda_contiguous("silu_mul_quantize", gate=gate, up=up, int_indices=int_indices_u16, fp_indices=fp_indices_u16)
-    _check_bits(bits)
-    if gate.shape != up.shape or gate.dtype != up.dtype:
-        raise RuntimeError("silu_mul_quantize: gate and up must have the same shape and dtype")
-    rows, cols = gate.shape
-    num_int, num_fp = int_indices_u16.numel(), fp_indices_u16.numel()
-    with torch.cuda.device(gate.device):
-        dst, meta, fp_x = _alloc_quantized(gate, num_int, num_fp, bits, wide)
-        check(load().quik_silu_mul_quantize_u16(ptr(gate), ptr(up), dtype_code(gate.dtype), rows, cols,
-                                                ptr(int_indices_u16), num_int, ptr(fp_indices_u16), num_fp, bits,
-                                                int(bool(wide)), ptr(dst), ptr(meta), ptr(fp_x), stream_of(gate)),
-              "silu_mul_quantize")
-    return dst, meta, fp_x
+    return host().quantize(2, gate, up, 0.0, int_indices_u16, fp_indices_u16, bits, wide)
 
 
 def find_meta(src, bits):
@@ -119,7 +69,7 @@ def find_meta(src, bits):
     _check_bits(bits)
     src = src.contiguous()
     rows, cols = src.shape
-    with torch.cuda.device(src.device):
+    with on_device(src):
         meta = torch.empty((2 * rows,), dtype=src.dtype, device=src.device)
         check(load().quik_asym_find_meta(ptr(src), dtype_code(src.dtype), rows, cols, bits, ptr(meta),
                                          stream_of(src)), "find_meta")
@@ -133,7 +83,7 @@ def quantizeOld(src, meta, bits):
     rows, cols = src.shape
     if meta.numel() != 2 * rows:
         raise RuntimeError(f"quantize: expected meta to have {2 * rows} elements, got {meta.numel()}")
-    with torch.cuda.device(src.device):
+    with on_device(src):
         if bits == 4:
             dst = torch.empty((rows, (cols + 1) // 2), dtype=torch.uint8, device=src.device)
         else:
@@ -164,7 +114,7 @@ def dequantize(x, meta, scale_col, wReduced, y, bits):
         raise RuntimeError(f"dequantize: expected wReduced to have size {cols} at dimension 1")
     if not (meta.dtype == scale_col.dtype == wReduced.dtype == y.dtype):
         raise RuntimeError("dequantize: meta, scale_col, wReduced and y must share one floating dtype")
-    with torch.cuda.device(x.device):
+    with on_device(x):
         out = torch.empty_like(y)
         check(load().quik_asym_dequantize(ptr(x), ptr(meta), ptr(scale_col), ptr(wReduced), ptr(y), ptr(out),
                                           dtype_code(y.dtype), rows, cols, bits, stream_of(x)), "dequantize")
@@ -184,7 +134,7 @@ def _fused(op, bits, A, B, scale_row, scale_col, shift_value, zero_row, w_reduce
         raise RuntimeError(f"{op}: A and B must have the same reduction size")
     if scale_row.numel() != M or scale_col.numel() != N or y.shape != (M, N):
         raise RuntimeError(f"{op}: scale_row / scale_col / y do not match A and B")
-    with torch.cuda.device(A.device):
+    with on_device(A):
         out = torch.empty((M, N), dtype=torch.float16, device=A.device)
         scratch, nbytes = None, 0
         if bits == 4:

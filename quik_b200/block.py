@@ -14,7 +14,7 @@ import math
 import torch
 import torch.nn.functional as F
 
-from ._lib import check, dtype_code, load, ptr, stream_of
+from ._lib import check, dtype_code, load, on_device, ptr, stream_of
 from .qlinear import MixedQLinear, SharedQuantizedInput
 from .workloads import rtn_clip_scales
 
@@ -108,7 +108,7 @@ class QuikLlamaBlock(torch.nn.Module):
         """The same rotation in one pass, in place on the q and k projections [s, heads*head_dim] (they are this
         block's own fresh outputs); bit-identical to ``_rope``."""
         c, sn = self._angles(s, q.device, q.dtype)
-        with torch.cuda.device(q.device):
+        with on_device(q):
             check(load().quik_rotary_inplace(ptr(q), ptr(k), ptr(c), ptr(sn), dtype_code(q.dtype), s, self.heads,
                                              self.kv_heads, self.head_dim, stream_of(q)), "rotary")
 

@@ -339,11 +339,20 @@ uint32_t make_idesc(int c_format, int ab_format, int m, int n) {
 }
 
 unsigned int *device_status_word() {
+  static std::atomic<unsigned int *> cached[kMaxDevices];      // the address of a device's word never changes
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  unsigned int *known = cached[dev].load();
+  if (known != nullptr) return known;
   void *p = nullptr;
   if (cudaGetSymbolAddress(&p, g_device_status) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
+  cached[dev].store(static_cast<unsigned int *>(p));
   return static_cast<unsigned int *>(p);
 }
 

@@ -1,0 +1,266 @@
+// CPython module quik_b200._host: the per-call host work of the layer (argument checks, output and workspace allocation,
+// the library call) in native code.
+//
+// A layer of few tokens runs for less time on the GPU (about 10 us) than its two library calls took to issue from Python:
+// attribute look-ups, four tensor allocations, device guards and two ctypes calls of 14 and 19 arguments were 49 us per layer,
+// so every workload of up to a few hundred tokens was bound by them.  The functions here take the tensors themselves and
+// reach the C ABI of libquik_b200.so through the addresses handed to init(); errors become the same RuntimeErrors.
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+
+#include "../../include/quik_b200.h"
+
+namespace {
+
+struct Abi {
+  decltype(&quik_asym_quantize_u16) quantize = nullptr;
+  decltype(&quik_rmsnorm_quantize_u16) rmsnorm_quantize = nullptr;
+  decltype(&quik_silu_mul_quantize_u16) silu_mul_quantize = nullptr;
+  decltype(&quik_mixed_linear_ld) linear = nullptr;
+  decltype(&quik_config_get) config_get = nullptr;
+  decltype(&quik_strerror) strerror_ = nullptr;
+  decltype(&quik_last_cuda_error) last_cuda_error = nullptr;
+} abi;
+
+void check(int status, const char *what) {
+  if (status == QUIK_OK) return;
+  std::string msg = std::string(what) + ": " + abi.strerror_(status);
+  if (status == QUIK_ERR_CUDA) msg += std::string(" [") + abi.last_cuda_error() + "]";
+  throw std::runtime_error(msg);
+}
+
+// the conditions of _lib.require_cuda_contiguous
+void require(const char *op, const char *name, const at::Tensor &t, const at::Tensor &first) {
+  if (!t.is_cuda())
+    throw std::runtime_error(std::string(op) + ": expected tensor for argument '" + name + "' to be on a CUDA device");
+  if (!t.is_contiguous())
+    throw std::runtime_error(std::string(op) + ": expected tensor for argument '" + name + "' to be contiguous");
+  if (t.device() != first.device())
+    throw std::runtime_error(std::string(op) + ": expected all tensors on the same GPU, got " + first.device().str() + " and " +
+                             t.device().str());
+}
+
+int dtype_code(at::ScalarType t) {
+  if (t == at::kHalf) return QUIK_F16;
+  if (t == at::kBFloat16) return QUIK_BF16;
+  throw std::runtime_error(std::string("expected a float16 or bfloat16 tensor, got ") + c10::toString(t));
+}
+
+void *ptr(const at::Tensor &t) { return t.numel() == 0 ? nullptr : t.data_ptr(); }
+
+const at::Tensor &tensor_arg(PyObject *o) {
+  if (!THPVariable_Check(o)) throw std::runtime_error("expected a tensor");
+  return THPVariable_Unpack(o);
+}
+// None -> undefined tensor
+at::Tensor optional_arg(PyObject *o) { return o == Py_None ? at::Tensor() : tensor_arg(o); }
+
+void expect(Py_ssize_t got, Py_ssize_t want) {
+  if (got != want) throw std::runtime_error("quik_b200._host: wrong number of arguments");
+}
+
+// where the quantizer's outputs are (the tensors or the workspace that hold them belong to the caller)
+struct Codes {
+  void *q, *meta, *fp_x;
+};
+
+constexpr int64_t align256(int64_t v) { return (v + 255) & ~(int64_t)255; }
+
+// Checks the arguments of a quantizer call.  Producer 0: none, 1: RMSNorm (aux = weight vector), 2: SiLU(x) * aux.
+const char *check_quantize(int producer, const at::Tensor &x, const at::Tensor &aux, const at::Tensor &ids, const at::Tensor &fp_ids,
+                           int bits) {
+  static const char *const ops[3] = {"quantize", "rmsnorm_quantize", "silu_mul_quantize"};
+  const char *op = ops[producer];
+  require(op, producer == 2 ? "gate" : (producer == 1 ? "x" : "src"), x, x);
+  if (producer) require(op, producer == 1 ? "norm_weight" : "up", aux, x);
+  require(op, "int_indices", ids, x);
+  require(op, "fp_indices", fp_ids, x);
+  if (bits != 4 && bits != 8) throw std::runtime_error("bits argument must be either 4 or 8");
+  if (x.dim() != 2) throw std::runtime_error(std::string(op) + ": expected a matrix");
+  if (producer == 1 && (aux.numel() != x.size(1) || aux.scalar_type() != x.scalar_type()))
+    throw std::runtime_error("rmsnorm_quantize: norm_weight must have one entry per column, of x's dtype");
+  if (producer == 2 && (!aux.sizes().equals(x.sizes()) || aux.scalar_type() != x.scalar_type()))
+    throw std::runtime_error("silu_mul_quantize: gate and up must have the same shape and dtype");
+  return op;
+}
+
+void launch_quantize(const char *op, int producer, const at::Tensor &x, const at::Tensor &aux, double eps, const at::Tensor &ids,
+                     const at::Tensor &fp_ids, int bits, bool wide, const Codes &c) {
+  void *st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  const int dt = dtype_code(x.scalar_type()), rows = (int)x.size(0), cols = (int)x.size(1);
+  const int num_int = (int)ids.numel(), num_fp = (int)fp_ids.numel();
+  const uint16_t *i16 = static_cast<const uint16_t *>(ptr(ids)), *f16 = static_cast<const uint16_t *>(ptr(fp_ids));
+  int rc;
+  if (producer == 0)
+    rc = abi.quantize(ptr(x), dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta, c.fp_x, st);
+  else if (producer == 1)
+    rc = abi.rmsnorm_quantize(ptr(x), ptr(aux), (float)eps, dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta,
+                              c.fp_x, st);
+  else
+    rc = abi.silu_mul_quantize(ptr(x), ptr(aux), dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta, c.fp_x, st);
+  check(rc, op);
+}
+
+// the layer's own tensors, as the module holds them
+struct Layer {
+  at::Tensor scales, reduced, fp_w, bias;
+  int64_t k_int, n, f;
+  int bits;
+};
+
+// [1, M, N] (or `out_buffer` with that leading dimension added, where the caller gave one)
+at::Tensor launch_linear(const at::Tensor &x, const Codes &c, bool q_packed, const void *w, bool w_packed, const Layer &l,
+                         const at::Tensor &out_buffer) {
+  const int64_t m = x.size(0);
+  at::Tensor result = out_buffer.defined() ? out_buffer.unsqueeze(0) : at::empty({1, m, l.n}, x.options());
+  const int64_t pitch = out_buffer.defined() ? out_buffer.stride(0) : l.n;
+  check(abi.linear(c.q, q_packed, w, w_packed, c.meta, ptr(l.scales), ptr(l.reduced), l.f > 0 ? c.fp_x : nullptr,
+                   l.f > 0 ? ptr(l.fp_w) : nullptr, l.bias.defined() ? ptr(l.bias) : nullptr, ptr(result), pitch,
+                   dtype_code(x.scalar_type()), (int)m, (int)l.n, (int)l.k_int, (int)l.f, l.bits,
+                   c10::cuda::getCurrentCUDAStream(x.device().index()).stream()),
+        "MixedQLinear.forward");
+  return result;
+}
+
+PyObject *py_init(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 7);
+  void *p[7];
+  for (int i = 0; i < 7; ++i) {
+    p[i] = PyLong_AsVoidPtr(a[i]);
+    if (p[i] == nullptr) throw std::runtime_error("quik_b200._host.init: a library function is missing");
+  }
+  abi.quantize = reinterpret_cast<decltype(abi.quantize)>(p[0]);
+  abi.rmsnorm_quantize = reinterpret_cast<decltype(abi.rmsnorm_quantize)>(p[1]);
+  abi.silu_mul_quantize = reinterpret_cast<decltype(abi.silu_mul_quantize)>(p[2]);
+  abi.linear = reinterpret_cast<decltype(abi.linear)>(p[3]);
+  abi.strerror_ = reinterpret_cast<decltype(abi.strerror_)>(p[4]);
+  abi.last_cuda_error = reinterpret_cast<decltype(abi.last_cuda_error)>(p[5]);
+  abi.config_get = reinterpret_cast<decltype(abi.config_get)>(p[6]);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// (producer, x, aux | None, eps, int_ids, fp_ids, bits, wide) -> (codes, meta, fp_x)
+PyObject *py_quantize(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 8);
+  const int producer = (int)PyLong_AsLong(a[0]), bits = (int)PyLong_AsLong(a[6]);
+  const double eps = PyFloat_AsDouble(a[3]);
+  const bool wide = PyObject_IsTrue(a[7]) == 1;
+  if (PyErr_Occurred()) return nullptr;
+  if (producer < 0 || producer > 2) throw std::runtime_error("quik_b200._host.quantize: producer");
+  const at::Tensor x = tensor_arg(a[1]), aux = optional_arg(a[2]), ids = tensor_arg(a[4]), fp_ids = tensor_arg(a[5]);
+  if (producer && !aux.defined()) throw std::runtime_error("expected a tensor");
+  at::Tensor q, meta, fp_x;
+  {
+    py::gil_scoped_release nogil;
+    const char *op = check_quantize(producer, x, aux, ids, fp_ids, bits);
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    const int64_t rows = x.size(0), num_int = ids.numel();
+    q = bits == 4 && !wide ? at::empty({rows, num_int / 2}, x.options().dtype(at::kByte))
+                           : at::empty({rows, num_int}, x.options().dtype(at::kChar));
+    meta = at::empty({2 * rows}, x.options());
+    fp_x = at::empty({rows, fp_ids.numel()}, x.options());
+    launch_quantize(op, producer, x, aux, eps, ids, fp_ids, bits, wide, Codes{ptr(q), ptr(meta), ptr(fp_x)});
+  }
+  PyObject *r = PyTuple_New(3);
+  if (!r) return nullptr;
+  PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(q)));
+  PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(std::move(meta)));
+  PyTuple_SET_ITEM(r, 2, THPVariable_Wrap(std::move(fp_x)));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// scales, reduced, fp_w | None, bias | None, k_int, n, f, bits at a[0..7]
+bool layer_args(PyObject *const *a, Layer *l) {
+  *l = Layer{tensor_arg(a[0]), tensor_arg(a[1]), optional_arg(a[2]), optional_arg(a[3]), PyLong_AsLongLong(a[4]),
+             PyLong_AsLongLong(a[5]), PyLong_AsLongLong(a[6]), (int)PyLong_AsLong(a[7])};
+  if (PyErr_Occurred()) return false;
+  if (l->f > 0 && !l->fp_w.defined()) throw std::runtime_error("expected a tensor");
+  return true;
+}
+
+// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w_packed, codes, q_packed, meta, fp_x):
+// the fused launch on a quantized input; x gives the number of tokens, the dtype and the device
+PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 16);
+  const at::Tensor x = tensor_arg(a[0]), out = optional_arg(a[1]), w = tensor_arg(a[10]), q = tensor_arg(a[12]),
+                   meta = tensor_arg(a[14]), fp_x = tensor_arg(a[15]);
+  const bool w_packed = PyObject_IsTrue(a[11]) == 1, q_packed = PyObject_IsTrue(a[13]) == 1;
+  Layer l;
+  if (!layer_args(a + 2, &l)) return nullptr;
+  at::Tensor result;
+  {
+    py::gil_scoped_release nogil;
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    result = launch_linear(x, Codes{ptr(q), ptr(meta), ptr(fp_x)}, q_packed, ptr(w), w_packed, l, out);
+  }
+  return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids):
+// quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  w: the weights in storage
+// format; w8: 4-bit weights one code per byte; None is returned, and nothing launched, where the settings ask for them and
+// they were not given.
+PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 14);
+  const at::Tensor given = tensor_arg(a[0]), out = optional_arg(a[1]), w = tensor_arg(a[10]), w8 = optional_arg(a[11]),
+                   ids = tensor_arg(a[12]), fp_ids = tensor_arg(a[13]);
+  Layer l;
+  if (!layer_args(a + 2, &l)) return nullptr;
+  at::Tensor result;
+  {
+    py::gil_scoped_release nogil;
+    const at::Tensor x = given.dim() == 3 ? given.select(0, 0) : given;      // the first matrix of a batch, as ever
+    const char *op = check_quantize(0, x, at::Tensor(), ids, fp_ids, l.bits);
+    const int64_t m = x.size(0);
+    // operand layouts by engine, as in MixedQLinear._operand_layouts
+    bool q_packed = false, w_packed = false;
+    if (l.bits == 4) {
+      const bool row_ok = l.k_int % 32 == 0;
+      const int small_m = abi.config_get(QUIK_CFG_SMALL_M);
+      if (m <= QUIK_STREAM_M_MAX && small_m != 0 && row_ok) {
+        w_packed = true;
+        q_packed = m <= QUIK_SMALL_M_MAX && small_m != 3;
+      } else {
+        q_packed = row_ok && abi.config_get(QUIK_CFG_GEMM_ENGINE) == QUIK_ENGINE_TCGEN05_TS;
+      }
+    }
+    const bool needs_w8 = l.bits == 4 && !w_packed;
+    if (!needs_w8 || w8.defined()) {
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const int64_t b_q = align256(m * ids.numel()), b_meta = align256(m * 4);
+      const at::Tensor ws = at::empty({b_q + b_meta + m * fp_ids.numel() * 2}, x.options().dtype(at::kByte));
+      unsigned char *base = static_cast<unsigned char *>(ptr(ws));
+      const Codes c{base, base + b_q, base + b_q + b_meta};
+      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !q_packed, c);
+      result = launch_linear(x, c, q_packed, ptr(needs_w8 ? w8 : w), w_packed, l, out);
+    }
+  }
+  if (!result.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"init", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_init)), METH_FASTCALL, "addresses of the C ABI"},
+    {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, "activation quantizer"},
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL, "fused launch"},
+    {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer)), METH_FASTCALL, "quantizer and fused launch"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of the layer", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from ._lib import check, load, ptr, require_cuda_contiguous, stream_of
+from ._lib import check, load, on_device, ptr, require_cuda_contiguous, stream_of
 
 __all__ = ["int4Matmul", "int8Matmul", "int4SpMatmul", "int8SpMatmul", "int4ReorderMeta", "int8ReorderMeta",
            "int4GenRandomSparseMeta", "int8GenRandomSparseMeta", "int4Uncompress", "int8Uncompress",
@@ -19,7 +19,7 @@ def int4Matmul(A, B):
     if A.shape[1] != B.shape[1]:
         raise RuntimeError("int4Matmul: A and B must have the same reduction size")
     M, N, K = A.shape[0], B.shape[0], A.shape[1] * 2
-    with torch.cuda.device(A.device):
+    with on_device(A):
         C = torch.empty((M, N), dtype=torch.int32, device=A.device)
         nbytes = load().quik_int4_matmul_scratch_bytes(M, N, K)
         scratch = torch.empty((max(nbytes, 1),), dtype=torch.uint8, device=A.device)
@@ -36,7 +36,7 @@ def int8Matmul(A, B):
     if A.shape[1] != B.shape[1]:
         raise RuntimeError("int8Matmul: A and B must have the same reduction size")
     M, N, K = A.shape[0], B.shape[0], A.shape[1]
-    with torch.cuda.device(A.device):
+    with on_device(A):
         C = torch.empty((M, N), dtype=torch.int32, device=A.device)
         check(load().quik_int8_matmul(ptr(A), ptr(B), ptr(C), M, N, K, stream_of(A)), "int8Matmul")
     return C
@@ -46,7 +46,7 @@ def unpack_int4(src):
     """Widen packed int4 [rows, K/2] (uint8) to int8 [rows, K]; low nibble first (include/int4.h:78-98)."""
     require_cuda_contiguous("unpack_int4", src=src)
     rows, cols = src.shape[0], src.shape[1] * 2
-    with torch.cuda.device(src.device):
+    with on_device(src):
         dst = torch.empty((rows, cols), dtype=torch.int8, device=src.device)
         check(load().quik_unpack_int4(ptr(src), ptr(dst), rows, cols, stream_of(src)), "unpack_int4")
     return dst

@@ -14,7 +14,6 @@ import torch
 from torch import Tensor
 
 from . import _lib, asymmetric, matmul, symmetric
-from ._lib import check, dtype_code, load, ptr, stream_of
 
 __all__ = ["two_compl", "pack_to_i4", "SharedQuantizedInput", "MixedQLinear"]
 
@@ -132,7 +131,7 @@ class MixedQLinear(torch.nn.Module):
 
     # ------------------------------------------------------------------ derived, lazily built operands
     def _cached(self, name, src: Tensor, make):
-        key = (src.data_ptr(), src._version, str(src.device))
+        key = (src.data_ptr(), src._version, src.get_device())
         ent = self._cache.get(name)
         if ent is None or ent[0] != key:
             ent = (key, make(src))
@@ -204,6 +203,8 @@ class MixedQLinear(torch.nn.Module):
 
         shared_input = self.shared_input
         if shared_input is None:
+            if self.fused and not self.symmetric and MixedQLinear.launch_hook is None:
+                return self._forward_one_call(x)
             shared_input = SharedQuantizedInput(1)
         if len(x.shape) == 3:
             x = x[0]
@@ -231,30 +232,46 @@ class MixedQLinear(torch.nn.Module):
             shared_input.qint_x, shared_input.meta, shared_input.fp_x = asymmetric.quantize_u16(
                 x, i16, f16, self.bits, wide)
             shared_input.wide = wide
-        q = shared_input.qint_x
         w = self.int_weight if (w_packed or self.bits == 8) else self._weight_codes_int8()
-        N = self.out_features
         hook = MixedQLinear.launch_hook
-        with torch.cuda.device(x.device):
-            ob = self.out_buffer
-            if ob is not None and tuple(ob.shape) == (M, N) and ob.dtype == x.dtype and ob.device == x.device \
-                    and ob.stride(1) == 1 and ob.stride(0) >= N:
-                out = ob                         # may be a column range of a wider row-major matrix
-            else:
-                out = torch.empty((M, N), dtype=x.dtype, device=x.device)
-            F = self.fp_features_num
-            if hook is not None:
-                hook(self, True)
-            check(load().quik_mixed_linear_ld(
-                ptr(q), int(q_packed), ptr(w), int(w_packed), ptr(shared_input.meta), ptr(self.weights_scales),
-                ptr(self.reduced_w), ptr(shared_input.fp_x) if F > 0 else None,
-                ptr(self.fp_weight) if F > 0 else None, ptr(self.bias) if self.bias is not None else None,
-                ptr(out), out.stride(0), dtype_code(x.dtype), M, N, self.int_features_num, F, self.bits, stream_of(x)),
-                "MixedQLinear.forward")
-            if hook is not None:
-                hook(self, False)
+        if hook is not None:
+            hook(self, True)
+        out = _lib.host().linear(x, self._out_buffer_for(x, M), *self._constants(), w, w_packed, shared_input.qint_x, q_packed,
+                                 shared_input.meta, shared_input.fp_x)
+        if hook is not None:
+            hook(self, False)
         shared_input.finish()
-        return out.reshape((1, *out.shape))
+        return out
+
+    def _out_buffer_for(self, x, M):
+        """The caller's output buffer (may be a column range of a wider row-major matrix) where it fits, else None."""
+        ob = self.out_buffer
+        if ob is not None and tuple(ob.shape) == (M, self.out_features) and ob.dtype == x.dtype \
+                and ob.device == x.device and ob.stride(1) == 1 and ob.stride(0) >= self.out_features:
+            return ob
+        return None
+
+    def _constants(self):
+        """The layer's own arguments of the native host path."""
+        b = self._buffers
+        try:
+            scales, reduced, bias = b["weights_scales"], b["reduced_w"], b["bias"]
+        except KeyError:          # replaced by something that is not a buffer
+            scales, reduced, bias = self.weights_scales, self.reduced_w, self.bias
+        f = self.fp_features_num
+        return (scales, reduced, self.fp_weight if f > 0 else None, bias, self.int_features_num, self.out_features, f, self.bits)
+
+    def _forward_one_call(self, x):
+        """The layer on its own input, [1, M, K] or [M, K]: quantizer and fused kernel from one native call."""
+        w = self.int_weight
+        ids, fp_ids = self._idx16()
+        M = x.shape[-2] if x.dim() > 1 else 0
+        wide = self._weight_codes_int8() if self.bits == 4 and M > _lib.STREAM_M_MAX else None
+        out = self._out_buffer_for(x, M)
+        res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids)
+        if res is None:          # the settings send this token count to the engine that takes one code per byte
+            res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids)
+        return res
 
     def _forward_unfused(self, x, shared_input):
         """The reference's operator sequence (experiments/qlinear.py:105-148)."""

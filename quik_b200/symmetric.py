@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from ._lib import check, load, ptr, require_cuda_contiguous, stream_of
+from ._lib import check, load, on_device, ptr, require_cuda_contiguous, stream_of
 from .asymmetric import _fused
 
 __all__ = ["quantize", "dequantize", "int4FusedDequantize", "int8FusedDequantize",
@@ -20,7 +20,7 @@ def quantize(src, scale, bits):
     rows, cols = src.shape
     if scale.shape[0] != rows:
         raise RuntimeError(f"quantize: expected scale to have size {rows} at dimension 0")
-    with torch.cuda.device(src.device):
+    with on_device(src):
         if bits == 4:
             dst = torch.empty((rows, (cols - 1) // 2 + 1), dtype=torch.uint8, device=src.device)
         else:
@@ -43,7 +43,7 @@ def dequantize(x, scale_row, scale_col, y, bits):
         raise RuntimeError("dequantize: x and y must have the same size")
     if scale_row.shape[0] != rows or scale_col.numel() != cols:
         raise RuntimeError("dequantize: scale sizes do not match x")
-    with torch.cuda.device(x.device):
+    with on_device(x):
         out = torch.empty_like(y)
         check(load().quik_sym_dequantize(ptr(x), bits, ptr(scale_row), ptr(scale_col), ptr(y), ptr(out), rows, cols,
                                          stream_of(x)), "dequantize")

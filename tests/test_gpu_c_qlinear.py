@@ -362,3 +362,38 @@ def test_layers_on_two_devices_of_one_process():
                 assert _lib.device_status() == 0
             outs.append((M, out[0].cpu()))
     assert torch.equal(outs[0][1], outs[2][1]) and torch.equal(outs[1][1], outs[3][1])      # cuda:0 == cuda:1
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K,N,F,bits", [(1, 1024, 264, 64, 4), (16, 1024, 264, 0, 8), (17, 1024, 264, 64, 4), (128, 1024, 130, 64, 4),
+                                          (129, 1024, 264, 64, 4), (300, 1024, 261, 32, 8), (9, 112, 24, 32, 4)])
+def test_single_native_call_equals_quantizer_and_layer_calls(M, K, N, F, bits, dtype):
+    """A layer without a shared input runs quantizer and fused kernel from one native call: same bits as the two calls of a
+    shared input, for matrices and batches of one, with the settings that send few tokens to the tensor-core GEMM, into a
+    caller's buffer; and it refuses what they refuse."""
+    case = make_layer("t", M, K, N, bits, F=F, seed=3, device=dev(), dtype=dtype, clip=False)
+    layer, x = case.module, case.x
+    one = layer(x)
+    assert one.shape == (1, M, N) and torch.equal(layer(x.unsqueeze(0)), one)
+    assert torch.equal(layer(torch.stack([x, x + 1])), one)               # a batch: its first matrix
+    layer.shared_input = SharedQuantizedInput(1)
+    assert torch.equal(layer(x), one)
+    layer.shared_input = None
+    try:
+        _lib.set_small_m(False)
+        off = layer(x)
+        layer.shared_input = SharedQuantizedInput(1)
+        assert torch.equal(layer(x), off)
+    finally:
+        _lib.set_small_m(True)
+        layer.shared_input = None
+    buf = torch.full((M, N + 8), -1.0, dtype=dtype, device=dev())
+    layer.out_buffer = buf[:, :N]
+    assert layer(x).data_ptr() == buf.data_ptr() and torch.equal(buf[:, :N], one[0]) and (buf[:, N:] == -1).all()
+    layer.out_buffer = None
+    assert layer(x[:0]).shape == (1, 0, N)
+    for bad in (x[:, :-2].contiguous(), x.float(), x.t()[: K // 2].t()):  # columns, dtype, not contiguous
+        with pytest.raises(RuntimeError):
+            layer(bad)
+    assert torch.equal(layer(x), one)
+    assert_device_clean()
