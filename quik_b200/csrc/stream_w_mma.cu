@@ -1,7 +1,7 @@
 // Weight-streaming fused layer for few tokens (M <= 16): TMA-fed shared-memory ring in front of mma.sync.
 //
 // Same problem and same outer structure as stream_w.cu (one 128-row slab of W per CTA, K split over a
-// thread-block cluster, outlier blocks to the cluster's leader, exact split-K reduction with red.shared::cluster),
+// thread-block cluster, outlier blocks to the cluster's first CTA, exact split-K reduction over shared memory),
 // but the consumers are the legacy warp-level tensor instructions, which accept this skinny shape (16 tokens x 8
 // weight rows x 32 codes per instruction) at a higher rate than tcgen05 accepts 128 x 16 x 32 ones, and which
 // take the packed int4 weights after a three-instruction nibble split instead of a trip through TMEM:
@@ -15,12 +15,14 @@
 //               out of the exact sum.  int8 / outliers: two chunks are the two k halves of one instruction.
 //               A warp releases a stage as soon as its operands are in registers.
 //   end         the two k-half warps of a row group write their int32 and fp32 partial sums into separate tiles in
-//               drained stages of the ring; the non-leading CTAs add theirs into the leader's tile
-//               (red.shared::cluster; integer addition, order-free); 256 threads of the leader add the tiles (the
-//               outlier halves in fixed order), apply the dequantize arithmetic of
-//               QUIK src/asymmetric/asymmetric.cu:134-146 and store out[m, n].
+//               drained stages of the ring; after a cluster barrier the 256 threads of CTA r add up the tiles of all CTAs
+//               (the outlier halves in fixed order) for its share of the tokens, apply the dequantize arithmetic of
+//               QUIK src/asymmetric/asymmetric.cu:134-146 and store out[m, n].  (Adding into the leader's tile with
+//               red.shared::cluster and finishing there alone cost 1.3 to 1.9 us per layer of four-way splits; the 16-token step of four Llama-2-7B layers took 52.9 instead of 51.0 us.)
 // Every mbarrier wait is bounded (device status word, see tcgen05_ptx.cuh).
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05_ptx.cuh"
@@ -36,9 +38,8 @@ constexpr int SM_STAGES_DEEP = 11;                  // ... with one CTA per SM (
 constexpr int SM_W_BYTES = SM_ROWS * 128;
 constexpr int SM_X_BYTES = SM_TOKENS * 128;
 constexpr int SM_STAGE_BYTES = SM_W_BYTES + SM_X_BYTES;
-constexpr int SM_RED_BYTES = SM_TOKENS * SM_ROWS * 4;
 constexpr int SM_AUX_BYTES = 1024;
-constexpr size_t sm_smem(int stages) { return 1024 + (size_t)stages * SM_STAGE_BYTES + SM_RED_BYTES + SM_AUX_BYTES; }
+constexpr size_t sm_smem(int stages) { return 1024 + (size_t)stages * SM_STAGE_BYTES + SM_AUX_BYTES; }
 static_assert(sm_smem(SM_STAGES_DEEP) <= 227 * 1024 && 2 * sm_smem(SM_STAGES) <= 227 * 1024, "shared-memory plan");
 static_assert(2 * SM_STAGES_DEEP * 8 + 4 <= 256, "barriers and the abort flag sit in front of the token scales");
 
@@ -99,8 +100,7 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
   const int STAGES = p.stages;
-  int *red = reinterpret_cast<int *>(tiles + STAGES * SM_STAGE_BYTES);     // [token][row] int32 sums of this CTA
-  unsigned char *aux = reinterpret_cast<unsigned char *>(red) + SM_RED_BYTES;
+  unsigned char *aux = tiles + STAGES * SM_STAGE_BYTES;
   uint64_t *full_bar = reinterpret_cast<uint64_t *>(aux);       // [STAGES] stage loaded
   uint64_t *empty_bar = full_bar + SM_STAGES_DEEP;                 // [STAGES] stage read by all 8 consumer warps
   volatile int *abort_flag = reinterpret_cast<volatile int *>(empty_bar + SM_STAGES_DEEP);
@@ -173,8 +173,6 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   }
   if (warp >= 1) {
     const int te = threadIdx.x - 32;
-    if (S > 1)       // only a cluster's leader receives remote sums; every CTA zeroes its tile all the same
-      for (int i = te; i < SM_TOKENS * SM_ROWS; i += 256) red[i] = 0;
     if (te < SM_TOKENS) {
       float s = 0.f, z = 0.f;
       if (te < p.M) {
@@ -186,15 +184,11 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
   }
   __syncthreads();
-  // The leader's reduction tile is zeroed: every thread arrives at the cluster barrier now (the TMA warp after its
-  // first load is under way); it is waited for before the first remote add.
-  if (S > 1 && warp != 0) cluster_arrive();
-
   // epilogue vectors of the weight row this thread finishes, fetched while the weights stream (kept in storage
   // format: converting here would wait for loads that take microseconds while the stream saturates HBM)
   T ep_scol = Traits<T>::from_float(0.f), ep_wred = ep_scol, ep_bias = ep_scol;
   const int ep_row = (threadIdx.x - 32) & (SM_ROWS - 1), ep_half = (threadIdx.x - 32) >> 7;   // valid for warps 1-8
-  if (warp >= 1 && rank == 0 && n0 + ep_row < p.N) {
+  if (warp >= 1 && n0 + ep_row < p.N) {
     ep_scol = static_cast<const T *>(p.scale_col)[n0 + ep_row];
     ep_wred = static_cast<const T *>(p.w_reduced)[n0 + ep_row];
     if (p.bias) ep_bias = static_cast<const T *>(p.bias)[n0 + ep_row];
@@ -229,7 +223,6 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     int i = pre;                          // those stages are complete or under way
     if (lane == 0 && pre == 0 && nb > 0) issue(i++, 0);
     __syncwarp();
-    if (S > 1) cluster_arrive();
     if (lane == 0) {
       int stage = i % STAGES;
       uint32_t phase = (uint32_t)((i / STAGES) & 1);
@@ -294,11 +287,10 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   dbg_t[3] = clock64();
   __syncwarp();
   const bool ok = !*abort_flag;
-  if (S > 1) cluster_wait();                    // every CTA of the cluster has started: the leader's tile is zero
   __syncthreads();                              // the ring has drained in this CTA: stage 0 may be reused
   // Partial sums leave the registers through shared memory: the two k-half warps of a row group write their 16 x 32
   // sums into separate tiles that reuse drained stages (row pitch 136 words: the paired 8-byte stores of a warp touch
-  // every bank once), the finishing thread of a weight row adds the two (and what other CTAs of the cluster sent).
+  // every bank once), the finishing thread of a weight row adds the two of every CTA of the cluster.
   constexpr int LD = SM_ROWS + 8;
   int *sumA = reinterpret_cast<int *>(tiles + 1 * SM_STAGE_BYTES), *sumB = reinterpret_cast<int *>(tiles + 2 * SM_STAGE_BYTES);
   float *fpA = fp_part, *fpB = reinterpret_cast<float *>(tiles + 3 * SM_STAGE_BYTES);
@@ -323,34 +315,39 @@ stream_w_mma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   }
   __syncthreads();
   if (S > 1) {
-    if (warp >= 1 && rank != 0 && ok) {         // one pass of remote adds per CTA: its 16 x 128 sums into the leader's tile
-      const uint32_t red_base = map_to_rank(smem_u32(red), 0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int m = 8 * ep_half + j;
-        red_add_cluster(red_base + (uint32_t)((m * SM_ROWS + ep_row) * 4), sumA[m * LD + ep_row] + sumB[m * LD + ep_row]);
-      }
-    }
     cluster_arrive();
-    cluster_wait();                             // all partial sums have reached the leader
+    cluster_wait();                             // the tiles of all CTAs are in place
   }
   dbg_t[4] = clock64();
-  if (warp >= 1 && rank == 0 && ok) {
+  if (warp >= 1 && ok && n0 + ep_row < p.N) {
     const int n = n0 + ep_row;
-    if (n < p.N) {
-      const float scol = Traits<T>::to_float(ep_scol), wred = Traits<T>::to_float(ep_wred), bias = Traits<T>::to_float(ep_bias);
-      T *out = static_cast<T *>(p.out);
+    const float scol = Traits<T>::to_float(ep_scol), wred = Traits<T>::to_float(ep_wred), bias = Traits<T>::to_float(ep_bias);
+    T *out = static_cast<T *>(p.out);
+    const uint32_t a0 = smem_u32(sumA), b0 = smem_u32(sumB);
+    const uint32_t fa = map_to_rank(smem_u32(fpA), 0), fb = map_to_rank(smem_u32(fpB), 0);      // the first CTA has the outliers
+    auto finish = [&](auto ctas) {              // this CTA's 16 / ctas tokens, two at a time
+      constexpr int C = decltype(ctas)::value;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int m = 8 * ep_half + j;
-        if (m < p.M) {
-          const int acc = sumA[m * LD + ep_row] + sumB[m * LD + ep_row] + (S > 1 ? red[m * SM_ROWS + ep_row] : 0);
-          // outlier sums of the two k halves in fixed order
-          const float add = fmaf(s_zs[m], wred, (p.nf > 0 ? fpA[m * LD + ep_row] + fpB[m * LD + ep_row] : 0.f) + bias);
-          out[(size_t)m * p.ldo + n] = Traits<T>::from_float(fmaf((float)acc, s_srow[m] * scol, add));
-        }
+      for (int i = 0; i < SM_TOKENS / C / 2; ++i) {
+        const int m = rank * (SM_TOKENS / C) + 2 * i + ep_half;
+        const uint32_t off = (uint32_t)((m * LD + ep_row) * 4);
+        int acc = 0;
+#pragma unroll
+        for (int s = 0; s < C; ++s) acc += ld_cluster_s32(map_to_rank(a0, s) + off) + ld_cluster_s32(map_to_rank(b0, s) + off);
+        // outlier sums of the two k halves in fixed order
+        const float fp = p.nf > 0 ? __int_as_float(ld_cluster_s32(fa + off)) + __int_as_float(ld_cluster_s32(fb + off)) : 0.f;
+        const float add = fmaf(s_zs[m], wred, fp + bias);
+        if (m < p.M) out[(size_t)m * p.ldo + n] = Traits<T>::from_float(fmaf((float)acc, s_srow[m] * scol, add));
       }
-    }
+    };
+    if (S == 1) finish(std::integral_constant<int, 1>());
+    else if (S == 2) finish(std::integral_constant<int, 2>());
+    else finish(std::integral_constant<int, 4>());
+  }
+  if (S > 1) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();                             // no CTA leaves while another reads its tiles
   }
   if (p.dbg && threadIdx.x == 32) {
     unsigned long long *d = p.dbg + (size_t)blockIdx.x * 16;
