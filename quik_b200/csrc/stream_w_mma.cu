@@ -18,7 +18,8 @@
 //               drained stages of the ring; after a cluster barrier the 256 threads of CTA r add up the tiles of all CTAs
 //               (the outlier halves in fixed order) for its share of the tokens, apply the dequantize arithmetic of
 //               QUIK src/asymmetric/asymmetric.cu:134-146 and store out[m, n].  (Adding into the leader's tile with
-//               red.shared::cluster and finishing there alone cost 1.3 to 1.9 us per layer of four-way splits; the 16-token step of four Llama-2-7B layers took 52.9 instead of 51.0 us.)
+//               red.shared::cluster and finishing there alone took 1.3 to 1.9 us of a layer split four ways; four
+//               Llama-2-7B layers at 16 tokens took 52.9 instead of 51.0 us.)
 // Every mbarrier wait is bounded (device status word, see tcgen05_ptx.cuh).
 #include <cuda.h>
 

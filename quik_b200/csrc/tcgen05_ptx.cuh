@@ -167,10 +167,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local_addr, uint32_t ra
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
 }
-// integer add into another CTA's shared memory (no return value)
-__device__ __forceinline__ void red_add_cluster(uint32_t cluster_addr, int v) {
-  asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ int ld_cluster_s32(uint32_t cluster_addr) {
   int v;
   asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");

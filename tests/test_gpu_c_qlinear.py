@@ -397,3 +397,18 @@ def test_single_native_call_equals_quantizer_and_layer_calls(M, K, N, F, bits, d
             layer(bad)
     assert torch.equal(layer(x), one)
     assert_device_clean()
+
+
+@pytest.mark.parametrize("K,N,F,bits", [(1088, 130, 64, 4), (4352, 512, 256, 4), (608, 264, 0, 8), (11264, 512, 256, 8)],
+                         ids=["int4", "int4_split", "int8", "int8_split"])
+@pytest.mark.parametrize("M", [17, 31, 33, 48, 64, 65, 80, 97, 112, 128])
+def test_streaming_engine_at_every_width(M, K, N, F, bits):
+    """The tcgen05 streaming engine pads the tokens to the next multiple of 16 and plans shared and tensor memory for that
+    width (two CTAs per SM up to 64); K whole or split over a cluster whose CTAs each finish a share of the tokens."""
+    case = make_layer("t", M, K, N, bits, F=F, seed=M, device=dev(), clip=False)
+    out = case.module(case.x.unsqueeze(0))[0]
+    assert rel_rms_err(out.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+    assert torch.equal(case.module(case.x.unsqueeze(0))[0], out)
+    few = case.module(case.x[:16].contiguous())[0]                       # other engine: exact integers, fp32 outlier product
+    assert rel_rms_err(out[:16].cpu(), few.cpu()) < 5e-3
+    assert_device_clean()
