@@ -138,6 +138,18 @@ template <> struct Traits<__half> {
   static __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
   static __device__ __forceinline__ __half from_float(float v) { return __float2half(v); }
   static __device__ __forceinline__ int to_int_rn(__half v) { return __half2int_rn(v); }
+  // two values in a word, the first one in the low half
+  static __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  static __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+    const __half2 h = __hmul2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  static __device__ __forceinline__ float unpack(uint32_t w, int high) {
+    return __half2float(__ushort_as_half((unsigned short)(high ? w >> 16 : w & 0xFFFFu)));
+  }
 };
 template <> struct Traits<__nv_bfloat16> {
   using T2 = __nv_bfloat162;
@@ -145,6 +157,15 @@ template <> struct Traits<__nv_bfloat16> {
   static __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
   static __device__ __forceinline__ __nv_bfloat16 from_float(float v) { return __float2bfloat16_rn(v); }
   static __device__ __forceinline__ int to_int_rn(__nv_bfloat16 v) { return __bfloat162int_rn(v); }
+  static __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  static __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&a), *reinterpret_cast<const __nv_bfloat162 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  static __device__ __forceinline__ float unpack(uint32_t w, int high) { return __uint_as_float(high ? w & 0xFFFF0000u : w << 16); }
 };
 
 __device__ __forceinline__ float warp_max(float v) {

@@ -30,7 +30,7 @@ __device__ __forceinline__ int quantize_code(T x, T zero, T scale) {
   return min(max(v, 0), kMaxQ) - kShift;
 }
 
-// ---- packed fp16 arithmetic for the quantizer's inner loops ---------------------------------------
+// ---- packed arithmetic for the quantizer's inner loops --------------------------------------------
 // Two gathered values travel in one 32-bit register.  Every step reproduces, per 16-bit half, exactly
 // what the scalar chain hsub -> hdiv -> half2int_rn -> clamp of the reference kernel produces:
 //   * __hsub2 rounds each half like __hsub;
@@ -51,6 +51,18 @@ __device__ __forceinline__ uint32_t codes_of_pair(uint32_t pair, __half2 zero2, 
   q = __hmin2(__hmax2(q, __float2half2_rn(0.f)), __float2half2_rn((float)((1 << BITS) - 1)));
   q = __hadd2(q, __float2half2_rn(1024.f));
   return *reinterpret_cast<const uint32_t *>(&q) & 0x00FF00FFu;      // code_lo | code_hi << 16, both unsigned
+}
+
+// bfloat16: the same product and clamp, rounded to an integer by adding 2^23 in fp32 (quotients of 8-bit significands keep an
+// even larger distance from a rounding boundary; all 2^14 pairs are checked in the same test).
+template <int BITS>
+__device__ __forceinline__ uint32_t codes_of_pair(uint32_t pair, __nv_bfloat162 zero2, float rcp_scale) {
+  const float2 f = __bfloat1622float2(__hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&pair), zero2));
+  const float2 q = __bfloat1622float2(__floats2bfloat162_rn(f.x * rcp_scale, f.y * rcp_scale));
+  constexpr float kMaxQ = (float)((1 << BITS) - 1);
+  const uint32_t a = __float_as_uint(fminf(fmaxf(q.x, 0.f), kMaxQ) + 8388608.f);
+  const uint32_t b = __float_as_uint(fminf(fmaxf(q.y, 0.f), kMaxQ) + 8388608.f);
+  return (a & 0xFFu) | ((b & 0xFFu) << 16);
 }
 
 // Four pair words (8 unsigned codes) -> output bytes.  PACKED: 8 nibbles in one word (code - 8 == code ^ 8
@@ -100,7 +112,7 @@ __global__ void __launch_bounds__(NTHR, NTHR == 256 ? (NC <= 4 ? 3 : 2) : 1)
 asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int_idx,
                          const IdxT *__restrict__ fp_idx, int rows, int cols, int num_int, int num_fp,
                          uint8_t *__restrict__ dst, T *__restrict__ meta, T *__restrict__ fp_x,
-                         int vec_load, int vec_store, int vec_ids, int nbuf, const T *__restrict__ aux, float eps) {
+                         int vec_load, int vec_store, int vec_ids, int vec_aux, int nbuf, const T *__restrict__ aux, float eps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float s_red[2][NTHR / 32];
   const int cols_pad = (cols + 7) & ~7;
@@ -182,10 +194,22 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
     __syncthreads();
   }
 
-  // ---- the producer of X, applied to the row in shared memory
+  // ---- the producer of X, applied to the row in shared memory: 16 bytes per access, the last cols % 8 values one by one
+  // (instruction issue bounds this part: 40 to 48 instructions per value with 2-byte accesses; [4096, 8192] RMSNorm 50.2 -> 42.0 us,
+  // SiLU 69.5 -> 60.1 us, [2048, 11008] SiLU 51.6 -> 46.9 us)
   if (PROD == 1) {
     float ss = 0.f;
-    for (int i = tid; i < cols; i += NTHR) {
+    const int nv = cols >> 3;
+    for (int i = tid; i < nv; i += NTHR) {
+      const uint4 v = reinterpret_cast<const uint4 *>(s_row)[i];
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = Traits<T>::unpack(w[j], 0), b = Traits<T>::unpack(w[j], 1);
+        ss = fmaf(b, b, fmaf(a, a, ss));
+      }
+    }
+    for (int i = 8 * nv + tid; i < cols; i += NTHR) {
       const float f = Traits<T>::to_float(s_row[i]);
       ss = fmaf(f, f, ss);
     }
@@ -197,15 +221,34 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
 #pragma unroll
     for (int w = 0; w < NTHR / 32; ++w) ss += s_red[0][w];
     const float rstd = rsqrtf(ss / (float)cols + eps);
-    for (int i = tid; i < cols; i += NTHR)
+    const int na = vec_aux ? nv : 0;
+    for (int i = tid; i < na; i += NTHR) {
+      const uint4 v = reinterpret_cast<const uint4 *>(s_row)[i], g = __ldg(reinterpret_cast<const uint4 *>(aux) + i);
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        w[j] = Traits<T>::mul2(Traits<T>::pack2(Traits<T>::unpack(w[j], 0) * rstd, Traits<T>::unpack(w[j], 1) * rstd), gw[j]);
+      reinterpret_cast<uint4 *>(s_row)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    for (int i = 8 * na + tid; i < cols; i += NTHR)
       s_row[i] = __hmul(Traits<T>::from_float(Traits<T>::to_float(s_row[i]) * rstd), aux[i]);
     __syncthreads();            // the transformed row is complete; s_red may be written again
   } else if (PROD == 2) {
     const T *s_arow = s_aux + (size_t)buf * cols_pad;
-    for (int i = tid; i < cols; i += NTHR) {
-      const float g = Traits<T>::to_float(s_row[i]);
-      s_row[i] = __hmul(Traits<T>::from_float(g / (1.f + expf(-g))), s_arow[i]);
+    auto silu = [](float g) { return g / (1.f + expf(-g)); };
+    const int nv = cols >> 3;
+    for (int i = tid; i < nv; i += NTHR) {
+      const uint4 v = reinterpret_cast<const uint4 *>(s_row)[i], u = reinterpret_cast<const uint4 *>(s_arow)[i];
+      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        w[j] = Traits<T>::mul2(Traits<T>::pack2(silu(Traits<T>::unpack(w[j], 0)), silu(Traits<T>::unpack(w[j], 1))), uw[j]);
+      reinterpret_cast<uint4 *>(s_row)[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    for (int i = 8 * nv + tid; i < cols; i += NTHR)
+      s_row[i] = __hmul(Traits<T>::from_float(silu(Traits<T>::to_float(s_row[i]))), s_arow[i]);
     __syncthreads();
   }
 
@@ -272,34 +315,12 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
   // ---- pass 2: quantize + pack
   uint8_t *drow = dst + (size_t)r * (kPacked ? (size_t)(num_int >> 1) : (size_t)num_int);
   const float rcp_scale = __frcp_rn(Traits<T>::to_float(scale));
+  const typename Traits<T>::T2 zero2 = {zero, zero};
   auto emit = [&](int c, const uint32_t (&p)[4]) {
-    uint32_t w0, w1;
-    if (Traits<T>::kIsHalf) {
-      const __half2 zero2 = __half2half2(*reinterpret_cast<const __half *>(&zero));
-      uint32_t codes[4];
+    uint32_t w0, w1, codes[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) codes[j] = codes_of_pair<BITS>(p[j], zero2, rcp_scale);
-      emit_codes<BITS, kPacked>(codes, w0, w1);
-    } else {
-      int v[8];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const T *e = reinterpret_cast<const T *>(&p[j]);
-        v[2 * j] = quantize_code<T, BITS>(e[0], zero, scale);
-        v[2 * j + 1] = quantize_code<T, BITS>(e[1], zero, scale);
-      }
-      if (kPacked) {
-        w0 = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) w0 |= (uint32_t)(v[j] & 0xF) << (4 * j);
-        w1 = 0;
-      } else {
-        w0 = (uint32_t)(v[0] & 0xFF) | ((uint32_t)(v[1] & 0xFF) << 8) | ((uint32_t)(v[2] & 0xFF) << 16) |
-             ((uint32_t)(v[3] & 0xFF) << 24);
-        w1 = (uint32_t)(v[4] & 0xFF) | ((uint32_t)(v[5] & 0xFF) << 8) | ((uint32_t)(v[6] & 0xFF) << 16) |
-             ((uint32_t)(v[7] & 0xFF) << 24);
-      }
-    }
+    for (int j = 0; j < 4; ++j) codes[j] = codes_of_pair<BITS>(p[j], zero2, rcp_scale);
+    emit_codes<BITS, kPacked>(codes, w0, w1);
     if (kPacked) {
       if (vec_store) {
         *reinterpret_cast<uint32_t *>(drow + (size_t)c * 4) = w0;
@@ -366,7 +387,7 @@ int launch_asym_rows_nc(const void *src, int rows, int cols, const void *int_idx
   QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, kern, static_cast<const T *>(src), static_cast<const IdxT *>(int_idx),
                                    static_cast<const IdxT *>(fp_idx), rows, cols, num_int, num_fp,
                                    static_cast<uint8_t *>(dst), static_cast<T *>(meta), static_cast<T *>(fp_x),
-                                   vec_load, vec_store, vec_ids, nbuf, static_cast<const T *>(pr.aux), pr.eps));
+                                   vec_load, vec_store, vec_ids, aligned16(pr.aux), nbuf, static_cast<const T *>(pr.aux), pr.eps));
   return check_launch("asym_quantize_row_kernel");
 }
 

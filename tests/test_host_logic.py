@@ -175,3 +175,13 @@ def test_reciprocal_product_rounds_like_the_fp16_quotient():
     for e in range(-11, 10):
         d = sig * np.float32(2.0 ** e)
         assert np.array_equal((d[:, None] / sig[None, :]).astype(np.float16), (d[:, None] * rcp[None, :]).astype(np.float16))
+
+
+def test_reciprocal_product_rounds_like_the_bfloat16_quotient():
+    """The same for bfloat16 (8-bit significands), whose quantizer takes the same shortcut."""
+    sig = (128 + torch.arange(128)).float() / 128
+    rcp = torch.from_numpy(np.float32(1) / sig.numpy())
+    for e in range(-11, 10):
+        d = sig * 2.0 ** e
+        quotient = (d.double()[:, None] / sig.double()[None, :]).float().bfloat16()
+        assert torch.equal(quotient, (d[:, None] * rcp[None, :]).bfloat16())
