@@ -106,8 +106,8 @@ int quik_selftest_bounded_wait(unsigned int limit_us, int *device_result, void *
 /* Diagnostics: when `device_buffer` (16 x uint64 per launched CTA, caller-owned device memory) is
  * non-NULL, every tcgen05 GEMM launch writes per-CTA cycle counters there: [0] MMA issue loop,
  * [1] of which waiting for a free accumulator region, [2] waiting for operands, [3] tiles of the CTA,
- * [4] epilogue waiting for an outlier product, [5] waiting for an integer product, [6] parking outlier
- * products, [7] final epilogues.  The ring streaming engine for few tokens (stream_w_mma) writes clock64 at [0] kernel
+ * [4] epilogue waiting for an outlier product, [5] waiting for an integer product, [6] rounding and keeping
+ * outlier products, [7] final epilogues.  The ring streaming engine for few tokens (stream_w_mma) writes clock64 at [0] kernel
  * entry, [1] after the wait for its predecessor, [2] first block consumed, [3] last block consumed, [4] after the
  * reduction, [5] end, then [6] its number of k-blocks, [7] its rank in the cluster, [8] the global timer at its end.
  * NULL switches it off (default).  No reference counterpart. */
@@ -267,9 +267,9 @@ int quik_fused_dequantize(const void *A, const void *B, int bits,
  *                                    packed weights are widened on chip on their way to the tensor cores;
  *   q packed,       w packed         weight streaming on mma.sync, direct loads or TMA ring by QUIK_CFG_SMALL_M
  *                                    (M <= QUIK_SMALL_M_MAX, K_int % 32 == 0).
- * The tensor-core engines use `out` as scratch while they run (the rounded outlier product + bias is parked there
- * before the dequantize step, as the reference's F.linear output is rounded, experiments/qlinear.py:124): `out` must
- * not alias any input.
+ * The tensor-core GEMMs round the outlier product + bias to the storage type before the dequantize step, as the reference's
+ * F.linear output is rounded (experiments/qlinear.py:124).  Finished tiles are stored while others are still being computed:
+ * `out` must not alias any input.
  * K_int % 16 == 0, F % 8 == 0. */
 #define QUIK_SMALL_M_MAX 16
 /* most tokens the tcgen05 weight-streaming engine takes (q one code per byte, w in storage format) */

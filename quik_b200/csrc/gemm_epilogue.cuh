@@ -1,7 +1,9 @@
 // Epilogue of the tiled tcgen05 GEMMs (gemm_tcgen05.cu, gemm_tcgen05_ts.cu): launch parameters and the work of
-// the eight epilogue warps of a CTA -- parking the outlier product, the dequantize arithmetic of
+// the epilogue warps of a CTA -- rounding the outlier product and keeping it, the dequantize arithmetic of
 // QUIK src/asymmetric/asymmetric.cu:134-146 and the stores of the finished tile.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "tcgen05_ptx.cuh"
 
@@ -11,14 +13,13 @@ namespace {
 
 constexpr int BLOCK_M = 128;
 constexpr int STAGE_K_BYTES = 128;           // one 128B-swizzle row of K per stage
-constexpr int NUM_EPI_THREADS = 256;         // eight epilogue warps
-constexpr int EPI_BUF_BYTES = 32 * 64;       // output staging of one epilogue warp: 32 rows x 64 bytes
+constexpr int EPI_BUF_BYTES = 32 * 32;       // output staging of one epilogue warp: 32 rows x 32 bytes
 constexpr int SMEM_LIMIT = 227 * 1024;
 
 struct GemmParams {
   int M, N;
   int block_n;                    // tile width: multiple of 16
-  int split_n;                    // columns of a tile that the first four epilogue warps take (multiple of 32 or block_n)
+  int split_n;                    // columns of a tile that each group of four epilogue warps takes (multiple of 32)
   int num_m_tiles, num_tiles;
   int int_kb, fp_kb;              // k-blocks per tile: integer (128 codes each) and outlier (64 elems)
   uint32_t idesc_int, idesc_fp;   // tcgen05 instruction descriptors
@@ -44,63 +45,60 @@ template <typename T> __device__ __forceinline__ float ldf(const void *p, size_t
   return Traits<T>::to_float(static_cast<const T *>(p)[i]);
 }
 
-// 32 consecutive values of type T: 16-byte vector access when `vec`, scalar with a column guard
-// otherwise.
-template <typename T>
-__device__ __forceinline__ void load_row32(const T *src, bool vec, int ncols_left, T (&v)[32]) {
-  if (vec) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) reinterpret_cast<uint4 *>(v)[j] = reinterpret_cast<const uint4 *>(src)[j];
-  } else {
-    for (int j = 0; j < 32; ++j) v[j] = (j < ncols_left) ? src[j] : Traits<T>::from_float(0.f);
+// ---------------------------------------------------------------------------------------------
+// Work of one CTA (or pair) = its tiles t_0, t_1, ...  Tensor memory holds two accumulator regions.  INT(t_j), the integer
+// product (s32), lives in region j & 1; FP(t_j), the outlier product (f32), is issued in the middle of INT(t_j) into the other
+// region, which the epilogue of t_{j-1} has left by then.  The epilogue warps round FP(t_j) + bias to T and keep it in
+// registers (drain), which frees that region for INT(t_{j+1}), and combine it with the integer product when that is complete
+// (finish).  So both hide behind integer products and only the last tile's finish has nothing to hide behind.
+// (Before, FP(t_{j+1}) was issued in the middle of INT(t_j) and its rounded value parked in the tile's place in `out` until
+// INT(t_{j+1}) was complete; fetching it back queued behind the operand loads that fill the SM's port to L2, the two parts of
+// the epilogue took 15 to 18 thousand cycles per 256 x 256 tile, and the first drain had nothing to hide behind.
+// Llama-2-7B at 2048 tokens: the issuing warp waited 23.4 thousand of 136 thousand cycles for a free region in the qkv layer and
+// 58 of 242 in gate+up, now 12.7 of 121 and 23.7 of 206; 87.5 -> 81.4 us and 155.4 -> 140.3 us.)
+// This walks the k-blocks in issue order; fn(j, fp, kb) returns false to stop.  `fp` is a compile-time flag (std::true_type /
+// std::false_type): a narrow tile's block occupies the tensor pipe for less than 200 cycles, the issuing warp has none to spare
+// for choosing between the two kinds of instruction.
+template <bool HAS_FP, typename Fn>
+__device__ __forceinline__ void for_each_block(int n_local, int int_kb, int fp_kb, Fn fn) {
+  const int int_half = (int_kb + 1) / 2;
+  for (int j = 0; j < n_local; ++j) {
+#pragma unroll 1
+    for (int part = 0; part < (HAS_FP ? 2 : 1); ++part) {
+      const int end = HAS_FP && part == 0 ? int_half : int_kb;
+      for (int kb = part == 0 ? 0 : int_half; kb < end; ++kb)
+        if (!fn(j, std::false_type(), kb)) return;
+      if (HAS_FP && part == 0)
+        for (int kb = 0; kb < fp_kb; ++kb)
+          if (!fn(j, std::true_type(), kb)) return;
+    }
   }
 }
-// eight fp32 values -> eight values of type T in one 16-byte word
-template <typename T>
-__device__ __forceinline__ uint4 pack8(const float *o) {
-  uint4 pk;
-  T *pe = reinterpret_cast<T *>(&pk);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) pe[e] = Traits<T>::from_float(o[e]);
-  return pk;
-}
-template <typename T>
-__device__ __forceinline__ void store_row32(T *dst, bool vec, int ncols_left, const float (&o)[32]) {
-  if (vec) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) reinterpret_cast<uint4 *>(dst)[j] = pack8<T>(o + 8 * j);
-  } else {
-    for (int j = 0; j < 32; ++j)
-      if (j < ncols_left) dst[j] = Traits<T>::from_float(o[j]);
+// What the first k-block of a product has to wait for: barrier and parity, or nullptr.  acc_empty[j & 1] completes when
+// finish(j) is done, fp_drained[j & 1] when drain(j) is.
+template <bool HAS_FP>
+__device__ __forceinline__ uint64_t *region_barrier(int j, bool fp, uint64_t *acc_empty, uint64_t *fp_drained, uint32_t &parity) {
+  if (HAS_FP) {
+    parity = (uint32_t)((j - 1) >> 1) & 1u;
+    return j == 0 ? nullptr : (fp ? acc_empty : fp_drained) + ((j - 1) & 1);
   }
+  parity = ((uint32_t)(j >> 1) & 1u) ^ 1u;
+  return acc_empty + (j & 1);
 }
 
-// ---------------------------------------------------------------------------------------------
-// One epilogue warp.  Warp (sub, half) owns rows [32*sub, 32*sub+32) of the CTA's 128 rows of the tile and the
-// columns [cb, cb + cn): the first split_n columns for half 0, the rest for half 1.  It walks them 32 at a time; the
-// last step of a range whose length is not a multiple of 32 holds 16 valid columns (`valid` below), the rest is
-// ignored.  Tile j of the CTA uses accumulator region j & 1 (region_stride tensor-memory columns apart) for both of
-// its products:
-//   drain(j)   the outlier product (f32) + bias, rounded to T, is parked in the tile's place in `out` (it stays in
-//              L2), which frees the region for the integer product;
-//   finish(j)  the integer product (s32) is combined with the parked value by the dequantize arithmetic and the
-//              result overwrites the parked value.
-// Where the outlier product of (this warp, tile) is parked: every full 32 x 32 chunk inside its own 32-row x 64-byte
-// block of `out` (so the final store of one chunk never touches the parked data of another), but permuted: the jj-th
-// 16-byte piece of lane L goes to row 8*jj + L/4, piece L%4 of the block, so one warp instruction writes 8 rows x 64
-// contiguous bytes (whole sectors) instead of 32 rows x 16 bytes.  The same lane reads its pieces back from the same
-// addresses; nobody else looks at them.  Chunks that touch the matrix edge or hold fewer than 32 valid columns keep
-// the plain row-per-lane layout with guards.
-template <typename T, bool HAS_FP, int CTAS>
+// One epilogue warp.  Warp (sub, group) owns rows [32*sub, 32*sub+32) of the CTA's 128 rows of the tile and the
+// columns [cb, cb + cn), COLS at most, of it (group g: the g-th split_n columns).  It walks them 16 at a time.
+template <typename T, bool HAS_FP, int CTAS, int COLS>
 struct EpilogueWarp {
+  static constexpr int CHUNKS = COLS / 16;
   const GemmParams &p;
   uint32_t tmem_base;
   int region_stride;                 // tensor-memory columns between the two accumulator regions
   int unit, num_units, rank;         // this CTA's unit (CTA or pair), number of units, rank inside the pair
-  int lane, sub, half;
+  int lane, sub;
   int cb, cn, cn32;
-  float *s_scol, *s_wred, *s_bias;   // [half_cap] each, private to this warp
-  unsigned char *s_stage;            // 32 x 64 bytes, private to this warp
+  float *s_scol, *s_wred, *s_bias;   // [COLS] each, private to this warp
+  unsigned char *s_stage;            // 32 x 32 bytes, private to this warp
   uint64_t *acc_full, *acc_empty, *fp_full, *fp_drained;
   volatile int *abort_flag;
   bool ok = true;
@@ -108,230 +106,233 @@ struct EpilogueWarp {
 
   __device__ __forceinline__ EpilogueWarp(const GemmParams &p_, uint32_t tmem_base_, int region_stride_, int unit_,
                                           int num_units_, int rank_, int e, int sub_, int lane_, float *s_vec,
-                                          int half_cap, unsigned char *s_out, uint64_t *acc_full_,
-                                          uint64_t *acc_empty_, uint64_t *fp_full_, uint64_t *fp_drained_,
-                                          volatile int *abort_flag_)
+                                          unsigned char *s_out, uint64_t *acc_full_, uint64_t *acc_empty_,
+                                          uint64_t *fp_full_, uint64_t *fp_drained_, volatile int *abort_flag_)
       : p(p_), tmem_base(tmem_base_), region_stride(region_stride_), unit(unit_), num_units(num_units_), rank(rank_),
-        lane(lane_), sub(sub_), half(e >> 2), acc_full(acc_full_), acc_empty(acc_empty_), fp_full(fp_full_),
-        fp_drained(fp_drained_), abort_flag(abort_flag_) {
-    cb = half ? p.split_n : 0;
-    cn = half ? p.block_n - p.split_n : p.split_n;
+        lane(lane_), sub(sub_), acc_full(acc_full_), acc_empty(acc_empty_), fp_full(fp_full_), fp_drained(fp_drained_),
+        abort_flag(abort_flag_) {
+    cb = min((e >> 2) * p.split_n, p.block_n);
+    cn = min(p.split_n, p.block_n - cb);
     cn32 = (cn + 31) & ~31;
-    s_scol = s_vec + e * 3 * half_cap;
-    s_wred = s_scol + half_cap;
-    s_bias = s_wred + half_cap;
+    s_scol = s_vec + e * 3 * COLS;
+    s_wred = s_scol + COLS;
+    s_bias = s_wred + COLS;
     s_stage = s_out + e * EPI_BUF_BYTES;
   }
 
-  __device__ __forceinline__ uint4 *parked_piece(T *sub_base, int c0, int jj) const {   // sub_base = &out[first row of warp][n0]
-    return reinterpret_cast<uint4 *>(sub_base + (size_t)(8 * jj + (lane >> 2)) * p.ldo + c0) + (lane & 3);
+  // this warp's part of tile j: first row, first column, valid columns from there on (<= 0: none)
+  struct Part {
+    int m0, n0, lim;
+  };
+  __device__ __forceinline__ Part part(int j) const {
+    const int tile = unit + j * num_units;
+    Part t;
+    t.m0 = (tile % p.num_m_tiles) * (BLOCK_M * CTAS) + rank * BLOCK_M + sub * 32;
+    t.n0 = (tile / p.num_m_tiles) * p.block_n + cb;
+    t.lim = min(p.N - t.n0, cn);
+    return t;
+  }
+  __device__ __forceinline__ uint32_t accumulators(int region) const {
+    return tmem_base + ((uint32_t)(sub * 32) << 16) + region * region_stride + cb;
+  }
+  __device__ __forceinline__ bool wait(uint64_t *bars, int j, long long &waited) {
+    const long long t0 = clock64();
+    ok = mbar_wait_warp(smem_u32(bars + (j & 1)), (uint32_t)(j >> 1) & 1u, abort_flag, p.status);
+    waited += clock64() - t0;
+    tc_fence_after();
+    return ok;
+  }
+  __device__ __forceinline__ void arrive(uint64_t *bars, int j) const {
+    tc_fence_before();
+    if (CTAS == 1) mbar_arrive(smem_u32(bars + (j & 1)));
+    else mbar_arrive_leader(smem_u32(bars + (j & 1)));
   }
 
-  // park T(outlier product + bias) of tile j in `out`
-  __device__ __forceinline__ void drain(int j) {
-    constexpr int TILE_M = BLOCK_M * CTAS;
-    const int tile = unit + j * num_units;
-    const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M + sub * 32;   // first row of this warp
-    const int n0 = (tile / p.num_m_tiles) * p.block_n + cb;
-    const int lim = min(p.N - n0, cn);       // valid columns from n0 on (<= 0: none)
-    const int r = j & 1;
+  // round and keep the outlier product of tile j
+  __device__ __forceinline__ void drain(int j, uint32_t (&keep)[COLS / 2]) {
+    const Part t = part(j);
     __syncwarp();
     for (int c = lane; c < cn32; c += 32)
-      s_bias[c] = (c < lim && p.bias) ? ldf<T>(p.bias, n0 + c) : 0.f;
+      s_bias[c] = (c < t.lim && p.bias) ? ldf<T>(p.bias, t.n0 + c) : 0.f;
     __syncwarp();
-    const long long tw = clock64();
-    const bool ready = mbar_wait(smem_u32(fp_full + r), (uint32_t)(j >> 1) & 1u, abort_flag, p.status);
-    if (!__all_sync(0xffffffffu, ready)) { ok = false; return; }
-    const long long tw1 = clock64();
-    e_wait_fp += tw1 - tw;
-    tc_fence_after();
-    const int row = m0 + lane;
-    const bool rows_in = m0 + 32 <= p.M;
-    T *sub_base = static_cast<T *>(p.out) + (size_t)m0 * p.ldo + n0;
-    const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16) + r * region_stride + cb;
-#pragma unroll 1
-    for (int c0 = 0; c0 < cn; c0 += 32) {
-      uint32_t f[32];
-      float o[32];
-      __syncwarp();                          // tcgen05.ld is warp-collective
-      tmem_ld32(taddr + c0, f);
-      tmem_ld_wait();
-      const int valid = lim - c0;            // warp-uniform
-      if (valid <= 0) continue;
+    if (!wait(fp_full, j, e_wait_fp)) return;
+    const long long t0 = clock64();
+    const uint32_t taddr = accumulators((j + 1) & 1);
+    uint32_t v[2][16];                       // the next 16 columns are on their way while these are worked on
+    if (t.lim > 0) tmem_ld16(taddr, v[0]);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(f[i]) + s_bias[c0 + i];
-      if (p.vec_out && rows_in && valid >= 32) {
+    for (int c = 0; c < CHUNKS; ++c) {
+      if (16 * c >= t.lim) break;            // warp-uniform
+      uint32_t (&f)[16] = v[c & 1];
+      tmem_ld_wait(f);
+      if (c + 1 < CHUNKS && 16 * (c + 1) < t.lim) tmem_ld16(taddr + 16 * (c + 1), v[(c + 1) & 1]);
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) *parked_piece(sub_base, c0, jj) = pack8<T>(o + 8 * jj);
-      } else if (row < p.M) {
-        T *dst = static_cast<T *>(p.out) + (size_t)row * p.ldo + n0 + c0;
-        if (p.vec_out) {                     // valid is a multiple of 8 here
+      for (int i = 0; i < 8; ++i)
+        keep[8 * c + i] = Traits<T>::pack2(__uint_as_float(f[2 * i]) + s_bias[16 * c + 2 * i],
+                                           __uint_as_float(f[2 * i + 1]) + s_bias[16 * c + 2 * i + 1]);
+    }
+    arrive(fp_drained, j);
+    e_drain += clock64() - t0;
+  }
+
+  // Two 16-byte pieces per lane (32 bytes of its row, ELEM-byte elements) -> memory at dst (row m0 of the warp), `bytes` of
+  // them valid.  Transposed through shared memory so that one warp instruction stores 16 rows x 32 contiguous bytes (whole
+  // sectors) instead of 32 rows x 16 bytes; rows without 16-byte alignment are stored element by element, still 32 contiguous
+  // bytes of a row at a time (one row per lane was a sector
+  // per element: 741 tokens through int4 5152 x 3333 took 85.6 us, now 22.6).
+  template <int ELEM>
+  __device__ __forceinline__ void store_row_pieces(uint4 p0, uint4 p1, unsigned char *dst, size_t pitch, int rows, int bytes) const {
+    __syncwarp();                            // the buffer has been read out
+    const int flip = (lane >> 2) & 1;        // swizzle: the eight lanes of a store phase touch every bank once
+    *reinterpret_cast<uint4 *>(s_stage + lane * 32 + 16 * flip) = p0;
+    *reinterpret_cast<uint4 *>(s_stage + lane * 32 + 16 * (flip ^ 1)) = p1;
+    __syncwarp();
+    if (p.vec_out) {
+      const int pc = lane & 1;
 #pragma unroll
-          for (int jj = 0; jj < 4; ++jj)
-            if (8 * jj < valid) reinterpret_cast<uint4 *>(dst)[jj] = pack8<T>(o + 8 * jj);
-        } else {
-          store_row32<T>(dst, false, valid, o);
+      for (int k = 0; k < 2; ++k) {
+        const int rr = 16 * k + (lane >> 1);
+        const uint4 piece = *reinterpret_cast<const uint4 *>(s_stage + rr * 32 + 16 * (pc ^ ((rr >> 2) & 1)));
+        if (16 * pc + 16 <= bytes && rr < rows) *reinterpret_cast<uint4 *>(dst + (size_t)rr * pitch + 16 * pc) = piece;
+      }
+    } else {
+      constexpr int PER_ROW = 32 / ELEM, ROWS = 32 / PER_ROW;
+      const int off = (lane % PER_ROW) * ELEM;
+#pragma unroll 4
+      for (int k = 0; k < 32 / ROWS; ++k) {
+        const int rr = ROWS * k + lane / PER_ROW;
+        const unsigned char *src = s_stage + rr * 32 + 16 * ((off >> 4) ^ ((rr >> 2) & 1)) + (off & 15);
+        if (off < bytes && rr < rows) {
+          if (ELEM == 2) *reinterpret_cast<uint16_t *>(dst + (size_t)rr * pitch + off) = *reinterpret_cast<const uint16_t *>(src);
+          else *reinterpret_cast<uint32_t *>(dst + (size_t)rr * pitch + off) = *reinterpret_cast<const uint32_t *>(src);
         }
       }
     }
-    tc_fence_before();
-    if (CTAS == 1) mbar_arrive(smem_u32(fp_drained + r));
-    else mbar_arrive_leader(smem_u32(fp_drained + r));
-    e_drain += clock64() - tw1;
   }
 
-  __device__ __forceinline__ void prefetch_parked(uint4 (&pk_next)[4], T *sub_base, const T *my_row, bool rows_in,
-                                                  bool row_ok, int lim, int c0) const {
-    if (!HAS_FP || p.mode != 1 || !p.vec_out) return;
-    const int valid = lim - c0;
-    if (rows_in && valid >= 32) {
+  // the addend y of this lane's row, chunk c; all lanes take part
+  __device__ __forceinline__ void load_y(const Part &t, int c, uint32_t *w) const {
+    const T *src = static_cast<const T *>(p.y) + (size_t)t.m0 * p.N + t.n0 + 16 * c;
+    const int rows = p.M - t.m0, valid = t.lim - 16 * c;
+    if (p.vec_y && valid >= 16) {
+      const uint4 *mine = reinterpret_cast<const uint4 *>(src + (size_t)max(0, min(lane, rows - 1)) * p.N);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) pk_next[jj] = *parked_piece(sub_base, c0, jj);
-    } else if (row_ok) {
+      for (int jj = 0; jj < 2; ++jj) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (lane < rows) v = mine[jj];
+        w[4 * jj] = v.x; w[4 * jj + 1] = v.y; w[4 * jj + 2] = v.z; w[4 * jj + 3] = v.w;
+      }
+    } else {
+      // half a warp fetches the 16 columns of a row (32 contiguous bytes); the staging buffer turns them
+      __syncwarp();
+      const int cc = lane & 15;
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const int rr = 2 * k + (lane >> 4);
+        T x = Traits<T>::from_float(0.f);
+        if (cc < valid && rr < rows) x = src[(size_t)rr * p.N + cc];
+        *reinterpret_cast<T *>(s_stage + rr * 32 + 16 * ((cc >> 3) ^ ((rr >> 2) & 1)) + 2 * (cc & 7)) = x;
+      }
+      __syncwarp();
+      const int flip = (lane >> 2) & 1;
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
-        if (8 * jj < valid) pk_next[jj] = reinterpret_cast<const uint4 *>(my_row + c0)[jj];
+      for (int jj = 0; jj < 2; ++jj) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(s_stage + lane * 32 + 16 * (flip ^ jj));
+        w[4 * jj] = v.x; w[4 * jj + 1] = v.y; w[4 * jj + 2] = v.z; w[4 * jj + 3] = v.w;
+      }
     }
   }
 
-  __device__ __forceinline__ void finish(int j) {
-    constexpr int TILE_M = BLOCK_M * CTAS;
-    const int tile = unit + j * num_units;
-    const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M + sub * 32;   // first row of this warp
-    const int n0 = (tile / p.num_m_tiles) * p.block_n + cb;
-    const int lim = min(p.N - n0, cn);
-    const int r = j & 1;
+  // `keep`: the kept outlier product, or room for the addend y of a tile without one
+  __device__ __forceinline__ void finish(int j, uint32_t (&keep)[COLS / 2]) {
+    const Part t = part(j);
+    const int row = t.m0 + lane;
+    float srow = 0.f, zs = 0.f;
+    // everything that comes from memory is fetched before waiting for the integer product: such a load queues behind the
+    // operand loads that fill the SM's port to L2 and takes 2 to 3 thousand cycles
     if (p.mode == 1) {
       __syncwarp();                         // previous readers of the vectors are done
       for (int c = lane; c < cn32; c += 32) {
-        const int col = n0 + c;
-        const bool in = c < lim;
+        const int col = t.n0 + c;
+        const bool in = c < t.lim;
         s_scol[c] = in ? ldf<T>(p.scale_col, col) : 0.f;
         s_wred[c] = (in && p.w_reduced) ? ldf<T>(p.w_reduced, col) : 0.f;
-        s_bias[c] = (in && p.bias && !HAS_FP) ? ldf<T>(p.bias, col) : 0.f;   // with outliers the drain added it
+        if (!HAS_FP) s_bias[c] = (in && p.bias) ? ldf<T>(p.bias, col) : 0.f;   // with outliers the drain added it
+      }
+      if (row < p.M) {
+        srow = ldf<T>(p.row_scale, (size_t)row * p.row_stride);
+        const float zrow = p.row_zero ? ldf<T>(p.row_zero, (size_t)row * p.row_stride) : 0.f;
+        zs = fmaf(p.shift_value, srow, zrow);
       }
       __syncwarp();
+      if (!HAS_FP && p.y != nullptr) {
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c)
+          if (16 * c < t.lim) load_y(t, c, keep + 8 * c);
+      }
     }
-    const int row = m0 + lane;
-    const bool row_ok = row < p.M;
-    const bool rows_in = m0 + 32 <= p.M;
-    T *sub_base = static_cast<T *>(p.out) + (size_t)m0 * p.ldo + n0;
-    const T *my_row = static_cast<const T *>(p.out) + (size_t)row * p.ldo + n0;
-    // The parked outlier product of the first 32 columns is fetched before waiting for the integer
-    // product, the following ones one step ahead, so their L2 latency stays off the critical path.
-    uint4 pk_next[4];
-    prefetch_parked(pk_next, sub_base, my_row, rows_in, row_ok, lim, 0);
-    const long long tw = clock64();
-    const bool ready = mbar_wait(smem_u32(acc_full + r), (uint32_t)(j >> 1) & 1u, abort_flag, p.status);
-    if (!__all_sync(0xffffffffu, ready)) { ok = false; return; }
-    const long long tw1 = clock64();
-    e_wait_acc += tw1 - tw;
-    tc_fence_after();
-    float srow = 0.f, zs = 0.f;
-    if (p.mode == 1 && row_ok) {
-      srow = ldf<T>(p.row_scale, (size_t)row * p.row_stride);
-      const float zrow = p.row_zero ? ldf<T>(p.row_zero, (size_t)row * p.row_stride) : 0.f;
-      zs = fmaf(p.shift_value, srow, zrow);
-    }
+    if (!wait(acc_full, j, e_wait_acc)) return;
+    const long long t1 = clock64();
     const int shift = p.acc_shift;
-    const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16) + r * region_stride + cb;
-#pragma unroll 1
-    for (int c0 = 0; c0 < cn; c0 += 32) {
-      uint32_t v[32];
-      uint4 pk[4];
+    const uint32_t taddr = accumulators(j & 1);
+    const int rows = p.M - t.m0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) pk[i] = pk_next[i];
+    for (int c = 0; c < CHUNKS; ++c) {
+      if (16 * c >= t.lim) break;            // warp-uniform
+      uint32_t v[16];
       __syncwarp();                          // tcgen05.ld is warp-collective: reconverge first
-      tmem_ld32(taddr + c0, v);
-      if (c0 + 32 < cn) prefetch_parked(pk_next, sub_base, my_row, rows_in, row_ok, lim, c0 + 32);
-      tmem_ld_wait();
-      const int valid = lim - c0;            // warp-uniform
-      if (valid <= 0) continue;
-      const int col0 = n0 + c0;
-      const size_t off = (size_t)row * p.N + col0;
+      tmem_ld16(taddr + 16 * c, v);
+      tmem_ld_wait(v);
+      const int valid = t.lim - 16 * c, col0 = t.n0 + 16 * c;
       if (p.mode == 0) {
-        if (!row_ok) continue;
-        if (p.vec_out) {                     // valid is a multiple of 4 here
-          int4 *dst = reinterpret_cast<int4 *>(p.C + off);
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (4 * i < valid)
-              dst[i] = make_int4((int)v[4 * i] >> shift, (int)v[4 * i + 1] >> shift, (int)v[4 * i + 2] >> shift,
-                                 (int)v[4 * i + 3] >> shift);
-        } else {
-          for (int i = 0; i < 32; ++i)
-            if (i < valid) p.C[off + i] = (int)v[i] >> shift;
-        }
+        for (int i = 0; i < 16; ++i) v[i] = (uint32_t)((int)v[i] >> shift);
+        int32_t *dst = p.C + (size_t)t.m0 * p.N + col0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          store_row_pieces<4>(make_uint4(v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3]),
+                              make_uint4(v[8 * h + 4], v[8 * h + 5], v[8 * h + 6], v[8 * h + 7]),
+                              reinterpret_cast<unsigned char *>(dst + 8 * h), (size_t)p.N * 4, rows, 4 * (valid - 8 * h));
         continue;
       }
-      float o[32];   // addend first, result later
-      if (HAS_FP) {
-        if (p.vec_out) {
-          const T *pe = reinterpret_cast<const T *>(pk);
+      float o[16];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = Traits<T>::to_float(pe[i]);   // pieces beyond `valid` are never stored
-        } else {
-          for (int i = 0; i < 32; ++i)
-            o[i] = (row_ok && i < valid) ? Traits<T>::to_float(my_row[c0 + i]) : 0.f;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = s_bias[c0 + i];
-      }
-      if (p.y != nullptr && row_ok) {
-        T yv[32];
-        load_row32<T>(static_cast<const T *>(p.y) + off, valid >= 32 && p.vec_y, valid, yv);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] += Traits<T>::to_float(yv[i]);
-      }
-#pragma unroll
-      for (int i4 = 0; i4 < 8; ++i4) {
-        const float4 sc4 = reinterpret_cast<const float4 *>(s_scol + c0)[i4];
-        const float4 wr4 = reinterpret_cast<const float4 *>(s_wred + c0)[i4];
+      for (int i4 = 0; i4 < 4; ++i4) {
+        const float4 sc4 = reinterpret_cast<const float4 *>(s_scol + 16 * c)[i4];
+        const float4 wr4 = reinterpret_cast<const float4 *>(s_wred + 16 * c)[i4];
         const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
         const float wr[4] = {wr4.x, wr4.y, wr4.z, wr4.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int i = 4 * i4 + q;
+          float a;
+          if (HAS_FP) {
+            a = Traits<T>::unpack(keep[8 * c + i / 2], i & 1);
+          } else {
+            a = s_bias[16 * c + i];
+            if (p.y != nullptr) a += Traits<T>::unpack(keep[8 * c + i / 2], i & 1);
+          }
           // out = acc * (s_row * s_col) + ((zero + shift * s_row) * w_red + addend), fused multiply-adds
-          o[i] = fmaf((float)((int)v[i] >> shift), srow * sc[q], fmaf(zs, wr[q], o[i]));
+          o[i] = fmaf((float)((int)v[i] >> shift), srow * sc[q], fmaf(zs, wr[q], a));
         }
       }
-      if (p.vec_out) {
-        // Transpose through shared memory so that one warp instruction stores 8 rows x 64 contiguous
-        // bytes (whole sectors) instead of 32 rows x 16 bytes: lane i writes its row as four 16-byte
-        // pieces (swizzled against bank conflicts), lane L then stores piece L%4 of rows 8k + L/4.
-        __syncwarp();                        // the previous chunk has been read out of the buffer
+      uint32_t w[8];
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj)
-          *reinterpret_cast<uint4 *>(s_stage + lane * 64 + ((jj ^ ((lane >> 1) & 3)) << 4)) = pack8<T>(o + 8 * jj);
-        __syncwarp();
-        const int pc = lane & 3;
-        const bool col_ok = 8 * pc + 8 <= valid;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int rr = 8 * k + (lane >> 2);
-          const uint4 piece = *reinterpret_cast<const uint4 *>(s_stage + rr * 64 + ((pc ^ ((rr >> 1) & 3)) << 4));
-          if (col_ok && m0 + rr < p.M)
-            *(reinterpret_cast<uint4 *>(static_cast<T *>(p.out) + (size_t)(m0 + rr) * p.ldo + col0) + pc) = piece;
-        }
-      } else if (row_ok) {
-        store_row32<T>(static_cast<T *>(p.out) + (size_t)row * p.ldo + col0, false, valid, o);
-      }
+      for (int i = 0; i < 8; ++i) w[i] = Traits<T>::pack2(o[2 * i], o[2 * i + 1]);
+      T *dst = static_cast<T *>(p.out) + (size_t)t.m0 * p.ldo + col0;
+      store_row_pieces<2>(make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]),
+                          reinterpret_cast<unsigned char *>(dst), (size_t)p.ldo * 2, rows, 2 * valid);
     }
-    tc_fence_before();
-    if (CTAS == 1) mbar_arrive(smem_u32(acc_empty + r));
-    else mbar_arrive_leader(smem_u32(acc_empty + r));
-    e_finish += clock64() - tw1;
+    arrive(acc_empty, j);
+    e_finish += clock64() - t1;
   }
 
-  // all tiles of this CTA, in the order that lets drain(j + 1) and finish(j) hide behind the products of tile j / j + 1
+  // all tiles of this CTA
   __device__ __forceinline__ void run(int n_local) {
-    if (HAS_FP && n_local > 0) drain(0);
+    uint32_t keep[COLS / 2];
     for (int j = 0; j < n_local && ok; ++j) {
-      if (HAS_FP && j + 1 < n_local) drain(j + 1);
-      if (!ok) break;
-      finish(j);
+      if (HAS_FP) drain(j, keep);
+      if (ok) finish(j, keep);
     }
   }
 
@@ -339,7 +340,7 @@ struct EpilogueWarp {
     unsigned long long *d = p.dbg + (size_t)cta * 16;
     d[4] = (unsigned long long)e_wait_fp;     // epilogue warp: waiting for an outlier product
     d[5] = (unsigned long long)e_wait_acc;    // ... waiting for an integer product
-    d[6] = (unsigned long long)e_drain;       // ... parking outlier products
+    d[6] = (unsigned long long)e_drain;       // ... rounding and keeping outlier products
     d[7] = (unsigned long long)e_finish;      // ... final epilogues
   }
 };
@@ -377,10 +378,8 @@ inline void fill_epilogue_params(GemmParams &p, const Epilogue &ep, int M, int N
   p.dbg = get_debug_counters();
   p.status = device_status_word();
 }
-inline int split_columns(int block_n) {
-  const int h = (block_n / 2 + 31) & ~31;
-  return h < block_n ? h : block_n;
-}
+// columns of a tile per group of four epilogue warps
+inline int split_columns(int block_n, int groups) { return (block_n / groups + 31) & ~31; }
 
 }  // namespace
 }  // namespace quik

@@ -14,11 +14,11 @@
 //             per row, 128B swizzle) into a ring of shared-memory stages, completion on mbarriers.
 //   warp 1    allocates TMEM; one elected lane issues tcgen05.mma (M=128 or 256, N=block_n, K=32
 //             bytes) from shared-memory descriptors and commits each stage back to the producer.
-//   warps 2-9 epilogue: tcgen05.ld the accumulators (32 lanes x 32 columns per warp and step),
+//   warps 2-9 epilogue: tcgen05.ld the accumulators (32 lanes x 16 columns per warp and step),
 //             apply the dequantize arithmetic in fp32 and store through a shared-memory transpose.
 // Outlier k-blocks (64 fp16 values = 128 bytes per row) travel through the same ring as the integer
 // k-blocks; TMEM holds two accumulator regions so the epilogue of tile i overlaps the MMAs of tile
-// i+1 (schedule in the comment above the kernel).
+// i+1 (schedule in gemm_epilogue.cuh).
 // The tile width block_n is a launch parameter (any multiple of 16 up to the kernel's capacity CAP_N,
 // which fixes the shared-memory and TMEM plan): the host picks it per problem so that the tiles fill
 // whole waves of CTAs (choose_tile below).
@@ -39,7 +39,8 @@ __device__ unsigned int g_device_status = 0;
 
 namespace {
 
-constexpr int NUM_THREADS = 320;              // TMA warp + MMA warp + 8 epilogue warps
+constexpr int EPI_WARPS = 8;
+constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;      // TMA warp + MMA warp + epilogue warps
 // Process-wide tuning knobs (quik_config_set): plain words, meant to be set once before the layers run; a
 // launch reads each of them once.
 std::atomic<int> g_tile_n{0};                                 // 0 = choose by shape, else a multiple of 16 in [32, 256]
@@ -50,28 +51,19 @@ std::atomic<unsigned long long *> g_dbg{nullptr};             // diagnostic coun
 
 // Shared-memory plan after the 1024-byte aligned ring of stages: 256 bytes of barriers etc. and the
 // per-warp epilogue vectors (rounded to 1024 together), then one output staging chunk per epilogue
-// warp (32 rows x 64 bytes).
-constexpr int AUX_BYTES(int cap_n) { return ((256 + 8 * 3 * (cap_n / 2) * 4) + 1023) / 1024 * 1024; }
+// warp (32 rows x 32 bytes).
+constexpr int EPI_COLS(int cap_n) { return cap_n / (EPI_WARPS / 4); }       // most columns per epilogue warp
+constexpr int AUX_BYTES(int cap_n) { return ((256 + EPI_WARPS * 3 * EPI_COLS(cap_n) * 4) + 1023) / 1024 * 1024; }
 constexpr int stage_bytes(int cap_n, int ctas) { return (BLOCK_M + cap_n / ctas) * STAGE_K_BYTES; }
 // Ring depth: as many stages as fit (at most 8).
 constexpr int num_stages(int cap_n, int ctas) {
-  const int n = (SMEM_LIMIT - 1024 - AUX_BYTES(cap_n) - 8 * EPI_BUF_BYTES) / stage_bytes(cap_n, ctas);
+  const int n = (SMEM_LIMIT - 1024 - AUX_BYTES(cap_n) - EPI_WARPS * EPI_BUF_BYTES) / stage_bytes(cap_n, ctas);
   return n > 8 ? 8 : n;
 }
 
 // ---------------------------------------------------------------------------------------------
-// Work of one CTA = its tiles t_0, t_1, ... (tile index blockIdx.x + j * gridDim.x).  TMEM holds
-// two accumulator regions (CAP_N columns apart); tile j uses region j & 1 for BOTH of its products,
-// one after the other:
-//   FP(t_j):  outlier k-blocks -> region (f32), drained by the epilogue warps, which round
-//             (product + bias) to T and park it in the tile's place in `out` (it stays in L2);
-//   INT(t_j): integer k-blocks -> same region (s32), then the final epilogue reads the parked
-//             value back (same thread, same address), applies the dequantize arithmetic and
-//             overwrites it.
-// The MMA issue order is FP(t_0), then for every j: first half of INT(t_j), FP(t_{j+1}), second half
-// of INT(t_j).  FP(t_{j+1}) and its drain therefore run in the shadow of INT(t_j), and the epilogue of
-// t_j in the shadow of INT(t_{j+1}): the tensor pipe never waits for an epilogue in steady state
-// although int32 and fp32 accumulators cannot share a region at the same time.
+// The tiles of a CTA are blockIdx.x + j * gridDim.x; their two accumulator regions in TMEM (CAP_N columns apart) and the order
+// of their products are described in gemm_epilogue.cuh.
 //
 // CTAS == 2: two CTAs on neighbouring SMs (a cluster of 2) work on one 256 x block_n tile.  Each
 // loads its own 128 rows of A and only its half of the B rows, so a CTA moves a third less operand
@@ -86,7 +78,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   constexpr int STAGE_BYTES = stage_bytes(CAP_N, CTAS);      // room for the widest tile; narrower ones use less of it
   constexpr int STAGES = num_stages(CAP_N, CTAS);
   constexpr int TMEM_ALLOC = 2 * CAP_N;                       // two accumulator regions, CAP_N columns apart
-  constexpr int HALF_CAP = CAP_N / 2;                         // most columns per epilogue warp
   constexpr int TILE_M = BLOCK_M * CTAS;
   const int bn = p.block_n;
   const int b_rows = bn / CTAS;                               // B rows this CTA loads per k-block
@@ -101,12 +92,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   uint64_t *acc_full = empty_bar + STAGES;                             // [2] integer product complete
   uint64_t *acc_empty = acc_full + 2;                                  // [2] region free again
   uint64_t *fp_full = acc_empty + 2;                                   // [2] outlier product complete
-  uint64_t *fp_drained = fp_full + 2;                                  // [2] outlier product parked
+  uint64_t *fp_drained = fp_full + 2;                                  // [2] outlier product kept, region free
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fp_drained + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // per-column epilogue vectors, one private copy per epilogue warp (no cross-warp barrier needed)
-  float *s_vec = reinterpret_cast<float *>(aux + 256);                 // [8][3][HALF_CAP], 16-byte aligned
-  // output staging: [8 warps][32 rows x 64 bytes], 1024-byte aligned
+  float *s_vec = reinterpret_cast<float *>(aux + 256);                 // [EPI_WARPS][3][EPI_COLS], 16-byte aligned
+  // output staging: [EPI_WARPS][32 rows x 32 bytes], 1024-byte aligned
   unsigned char *s_out = tiles + STAGES * STAGE_BYTES + AUX_BYTES(CAP_N);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -119,9 +110,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), NUM_EPI_THREADS * CTAS);    // epilogue threads of the whole pair
+      mbar_init(smem_u32(acc_empty + s), 32 * EPI_WARPS * CTAS);    // epilogue threads of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
-      mbar_init(smem_u32(fp_drained + s), NUM_EPI_THREADS * CTAS);
+      mbar_init(smem_u32(fp_drained + s), 32 * EPI_WARPS * CTAS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -147,49 +138,39 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int rank = CTAS == 2 ? (int)cluster_ctarank() : 0;
   const int unit = (int)blockIdx.x / CTAS, num_units = (int)gridDim.x / CTAS;    // a unit = CTA or CTA pair
   const int n_local = (p.num_tiles - unit + num_units - 1) / num_units;           // tiles of this unit
-  const int int_half = (p.int_kb + 1) / 2;
 
   if (warp == 0) {
     // ================= TMA producer =================
     const bool elected = elect_one();
     int stage = 0;
     uint32_t phase = 0;
-    bool ok = true;
     // The token operand A is read again by every column tile of the launch and fits in L2: its lines are marked to
     // be evicted last, so that data streaming through L2 meanwhile (the weights, the outputs, a tensor-parallel
     // rank's peer copies) does not push it out.
     const uint64_t keep = l2_policy_evict_last();
     const bool hint = p.l2_hint != 0;
-    // one k-block range of one product of tile j into the ring
-    auto feed = [&](int j, bool fp, int kb0, int kb1) {
+    for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
+      constexpr bool fp = decltype(is_fp)::value;
       const int tile = unit + j * num_units;
       const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M;      // this CTA's rows of A
       const int n0 = (tile / p.num_m_tiles) * bn + rank * b_rows;           // this CTA's rows of B
-      for (int kb = kb0; kb < kb1; ++kb) {
-        ok = mbar_wait_warp(smem_u32(empty_bar + stage), phase ^ 1, abort_flag, p.status);
-        if (!ok) return;
-        if (elected) {
-          const uint32_t fb = smem_u32(full_bar + stage);
-          const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
-          if (rank == 0) mbar_expect_tx(fb, stage_tx);
-          if (fp) {
-            tma_load_2d<CTAS>(sa, &tmap_fa, fb, kb * 64, m0);
-            tma_load_2d<CTAS>(sa + A_BYTES, &tmap_fb, fb, kb * 64, n0);
-          } else {
-            if (hint) tma_load_2d_policy<CTAS>(sa, &tmap_a, fb, kb * STAGE_K_BYTES, m0, keep);
-            else tma_load_2d<CTAS>(sa, &tmap_a, fb, kb * STAGE_K_BYTES, m0);
-            tma_load_2d<CTAS>(sa + A_BYTES, &tmap_b, fb, kb * STAGE_K_BYTES, n0);
-          }
+      if (!mbar_wait_warp(smem_u32(empty_bar + stage), phase ^ 1, abort_flag, p.status)) return false;
+      if (elected) {
+        const uint32_t fb = smem_u32(full_bar + stage);
+        const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
+        if (rank == 0) mbar_expect_tx(fb, stage_tx);
+        if (fp) {
+          tma_load_2d<CTAS>(sa, &tmap_fa, fb, kb * 64, m0);
+          tma_load_2d<CTAS>(sa + A_BYTES, &tmap_fb, fb, kb * 64, n0);
+        } else {
+          if (hint) tma_load_2d_policy<CTAS>(sa, &tmap_a, fb, kb * STAGE_K_BYTES, m0, keep);
+          else tma_load_2d<CTAS>(sa, &tmap_a, fb, kb * STAGE_K_BYTES, m0);
+          tma_load_2d<CTAS>(sa + A_BYTES, &tmap_b, fb, kb * STAGE_K_BYTES, n0);
         }
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-    };
-    if (HAS_FP && n_local > 0) feed(0, true, 0, p.fp_kb);
-    for (int j = 0; j < n_local && ok; ++j) {
-      feed(j, false, 0, int_half);
-      if (HAS_FP && ok && j + 1 < n_local) feed(j + 1, true, 0, p.fp_kb);
-      if (ok) feed(j, false, int_half, p.int_kb);
-    }
+      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      return true;
+    });
     __syncwarp();
   } else if (warp == 1) {
     // ================= MMA issuer (pair leader only) =================
@@ -204,58 +185,37 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint64_t da0 = make_smem_desc(smem_u32(tiles)), db0 = make_smem_desc(smem_u32(tiles) + A_BYTES);
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
       long long w_region = 0, w_full = 0;
       const long long t_begin = clock64();
-      // one k-block of one product into the accumulator at `d`
-      auto block = [&](bool fp, uint32_t d, uint32_t idesc, bool first) {
+      for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
+      constexpr bool fp = decltype(is_fp)::value;
+        if (kb == 0) {
+          const long long t0 = dbg ? clock64() : 0;
+          uint32_t parity;
+          const uint64_t *bar = region_barrier<HAS_FP>(j, fp, acc_empty, fp_drained, parity);
+          if (bar != nullptr && !mbar_wait_warp(smem_u32(bar), parity, abort_flag, p.status)) return false;
+          if (dbg) w_region += clock64() - t0;
+        }
         const long long t1 = dbg ? clock64() : 0;
-        ok = mbar_wait_warp(smem_u32(full_bar + stage), phase, abort_flag, p.status);
+        if (!mbar_wait_warp(smem_u32(full_bar + stage), phase, abort_flag, p.status)) return false;
         if (dbg) w_full += clock64() - t1;
-        if (!ok) return;
         tc_fence_after();
         if (elected) {
           // stage bases and 32-byte K steps inside the swizzled row are offsets of the 16-byte start-address field
           const uint64_t da = da0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), db = db0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
+          const uint32_t d = tmem_base + ((fp ? j + 1 : j) & 1) * CAP_N;
 #pragma unroll
           for (int k = 0; k < STAGE_K_BYTES / 32; ++k) {
-            if (fp) mma_f16<CTAS>(d, da + 2 * k, db + 2 * k, idesc, (k > 0 || !first) ? 1u : 0u);
-            else mma_i8<CTAS>(d, da + 2 * k, db + 2 * k, idesc, (k > 0 || !first) ? 1u : 0u);
+            if (fp) mma_f16<CTAS>(d, da + 2 * k, db + 2 * k, p.idesc_fp, (k > 0 || kb > 0) ? 1u : 0u);
+            else mma_i8<CTAS>(d, da + 2 * k, db + 2 * k, p.idesc_int, (k > 0 || kb > 0) ? 1u : 0u);
           }
           mma_commit<CTAS>(smem_u32(empty_bar + stage));    // stage reusable once these MMAs retire
+          if (fp && kb == p.fp_kb - 1) mma_commit<CTAS>(smem_u32(fp_full + (j & 1)));
+          if (!fp && kb == p.int_kb - 1) mma_commit<CTAS>(smem_u32(acc_full + (j & 1)));
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
-      };
-      // waits until the accumulator region may be overwritten: after the previous tile's epilogue (outlier product, or
-      // integer product of an outlier-free layer), or after this tile's drain
-      auto region_free = [&](uint64_t *bar, uint32_t parity) {
-        const long long t0 = dbg ? clock64() : 0;
-        ok = mbar_wait_warp(smem_u32(bar), parity, abort_flag, p.status);
-        if (dbg) w_region += clock64() - t0;
-        tc_fence_after();
-      };
-      auto issue_fp = [&](int j) {
-        const int r = j & 1;
-        region_free(acc_empty + r, ((uint32_t)(j >> 1) & 1u) ^ 1u);
-        for (int kb = 0; kb < p.fp_kb && ok; ++kb) block(true, tmem_base + r * CAP_N, p.idesc_fp, kb == 0);
-        if (ok && elected) mma_commit<CTAS>(smem_u32(fp_full + r));
-      };
-      auto issue_int = [&](int j, int kb0, int kb1) {
-        const int r = j & 1;
-        for (int kb = kb0; kb < kb1 && ok; ++kb) block(false, tmem_base + r * CAP_N, p.idesc_int, kb == 0);
-      };
-      if (HAS_FP && n_local > 0) issue_fp(0);
-      for (int j = 0; j < n_local && ok; ++j) {
-        const uint32_t use_parity = (uint32_t)(j >> 1) & 1u;
-        if (HAS_FP) region_free(fp_drained + (j & 1), use_parity);
-        else region_free(acc_empty + (j & 1), use_parity ^ 1u);
-        if (!ok) break;
-        issue_int(j, 0, int_half);
-        if (HAS_FP && j + 1 < n_local && ok) issue_fp(j + 1);
-        if (!ok) break;
-        issue_int(j, int_half, p.int_kb);
-        if (ok && elected) mma_commit<CTAS>(smem_u32(acc_full + (j & 1)));
-      }
+        return true;
+      });
       if (dbg && lane == 0) {
         unsigned long long *d = p.dbg + (size_t)blockIdx.x * 16;
         d[0] = (unsigned long long)(clock64() - t_begin);   // MMA warp: issue loop
@@ -266,8 +226,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else {
     // ================= epilogue (warps 2..9): gemm_epilogue.cuh =================
-    EpilogueWarp<T, HAS_FP, CTAS> ew(p, tmem_base, CAP_N, unit, num_units, rank, warp - 2, warp & 3, lane, s_vec,
-                                     HALF_CAP, s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
+    EpilogueWarp<T, HAS_FP, CTAS, EPI_COLS(CAP_N)> ew(p, tmem_base, CAP_N, unit, num_units, rank, warp - 2, warp & 3, lane, s_vec,
+                                                      s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
     ew.run(n_local);
     if (p.dbg && warp == 2 && lane == 0) ew.write_counters((int)blockIdx.x);
   }
@@ -360,7 +320,7 @@ namespace {
 
 constexpr size_t smem_bytes(int cap_n, int ctas) {
   return 1024 /*align slack*/ + (size_t)num_stages(cap_n, ctas) * stage_bytes(cap_n, ctas) + AUX_BYTES(cap_n) +
-         8 * EPI_BUF_BYTES;
+         EPI_WARPS * EPI_BUF_BYTES;
 }
 
 // Largest number of CTA pairs that can be resident at once (0 if pairs cannot be launched).
@@ -422,12 +382,13 @@ int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tf
 }
 
 // ---- tile shape per problem -------------------------------------------------------------------
-// A launch is a number of waves of equally sized tiles over the resident units (CTAs or CTA pairs).  Measured on the
-// Llama-2 shapes (7B at 2048 tokens, 70B at 4096, and their column shards for 2/4/8 GPUs): the time of a tile hardly
-// depends on its width -- a tcgen05.mma with both operands in shared memory occupies its issuing thread ~217 cycles
-// whatever its N -- so per k-block a tile costs about kBlockClk + kColClk * block_n cycles.  A narrower tile is
-// therefore almost as expensive as the widest one and only pays where it saves a whole wave; among widths with the
-// same number of waves the narrowest wins by a little.
+// A launch is a number of waves of equally sized tiles over the resident units (CTAs or CTA pairs).  The time of a tile depends
+// little on its width: a k-block of a pair moves 16 KB of A and 64 * block_n bytes of B per CTA through the SM's 64-byte port to
+// L2 (a sweep over 30 problems of 160 to 2048 tokens fits 179 + 0.50 * block_n ns, single CTAs 215 + 0.67 * block_n), so per
+// k-block a tile costs about kBlockClk + kColClk * block_n cycles.  A narrower tile is therefore almost as expensive as the
+// widest one and only pays where it saves a whole wave; among widths with the same number of waves the narrowest wins by a
+// little.  In that sweep the choice was within 2 % of the best width for all but three problems (10 % for 160 tokens through
+// 4096 x 4096).
 constexpr double kBlockClk = 366.0;
 constexpr double kColClk = 0.45;
 constexpr double kTileFixedClk = 1500.0;
@@ -514,7 +475,7 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   fill_epilogue_params(p, ep, M, N);
   if (p.status == nullptr) return QUIK_ERR_CUDA;
   p.block_n = block_n;
-  p.split_n = split_columns(block_n);
+  p.split_n = split_columns(block_n, EPI_WARPS / 4);
   p.num_m_tiles = m_tiles;
   p.num_tiles = m_tiles * ((N + block_n - 1) / block_n);
   p.idesc_int = make_idesc(2, 1, tile_m, block_n);                              // S32 accumulate, signed 8-bit operands

@@ -28,6 +28,7 @@ namespace quik {
 namespace {
 
 constexpr int TS_THREADS = 448;
+constexpr int TS_EPI_WARPS = 8;
 constexpr int TS_MAX_N = 224;                 // 2 x 224 accumulator columns + 2 operand slots = 512
 constexpr int TS_HALF_CAP = 128;              // most columns per epilogue warp
 constexpr int TS_A_BYTES = BLOCK_M * STAGE_K_BYTES;           // room for an unpacked k-block of A (packed: first half)
@@ -35,29 +36,11 @@ constexpr int TS_MAX_SLOTS = 4;
 constexpr int TS_AUX_BYTES = ((512 + 8 * 3 * TS_HALF_CAP * 4) + 1023) / 1024 * 1024;
 constexpr int ts_stage_bytes(int ctas) { return TS_A_BYTES + (TS_MAX_N / ctas) * STAGE_K_BYTES; }
 constexpr int ts_num_stages(int ctas) {
-  const int n = (SMEM_LIMIT - 1024 - TS_AUX_BYTES - 8 * EPI_BUF_BYTES) / ts_stage_bytes(ctas);
+  const int n = (SMEM_LIMIT - 1024 - TS_AUX_BYTES - TS_EPI_WARPS * EPI_BUF_BYTES) / ts_stage_bytes(ctas);
   return n > 8 ? 8 : n;
 }
 constexpr size_t ts_smem_bytes(int ctas) {
-  return 1024 + (size_t)ts_num_stages(ctas) * ts_stage_bytes(ctas) + TS_AUX_BYTES + 8 * EPI_BUF_BYTES;
-}
-
-// The k-blocks of a CTA in issue order: outlier blocks of tile 0; then per tile j the first half of its integer
-// blocks, the outlier blocks of tile j + 1, the second half of its integer blocks (so that the drain of tile j + 1 and
-// the epilogue of tile j hide behind integer products).  fn(j, fp, kb) returns false to stop.
-template <bool HAS_FP, typename Fn>
-__device__ __forceinline__ void for_each_block(int n_local, int int_kb, int fp_kb, Fn fn) {
-  const int int_half = (int_kb + 1) / 2;
-  bool ok = true;
-  auto range = [&](int j, bool fp, int kb0, int kb1) {
-    for (int kb = kb0; kb < kb1 && ok; ++kb) ok = fn(j, fp, kb);
-  };
-  if (HAS_FP && n_local > 0) range(0, true, 0, fp_kb);
-  for (int j = 0; j < n_local && ok; ++j) {
-    range(j, false, 0, int_half);
-    if (HAS_FP && j + 1 < n_local) range(j + 1, true, 0, fp_kb);
-    range(j, false, int_half, int_kb);
-  }
+  return 1024 + (size_t)ts_num_stages(ctas) * ts_stage_bytes(ctas) + TS_AUX_BYTES + TS_EPI_WARPS * EPI_BUF_BYTES;
 }
 
 template <typename T, bool HAS_FP, int CTAS, bool A_PACKED>
@@ -86,7 +69,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   uint64_t *acc_full = a_empty + TS_MAX_SLOTS;                         // [2] integer product complete
   uint64_t *acc_empty = acc_full + 2;                                  // [2] region free again
   uint64_t *fp_full = acc_empty + 2;                                   // [2] outlier product complete
-  uint64_t *fp_drained = fp_full + 2;                                  // [2] outlier product parked
+  uint64_t *fp_drained = fp_full + 2;                                  // [2] outlier product kept, region free
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fp_drained + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   float *s_vec = reinterpret_cast<float *>(aux + 512);                 // [8][3][TS_HALF_CAP]
@@ -107,9 +90,9 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), NUM_EPI_THREADS * CTAS);    // epilogue threads of the whole pair
+      mbar_init(smem_u32(acc_empty + s), 32 * TS_EPI_WARPS * CTAS);    // epilogue threads of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
-      mbar_init(smem_u32(fp_drained + s), NUM_EPI_THREADS * CTAS);
+      mbar_init(smem_u32(fp_drained + s), 32 * TS_EPI_WARPS * CTAS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -141,7 +124,8 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, bool fp, int kb) {
+      for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
+        constexpr bool fp = decltype(is_fp)::value;
         const int tile = unit + j * num_units;
         const int m0 = (tile % p.num_m_tiles) * TILE_M + rank * BLOCK_M;      // this CTA's rows of A
         const int n0 = (tile / p.num_m_tiles) * bn + rank * b_rows;           // this CTA's rows of B
@@ -168,17 +152,15 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       uint32_t phase = 0, slot_phase = 0;
       long long w_region = 0, w_full = 0, w_a = 0;
       const long long t_begin = clock64();
-      for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, bool fp, int kb) {
+      for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
+        constexpr bool fp = decltype(is_fp)::value;
         const int r = j & 1;
-        const uint32_t use_parity = (uint32_t)(j >> 1) & 1u;
-        const uint32_t d = tmem_base + r * bn;
+        const uint32_t d = tmem_base + ((fp ? j + 1 : j) & 1) * bn;
         if (kb == 0) {
-          // the region must be free: after the previous tile's epilogue (outlier product, or integer product of
-          // an outlier-free layer), or after this tile's drain
-          const bool after_drain = HAS_FP && !fp;
-          const uint32_t bar = smem_u32((after_drain ? fp_drained : acc_empty) + r);
+          uint32_t parity;
+          const uint64_t *bar = region_barrier<HAS_FP>(j, fp, acc_empty, fp_drained, parity);
           const long long t0 = clock64();
-          if (!mbar_wait(bar, after_drain ? use_parity : (use_parity ^ 1u), abort_flag, p.status)) return false;
+          if (bar != nullptr && !mbar_wait(smem_u32(bar), parity, abort_flag, p.status)) return false;
           w_region += clock64() - t0;
         }
         const long long t1 = clock64();
@@ -221,7 +203,8 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     int stage = 0, slot = 0;
     uint32_t phase = 0, slot_phase = 0;
     long long c_full = 0, c_slot = 0;
-    for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, bool fp, int kb) {
+    for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
+        constexpr bool fp = decltype(is_fp)::value;
       const long long t0 = clock64();
       const bool landed = mbar_wait(smem_u32(a_bar + stage), phase, abort_flag, p.status);
       if (!__all_sync(0xffffffffu, landed)) return false;
@@ -275,8 +258,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
   } else {
     // ================= epilogue (warps 6..13): gemm_epilogue.cuh =================
-    EpilogueWarp<T, HAS_FP, CTAS> ew(p, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec, TS_HALF_CAP,
-                                     s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
+    EpilogueWarp<T, HAS_FP, CTAS, TS_HALF_CAP> ew(p, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec, s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
     ew.run(n_local);
     if (p.dbg && warp == 6 && lane == 0) ew.write_counters((int)blockIdx.x);
   }
@@ -400,7 +382,7 @@ int launch_gemm_tcgen05_ts(const void *A, int a_packed, const int8_t *B, int M, 
   fill_epilogue_params(p, ep, M, N);
   if (p.status == nullptr) return QUIK_ERR_CUDA;
   p.block_n = block_n;
-  p.split_n = split_columns(block_n);
+  p.split_n = split_columns(block_n, TS_EPI_WARPS / 4);
   p.num_m_tiles = m_tiles;
   p.num_tiles = m_tiles * ((N + block_n - 1) / block_n);
   p.idesc_int = make_idesc(2, 1, tile_m, block_n);

@@ -412,3 +412,27 @@ def test_streaming_engine_at_every_width(M, K, N, F, bits):
     few = case.module(case.x[:16].contiguous())[0]                       # other engine: exact integers, fp32 outlier product
     assert rel_rms_err(out[:16].cpu(), few.cpu()) < 5e-3
     assert_device_clean()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("engine", [_lib.ENGINE_TCGEN05, _lib.ENGINE_TCGEN05_TS], ids=["smem_operands", "tmem_operand"])
+@pytest.mark.parametrize("N", [3600, 3599, 3602])
+@pytest.mark.parametrize("F", [64, 0])
+def test_many_tiles_per_cta_and_ragged_rows(N, F, engine, dtype):
+    """Four tiles of 32 columns per CTA or pair, so that both accumulator regions change hands several times, with integer
+    products of one and of three k-blocks; output rows with 16-byte, 2-byte and 4-byte alignment, the last tile ragged in
+    both directions."""
+    for K in (64 + F, 320 + F):
+        case = make_layer("t", 300, K, N, 4, F=F, seed=N, device=dev(), dtype=dtype, clip=False)
+        try:
+            _lib.set_engine(engine)
+            _lib.set_tile_n(32)
+            for pair in (2, 1):
+                _lib.set_cta_pair(pair)
+                out = case.module(case.x.unsqueeze(0))[0]
+                assert rel_rms_err(out.cpu(), _oracle_out(case, round_y=True)) < (TOL_RMS if dtype == torch.float16 else 4e-2)
+        finally:
+            _lib.set_engine(_lib.ENGINE_AUTO)
+            _lib.set_tile_n(0)
+            _lib.set_cta_pair(0)
+    assert_device_clean()
