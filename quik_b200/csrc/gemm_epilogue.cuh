@@ -51,11 +51,11 @@ template <typename T> __device__ __forceinline__ float ldf(const void *p, size_t
 // region, which the epilogue of t_{j-1} has left by then.  The epilogue warps round FP(t_j) + bias to T and keep it in
 // registers (drain), which frees that region for INT(t_{j+1}), and combine it with the integer product when that is complete
 // (finish).  So both hide behind integer products and only the last tile's finish has nothing to hide behind.
-// (Before, FP(t_{j+1}) was issued in the middle of INT(t_j) and its rounded value parked in the tile's place in `out` until
-// INT(t_{j+1}) was complete; fetching it back queued behind the operand loads that fill the SM's port to L2, the two parts of
-// the epilogue took 15 to 18 thousand cycles per 256 x 256 tile, and the first drain had nothing to hide behind.
-// Llama-2-7B at 2048 tokens: the issuing warp waited 23.4 thousand of 136 thousand cycles for a free region in the qkv layer and
-// 58 of 242 in gate+up, now 12.7 of 121 and 23.7 of 206; 87.5 -> 81.4 us and 155.4 -> 140.3 us.)
+// (Before, FP(t_{j+1}) was issued in the middle of INT(t_j), its rounded value parked in the tile's place in `out` until
+// INT(t_{j+1}) was complete and fetched back in the epilogue, and the first drain had nothing to hide behind.  Llama-2-7B at 2048
+// tokens, before and now: drain 6.1 -> 3.6 and finish 9.2 -> 8.6 thousand cycles per 256 x 224 tile, the issuing warp waits for a
+// free region 23.4 of 136 -> 12.7 of 121 thousand cycles in the qkv layer and 58 of 242 -> 23.7 of 206 in gate+up; 87.5 -> 81.4 us
+// and 155.4 -> 140.3 us.)
 // This walks the k-blocks in issue order; fn(j, fp, kb) returns false to stop.  `fp` is a compile-time flag (std::true_type /
 // std::false_type): a narrow tile's block occupies the tensor pipe for less than 200 cycles, the issuing warp has none to spare
 // for choosing between the two kinds of instruction.
@@ -248,8 +248,7 @@ struct EpilogueWarp {
     const Part t = part(j);
     const int row = t.m0 + lane;
     float srow = 0.f, zs = 0.f;
-    // everything that comes from memory is fetched before waiting for the integer product: such a load queues behind the
-    // operand loads that fill the SM's port to L2 and takes 2 to 3 thousand cycles
+    // everything that comes from memory is fetched before waiting for the integer product
     if (p.mode == 1) {
       __syncwarp();                         // previous readers of the vectors are done
       for (int c = lane; c < cn32; c += 32) {

@@ -383,9 +383,9 @@ int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tf
 
 // ---- tile shape per problem -------------------------------------------------------------------
 // A launch is a number of waves of equally sized tiles over the resident units (CTAs or CTA pairs).  The time of a tile depends
-// little on its width: a k-block of a pair moves 16 KB of A and 64 * block_n bytes of B per CTA through the SM's 64-byte port to
-// L2 (a sweep over 30 problems of 160 to 2048 tokens fits 179 + 0.50 * block_n ns, single CTAs 215 + 0.67 * block_n), so per
-// k-block a tile costs about kBlockClk + kColClk * block_n cycles.  A narrower tile is therefore almost as expensive as the
+// little on its width: a k-block of a pair moves 16 KB of A and 64 * block_n bytes of B per CTA from L2 (a sweep over 30 problems
+// of 160 to 2048 tokens fits 179 + 0.50 * block_n ns, single CTAs 215 + 0.67 * block_n, 15 to 18 TB/s over the chip), so per k-block
+// a tile costs about kBlockClk + kColClk * block_n cycles.  A narrower tile is therefore almost as expensive as the
 // widest one and only pays where it saves a whole wave; among widths with the same number of waves the narrowest wins by a
 // little.  In that sweep the choice was within 2 % of the best width for all but three problems (10 % for 160 tokens through
 // 4096 x 4096).
