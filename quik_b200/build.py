@@ -1,10 +1,11 @@
-"""Build libquik_b200.so in-tree with nvcc for sm_100a.
+"""Build libquik_b200.so in-tree with nvcc for sm_100a, and the CPython module _host (csrc/host_ext.cpp) with g++.
 
     python -m quik_b200.build            # build if sources are newer than the library
     python -m quik_b200.build --force
 
 The library is a plain C-ABI shared object (see include/quik_b200.h); it links the CUDA
-runtime statically and needs no GPU to build or to load.
+runtime statically and needs no GPU to build or to load.  _host is built against the headers and libraries of the torch that
+is installed; neither depends on the other at link time.
 """
 from __future__ import annotations
 
