@@ -58,9 +58,9 @@ def test_fused_forward_matches_oracle(dtype, M, K, N, F, bits):
 def test_fused_layer_writes_only_its_columns(M, K, N, F, bits, tile, pair, engine, col_pad):
     """The layer's output is a window of a poisoned slab (rows and columns of padding on every side, handed over as
     `out_buffer` with a row pitch wider than N): the window equals the plain forward bit for bit and the padding is
-    untouched.  col_pad = 8 keeps the window 16-byte aligned (vector stores, parked outlier products in the
-    permuted layout), col_pad = 3 does not (scalar stores); the tile widths end a warp's column range with a
-    16-column step.  Covers the ragged-edge stores and the parked-tile writes of the tiled kernel and the stores of
+    untouched.  col_pad = 8 keeps the window 16-byte aligned (vector stores), col_pad = 3 does not (element
+    stores); the tile widths end a warp's column range with a
+    16-column step.  Covers the ragged-edge stores of the tiled kernel and the stores of
     the weight-streaming engines (16 and 100 tokens)."""
     case = make_layer("t", M, K, N, bits, F=F, seed=M + N, device=dev(), clip=False)
     row_pad = 5
