@@ -195,21 +195,14 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
   }
 
   // ---- the producer of X, applied to the row in shared memory: 16 bytes per access, the last cols % 8 values one by one
-  // (instruction issue bounds this part: 40 to 48 instructions per value with 2-byte accesses; [4096, 8192] RMSNorm 50.2 -> 42.0 us,
+  // (instruction issue bounds this part: 40 to 48 instructions per value with 2-byte accesses; [4096, 8192] RMSNorm 50.2 -> 43.7 us,
   // SiLU 69.5 -> 60.1 us, [2048, 11008] SiLU 51.6 -> 46.9 us)
   if (PROD == 1) {
+    // The sum of squares keeps its order, thread t adding columns t, t + NTHR, ...: another order moves the last bit of rstd,
+    // and with it single values across a step of the quantization grid.
     float ss = 0.f;
-    const int nv = cols >> 3;
-    for (int i = tid; i < nv; i += NTHR) {
-      const uint4 v = reinterpret_cast<const uint4 *>(s_row)[i];
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float a = Traits<T>::unpack(w[j], 0), b = Traits<T>::unpack(w[j], 1);
-        ss = fmaf(b, b, fmaf(a, a, ss));
-      }
-    }
-    for (int i = 8 * nv + tid; i < cols; i += NTHR) {
+#pragma unroll 4
+    for (int i = tid; i < cols; i += NTHR) {
       const float f = Traits<T>::to_float(s_row[i]);
       ss = fmaf(f, f, ss);
     }
@@ -221,7 +214,7 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
 #pragma unroll
     for (int w = 0; w < NTHR / 32; ++w) ss += s_red[0][w];
     const float rstd = rsqrtf(ss / (float)cols + eps);
-    const int na = vec_aux ? nv : 0;
+    const int na = vec_aux ? cols >> 3 : 0;
     for (int i = tid; i < na; i += NTHR) {
       const uint4 v = reinterpret_cast<const uint4 *>(s_row)[i], g = __ldg(reinterpret_cast<const uint4 *>(aux) + i);
       uint32_t w[4] = {v.x, v.y, v.z, v.w};

@@ -173,6 +173,45 @@ def test_rmsnorm_quantize_matches_norm_then_quantize(dtype, M, K, F, bits, wide)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shift", [0, 1], ids=["aligned_norm", "unaligned_norm"])
+@pytest.mark.parametrize("M,K,F,bits,wide", [(300, 4096, 256, 4, True), (16, 4096, 256, 4, False), (2048, 1088, 64, 8, True),
+                                            (129, 11008, 256, 8, True), (149, 28672, 256, 8, True), (333, 2058, 32, 4, True),
+                                            (40, 2058, 32, 8, True)])
+def test_rmsnorm_quantize_keeps_the_order_of_its_sum(dtype, shift, M, K, F, bits, wide):
+    """The row statistic is summed in one fixed order: thread t of the row's CTA adds the squares of columns t, t + threads,
+    ..., the 32 sums of a warp fold by halves, the warps' sums are added in turn.  In that order torch gives the same fp32
+    statistic (the squares are exact in fp32), and so the same codes, meta and outliers bit for bit.  Row lengths that are
+    no multiple of 8 and norm weights off a 16-byte boundary take the element-wise paths."""
+    g = torch.Generator().manual_seed(M + K)
+    perm = torch.randperm(K, generator=g)
+    ids, fp_ids = perm[F:].sort()[0], perm[:F].sort()[0]
+    x = torch.randn(M, K, generator=g)
+    x[:, fp_ids] *= 20
+    x = (x * 1.7).to(dtype).to(dev())
+    w = (1.0 + 0.1 * torch.randn(K + shift, generator=g)).to(dtype).to(dev())[shift:]
+    i16, f16 = (t.to(torch.int16).to(dev()) for t in (ids, fp_ids))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    threads = 512 if M <= sms or K * 4 > 100 * 1024 else 256
+    sq = torch.nn.functional.pad(x.float().pow(2), (0, -K % threads)).view(M, -1, threads)
+    part = torch.zeros(M, threads, device=dev())
+    for i in range(sq.shape[1]):
+        part = part + sq[:, i]
+    part = part.view(M, threads // 32, 32)
+    for half in (16, 8, 4, 2, 1):
+        part = part[..., :half] + part[..., half:]
+    total = torch.zeros(M, 1, device=dev())
+    for i in range(threads // 32):
+        total = total + part[:, i]
+    mean = total / torch.full_like(total, K)                  # a division (a scalar divisor would become a product)
+    normed = (x.float() * torch.rsqrt(mean + 1e-5)).to(dtype) * w
+    got = asymmetric.rmsnorm_quantize_u16(x, w, 1e-5, i16, f16, bits, wide)
+    torch.cuda.synchronize()
+    for a, b in zip(got, asymmetric.quantize_u16(normed, i16, f16, bits, wide)):
+        assert torch.equal(a, b)
+    assert_device_clean()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("M,K,F,bits,wide", [(300, 11008, 256, 8, True), (16, 1408, 64, 8, True), (2048, 1408, 64, 4, True),
                                             (9, 608, 32, 4, False)])
 def test_silu_mul_quantize_matches_activation_then_quantize(dtype, M, K, F, bits, wide):
