@@ -159,6 +159,15 @@ int quik_silu_mul_quantize_u16(const void *gate, const void *up, int dtype, int 
                                const uint16_t *fp_indices, int num_fp, int bits, int wide,
                                void *dst, void *meta, void *fp_x, void *stream);
 
+/* The three calls above as a layer makes them: producer 0 = none (aux unused), 1 = RMSNorm (aux = norm_weight),
+ * 2 = SiLU(x) * aux.  ids_settled != 0 states that both id arrays were complete on the device before this call was made (a
+ * captured launch: before its graph is launched), e.g. because they were uploaded by a synchronous copy: the kernel then
+ * fetches them while its predecessor in the stream still runs.  With 0, as in the calls above, they may be written by any
+ * earlier work of the stream. */
+int quik_layer_quantize(int producer, const void *x, const void *aux, float eps, int dtype, int rows, int cols,
+                        const uint16_t *int_indices, int num_int, const uint16_t *fp_indices, int num_fp,
+                        int bits, int wide, int ids_settled, void *dst, void *meta, void *fp_x, void *stream);
+
 /* quik.asymmetric.find_meta (src/asymmetric/asymmetric.cpp:40-44, asymmetric.cu:263-338):
  * meta[2r] = T(fmaxf((max_r - min_r) / (2^bits - 1), 1e-6f)), meta[2r+1] = min_r. */
 int quik_asym_find_meta(const void *src, int dtype, int rows, int cols, int bits,

@@ -40,6 +40,7 @@ SIGNATURES = {
     "quik_asym_quantize_u16": (_i, [_vp, _i, _i, _i, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
     "quik_rmsnorm_quantize_u16": (_i, [_vp, _vp, _f, _i, _i, _i, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
     "quik_silu_mul_quantize_u16": (_i, [_vp, _vp, _i, _i, _i, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
+    "quik_layer_quantize": (_i, [_i, _vp, _vp, _f, _i, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp]),
     "quik_asym_find_meta": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),
     "quik_asym_quantize_old": (_i, [_vp, _i, _vp, _i, _i, _i, _vp, _vp]),
     "quik_asym_dequantize": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
@@ -92,8 +93,7 @@ def host():
             raise RuntimeError(f"quik_b200._host is missing or does not load ({e}): build it with "
                                "`python -m quik_b200.build`") from e
         mod.init(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
-            "quik_asym_quantize_u16", "quik_rmsnorm_quantize_u16", "quik_silu_mul_quantize_u16", "quik_mixed_linear_ld",
-            "quik_strerror", "quik_last_cuda_error", "quik_config_get")))
+            "quik_layer_quantize", "quik_mixed_linear_ld", "quik_strerror", "quik_last_cuda_error", "quik_config_get")))
         _host = mod
     return _host
 

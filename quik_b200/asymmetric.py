@@ -48,18 +48,18 @@ def quantize(src, int_indices, fp_indices, bits):
 def quantize_u16(src, int_indices_u16, fp_indices_u16, bits, wide):
     """Layer-internal form of :func:`quantize`: 16-bit column ids (stored in int16 tensors) and an
     optional one-code-per-byte layout for 4-bit codes (the tensor-core GEMM operand)."""
-    return host().quantize(0, src, None, 0.0, int_indices_u16, fp_indices_u16, bits, wide)
+    return host().quantize(0, src, None, 0.0, int_indices_u16, fp_indices_u16, bits, wide, False)
 
 
 def rmsnorm_quantize_u16(x, norm_weight, eps, int_indices_u16, fp_indices_u16, bits, wide):
     """quantize_u16(rmsnorm(x) * norm_weight) in one pass over ``x``: the normalised matrix is never written
     (LlamaRMSNorm arithmetic: fp32 statistics, rounded to x.dtype, times the weight in x.dtype)."""
-    return host().quantize(1, x, norm_weight, eps, int_indices_u16, fp_indices_u16, bits, wide)
+    return host().quantize(1, x, norm_weight, eps, int_indices_u16, fp_indices_u16, bits, wide, False)
 
 
 def silu_mul_quantize_u16(gate, up, int_indices_u16, fp_indices_u16, bits, wide):
     """quantize_u16(silu(gate) * up) in one pass over ``gate`` and ``up``: the activated matrix is never written."""
-    return host().quantize(2, gate, up, 0.0, int_indices_u16, fp_indices_u16, bits, wide)
+    return host().quantize(2, gate, up, 0.0, int_indices_u16, fp_indices_u16, bits, wide, False)
 
 
 def find_meta(src, bits):

@@ -178,37 +178,41 @@ int quik_asym_quantize(const void *src, int dtype, int rows, int cols, const int
                        void *stream) {
   int rc = check_quantize_args(src, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x);
   if (rc != QUIK_OK) return rc;
-  return launch_asym_quantize(src, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, 8, bits, 0, dst,
-                              meta, fp_x, static_cast<cudaStream_t>(stream));
+  return launch_asym_quantize(src, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x,
+                              static_cast<cudaStream_t>(stream));
+}
+
+int quik_layer_quantize(int producer, const void *x, const void *aux, float eps, int dtype, int rows, int cols,
+                        const uint16_t *int_indices, int num_int, const uint16_t *fp_indices, int num_fp, int bits, int wide,
+                        int ids_settled, void *dst, void *meta, void *fp_x, void *stream) {
+  if (producer < 0 || producer > 2) return QUIK_ERR_UNSUPPORTED;
+  int rc = check_quantize_args(x, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x);
+  if (rc != QUIK_OK) return rc;
+  if (rows > 0 && producer != 0 && !aux) return QUIK_ERR_NULL;
+  return launch_asym_quantize_u16(producer, x, producer == 0 ? nullptr : aux, eps, dtype, rows, cols, int_indices, num_int,
+                                  fp_indices, num_fp, bits, wide, ids_settled, dst, meta, fp_x,
+                                  static_cast<cudaStream_t>(stream));
 }
 
 int quik_asym_quantize_u16(const void *src, int dtype, int rows, int cols, const uint16_t *int_indices, int num_int,
                            const uint16_t *fp_indices, int num_fp, int bits, int wide, void *dst, void *meta,
                            void *fp_x, void *stream) {
-  int rc = check_quantize_args(src, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x);
-  if (rc != QUIK_OK) return rc;
-  return launch_asym_quantize(src, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, 2, bits, wide, dst,
-                              meta, fp_x, static_cast<cudaStream_t>(stream));
+  return quik_layer_quantize(0, src, nullptr, 0.f, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, wide, 0,
+                             dst, meta, fp_x, stream);
 }
 
 int quik_rmsnorm_quantize_u16(const void *x, const void *norm_weight, float eps, int dtype, int rows, int cols,
                               const uint16_t *int_indices, int num_int, const uint16_t *fp_indices, int num_fp, int bits,
                               int wide, void *dst, void *meta, void *fp_x, void *stream) {
-  int rc = check_quantize_args(x, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x);
-  if (rc != QUIK_OK) return rc;
-  if (rows > 0 && !norm_weight) return QUIK_ERR_NULL;
-  return launch_asym_quantize_fused(1, x, norm_weight, eps, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp,
-                                    bits, wide, dst, meta, fp_x, static_cast<cudaStream_t>(stream));
+  return quik_layer_quantize(1, x, norm_weight, eps, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, wide, 0,
+                             dst, meta, fp_x, stream);
 }
 
 int quik_silu_mul_quantize_u16(const void *gate, const void *up, int dtype, int rows, int cols,
                                const uint16_t *int_indices, int num_int, const uint16_t *fp_indices, int num_fp, int bits,
                                int wide, void *dst, void *meta, void *fp_x, void *stream) {
-  int rc = check_quantize_args(gate, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, dst, meta, fp_x);
-  if (rc != QUIK_OK) return rc;
-  if (rows > 0 && !up) return QUIK_ERR_NULL;
-  return launch_asym_quantize_fused(2, gate, up, 0.f, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits,
-                                    wide, dst, meta, fp_x, static_cast<cudaStream_t>(stream));
+  return quik_layer_quantize(2, gate, up, 0.f, dtype, rows, cols, int_indices, num_int, fp_indices, num_fp, bits, wide, 0, dst,
+                             meta, fp_x, stream);
 }
 
 int quik_asym_find_meta(const void *src, int dtype, int rows, int cols, int bits, void *meta, void *stream) {

@@ -180,13 +180,12 @@ __device__ __forceinline__ float warp_min(float v) {
 }
 
 // ---- launchers implemented in the individual .cu files ---------------------------------------
-int launch_asym_quantize(const void *src, int dtype, int rows, int cols, const void *int_idx,
-                         int num_int, const void *fp_idx, int num_fp, int idx_bytes, int bits,
-                         int wide, void *dst, void *meta, void *fp_x, cudaStream_t st);
-// quantizer with the producer of X fused in (quantize.cu): prod 1 = RMSNorm (aux = weight vector), 2 = SiLU(src) * aux
-int launch_asym_quantize_fused(int prod, const void *src, const void *aux, float eps, int dtype, int rows, int cols,
-                               const void *int_idx, int num_int, const void *fp_idx, int num_fp, int bits, int wide,
-                               void *dst, void *meta, void *fp_x, cudaStream_t st);
+int launch_asym_quantize(const void *src, int dtype, int rows, int cols, const int64_t *int_idx, int num_int,
+                         const int64_t *fp_idx, int num_fp, int bits, void *dst, void *meta, void *fp_x, cudaStream_t st);
+// the same with 16-bit ids and the producer of X fused in: prod 0 = none, 1 = RMSNorm (aux = weight vector), 2 = SiLU(src) * aux
+int launch_asym_quantize_u16(int prod, const void *src, const void *aux, float eps, int dtype, int rows, int cols,
+                             const void *int_idx, int num_int, const void *fp_idx, int num_fp, int bits, int wide,
+                             int early_ids, void *dst, void *meta, void *fp_x, cudaStream_t st);
 int launch_find_meta(const void *src, int dtype, int rows, int cols, int bits, void *meta,
                      cudaStream_t st);
 int launch_quantize_old(const void *src, int dtype, const void *meta, int rows, int cols, int bits,

@@ -19,9 +19,7 @@
 namespace {
 
 struct Abi {
-  decltype(&quik_asym_quantize_u16) quantize = nullptr;
-  decltype(&quik_rmsnorm_quantize_u16) rmsnorm_quantize = nullptr;
-  decltype(&quik_silu_mul_quantize_u16) silu_mul_quantize = nullptr;
+  decltype(&quik_layer_quantize) quantize = nullptr;
   decltype(&quik_mixed_linear_ld) linear = nullptr;
   decltype(&quik_config_get) config_get = nullptr;
   decltype(&quik_strerror) strerror_ = nullptr;
@@ -91,20 +89,12 @@ const char *check_quantize(int producer, const at::Tensor &x, const at::Tensor &
 }
 
 void launch_quantize(const char *op, int producer, const at::Tensor &x, const at::Tensor &aux, double eps, const at::Tensor &ids,
-                     const at::Tensor &fp_ids, int bits, bool wide, const Codes &c) {
+                     const at::Tensor &fp_ids, int bits, bool wide, bool settled, const Codes &c) {
   void *st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  const int dt = dtype_code(x.scalar_type()), rows = (int)x.size(0), cols = (int)x.size(1);
-  const int num_int = (int)ids.numel(), num_fp = (int)fp_ids.numel();
-  const uint16_t *i16 = static_cast<const uint16_t *>(ptr(ids)), *f16 = static_cast<const uint16_t *>(ptr(fp_ids));
-  int rc;
-  if (producer == 0)
-    rc = abi.quantize(ptr(x), dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta, c.fp_x, st);
-  else if (producer == 1)
-    rc = abi.rmsnorm_quantize(ptr(x), ptr(aux), (float)eps, dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta,
-                              c.fp_x, st);
-  else
-    rc = abi.silu_mul_quantize(ptr(x), ptr(aux), dt, rows, cols, i16, num_int, f16, num_fp, bits, wide, c.q, c.meta, c.fp_x, st);
-  check(rc, op);
+  check(abi.quantize(producer, ptr(x), producer ? ptr(aux) : nullptr, (float)eps, dtype_code(x.scalar_type()), (int)x.size(0),
+                     (int)x.size(1), static_cast<const uint16_t *>(ptr(ids)), (int)ids.numel(),
+                     static_cast<const uint16_t *>(ptr(fp_ids)), (int)fp_ids.numel(), bits, wide, settled, c.q, c.meta, c.fp_x, st),
+        op);
 }
 
 // the layer's own tensors, as the module holds them
@@ -130,30 +120,28 @@ at::Tensor launch_linear(const at::Tensor &x, const Codes &c, bool q_packed, con
 
 PyObject *py_init(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 7);
-  void *p[7];
-  for (int i = 0; i < 7; ++i) {
+  expect(n, 5);
+  void *p[5];
+  for (int i = 0; i < 5; ++i) {
     p[i] = PyLong_AsVoidPtr(a[i]);
     if (p[i] == nullptr) throw std::runtime_error("quik_b200._host.init: a library function is missing");
   }
   abi.quantize = reinterpret_cast<decltype(abi.quantize)>(p[0]);
-  abi.rmsnorm_quantize = reinterpret_cast<decltype(abi.rmsnorm_quantize)>(p[1]);
-  abi.silu_mul_quantize = reinterpret_cast<decltype(abi.silu_mul_quantize)>(p[2]);
-  abi.linear = reinterpret_cast<decltype(abi.linear)>(p[3]);
-  abi.strerror_ = reinterpret_cast<decltype(abi.strerror_)>(p[4]);
-  abi.last_cuda_error = reinterpret_cast<decltype(abi.last_cuda_error)>(p[5]);
-  abi.config_get = reinterpret_cast<decltype(abi.config_get)>(p[6]);
+  abi.linear = reinterpret_cast<decltype(abi.linear)>(p[1]);
+  abi.strerror_ = reinterpret_cast<decltype(abi.strerror_)>(p[2]);
+  abi.last_cuda_error = reinterpret_cast<decltype(abi.last_cuda_error)>(p[3]);
+  abi.config_get = reinterpret_cast<decltype(abi.config_get)>(p[4]);
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
 
-// (producer, x, aux | None, eps, int_ids, fp_ids, bits, wide) -> (codes, meta, fp_x)
+// (producer, x, aux | None, eps, int_ids, fp_ids, bits, wide, ids_settled) -> (codes, meta, fp_x)
 PyObject *py_quantize(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 8);
+  expect(n, 9);
   const int producer = (int)PyLong_AsLong(a[0]), bits = (int)PyLong_AsLong(a[6]);
   const double eps = PyFloat_AsDouble(a[3]);
-  const bool wide = PyObject_IsTrue(a[7]) == 1;
+  const bool wide = PyObject_IsTrue(a[7]) == 1, settled = PyObject_IsTrue(a[8]) == 1;
   if (PyErr_Occurred()) return nullptr;
   if (producer < 0 || producer > 2) throw std::runtime_error("quik_b200._host.quantize: producer");
   const at::Tensor x = tensor_arg(a[1]), aux = optional_arg(a[2]), ids = tensor_arg(a[4]), fp_ids = tensor_arg(a[5]);
@@ -168,7 +156,7 @@ PyObject *py_quantize(PyObject *, PyObject *const *a, Py_ssize_t n) {
                            : at::empty({rows, num_int}, x.options().dtype(at::kChar));
     meta = at::empty({2 * rows}, x.options());
     fp_x = at::empty({rows, fp_ids.numel()}, x.options());
-    launch_quantize(op, producer, x, aux, eps, ids, fp_ids, bits, wide, Codes{ptr(q), ptr(meta), ptr(fp_x)});
+    launch_quantize(op, producer, x, aux, eps, ids, fp_ids, bits, wide, settled, Codes{ptr(q), ptr(meta), ptr(fp_x)});
   }
   PyObject *r = PyTuple_New(3);
   if (!r) return nullptr;
@@ -209,7 +197,8 @@ PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids):
-// quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  w: the weights in storage
+// quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  The ids are settled (see
+// quik_layer_quantize).  w: the weights in storage
 // format; w8: 4-bit weights one code per byte; None is returned, and nothing launched, where the settings ask for them and
 // they were not given.
 PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
@@ -244,7 +233,7 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
       const at::Tensor ws = at::empty({b_q + b_meta + m * fp_ids.numel() * 2}, x.options().dtype(at::kByte));
       unsigned char *base = static_cast<unsigned char *>(ptr(ws));
       const Codes c{base, base + b_q, base + b_q + b_meta};
-      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !q_packed, c);
+      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !q_packed, true, c);
       result = launch_linear(x, c, q_packed, ptr(needs_w8 ? w8 : w), w_packed, l, out);
     }
   }

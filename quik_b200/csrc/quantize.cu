@@ -88,6 +88,24 @@ __device__ __forceinline__ void emit_codes(const uint32_t (&c)[4], uint32_t &w0,
   }
 }
 
+// Column ids.  Volatile, so that they stay behind griddepcontrol.wait where that comes first (the compiler may move an ordinary
+// load of memory that is declared constant for the kernel's lifetime ahead of it).
+__device__ __forceinline__ uint32_t ld_id(const uint16_t *p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_id(const int64_t *p) {
+  int64_t v;
+  asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(p));
+  return (uint32_t)v;
+}
+__device__ __forceinline__ uint4 ld_ids8(const void *p) {      // 16 bytes
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // ---- one CTA per row at a time ------------------------------------------------------------------------
 // 256 threads share a row: each thread gathers a few chunks of 8 values (kept in registers between the
 // max/min pass and the quantize pass), the row's max/min go through one block-wide reduction.  A CTA walks
@@ -112,7 +130,8 @@ __global__ void __launch_bounds__(NTHR, NTHR == 256 ? (NC <= 4 ? 3 : 2) : 1)
 asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int_idx,
                          const IdxT *__restrict__ fp_idx, int rows, int cols, int num_int, int num_fp,
                          uint8_t *__restrict__ dst, T *__restrict__ meta, T *__restrict__ fp_x,
-                         int vec_load, int vec_store, int vec_ids, int vec_aux, int nbuf, const T *__restrict__ aux, float eps) {
+                         int vec_load, int vec_store, int vec_ids, int vec_aux, int nbuf, const T *__restrict__ aux, float eps,
+                         int early_ids) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float s_red[2][NTHR / 32];
   const int cols_pad = (cols + 7) & ~7;
@@ -139,23 +158,23 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
   // ids of chunk c as four words of two 16-bit ids; the pad of the last chunk repeats the first id
   auto load_ids = [&](int c, uint32_t (&w)[4]) {
     if (vec_ids) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(int_idx) + c);
+      const uint4 v = ld_ids8(int_idx + 8 * (size_t)c);
       w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int i0 = c * 8 + 2 * j, i1 = i0 + 1;
-        const uint32_t a = (uint32_t)int_idx[i0 < num_int ? i0 : 0], b = (uint32_t)int_idx[i1 < num_int ? i1 : 0];
+        const uint32_t a = ld_id(int_idx + (i0 < num_int ? i0 : 0)), b = ld_id(int_idx + (i1 < num_int ? i1 : 0));
         w[j] = (a & 0xffffu) | (b << 16);
       }
     }
   };
-  // 16-bit ids belong to the layer, like its weights: they are fetched before waiting for the producer of `src` (one memory
-  // latency less per launch: 2.5 -> 2.3 us for 16 rows of 4096 columns, 3.35 -> 3.05 us for 11008); ids of the reference's
-  // operator are an argument like any other
-  constexpr bool kLayerIds = sizeof(IdxT) == 2;
+  // Ids are an argument like any other: what an earlier launch of the stream wrote there is visible after the wait only.  Where
+  // the caller vouches that no launch writes them (a layer's own 16-bit ids, uploaded once) they are fetched before it: one memory
+  // latency less per launch, 2.5 -> 2.3 us for 16 rows of 4096 columns, 3.35 -> 3.05 us for 11008.
+  const bool early = sizeof(IdxT) == 2 && early_ids;
   uint32_t ids[NC][4];
-  if (!kLayerIds) {
+  if (!early) {
     pdl_wait();
     if (vec_load && nbuf == 2 && (int)blockIdx.x < rows) prefetch_row(blockIdx.x, 0);
   }
@@ -164,7 +183,7 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
     const int c = tid + NTHR * it;
     if (c < num_chunks) load_ids(c, ids[it]);
   }
-  if (kLayerIds) {
+  if (early) {
     pdl_wait();     // the producer of `src` has completed
     if (vec_load && nbuf == 2 && (int)blockIdx.x < rows) prefetch_row(blockIdx.x, 0);
   }
@@ -352,6 +371,7 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
 struct RowProducer {
   const void *aux;     // PROD 1: norm weight [cols]; PROD 2: second matrix [rows, cols]
   float eps;
+  int early_ids;       // the 16-bit ids may be read before the launch's predecessor has completed
 };
 
 template <typename T, int BITS, bool WIDE, typename IdxT, int NC, int NTHR, int PROD>
@@ -380,7 +400,8 @@ int launch_asym_rows_nc(const void *src, int rows, int cols, const void *int_idx
   QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, kern, static_cast<const T *>(src), static_cast<const IdxT *>(int_idx),
                                    static_cast<const IdxT *>(fp_idx), rows, cols, num_int, num_fp,
                                    static_cast<uint8_t *>(dst), static_cast<T *>(meta), static_cast<T *>(fp_x),
-                                   vec_load, vec_store, vec_ids, aligned16(pr.aux), nbuf, static_cast<const T *>(pr.aux), pr.eps));
+                                   vec_load, vec_store, vec_ids, aligned16(pr.aux), nbuf, static_cast<const T *>(pr.aux), pr.eps,
+                                   pr.early_ids));
   return check_launch("asym_quantize_row_kernel");
 }
 
@@ -511,28 +532,27 @@ inline int ew_grid(size_t total, int threads) {
 
 }  // namespace
 
-int launch_asym_quantize(const void *src, int dtype, int rows, int cols, const void *int_idx,
-                         int num_int, const void *fp_idx, int num_fp, int idx_bytes, int bits,
-                         int wide, void *dst, void *meta, void *fp_x, cudaStream_t st) {
+int launch_asym_quantize(const void *src, int dtype, int rows, int cols, const int64_t *int_idx, int num_int,
+                         const int64_t *fp_idx, int num_fp, int bits, void *dst, void *meta, void *fp_x, cudaStream_t st) {
   if (rows == 0) return QUIK_OK;
-  const RowProducer none{nullptr, 0.f};
-  if (dtype == QUIK_F16) {
-    return idx_bytes == 8
-               ? dispatch_bits<__half, int64_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st)
-               : dispatch_bits<__half, uint16_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st);
-  }
-  return idx_bytes == 8
-             ? dispatch_bits<__nv_bfloat16, int64_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st)
-             : dispatch_bits<__nv_bfloat16, uint16_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st);
+  const RowProducer none{nullptr, 0.f, 0};
+  if (dtype == QUIK_F16)
+    return dispatch_bits<__half, int64_t, 0>(bits, 0, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st);
+  return dispatch_bits<__nv_bfloat16, int64_t, 0>(bits, 0, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, none, st);
 }
 
-// The quantizer with the producer of X fused in (16-bit column ids only): prod 1 = RMSNorm with weight vector `aux` and
-// `eps`, prod 2 = SiLU(src) * aux with a second matrix `aux`.
-int launch_asym_quantize_fused(int prod, const void *src, const void *aux, float eps, int dtype, int rows, int cols,
-                               const void *int_idx, int num_int, const void *fp_idx, int num_fp, int bits, int wide,
-                               void *dst, void *meta, void *fp_x, cudaStream_t st) {
+// The quantizer with 16-bit column ids and the producer of X fused in: prod 0 = none, 1 = RMSNorm with weight vector `aux` and
+// `eps`, 2 = SiLU(src) * aux with a second matrix `aux`.
+int launch_asym_quantize_u16(int prod, const void *src, const void *aux, float eps, int dtype, int rows, int cols,
+                             const void *int_idx, int num_int, const void *fp_idx, int num_fp, int bits, int wide,
+                             int early_ids, void *dst, void *meta, void *fp_x, cudaStream_t st) {
   if (rows == 0) return QUIK_OK;
-  const RowProducer pr{aux, eps};
+  const RowProducer pr{aux, eps, early_ids};
+  if (prod == 0) {
+    if (dtype == QUIK_F16)
+      return dispatch_bits<__half, uint16_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, pr, st);
+    return dispatch_bits<__nv_bfloat16, uint16_t, 0>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, pr, st);
+  }
   if (prod == 1) {
     if (dtype == QUIK_F16)
       return dispatch_bits<__half, uint16_t, 1>(bits, wide, src, rows, cols, int_idx, num_int, fp_idx, num_fp, dst, meta, fp_x, pr, st);

@@ -168,6 +168,12 @@ class MixedQLinear(torch.nn.Module):
             return (M <= _lib.SMALL_M_MAX and small_m_mode != _lib.SMALL_M_TCGEN05), True
         return (row_ok and _lib.config_get(_lib.CFG_GEMM_ENGINE) == _lib.ENGINE_TCGEN05_TS), False
 
+    def _quantize(self, producer, x, aux, eps, wide):
+        """(codes, meta, outliers) of producer(x) with this layer's columns; its ids are settled: ``_to_u16`` made them on the
+        host and copied them synchronously."""
+        i16, f16 = self._idx16()
+        return _lib.host().quantize(producer, x, aux, eps, i16, f16, self.bits, wide, True)
+
     def _fill_shared(self, quantized, wide):
         shared_input = self.shared_input
         if shared_input is None:
@@ -181,18 +187,14 @@ class MixedQLinear(torch.nn.Module):
         own quantizer; pass them any tensor of x's shape, dtype and device (it is not read)."""
         x2 = x[0] if x.dim() == 3 else x
         q_packed, _ = self._operand_layouts(x2.shape[0])
-        i16, f16 = self._idx16()
-        self._fill_shared(asymmetric.rmsnorm_quantize_u16(x2.contiguous(), norm_weight, eps, i16, f16, self.bits,
-                                                          not q_packed), not q_packed)
+        self._fill_shared(self._quantize(1, x2.contiguous(), norm_weight, eps, not q_packed), not q_packed)
 
     def quantize_silu_mul(self, gate, up):
         """Quantizes SiLU(gate) * up straight into this layer's shared input (see :meth:`quantize_rmsnorm`)."""
         g2 = gate[0] if gate.dim() == 3 else gate
         u2 = up[0] if up.dim() == 3 else up
         q_packed, _ = self._operand_layouts(g2.shape[0])
-        i16, f16 = self._idx16()
-        self._fill_shared(asymmetric.silu_mul_quantize_u16(g2.contiguous(), u2.contiguous(), i16, f16, self.bits,
-                                                           not q_packed), not q_packed)
+        self._fill_shared(self._quantize(2, g2.contiguous(), u2.contiguous(), 0.0, not q_packed), not q_packed)
 
     # ------------------------------------------------------------------ forward
     def forward(self, x):
@@ -228,9 +230,7 @@ class MixedQLinear(torch.nn.Module):
             raise RuntimeError("MixedQLinear: the shared quantized input was written in another code layout than this "
                                "member needs (the members of a group must run on the same engine)")
         if shared_input.qint_x is None:
-            i16, f16 = self._idx16()
-            shared_input.qint_x, shared_input.meta, shared_input.fp_x = asymmetric.quantize_u16(
-                x, i16, f16, self.bits, wide)
+            shared_input.qint_x, shared_input.meta, shared_input.fp_x = self._quantize(0, x, None, 0.0, wide)
             shared_input.wide = wide
         w = self.int_weight if (w_packed or self.bits == 8) else self._weight_codes_int8()
         hook = MixedQLinear.launch_hook

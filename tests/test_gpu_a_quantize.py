@@ -156,3 +156,48 @@ def test_error_paths_raise_like_the_reference():
         quik.matmul.int8Matmul(x, x)                                               # wrong dtype
     with pytest.raises(NotImplementedError):
         quik.matmul.int4SpMatmul(None, None, None)
+
+
+@pytest.mark.parametrize("producer", [0, 1, 2], ids=["plain", "rmsnorm", "silu"])
+@pytest.mark.parametrize("M,K,F", [(1, 4096, 256), (300, 4096, 256), (40, 2058, 32), (5, 28672, 0)])
+def test_column_ids_written_on_the_same_stream_are_seen(M, K, F, producer):
+    """Column ids are an argument of the 16-bit-id operators: ids that a kernel writes on the stream directly before the call
+    are the ones that are used (the kernel is launched to overlap its predecessor).  The buffers hold another valid choice of
+    columns before, so a read that came too early would show as that choice's result."""
+    import quik
+    from quik_b200 import _lib
+    A = quik.asymmetric
+    x, up = outlier_x(M, K, torch.arange(0), torch.float16).to(dev()), outlier_x(M, K, torch.arange(0), torch.float16, 1).to(dev())
+    norm = torch.linspace(0.5, 1.5, K, dtype=torch.float16, device=dev())
+
+    def call(i16, f16):
+        if producer == 0:
+            return A.quantize_u16(x, i16, f16, 4, True)
+        if producer == 1:
+            return A.rmsnorm_quantize_u16(x, norm, 1e-5, i16, f16, 4, True)
+        return A.silu_mul_quantize_u16(x, up, i16, f16, 4, True)
+    choices = [tuple(t.to(torch.int16).to(dev()) for t in make_indices(K, F, "shuffled", seed)) for seed in (0, 1)]
+    want = [call(*c) for c in choices]
+    assert not torch.equal(want[0][0], want[1][0])
+    torch.cuda.synchronize()
+    i16, f16 = choices[0][0].clone(), choices[0][1].clone()
+    got = []
+    for rep in range(12):
+        new_i, new_f = choices[(rep + 1) & 1]
+        if F:
+            torch.bitwise_or(new_f, 0, out=f16)
+        torch.bitwise_or(new_i, 0, out=i16)          # the launch that precedes the call
+        got.append(call(i16, f16))
+    torch.cuda.synchronize()
+    for rep, g in enumerate(got):
+        for a, b in zip(g, want[(rep + 1) & 1]):
+            assert torch.equal(a, b)
+    # ids stated to be settled (how a layer launches it): the same result
+    q, meta, fp_x = (torch.empty_like(t) for t in want[0])
+    aux = (None, norm, up)[producer]
+    _lib.check(_lib.load().quik_layer_quantize(
+        producer, x.data_ptr(), None if aux is None else aux.data_ptr(), 1e-5, _lib.F16, M, K, choices[0][0].data_ptr(), K - F,
+        _lib.ptr(choices[0][1]), F, 4, 1, 1, q.data_ptr(), meta.data_ptr(), _lib.ptr(fp_x), _lib.stream_of(x)), "layer_quantize")
+    for a, b in zip((q, meta, fp_x), want[0]):
+        assert torch.equal(a, b)
+    assert_device_clean()
