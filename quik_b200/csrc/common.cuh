@@ -122,7 +122,7 @@ void set_mma_issuers(int n);           // kept for callers of QUIK_CFG_MMA_ISSUE
 int get_mma_issuers();
 void set_l2_hint(int on);               // token-operand loads of the tiled GEMM carry an L2 evict-last hint
 int get_l2_hint();
-void set_stream_preload(int on);        // weight-streaming engines load their first weight tiles before waiting for the predecessor
+void set_stream_preload(int on);        // the ring streaming engine (stream_w_mma) loads its first weight tiles before waiting for the predecessor
 int get_stream_preload();
 void set_stream_ring(int mode);         // ring depth policy of the mma.sync streaming engine (QUIK_CFG_STREAM_RING)
 int get_stream_ring();

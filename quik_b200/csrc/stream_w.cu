@@ -81,7 +81,6 @@ struct StreamParams {
   int ntok;                       // tokens rounded up to a multiple of 16: the MMA's N
   int stages, stage_bytes, x_bytes;
   int a_slots, d_int, d_fp, tmem_cols;
-  int preload;                    // 1: the weight tiles of the first ring fill are loaded before waiting for the predecessor
   uint32_t idesc_int, idesc_fp;
   const void *meta, *scale_col, *w_reduced, *bias;
   void *out;
@@ -126,34 +125,27 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   const int n_int = nb - n_fp;
   const int kb_first = c0 + n_fp - p.nf;                           // first integer k-block
 
-  // one block of the sequence into its stage: the weight tile and the token tile(s) are requested separately, the stage's
-  // byte count with the weights
-  auto load_weights = [&](int i, int stage) {
-    const uint32_t fb = smem_u32(full_bar + stage), sw = smem_u32(tiles + stage * STAGE_BYTES);
+  // one block of the sequence, weight tile and token tile(s), into its stage
+  auto load_block = [&](int i, int stage) {
+    const uint32_t fb = smem_u32(full_bar + stage), sw = smem_u32(tiles + stage * STAGE_BYTES), sx = sw + SW_W_BYTES;
     if (i < n_fp) {
       mbar_expect_tx(fb, SW_W_BYTES + X_BYTES);
       tma_load_2d<1>(sw, &tm_fw, fb, (c0 + i) * 64, n0);
-    } else {
-      mbar_expect_tx(fb, STAGE_BYTES);
-      tma_load_2d<1>(sw, &tm_w, fb, (kb_first + i - n_fp) * 128, n0);
-    }
-  };
-  auto load_tokens = [&](int i, int stage) {
-    const uint32_t fb = smem_u32(full_bar + stage), sx = smem_u32(tiles + stage * STAGE_BYTES) + SW_W_BYTES;
-    if (i < n_fp) {
       tma_load_2d<1>(sx, &tm_fx, fb, (c0 + i) * 64, 0);
-    } else if (BITS == 4) {                                            // 128 packed bytes of W = 256 codes
-      tma_load_2d<1>(sx, &tm_x, fb, (kb_first + i - n_fp) * 256, 0);
-      tma_load_2d<1>(sx + X_BYTES, &tm_x, fb, (kb_first + i - n_fp) * 256 + 128, 0);
+      return;
+    }
+    const int kb = kb_first + i - n_fp;
+    mbar_expect_tx(fb, STAGE_BYTES);
+    tma_load_2d<1>(sw, &tm_w, fb, kb * 128, n0);
+    if (BITS == 4) {                                                   // 128 packed bytes of W = 256 codes
+      tma_load_2d<1>(sx, &tm_x, fb, kb * 256, 0);
+      tma_load_2d<1>(sx + X_BYTES, &tm_x, fb, kb * 256 + 128, 0);
     } else {
-      tma_load_2d<1>(sx, &tm_x, fb, (kb_first + i - n_fp) * 128, 0);
+      tma_load_2d<1>(sx, &tm_x, fb, kb * 128, 0);
     }
   };
 
   pdl_launch_dependents();
-  // The weights are constants of the layer, nothing the predecessor writes: the first ring fill of weight tiles is
-  // requested before waiting for it (it produces the token codes), so the weight stream starts while it runs.
-  const int pre = p.preload ? (nb < STAGES ? nb : STAGES) : 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(full_bar + s), 1);
@@ -167,18 +159,31 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    for (int i = 0; i < pre; ++i) load_weights(i, i);
+    prefetch_tmap(&tm_w);
     prefetch_tmap(&tm_x);
-    if (p.nf > 0) prefetch_tmap(&tm_fx);
+    if (p.nf > 0) {
+      prefetch_tmap(&tm_fw);
+      prefetch_tmap(&tm_fx);
+    }
   }
   if (warp == 1) {
     tmem_alloc<1>(smem_u32(tmem_slot), p.tmem_cols);
     tmem_relinquish<1>();
   }
+  if (warp == 0) {
+    // Ask L2 for the weight tiles of the first ring fill while the producer of the token codes may still run (more tiles
+    // measured slower: their requests delay the first loads).  The loads themselves come after the wait: an earlier launch of
+    // the stream may have written the weights.  Loading the first ring fill into shared memory here gave nothing: four
+    // layers of Llama-2-7B at 20 / 64 / 128 tokens 70.9 / 75.3 / 97.5 us, with the prefetch 71.5 / 75.8 / 97.3 us, with
+    // neither 74.3 / 78.2 / 97.7 us.
+    __syncwarp();
+    for (int i = lane; i < (nb < STAGES ? nb : STAGES); i += 32) {
+      if (i < n_fp) tma_prefetch_2d(&tm_fw, (c0 + i) * 64, n0);
+      else tma_prefetch_2d(&tm_w, (kb_first + i - n_fp) * 128, n0);
+    }
+  }
   __syncwarp();
-  pdl_wait();      // below: reads of what the predecessor wrote
-  if (threadIdx.x == 0)
-    for (int i = 0; i < pre; ++i) load_tokens(i, i);
+  pdl_wait();      // first global access below
   if (worker) {
     const int te = threadIdx.x - 64;
     if (te < p.ntok) {
@@ -209,16 +214,13 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   }
 
   if (warp == 0) {
-    // ================= TMA producer: the blocks after the first ring fill, in order =================
+    // ================= TMA producer =================
     const bool elected = elect_one();
-    int stage = pre == STAGES ? 0 : pre;
-    uint32_t phase = pre == STAGES ? 1u : 0u;
-    for (int i = pre; i < nb; ++i) {
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < nb; ++i) {
       if (!mbar_wait_warp(smem_u32(empty_bar + stage), phase ^ 1, abort_flag, p.status)) break;
-      if (elected) {
-        load_weights(i, stage);
-        load_tokens(i, stage);
-      }
+      if (elected) load_block(i, stage);
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
     __syncwarp();
@@ -479,7 +481,6 @@ int launch_stream_w(const void *q, const void *w, int bits, int M, int N, int K_
   p.d_int = plan.d_int;
   p.d_fp = plan.d_fp;
   p.tmem_cols = plan.tmem_cols;
-  p.preload = get_stream_preload() != 0;
   p.idesc_int = make_idesc(2, 1, SW_ROWS, ntok);
   p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, SW_ROWS, ntok);
   p.meta = ep.meta;
