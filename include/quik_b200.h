@@ -61,7 +61,9 @@ extern "C" {
 /* Programmatic dependent launch of the layer's kernels (quantizer, GEMM, weight streaming): 1 (default) a
  * kernel may start, set up and ask L2 to prefetch its weights while its predecessor in the stream still runs;
  * it waits for the predecessor's completion before its first global load or store, so results are those of
- * plain stream order; 0 launches in plain stream order. */
+ * plain stream order.  Two exceptions read constants before that wait: the ring streaming engine the weights (see
+ * QUIK_CFG_STREAM_PRELOAD), and quik_layer_quantize the column ids where its caller states that they are settled.
+ * 0 launches in plain stream order. */
 #define QUIK_CFG_PDL           5
 /* Accepted (1 or 2) for callers that set it and without effect: one warp issues every product of the tcgen05 engine, which
  * keeps the tensor pipe busy (512 to 545 cycles per 256 x 256 x 128 block of a CTA pair, 512 being the pipe's own time). */
@@ -70,10 +72,13 @@ extern "C" {
  * evict-last hint, so that data streaming through L2 meanwhile does not push it out; 0 (default): plain loads. */
 #define QUIK_CFG_L2_HINT       7
 /* Weight-streaming engine behind the TMA ring (few tokens).  The weights are constants of the layer, so their loads need
- * not wait for the kernel that produces the token codes.  1 (default): the weight tiles of the first ring fill are
+ * not wait for the kernel that produces the token codes.  1 (default): the weight tiles (w, fp_w) of the first ring fill are
  * loaded before that wait, the token tiles of the same stages after it (measured 56.8 against 58.1 us for the four
- * Llama-2-7B layers at 16 tokens); 0: only an L2 prefetch of the first tiles precedes the wait; 2: like 1 plus an L2
- * prefetch of the later tiles (measured slower: 60.7 us). */
+ * Llama-2-7B layers at 16 tokens).  The weights must therefore be settled: complete on the device when the call is made
+ * (a captured launch: when its graph is launched), or followed on the stream by an ordinary kernel or copy, one without
+ * programmatic dependence, before this library's launches.  0: only an L2 prefetch of the first tiles precedes the wait,
+ * the weights may be written by any earlier work of the stream; 2: like 1 plus an L2 prefetch of the later tiles
+ * (measured slower: 60.7 us). */
 #define QUIK_CFG_STREAM_PRELOAD 8
 /* Ring depth of the same engine: a CTA streams at (bytes in flight) / (loaded DRAM latency), and a grid of at most one
  * CTA per SM would leave half of every SM's shared memory unused with the 5-stage ring that two CTAs per SM share.
@@ -276,6 +281,7 @@ int quik_fused_dequantize(const void *A, const void *B, int bits,
  *                                    packed weights are widened on chip on their way to the tensor cores;
  *   q packed,       w packed         weight streaming on mma.sync, direct loads or TMA ring by QUIK_CFG_SMALL_M
  *                                    (M <= QUIK_SMALL_M_MAX, K_int % 32 == 0).
+ * For M <= QUIK_SMALL_M_MAX the ring engine expects settled weights (QUIK_CFG_STREAM_PRELOAD).
  * The tensor-core GEMMs round the outlier product + bias to the storage type before the dequantize step, as the reference's
  * F.linear output is rounded (experiments/qlinear.py:124).  Finished tiles are stored while others are still being computed:
  * `out` must not alias any input.

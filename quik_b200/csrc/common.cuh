@@ -74,8 +74,10 @@ int ensure_smem(PerDeviceSmem &st, Kern kern, size_t smem, int threads = 0, int 
 // while its predecessor in the stream is still running: it sets up (barriers, TMEM, descriptors), asks L2 to
 // prefetch its weights (a prefetch returns nothing to the SM and L2 is coherent, so this is safe whoever
 // writes that memory) and only then waits for the predecessor to complete (pdl_wait) before its first global
-// load or store.  Every kernel launched through LaunchCfg must call pdl_wait() before that point.
-// QUIK_CFG_PDL = 0 restores plain stream order.
+// load or store.  Every kernel launched through LaunchCfg must call pdl_wait() before that point; only what the caller
+// has declared settled may be loaded earlier (the ring streaming engine's weights, a layer's column ids): because every
+// kernel signals its dependents before its own wait, what any earlier launch of the stream wrote is certain to be visible
+// after the wait only.  QUIK_CFG_PDL = 0 restores plain stream order.
 bool pdl_enabled();                                      // abi.cu
 
 struct LaunchCfg {

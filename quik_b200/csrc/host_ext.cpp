@@ -12,6 +12,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstring>
 #include <string>
 
 #include "../../include/quik_b200.h"
@@ -104,6 +105,41 @@ struct Layer {
   int bits;
 };
 
+// True at first and after the integer or outlier weights (fp_w may be undefined) were replaced or written in place since the last
+// call with this record, by address and version; always for inference tensors, which count no versions.
+constexpr size_t kSeenBytes = 4 * sizeof(int64_t);
+struct Seen {
+  int64_t v[4] = {0, 0, 0, 0};
+  bool known = true;
+  Seen(const at::Tensor &w, const at::Tensor &fp_w) {
+    const at::Tensor *const t[2] = {&w, &fp_w};
+    for (int i = 0; i < 2; ++i) {
+      if (!t[i]->defined()) continue;
+      known = known && !t[i]->is_inference();
+      v[2 * i] = (int64_t)(intptr_t)ptr(*t[i]);
+      v[2 * i + 1] = known ? (int64_t)t[i]->_version() : 0;
+    }
+  }
+  bool changed(const char *record) const { return !known || std::memcmp(record, v, kSeenBytes) != 0; }
+};
+char *seen_arg(PyObject *o) {
+  if (!PyByteArray_Check(o) || PyByteArray_GET_SIZE(o) != (Py_ssize_t)kSeenBytes) throw std::runtime_error("expected a record of 32 bytes");
+  return PyByteArray_AS_STRING(o);
+}
+// Before a launch for few tokens.  The ring streaming engine loads its first weight tiles before it waits for the stream's earlier
+// launches (QUIK_CFG_STREAM_PRELOAD), which may just have written them: after a change of the weights an ordinary launch goes
+// first.  It starts when all earlier ones have completed, and the layer's launches start when it has.  Called with the GIL held:
+// no other thread takes the weights for settled before that launch is in the stream.
+void settle_weights(const at::Tensor &x, const at::Tensor &w, const at::Tensor &fp_w, char *record) {
+  const int64_t rows = x.dim() >= 2 ? x.size(-2) : 0;
+  if (rows > QUIK_SMALL_M_MAX || !w.is_cuda()) return;
+  const Seen now(w, fp_w);
+  if (!now.changed(record)) return;
+  const c10::cuda::OptionalCUDAGuard guard(w.device());
+  at::zeros({1}, w.options());
+  std::memcpy(record, now.v, kSeenBytes);
+}
+
 // [1, M, N] (or `out_buffer` with that leading dimension added, where the caller gave one)
 at::Tensor launch_linear(const at::Tensor &x, const Codes &c, bool q_packed, const void *w, bool w_packed, const Layer &l,
                          const at::Tensor &out_buffer) {
@@ -176,16 +212,17 @@ bool layer_args(PyObject *const *a, Layer *l) {
   return true;
 }
 
-// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w_packed, codes, q_packed, meta, fp_x):
+// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w_packed, codes, q_packed, meta, fp_x, seen):
 // the fused launch on a quantized input; x gives the number of tokens, the dtype and the device
 PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 16);
+  expect(n, 17);
   const at::Tensor x = tensor_arg(a[0]), out = optional_arg(a[1]), w = tensor_arg(a[10]), q = tensor_arg(a[12]),
                    meta = tensor_arg(a[14]), fp_x = tensor_arg(a[15]);
   const bool w_packed = PyObject_IsTrue(a[11]) == 1, q_packed = PyObject_IsTrue(a[13]) == 1;
   Layer l;
   if (!layer_args(a + 2, &l)) return nullptr;
+  settle_weights(x, w, l.fp_w, seen_arg(a[16]));
   at::Tensor result;
   {
     py::gil_scoped_release nogil;
@@ -196,18 +233,19 @@ PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids):
+// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids, seen):
 // quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  The ids are settled (see
 // quik_layer_quantize).  w: the weights in storage
 // format; w8: 4-bit weights one code per byte; None is returned, and nothing launched, where the settings ask for them and
 // they were not given.
 PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 14);
+  expect(n, 15);
   const at::Tensor given = tensor_arg(a[0]), out = optional_arg(a[1]), w = tensor_arg(a[10]), w8 = optional_arg(a[11]),
                    ids = tensor_arg(a[12]), fp_ids = tensor_arg(a[13]);
   Layer l;
   if (!layer_args(a + 2, &l)) return nullptr;
+  settle_weights(given, w, l.fp_w, seen_arg(a[14]));
   at::Tensor result;
   {
     py::gil_scoped_release nogil;
@@ -242,11 +280,25 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (seen, w, fp_w | None) -> whether the weights differ from the record, which holds them afterwards
+PyObject *py_weights_changed(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 3);
+  char *record = seen_arg(a[0]);
+  const Seen now(tensor_arg(a[1]), optional_arg(a[2]));
+  const bool changed = now.changed(record);
+  std::memcpy(record, now.v, kSeenBytes);
+  return PyBool_FromLong(changed);
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
     {"init", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_init)), METH_FASTCALL, "addresses of the C ABI"},
     {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, "activation quantizer"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL, "fused launch"},
     {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer)), METH_FASTCALL, "quantizer and fused launch"},
+    {"weights_changed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_weights_changed)), METH_FASTCALL,
+     "weights against a record"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of the layer", -1, methods};
 

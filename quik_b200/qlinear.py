@@ -73,6 +73,8 @@ class MixedQLinear(torch.nn.Module):
     # optional caller-owned output buffer [M, out_features] (e.g. symmetric memory of a tensor-parallel
     # group); used by the fused path when its shape, dtype and device match
     out_buffer = None
+    # weights of the last call for few tokens (see _host.weights_changed); every layer has its own
+    _seen = bytearray(32)
 
     def __init__(self, in_features, out_features, shared_input=None,
                  fp_features_num=0, symm=False, bits=4, dtype=torch.float16):
@@ -101,6 +103,7 @@ class MixedQLinear(torch.nn.Module):
         if not self.symmetric:
             self.register_buffer('reduced_w', torch.zeros((1, self.out_features), dtype=dtype))
         self._cache = {}
+        self._seen = bytearray(32)
 
     @classmethod
     def concat(cls, modules):
@@ -237,7 +240,7 @@ class MixedQLinear(torch.nn.Module):
         if hook is not None:
             hook(self, True)
         out = _lib.host().linear(x, self._out_buffer_for(x, M), *self._constants(), w, w_packed, shared_input.qint_x, q_packed,
-                                 shared_input.meta, shared_input.fp_x)
+                                 shared_input.meta, shared_input.fp_x, self._seen)
         if hook is not None:
             hook(self, False)
         shared_input.finish()
@@ -268,9 +271,9 @@ class MixedQLinear(torch.nn.Module):
         M = x.shape[-2] if x.dim() > 1 else 0
         wide = self._weight_codes_int8() if self.bits == 4 and M > _lib.STREAM_M_MAX else None
         out = self._out_buffer_for(x, M)
-        res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids)
+        res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids, self._seen)
         if res is None:          # the settings send this token count to the engine that takes one code per byte
-            res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids)
+            res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids, self._seen)
         return res
 
     def _forward_unfused(self, x, shared_input):

@@ -476,3 +476,49 @@ def test_weights_written_on_the_same_stream_are_seen(M, K, N, F, bits):
     for rep, out in enumerate(got):
         assert torch.equal(out, want[rep & 1]), rep
     assert_device_clean()
+
+
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("M,bits", [(16, 4), (3, 8), (128, 4)])
+def test_few_tokens_after_an_in_place_update_of_the_weights(M, bits, shared):
+    """The module directly after in-place updates of its weights by kernels of the same stream, at sizes where few tokens go
+    to the ring engine, which reads weights ahead of the stream's earlier launches (16 MiB packed, 32 MiB int8): the results
+    are those of plain stream order; so are a call without an update in between and one captured together with its update."""
+    case = make_layer("t", M, 4096 + 64, 8192, bits, F=64, seed=M, device=dev(), clip=False)
+    layer, x = case.module, case.x
+    w0, f0 = layer.int_weight.clone(), layer.fp_weight.clone()
+    layer.shared_input = SharedQuantizedInput(1) if shared else None
+
+    def update(flip):
+        torch.mul(f0, -1 if flip else 1, out=layer.fp_weight)
+        torch.bitwise_xor(w0, 0x11 if flip else 0, out=layer.int_weight)
+
+    want = []
+    try:
+        _lib.set_pdl(False)
+        for flip in (0, 1):
+            update(flip)
+            want.append(layer(x).clone())
+    finally:
+        _lib.set_pdl(True)
+    torch.cuda.synchronize()
+    got = []
+    for rep in range(8):
+        update(rep & 1)
+        got.append((layer(x), layer(x)))
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            update(0)
+            a = layer(x)
+            update(1)
+            b = layer(x)
+        for _ in range(3):
+            g.replay()
+    torch.cuda.synchronize()
+    for rep, pair in enumerate(got):
+        assert all(torch.equal(out, want[rep & 1]) for out in pair), rep
+    assert torch.equal(a, want[0]) and torch.equal(b, want[1])
+    assert_device_clean()

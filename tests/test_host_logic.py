@@ -185,3 +185,30 @@ def test_reciprocal_product_rounds_like_the_bfloat16_quotient():
         d = sig * 2.0 ** e
         quotient = (d.double()[:, None] / sig.double()[None, :]).float().bfloat16()
         assert torch.equal(quotient, (d[:, None] * rcp[None, :]).bfloat16())
+
+
+def test_changed_weights_are_noticed():
+    """A layer for few tokens has to know when its weights were written since its last call: at first, in place, replaced,
+    through either weight tensor; not otherwise."""
+    from quik_b200 import _lib
+    layer = qlinear.MixedQLinear(96, 8, fp_features_num=32, bits=4)
+    assert layer._seen is not qlinear.MixedQLinear(96, 8)._seen
+
+    def changed():
+        return _lib.host().weights_changed(layer._seen, layer.int_weight, layer.fp_weight)
+    assert changed() and not changed()
+    layer.int_weight.zero_()
+    assert changed() and not changed()
+    layer.fp_weight.mul_(2)
+    assert changed() and not changed()
+    layer.int_weight = layer.int_weight.clone()
+    assert changed() and not changed()
+    layer.load_state_dict(layer.state_dict())
+    assert changed() and not changed()
+    with torch.inference_mode():
+        layer.int_weight = layer.int_weight.clone()           # counts no versions: never taken for settled
+    assert changed() and changed()
+    seen = bytearray(32)
+    assert _lib.host().weights_changed(seen, layer.fp_weight, None) and not _lib.host().weights_changed(seen, layer.fp_weight, None)
+    with pytest.raises(RuntimeError):
+        _lib.host().weights_changed(bytearray(8), layer.fp_weight, None)
