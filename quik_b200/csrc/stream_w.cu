@@ -343,7 +343,7 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   auto load_int = [&](int tok0, uint32_t (&acc)[8]) {
     if (n_int > 0) {
       tmem_ld8(tmem_base + lane_base + p.d_int + tok0, acc);
-      tmem_ld_wait();
+      tmem_ld_wait(acc);
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0;
@@ -374,7 +374,7 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         for (int j = 0; j < 8; ++j) sum_i[(tok0 + j) * SW_ROWS + row] = (int)acc[j];
         if (n_fp > 0) {
           tmem_ld8(tmem_base + lane_base + p.d_fp + tok0, acc);
-          tmem_ld_wait();
+          tmem_ld_wait(acc);
 #pragma unroll
           for (int j = 0; j < 8; ++j) sum_f[(tok0 + j) * SW_ROWS + row] = __uint_as_float(acc[j]);
         }
@@ -403,12 +403,13 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       const int tok0 = h * (p.ntok / 2) + 8 * c;
       if (tok0 >= p.M) break;                        // warp-uniform
       uint32_t acc_i[8], acc_f[8];
-      load_int(tok0, acc_i);                         // tcgen05.ld is warp-collective: all lanes, also rows beyond N
+      __syncwarp();                                  // tcgen05.ld is warp-collective: all lanes, also rows beyond N, converged
+      load_int(tok0, acc_i);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc_f[j] = 0;
       if (n_fp > 0) {
         tmem_ld8(tmem_base + lane_base + p.d_fp + tok0, acc_f);
-        tmem_ld_wait();
+        tmem_ld_wait(acc_f);
       }
       if (n < p.N) {
 #pragma unroll
