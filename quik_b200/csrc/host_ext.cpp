@@ -98,6 +98,32 @@ void launch_quantize(const char *op, int producer, const at::Tensor &x, const at
         op);
 }
 
+// Operand layouts of a layer of `bits` with k_int integer columns for m tokens, which is to say the engine that the fused launch
+// will use (the C side picks it from them, include/quik_b200.h):
+//   up to STREAM_M_MAX tokens: weight streaming, the weights stay in their storage format; the tcgen05 streaming engine takes
+//     the token codes one per byte, the mma.sync engines (up to SMALL_M_MAX tokens, the default for 4-bit layers) packed
+//     like the weights;
+//   more tokens: tensor-core GEMM on weight codes one per byte; the quantizer writes the token codes one per byte too,
+//     except when the engine with the token operand in tensor memory is selected: it takes 4-bit token codes packed (the
+//     reference layout) and widens them on chip.
+// (a packed 4-bit row must be a multiple of 16 bytes for these engines; otherwise both operands one per byte)
+struct Layouts {
+  bool q_packed = false, w_packed = false;
+};
+Layouts operand_layouts(int bits, int64_t k_int, int64_t m) {
+  Layouts r;
+  if (bits == 8) return r;
+  const bool row_ok = k_int % 32 == 0;
+  const int small_m = abi.config_get(QUIK_CFG_SMALL_M);
+  if (m <= QUIK_STREAM_M_MAX && small_m != 0 && row_ok) {
+    r.w_packed = true;
+    r.q_packed = m <= QUIK_SMALL_M_MAX && small_m != 3;
+  } else {
+    r.q_packed = row_ok && abi.config_get(QUIK_CFG_GEMM_ENGINE) == QUIK_ENGINE_TCGEN05_TS;
+  }
+  return r;
+}
+
 // the layer's own tensors, as the module holds them
 struct Layer {
   at::Tensor scales, reduced, fp_w, bias;
@@ -252,31 +278,32 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
     const at::Tensor x = given.dim() == 3 ? given.select(0, 0) : given;      // the first matrix of a batch, as ever
     const char *op = check_quantize(0, x, at::Tensor(), ids, fp_ids, l.bits);
     const int64_t m = x.size(0);
-    // operand layouts by engine, as in MixedQLinear._operand_layouts
-    bool q_packed = false, w_packed = false;
-    if (l.bits == 4) {
-      const bool row_ok = l.k_int % 32 == 0;
-      const int small_m = abi.config_get(QUIK_CFG_SMALL_M);
-      if (m <= QUIK_STREAM_M_MAX && small_m != 0 && row_ok) {
-        w_packed = true;
-        q_packed = m <= QUIK_SMALL_M_MAX && small_m != 3;
-      } else {
-        q_packed = row_ok && abi.config_get(QUIK_CFG_GEMM_ENGINE) == QUIK_ENGINE_TCGEN05_TS;
-      }
-    }
-    const bool needs_w8 = l.bits == 4 && !w_packed;
+    const Layouts lay = operand_layouts(l.bits, l.k_int, m);
+    const bool needs_w8 = l.bits == 4 && !lay.w_packed;
     if (!needs_w8 || w8.defined()) {
       const c10::cuda::OptionalCUDAGuard guard(x.device());
       const int64_t b_q = align256(m * ids.numel()), b_meta = align256(m * 4);
       const at::Tensor ws = at::empty({b_q + b_meta + m * fp_ids.numel() * 2}, x.options().dtype(at::kByte));
       unsigned char *base = static_cast<unsigned char *>(ptr(ws));
       const Codes c{base, base + b_q, base + b_q + b_meta};
-      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !q_packed, true, c);
-      result = launch_linear(x, c, q_packed, ptr(needs_w8 ? w8 : w), w_packed, l, out);
+      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !lay.q_packed, true, c);
+      result = launch_linear(x, c, lay.q_packed, ptr(needs_w8 ? w8 : w), lay.w_packed, l, out);
     }
   }
   if (!result.defined()) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// (bits, k_int, m) -> (token codes packed, weight codes packed)
+PyObject *py_operand_layouts(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 3);
+  const int bits = (int)PyLong_AsLong(a[0]);
+  const int64_t k_int = PyLong_AsLongLong(a[1]), m = PyLong_AsLongLong(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  const Layouts r = operand_layouts(bits, k_int, m);
+  return PyTuple_Pack(2, r.q_packed ? Py_True : Py_False, r.w_packed ? Py_True : Py_False);
   END_HANDLE_TH_ERRORS
 }
 
@@ -297,6 +324,8 @@ PyMethodDef methods[] = {
     {"quantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize)), METH_FASTCALL, "activation quantizer"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL, "fused launch"},
     {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer)), METH_FASTCALL, "quantizer and fused launch"},
+    {"operand_layouts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_operand_layouts)), METH_FASTCALL,
+     "operand layouts for a token count"},
     {"weights_changed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_weights_changed)), METH_FASTCALL,
      "weights against a record"},
     {nullptr, nullptr, 0, nullptr}};

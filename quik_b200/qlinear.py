@@ -162,14 +162,7 @@ class MixedQLinear(torch.nn.Module):
 
     def _operand_layouts(self, M):
         """(token codes packed?, weight codes packed?) for M tokens: which engine the fused launch will use."""
-        small_m_mode = _lib.config_get(_lib.CFG_SMALL_M)
-        row_ok = self.bits == 8 or self.int_features_num % 32 == 0
-        stream = M <= _lib.STREAM_M_MAX and small_m_mode != _lib.SMALL_M_OFF and row_ok
-        if self.bits == 8:
-            return False, False
-        if stream:
-            return (M <= _lib.SMALL_M_MAX and small_m_mode != _lib.SMALL_M_TCGEN05), True
-        return (row_ok and _lib.config_get(_lib.CFG_GEMM_ENGINE) == _lib.ENGINE_TCGEN05_TS), False
+        return _lib.host().operand_layouts(self.bits, self.int_features_num, M)
 
     def _quantize(self, producer, x, aux, eps, wide):
         """(codes, meta, outliers) of producer(x) with this layer's columns; its ids are settled: ``_to_u16`` made them on the
@@ -219,14 +212,6 @@ class MixedQLinear(torch.nn.Module):
             return self._forward_unfused(x, shared_input)
 
         M = x.shape[0]
-        # Operand layouts by engine (the C side picks the engine from them, include/quik_b200.h):
-        #   up to STREAM_M_MAX tokens: weight streaming, the weights stay in their storage format; the tcgen05
-        #     streaming engine takes the token codes one per byte, the mma.sync engines (up to SMALL_M_MAX tokens, the
-        #     default for 4-bit layers) packed like the weights;
-        #   more tokens: tensor-core GEMM on weight codes one per byte; the quantizer writes the token codes one per
-        #     byte too, except when the engine with the token operand in tensor memory is selected: it takes 4-bit
-        #     token codes packed (the reference layout) and widens them on chip.
-        # (a packed 4-bit row must be a multiple of 16 bytes for these engines; otherwise both operands one per byte)
         q_packed, w_packed = self._operand_layouts(M)
         wide = not q_packed
         if shared_input.qint_x is not None and self.bits == 4 and shared_input.wide != wide:
@@ -269,10 +254,10 @@ class MixedQLinear(torch.nn.Module):
         w = self.int_weight
         ids, fp_ids = self._idx16()
         M = x.shape[-2] if x.dim() > 1 else 0
-        wide = self._weight_codes_int8() if self.bits == 4 and M > _lib.STREAM_M_MAX else None
+        wide = self._weight_codes_int8() if self.bits == 4 and not self._operand_layouts(M)[1] else None
         out = self._out_buffer_for(x, M)
         res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids, self._seen)
-        if res is None:          # the settings send this token count to the engine that takes one code per byte
+        if res is None:          # a setting that another thread has changed since asks for weight codes one per byte
             res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids, self._seen)
         return res
 

@@ -212,3 +212,25 @@ def test_changed_weights_are_noticed():
     assert _lib.host().weights_changed(seen, layer.fp_weight, None) and not _lib.host().weights_changed(seen, layer.fp_weight, None)
     with pytest.raises(RuntimeError):
         _lib.host().weights_changed(bytearray(8), layer.fp_weight, None)
+
+
+def test_operand_layouts_by_engine():
+    """One rule picks the operand layouts, for a layer's single native call and for members of a shared input alike."""
+    from quik_b200 import _lib
+    lay = lambda bits, k, m: qlinear.MixedQLinear(k, 8, bits=bits)._operand_layouts(m)
+    try:
+        for m in (0, 1, 16, 17, 128, 129, 4096):
+            assert lay(8, 64, m) == (False, False)
+            assert lay(4, 64, m) == (m <= 16, m <= 128)
+            assert lay(4, 48, m) == (False, False)            # a packed row is no multiple of 16 bytes
+        _lib.set_small_m(_lib.SMALL_M_TCGEN05)
+        assert lay(4, 64, 16) == (False, True)
+        _lib.set_small_m(_lib.SMALL_M_OFF)
+        assert lay(4, 64, 16) == (False, False)
+        _lib.set_engine(_lib.ENGINE_TCGEN05_TS)
+        assert lay(4, 64, 16) == (True, False) and lay(4, 48, 16) == (False, False)
+        _lib.set_small_m(True)
+        assert lay(4, 64, 16) == (True, True) and lay(4, 64, 129) == (True, False) and lay(8, 64, 129) == (False, False)
+    finally:
+        _lib.set_small_m(True)
+        _lib.set_engine(_lib.ENGINE_AUTO)
