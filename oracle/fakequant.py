@@ -109,14 +109,14 @@ class FakeQuantLinear:
             self.fp_idx = order[-fp_features:]
             self.q_idx = order[:-fp_features]
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def linear_input(self, x: torch.Tensor) -> torch.Tensor:
+        """What the linear multiplies: x with its integer columns fake-quantized."""
         dt = x.dtype
         if self.bits == 16:
-            return torch.nn.functional.linear(x, self.weight).to(dt)
+            return x
         if self.fp_features_num == 0:
             scale, zero, maxq = act_find_params(x, self.bits)
-            xq = asymmetric_fake_quantize(x, scale, zero, maxq).to(dt)
-            return torch.nn.functional.linear(xq, self.weight).to(dt)
+            return asymmetric_fake_quantize(x, scale, zero, maxq).to(dt)
         mixed = torch.zeros_like(x)
         qf = x[..., self.q_idx]
         ff = x[..., self.fp_idx]
@@ -124,6 +124,9 @@ class FakeQuantLinear:
         qf = asymmetric_fake_quantize(qf, scale, zero, maxq).to(dt)
         mixed[..., self.q_idx] = qf
         mixed[..., self.fp_idx] = ff
-        return torch.nn.functional.linear(mixed, self.weight).to(dt)
+        return mixed
+
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
+        return torch.nn.functional.linear(self.linear_input(x), self.weight).to(x.dtype)
 
     __call__ = forward
