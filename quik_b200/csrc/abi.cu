@@ -18,6 +18,7 @@ std::atomic<int> g_small_m{1};
 std::atomic<int> g_stream_preload{1};
 std::atomic<int> g_stream_ring{2};
 std::atomic<int> g_pdl{1};
+std::atomic<int> g_mma_issuers{1};       // nothing reads it but quik_config_get
 }  // namespace
 
 void set_cuda_error(cudaError_t e, const char *where) {
@@ -106,7 +107,7 @@ int quik_config_set(int key, int value) {
   }
   if (key == QUIK_CFG_MMA_ISSUERS) {
     if (value < 1 || value > 2) return QUIK_ERR_UNSUPPORTED;
-    set_mma_issuers(value);
+    g_mma_issuers = value;
     return QUIK_OK;
   }
   if (key == QUIK_CFG_L2_HINT) {
@@ -130,7 +131,7 @@ int quik_config_get(int key) {
   if (key == QUIK_CFG_SMALL_M) return g_small_m;
   if (key == QUIK_CFG_PDL) return g_pdl;
   if (key == QUIK_CFG_CTA_PAIR) return get_cta_pair();
-  if (key == QUIK_CFG_MMA_ISSUERS) return get_mma_issuers();
+  if (key == QUIK_CFG_MMA_ISSUERS) return g_mma_issuers;
   if (key == QUIK_CFG_L2_HINT) return get_l2_hint();
   if (key == QUIK_CFG_STREAM_PRELOAD) return g_stream_preload;
   if (key == QUIK_CFG_STREAM_RING) return g_stream_ring;

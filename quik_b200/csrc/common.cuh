@@ -120,8 +120,6 @@ void choose_tile(int M, int N, int kblocks, int *ctas_out, int *bn_out);
 void set_tile_n(int n);               // 0 = by shape, else a multiple of 16 in [32, 256]
 int get_tile_n();
 void set_cta_pair(int mode);           // 0 = by shape, 1 = never, 2 = always
-void set_mma_issuers(int n);           // kept for callers of QUIK_CFG_MMA_ISSUERS; no effect
-int get_mma_issuers();
 void set_l2_hint(int on);               // token-operand loads of the tiled GEMM carry an L2 evict-last hint
 int get_l2_hint();
 void set_stream_preload(int on);        // the ring streaming engine (stream_w_mma) loads its first weight tiles before waiting for the predecessor

@@ -46,7 +46,6 @@ constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;      // TMA warp + MMA warp + e
 std::atomic<int> g_tile_n{0};                                 // 0 = choose by shape, else a multiple of 16 in [32, 256]
 std::atomic<int> g_cta_pair{0};                               // 0 = by shape, 1 = never, 2 = always
 std::atomic<int> g_l2_hint{0};                                // 1 = token-operand loads carry an L2 evict-last hint
-std::atomic<int> g_issuers{1};                                // kept for callers of QUIK_CFG_MMA_ISSUERS; no effect
 std::atomic<unsigned long long *> g_dbg{nullptr};             // diagnostic counters (device memory), off by default
 
 // Shared-memory plan after the 1024-byte aligned ring of stages: 256 bytes of barriers etc. and the
@@ -439,8 +438,6 @@ void set_debug_counters(void *buf) { g_dbg.store(static_cast<unsigned long long 
 unsigned long long *get_debug_counters() { return g_dbg.load(); }
 void set_l2_hint(int on) { g_l2_hint.store(on ? 1 : 0); }
 int get_l2_hint() { return g_l2_hint.load(); }
-void set_mma_issuers(int n) { g_issuers.store(n); }
-int get_mma_issuers() { return g_issuers.load(); }
 void set_cta_pair(int mode) { g_cta_pair.store(mode); }
 int get_cta_pair() { return g_cta_pair.load(); }
 
