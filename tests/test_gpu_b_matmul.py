@@ -82,7 +82,8 @@ def test_int8_matmul_writes_only_its_output(engine, M, N, K):
 @pytest.mark.parametrize("tile,pair", [(0, 0), (256, 2), (256, 1), (240, 2), (128, 1)])
 @pytest.mark.parametrize("M,N,K", [(2048, 1024, 4096), (300, 520, 10752), (257, 264, 2048), (129, 4100, 28672)])
 def test_long_sums_are_exact_per_tile_and_pair(M, N, K, tile, pair):
-    """Long sums (K of 2048 to 28672) through each tile shape: the int32 result is the exact product, run after run.  Extreme codes (-128 / 127 mixed in) make every partial sum matter."""
+    """Long sums (K of 2048 to 28672) through each tile shape: the int32 result is the exact product, run after run.  Extreme
+    codes (-128 / 127 mixed in) make every partial sum matter."""
     import quik
     g = torch.Generator().manual_seed(M + N + K + tile)
     a = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8)

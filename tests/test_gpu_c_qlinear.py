@@ -392,9 +392,12 @@ def test_single_native_call_equals_quantizer_and_layer_calls(M, K, N, F, bits, d
     assert layer(x).data_ptr() == buf.data_ptr() and torch.equal(buf[:, :N], one[0]) and (buf[:, N:] == -1).all()
     layer.out_buffer = None
     assert layer(x[:0]).shape == (1, 0, N)
-    for bad in (x[:, :-2].contiguous(), x.float(), x.t()[: K // 2].t()):  # columns, dtype, not contiguous
-        with pytest.raises(RuntimeError):
+    for bad, why in ((x[:, :-2].contiguous(), "column counts"), (x.float(), "float16 or bfloat16")):
+        with pytest.raises(RuntimeError, match=why):
             layer(bad)
+    if M > 1:                                                             # the right shape at a wider pitch
+        with pytest.raises(RuntimeError, match="to be contiguous"):
+            layer(torch.nn.functional.pad(x, (0, 8))[:, :K])
     assert torch.equal(layer(x), one)
     assert_device_clean()
 
@@ -521,4 +524,23 @@ def test_few_tokens_after_an_in_place_update_of_the_weights(M, bits, shared):
     for rep, pair in enumerate(got):
         assert all(torch.equal(out, want[rep & 1]) for out in pair), rep
     assert torch.equal(a, want[0]) and torch.equal(b, want[1])
+    assert_device_clean()
+
+
+@pytest.mark.parametrize("N,bits", [(8192, 4), (1000, 4), (8192, 8)])
+def test_ring_engine_settings_give_the_same_bits(N, bits):
+    """The ring engine with its weights loaded before or after the wait, or also asked of L2, and with either ring depth."""
+    case = make_layer("t", 16, 4096 + 64, N, bits, F=64, seed=N, device=dev(), clip=False)
+    try:
+        _lib.set_small_m(_lib.SMALL_M_TMA_MMA)
+        want = case.module(case.x)
+        for key, values in ((_lib.CFG_STREAM_PRELOAD, (0, 2, 1)), (_lib.CFG_STREAM_RING, (0, 1, 2))):
+            for v in values:
+                _lib.check(_lib.load().quik_config_set(key, v), "quik_config_set")
+                for _ in range(3):
+                    assert torch.equal(case.module(case.x), want)
+    finally:
+        _lib.set_small_m(True)
+        _lib.check(_lib.load().quik_config_set(_lib.CFG_STREAM_PRELOAD, 1), "quik_config_set")
+        _lib.check(_lib.load().quik_config_set(_lib.CFG_STREAM_RING, 2), "quik_config_set")
     assert_device_clean()

@@ -236,6 +236,29 @@ def test_silu_mul_quantize_matches_activation_then_quantize(dtype, M, K, F, bits
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K,F,bits,wide", [(333, 2058, 32, 4, True), (40, 2058, 32, 8, True), (40, 14, 4, 4, False)])
+def test_silu_mul_quantize_of_ragged_rows(dtype, M, K, F, bits, wide):
+    """Rows whose length is no multiple of 8, and matrices off a 16-byte boundary, take element-wise paths; the producer works
+    column by column, so the result is that of the same columns inside longer, aligned rows (the extra columns being outliers)."""
+    g = torch.Generator().manual_seed(M + K)
+    perm = torch.randperm(K, generator=g)
+    pad = -K % 8
+    ids, fp_ids = perm[F:].sort()[0], perm[:F].sort()[0]
+    wide_fp = torch.cat([fp_ids, torch.arange(K, K + pad)])
+    i16, f16, w16 = (t.to(torch.int16).to(dev()) for t in (ids, fp_ids, wide_fp))
+    gate, up = ((2.0 * torch.randn(M, K + pad, generator=g)).to(dtype).to(dev()) for _ in range(2))
+
+    def shifted(t):                      # the same values, one element off a 16-byte boundary
+        flat = torch.empty(t.numel() + 1, dtype=dtype, device=dev())[1:].view(t.shape)
+        return flat.copy_(t)
+    want = asymmetric.silu_mul_quantize_u16(gate, up, i16, w16, bits, wide)
+    for args in ((shifted(gate), up, i16, w16), (gate, shifted(up), i16, w16), (gate[:, :K].contiguous(), up[:, :K].contiguous(), i16, f16)):
+        q, meta, fp_x = asymmetric.silu_mul_quantize_u16(*args, bits, wide)
+        assert torch.equal(q, want[0]) and torch.equal(meta, want[1]) and torch.equal(fp_x, want[2][:, :fp_x.shape[1]])
+    assert_device_clean()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,head_dim,seq", [(8, 8, 64, 33), (32, 8, 128, 257), (4, 2, 16, 5)])
 def test_rotary_inplace_is_bit_identical_to_the_torch_expression(dtype, heads, kv_heads, head_dim, seq):
     """quik_rotary_inplace against x * cos + rotate_half(x) * sin in torch (transformers' apply_rotary_pos_emb
