@@ -46,17 +46,16 @@ import torch  # noqa: E402
 METRIC = "MixedQLinear TOPS (Llama-2 linear shapes, fused quantize+GEMM+dequant)"
 L2_BYTES = 126e6
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of gemm_tcgen05_kernel from `ncu --set full` captures of
-# single bench steps, key = (M, K, N); the files under profiles/ named here hold the captures' figures and commands
+# single bench steps, key = (M, K, N)
 NCU_TRAFFIC_BYTES = {
     (2048, 4096, 12288): 84.55e6, (2048, 4096, 4096): 26.88e6, (2048, 4096, 22016): 178.77e6, (2048, 11008, 4096): 84.54e6,
 }
-NCU_TRAFFIC_SOURCE = "profiles/gemm_tcgen05_llama7b_m2048.md"
+NCU_TRAFFIC_SOURCE = "ncu capture of one step of the Llama-2-7B layers at 2048 tokens"
 # The 70B layers at M = 4096 hold up to 1.3 GB per launch, more than a full-section capture should; one layer of them
 # was captured (o, 8192 -> 8192: 281.0 MB of DRAM traffic for 266.6 MB of algorithmic bytes) and the others are scaled
 # from it by their algorithmic bytes (operands and outputs cross HBM once in every layer: traffic grows in proportion).
 NCU_TRAFFIC_RATIO_70B = 281.0 / 266.6
-NCU_TRAFFIC_RATIO_SOURCE = ("profiles/gemm_tcgen05_llama70b_m4096.md (capture of the o layer; the other layers scaled "
-                            "by algorithmic bytes)")
+NCU_TRAFFIC_RATIO_SOURCE = "ncu capture of the Llama-2-70B o layer at 4096 tokens; the other layers scaled by algorithmic bytes"
 
 
 def parse_args():

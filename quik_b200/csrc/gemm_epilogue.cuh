@@ -178,8 +178,8 @@ struct EpilogueWarp {
   // Two 16-byte pieces per lane (32 bytes of its row, ELEM-byte elements) -> memory at dst (row m0 of the warp), `bytes` of
   // them valid.  Transposed through shared memory so that one warp instruction stores 16 rows x 32 contiguous bytes (whole
   // sectors) instead of 32 rows x 16 bytes; rows without 16-byte alignment are stored element by element, still 32 contiguous
-  // bytes of a row at a time (one row per lane was a sector
-  // per element: 741 tokens through int4 5152 x 3333 took 85.6 us, now 22.6).
+  // bytes of a row at a time (one row per lane was a sector per element: 741 tokens through int4 5152 x 3333 took 85.6 us,
+  // now 22.6).
   template <int ELEM>
   __device__ __forceinline__ void store_row_pieces(uint4 p0, uint4 p1, unsigned char *dst, size_t pitch, int rows, int bytes) const {
     __syncwarp();                            // the buffer has been read out

@@ -187,7 +187,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       long long w_region = 0, w_full = 0;
       const long long t_begin = clock64();
       for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
-      constexpr bool fp = decltype(is_fp)::value;
+        constexpr bool fp = decltype(is_fp)::value;
         if (kb == 0) {
           const long long t0 = dbg ? clock64() : 0;
           uint32_t parity;

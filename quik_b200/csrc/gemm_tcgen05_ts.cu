@@ -5,13 +5,12 @@
 // src/asymmetric/asymmetric.cu:134-146), but the A operand (the activation codes, or the outlier activations) does not
 // go from shared memory to the tensor core through a shared-memory descriptor.  Four warps move every k-block of A from
 // its shared-memory stage into a small ring of tensor-memory slots (tcgen05.st), and the products are issued in the
-// form that reads A from tensor memory and only B through a descriptor.  Two things follow:
-//   * one thread issues tcgen05.mma of this form at the tensor pipe's full rate (128 cycles for 128 x 256 x 32 bytes
-//     per SM), whereas with both operands in shared memory one thread needs ~217 cycles per instruction whatever its
-//     size (measured), which bounded the other kernel;
-//   * 4-bit activation codes travel packed (the reference layout, two per byte, include/int4.h:78-98) from HBM
-//     through L2 into shared memory -- half the bytes -- and are widened to signed bytes on their way into tensor
-//     memory (each byte = 16 x code; the factor is shifted out of the exact int32 sums in the epilogue).
+// form that reads A from tensor memory and only B through a descriptor.  So 4-bit activation codes travel packed (the
+// reference layout, two per byte, include/int4.h:78-98) from HBM through L2 into shared memory -- half the bytes -- and are
+// widened to signed bytes on their way into tensor memory (each byte = 16 x code; the factor is shifted out of the exact int32
+// sums in the epilogue).  A comparison engine: tensor memory has room for two operand slots beside two accumulator
+// regions, too few to hide the hand-over, and it measured 822 (pairs) / 1286 (single CTAs) against 2081 TOPS on the Llama-2-7B
+// step; the other kernel has become faster since by issuing with a whole warp, which this one does not do.
 //
 // Roles of a CTA (448 threads): warp 0 TMA producer, warp 1 TMEM allocation + MMA issue, warps 2-5 operand transfer
 // (one per tensor-memory lane quarter), warps 6-13 epilogue (gemm_epilogue.cuh).  Tensor memory (512 columns): two
@@ -73,7 +72,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fp_drained + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   float *s_vec = reinterpret_cast<float *>(aux + 512);                 // [8][3][TS_HALF_CAP]
-  unsigned char *s_out = aux + TS_AUX_BYTES;                           // [8][32 x 64 bytes]
+  unsigned char *s_out = aux + TS_AUX_BYTES;                           // [8][32 x 32 bytes]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -204,7 +203,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     uint32_t phase = 0, slot_phase = 0;
     long long c_full = 0, c_slot = 0;
     for_each_block<HAS_FP>(n_local, p.int_kb, p.fp_kb, [&](int j, auto is_fp, int kb) {
-        constexpr bool fp = decltype(is_fp)::value;
+      constexpr bool fp = decltype(is_fp)::value;
       const long long t0 = clock64();
       const bool landed = mbar_wait(smem_u32(a_bar + stage), phase, abort_flag, p.status);
       if (!__all_sync(0xffffffffu, landed)) return false;

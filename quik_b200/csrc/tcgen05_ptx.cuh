@@ -228,8 +228,7 @@ __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint
                  ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Same products with the A operand read from tensor memory (128 lanes x 8 columns of 32 bits per instruction = 32 bytes
-// of K per row; with CTAS == 2 each CTA's rows come from its own tensor memory at the same address).  A single thread
-// issues these at the tensor pipe's full rate, which it cannot do with both operands described in shared memory.
+// of K per row; with CTAS == 2 each CTA's rows come from its own tensor memory at the same address).
 template <int CTAS>
 __device__ __forceinline__ void mma_i8_ts(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   if (CTAS == 1)
