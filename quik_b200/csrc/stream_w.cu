@@ -28,6 +28,8 @@
 // loops, the cluster barriers are still passed by every thread, TMEM is released and the kernel returns.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tcgen05_ptx.cuh"
 
@@ -384,15 +386,36 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     cluster_arrive();
     cluster_wait();                                  // the sums of all CTAs are in place
     if (worker && have && n < p.N) {
-      const int t1 = min(p.M, (rank + 1) * p.ntok / S);
+      // This CTA's share of the tokens, every second one from h on.  All loads of a batch are under way before the first is
+      // used: one at a time they cost 0.2 us per token (80 tokens, 33 slabs of 1600 int4 columns: 14.2 -> 9.7 us).
+      const int t0 = rank * p.ntok / S + h, last = min(p.M, (rank + 1) * p.ntok / S) - 1;
       const uint32_t own_i = smem_u32(sum_i), fp0 = map_to_rank(smem_u32(sum_f), 0);
-      for (int m = rank * p.ntok / S + h; m < t1; m += 2) {
-        const uint32_t off = (uint32_t)((m * SW_ROWS + row) * 4);
-        int acc = 0;
-#pragma unroll 4
-        for (int s = 0; s < S; ++s) acc += ld_cluster_s32(map_to_rank(own_i, s) + off);
-        finish(m, acc, p.nf > 0 ? __int_as_float(ld_cluster_s32(fp0 + off)) : 0.f);
-      }
+      auto finish_share = [&](auto ctas) {
+        constexpr int C = decltype(ctas)::value, U = 32 / C;
+        for (int m0 = t0; m0 <= last; m0 += 2 * U) {
+          int v[C][U], f[U];
+#pragma unroll
+          for (int s = 0; s < C; ++s) {
+            const uint32_t theirs = map_to_rank(own_i, s);
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[s][u] = ld_cluster_s32(theirs + (uint32_t)((min(m0 + 2 * u, last) * SW_ROWS + row) * 4));
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            f[u] = p.nf > 0 ? ld_cluster_s32(fp0 + (uint32_t)((min(m0 + 2 * u, last) * SW_ROWS + row) * 4)) : 0;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (m0 + 2 * u > last) break;
+            int acc = 0;
+#pragma unroll
+            for (int s = 0; s < C; ++s) acc += v[s][u];
+            finish(m0 + 2 * u, acc, __int_as_float(f[u]));
+          }
+        }
+      };
+      if (S == 2) finish_share(std::integral_constant<int, 2>());
+      else if (S == 4) finish_share(std::integral_constant<int, 4>());
+      else finish_share(std::integral_constant<int, 8>());
     }
     __syncwarp();
     cluster_arrive();
