@@ -60,7 +60,7 @@ inline StreamPlan plan_stream(int bits, int ntok, int slabs, int sms) {
   c.tmem_cols = c.ctas_per_sm == 2 ? 256 : 512;
   const int d_cols = ntok <= 32 ? 32 : (ntok <= 64 ? 64 : 128);
   c.d_fp = c.tmem_cols - d_cols;                                         // f32 accumulator
-  c.d_int = c.d_fp - d_cols;                                             // s32 accumulator
+  c.d_int = c.d_fp - (bits == 8 ? 2 : 1) * d_cols;                       // s32 accumulator; int8: two, d_cols apart
   c.a_slots = bits == 4 ? c.d_int / SW_A_COLS : 0;                       // ring of widened W k-blocks, from column 0 on
   if (c.a_slots > 4) c.a_slots = 4;
   c.x_bytes = ntok * 128;                                                // one 128-byte k-block of the token operand
@@ -151,13 +151,13 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(full_bar + s), 1);
-      mbar_init(smem_u32(empty_bar + s), 1 + (BITS == 4 ? 8 : 0));   // MMA commit (+ the 8 widening warps)
+      mbar_init(smem_u32(empty_bar + s), 1 + (BITS == 4 ? 8 : 1));   // MMA commit, and the 8 widening warps or the other issuer
     }
     for (int s = 0; s < p.a_slots; ++s) {
       mbar_init(smem_u32(a_full + s), 8);
       mbar_init(smem_u32(a_empty + s), 1);
     }
-    mbar_init(smem_u32(acc_full), 1);
+    mbar_init(smem_u32(acc_full), BITS == 8 ? 2 : 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -226,12 +226,17 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp == 1 || (BITS == 8 && warp == 2)) {
     // ================= MMA issuer =================
     // The loop's exits are warp votes, so its counters and the descriptors made from them are uniform over the warp and
     // the elected lane issues back to back.  (A loop inside a `lane == 0` branch issued one instruction every ~62 ns.)
+    // Waiting for a stage and issuing its four products still takes one warp 600 cycles, more than an int8 block takes to arrive:
+    // two warps (the second has nothing else to do until the epilogue) take the int8 blocks in turn, each into an
+    // accumulator of its own (75 slabs of 10752 int8 columns, 33 / 64 tokens: 34.3 / 35.4 -> 31.2 / 31.9 us).
+    const int me = warp - 1;
     const bool elected = elect_one();
     const uint64_t dw0 = make_smem_desc(smem_u32(tiles));
+    const uint32_t d_int = tmem_base + p.d_int + me * ((p.d_fp - p.d_int) / 2);
     int stage = 0, slot = 0;
     uint32_t phase = 0, slot_phase = 0;
     long long w_full = 0, w_a = 0;
@@ -241,6 +246,13 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       const long long t0 = dbg ? clock64() : 0;
       if (!mbar_wait_warp(smem_u32(full_bar + stage), phase, abort_flag, p.status)) break;
       if (dbg) w_full += clock64() - t0;
+      if (BITS == 8 && me != (i < n_fp ? 0 : (i - n_fp) & 1)) {
+        // the other warp's block.  A stage is filled again only when both have seen it: a barrier's phase is one bit, so a warp
+        // may neither miss a fill nor fall behind by two.
+        if (elected) mbar_arrive(smem_u32(empty_bar + stage));
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        continue;
+      }
       const uint64_t dw = dw0 + (uint32_t)(stage * (STAGE_BYTES >> 4));      // 16-byte units of the start-address field
       const uint64_t dx = dw + (SW_W_BYTES >> 4);
       if (i < n_fp) {
@@ -254,7 +266,7 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         if (elected)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            mma_i8<1>(tmem_base + p.d_int, dw + 2 * k, dx + 2 * k, p.idesc_int, (i > n_fp || k > 0) ? 1u : 0u);
+            mma_i8<1>(d_int, dw + 2 * k, dx + 2 * k, p.idesc_int, (i > n_fp + 1 || k > 0) ? 1u : 0u);
       } else {
         const long long t1 = dbg ? clock64() : 0;
         if (!mbar_wait_warp(smem_u32(a_full + slot), slot_phase, abort_flag, p.status)) break;
@@ -265,7 +277,7 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           const uint32_t a = tmem_base + slot * SW_A_COLS;
 #pragma unroll
           for (int k = 0; k < 8; ++k)      // 32 codes = 8 TMEM columns of A per instruction
-            mma_i8_ts<1>(tmem_base + p.d_int, a + 8 * k, (k < 4 ? dx : dx1) + 2 * (k & 3), p.idesc_int,
+            mma_i8_ts<1>(d_int, a + 8 * k, (k < 4 ? dx : dx1) + 2 * (k & 3), p.idesc_int,
                          (i > n_fp || k > 0) ? 1u : 0u);
           mma_commit<1>(smem_u32(a_empty + slot));
         }
@@ -276,7 +288,7 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     if (elected) mma_commit<1>(smem_u32(acc_full));     // also after an aborted loop: the epilogue wait ends either way
     __syncwarp();
-    if (dbg && lane == 0) {
+    if (dbg && me == 0 && lane == 0) {
       unsigned long long *d = p.dbg + (size_t)blockIdx.x * 16;
       d[0] = (unsigned long long)(clock64() - t_begin);   // MMA warp: issue loop
       d[1] = (unsigned long long)w_full;                  // ... waiting for a loaded stage
@@ -346,6 +358,13 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     if (n_int > 0) {
       tmem_ld8(tmem_base + lane_base + p.d_int + tok0, acc);
       tmem_ld_wait(acc);
+      if (BITS == 8 && n_int > 1) {
+        uint32_t second[8];
+        tmem_ld8(tmem_base + lane_base + (p.d_int + p.d_fp) / 2 + tok0, second);
+        tmem_ld_wait(second);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += second[j];
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0;
