@@ -28,6 +28,7 @@
 // loops, the cluster barriers are still passed by every thread, TMEM is released and the kernel returns.
 #include <cuda.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -45,18 +46,16 @@ constexpr int SW_AUX_BYTES = 2048;                 // barriers, then the token s
 constexpr int SW_SMEM_SM = 227 * 1024;
 
 // Sizes that depend on the number of tokens (the MMA's N, a multiple of 16): shared-memory ring and tensor-memory plan.
-// Up to 64 tokens two CTAs share an SM (256 tensor-memory columns and at most 113 KB each), beyond that one CTA has it;
-// from 33 tokens on also where the slabs alone occupy more than half of the SMs, but not all twice: a whole K and the deeper ring
-// of one CTA per SM then beat a split K (64 tokens: 14.4 against 19.8 us for 96 slabs of 4096 int4 columns, 22.9 against 26.4 us
-// for 80 slabs of 8192; for 64 slabs 20.9 against 17.0 us, for 172 slabs 28.2 against 20.3 us).
+// Up to 64 tokens two CTAs may share an SM (256 tensor-memory columns and at most 113 KB each; the rule is in launch_stream_w),
+// beyond that one CTA has it.
 struct StreamPlan {
   int ctas_per_sm, tmem_cols, a_slots, d_int, d_fp;
   int x_bytes, stage_bytes, stages;
   size_t smem;
 };
-inline StreamPlan plan_stream(int bits, int ntok, int slabs, int sms) {
+inline StreamPlan plan_stream(int bits, int ntok, int ctas_per_sm) {
   StreamPlan c{};
-  c.ctas_per_sm = ntok <= 32 || (ntok <= 64 && (2 * slabs <= sms || slabs > sms)) ? 2 : 1;
+  c.ctas_per_sm = ctas_per_sm;
   c.tmem_cols = c.ctas_per_sm == 2 ? 256 : 512;
   const int d_cols = ntok <= 32 ? 32 : (ntok <= 64 ? 64 : 128);
   c.d_fp = c.tmem_cols - d_cols;                                         // f32 accumulator
@@ -474,6 +473,36 @@ stream_w_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   }
 }
 
+// Clusters of `size` CTAs (2, 4 or 8) that run at once on the current device.  Fewer than SMs x CTAs per SM / size: a cluster has
+// to fit the SMs of one processing cluster of the GPU.  The occupancy call answers that for one CTA per SM (74, 33 and 15 on a
+// GPU of 148 SMs; it does not know that two of these kernels fit an SM).  With two per SM a cluster takes half as many SMs:
+// measured by the launch time's jump, 33 clusters of eight run at once and 69 to 71 of four (of 74: launches overlap and leave
+// gaps).  Counting slots alone sent 72 to 74 slabs to a second wave: 19.8 us for 64 tokens of 4096 int4 columns, now 12.7.
+int resident_clusters(int ctas_per_sm, int size) {
+  if (ctas_per_sm == 2) {
+    if (size == 2) return num_sms();
+    const int r = resident_clusters(1, size / 2);
+    return size == 4 ? r - r / 14 : r;
+  }
+  static std::atomic<int> cached[kMaxDevices][4];        // 0 = not asked yet, else the answer + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  std::atomic<int> &known = cached[dev][size == 2 ? 1 : (size == 4 ? 2 : 3)];
+  int n = known.load() - 1;
+  if (n >= 0) return n;
+  auto kern = stream_w_kernel<__half, 8>;                // the others take the same room
+  LaunchCfg lc(dim3(2 * size * num_sms()), dim3(SW_THREADS), 200 * 1024, nullptr, size);
+  lc.cfg.numAttrs = 1;                                   // the cluster shape only
+  n = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_SM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &lc.cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known.store(n + 1);
+  return n;
+}
+
 template <typename T, int BITS>
 int launch_t(const CUtensorMap &tw, const CUtensorMap &tx, const CUtensorMap &tfw, const CUtensorMap &tfx,
              const StreamParams &p, int slabs, size_t smem, cudaStream_t st) {
@@ -509,13 +538,31 @@ int launch_stream_w(const void *q, const void *w, int bits, int M, int N, int K_
   p.nk = (w_row_bytes + 127) / 128;
   p.nf = has_fp ? (ep.F + 63) / 64 : 0;
   const int slabs = (N + SW_ROWS - 1) / SW_ROWS;
-  // Split K over a cluster while all CTAs still fit on the GPU at once, every CTA keeps at least two k-blocks and
-  // the outlier blocks all fall to the first CTA.
-  const StreamPlan plan = plan_stream(bits, ntok, slabs, num_sms());
-  const int total = p.nk + p.nf, slots = plan.ctas_per_sm * num_sms();
-  int splits = 1;
-  while (splits < 8 && slabs * splits * 2 <= slots && total / (splits * 2) >= (p.nf > 2 ? p.nf : 2)) splits *= 2;
-  p.splits = splits;
+  // Split K over a cluster while all CTAs still run at once, every CTA keeps at least two k-blocks and the outlier
+  // blocks all fall to the first CTA.
+  const int total = p.nk + p.nf;
+  auto choose_splits = [&](int ctas_per_sm) {
+    int s = 1;
+    while (s < 8 && total / (s * 2) >= (p.nf > 2 ? p.nf : 2) && slabs <= resident_clusters(ctas_per_sm, s * 2)) s *= 2;
+    return s;
+  };
+  int per_sm = 1;
+  p.splits = choose_splits(1);
+  if (ntok <= 64) {
+    // Two CTAs per SM, each with half of the ring, or one?  More slabs than SMs: two (172 slabs of 4096 int4 columns, 48 tokens:
+    // 19.3 against 27.6 us).  Otherwise two only where they allow a deeper split of a long K: each CTA starts and
+    // finishes its own pipeline, so up to 20 blocks per CTA one is as good or better (96 slabs of 4096 int4 columns, 33 / 64
+    // tokens: 14.2 / 14.7 against 15.2 / 16.2 us; 40 slabs 11.1 / 11.6 against 11.2 / 11.8), beyond that two keep the widening
+    // warps busier (40 slabs of 11008 columns 16.8 / 18.1 against 18.3 / 18.8 us, 120 slabs 26.1 / 27.4 against 29.9 /
+    // 30.2); int8 blocks need no widening and gain only while most CTAs still have an SM for themselves (40 and 96
+    // slabs of 11008 columns, 33 tokens: 17.1 against 19.7 and 29.6 against 31.3 us, 120 slabs: 33.3 against 32.1).
+    const int s2 = choose_splits(2), sms = num_sms();
+    if (slabs > sms || (s2 > p.splits && total / p.splits > 20 && (bits == 4 || 5 * slabs * s2 <= 7 * sms))) {
+      per_sm = 2;
+      p.splits = s2;
+    }
+  }
+  const StreamPlan plan = plan_stream(bits, ntok, per_sm);
   p.ntok = ntok;
   p.stages = plan.stages;
   p.stage_bytes = plan.stage_bytes;

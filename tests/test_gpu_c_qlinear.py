@@ -544,3 +544,25 @@ def test_ring_engine_settings_give_the_same_bits(N, bits):
         _lib.check(_lib.load().quik_config_set(_lib.CFG_STREAM_PRELOAD, 1), "quik_config_set")
         _lib.check(_lib.load().quik_config_set(_lib.CFG_STREAM_RING, 2), "quik_config_set")
     assert_device_clean()
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("slabs,K,F", [(1, 96, 64), (3, 160, 0), (2, 352, 64), (15, 2304, 64), (16, 2304, 64), (34, 2304, 64), (70, 1088, 64),
+                                       (74, 2304, 64), (75, 4352, 256), (96, 5632, 64), (149, 1088, 64)])
+def test_streaming_engine_splits_and_short_sums(slabs, K, F, bits):
+    """One to a few integer blocks (the two int8 issuing warps then have none, one or several each), and numbers of 128-row slabs on
+    both sides of every line of the rule for splits and CTAs per SM.  The sums are integers: the rows of a call equal those of
+    a call for other token counts, which run another split, another plan or (up to 16 tokens) another engine, up to the
+    place of the rounding; the smallest layers are compared with the oracle."""
+    N = 128 * slabs - 5
+    case = make_layer("t", 128, K, N, bits, F=F, seed=slabs, device=dev(), clip=False)
+    ref = case.module(case.x)[0]
+    if slabs <= 16:
+        assert rel_rms_err(ref.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+    few = case.module(case.x[:16].contiguous())[0]
+    assert rel_rms_err(ref[:16].cpu(), few.cpu()) < 5e-3
+    for M in (17, 32, 33, 64, 65, 97):
+        out = case.module(case.x[:M].contiguous())[0]
+        assert torch.equal(case.module(case.x[:M].contiguous())[0], out)
+        assert rel_rms_err(out.cpu(), ref[:M].cpu()) < 5e-3
+    assert_device_clean()
