@@ -9,13 +9,13 @@
 //                                                                                asymmetric.cu:134-146
 // or stores acc_i as int32 (mode 0).
 //
-// Structure (one persistent CTA per SM or one CTA pair per two SMs, 320 threads per CTA):
+// Structure (one persistent CTA per SM or one CTA pair per two SMs, 384 threads per CTA):
 //   warp 0    TMA producer: cp.async.bulk.tensor.2d loads of the A / B k-blocks (128 bytes of K
 //             per row, 128B swizzle) into a ring of shared-memory stages, completion on mbarriers.
 //   warp 1    allocates TMEM; one elected lane issues tcgen05.mma (M=128 or 256, N=block_n, K=32
 //             bytes) from shared-memory descriptors and commits each stage back to the producer.
-//   warps 2-9 epilogue: tcgen05.ld the accumulators (32 lanes x 16 columns per warp and step),
-//             apply the dequantize arithmetic in fp32 and store through a shared-memory transpose.
+//   warps 4-11 epilogue: tcgen05.ld the accumulators (32 lanes x 16 columns per warp and step),
+//             apply the dequantize arithmetic in fp32 and store through shared memory (bulk stores where rows allow).
 // Outlier k-blocks (64 fp16 values = 128 bytes per row) travel through the same ring as the integer
 // k-blocks; TMEM holds two accumulator regions so the epilogue of tile i overlaps the MMAs of tile
 // i+1 (schedule in gemm_epilogue.cuh).
@@ -40,7 +40,11 @@ __device__ unsigned int g_device_status = 0;
 namespace {
 
 constexpr int EPI_WARPS = 8;
-constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;      // TMA warp + MMA warp + epilogue warps
+constexpr int NUM_THREADS = 128 + 32 * EPI_WARPS;     // TMA warp, MMA warp, two that only fill their warpgroup, epilogue warps
+// Registers per thread once the roles part: the launch gives 168 to each of 384 threads; the first four warps hand most of theirs to
+// the epilogue warps, which keep 64 words of the outlier product and work on two chunks of an accumulator at once.
+constexpr int REGS_LAUNCH = 168, REGS_ISSUE = 72, REGS_EPILOGUE = 216;
+static_assert(128 * REGS_ISSUE + 32 * EPI_WARPS * REGS_EPILOGUE <= NUM_THREADS * REGS_LAUNCH, "register split");
 // Process-wide tuning knobs (quik_config_set): plain words, meant to be set once before the layers run; a
 // launch reads each of them once.
 std::atomic<int> g_tile_n{0};                                 // 0 = choose by shape, else a multiple of 16 in [32, 256]
@@ -49,8 +53,8 @@ std::atomic<int> g_l2_hint{0};                                // 1 = token-opera
 std::atomic<unsigned long long *> g_dbg{nullptr};             // diagnostic counters (device memory), off by default
 
 // Shared-memory plan after the 1024-byte aligned ring of stages: 256 bytes of barriers etc. and the
-// per-warp epilogue vectors (rounded to 1024 together), then one output staging chunk per epilogue
-// warp (32 rows x 32 bytes).
+// per-warp epilogue vectors (rounded to 1024 together), then the output staging of each epilogue
+// warp.
 constexpr int EPI_COLS(int cap_n) { return cap_n / (EPI_WARPS / 4); }       // most columns per epilogue warp
 constexpr int AUX_BYTES(int cap_n) { return ((256 + EPI_WARPS * 3 * EPI_COLS(cap_n) * 4) + 1023) / 1024 * 1024; }
 constexpr int stage_bytes(int cap_n, int ctas) { return (BLOCK_M + cap_n / ctas) * STAGE_K_BYTES; }
@@ -68,11 +72,13 @@ constexpr int num_stages(int cap_n, int ctas) {
 // loads its own 128 rows of A and only its half of the B rows, so a CTA moves a third less operand
 // data per multiply-accumulate than alone.  The leader (cluster rank 0) issues the MMAs for the pair
 // and owns the barriers that count loads and region releases; commits reach both CTAs.
-template <typename T, int CAP_N, bool HAS_FP, int CTAS>
+// KIND: what becomes of the integer product, see EpilogueWarp.
+template <typename T, int CAP_N, int KIND, int CTAS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_fa, const __grid_constant__ CUtensorMap tmap_fb,
-                    const GemmParams p) {
+                    const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
+  constexpr bool HAS_FP = KIND == 2;
   constexpr int A_BYTES = BLOCK_M * STAGE_K_BYTES;
   constexpr int STAGE_BYTES = stage_bytes(CAP_N, CTAS);      // room for the widest tile; narrower ones use less of it
   constexpr int STAGES = num_stages(CAP_N, CTAS);
@@ -96,7 +102,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // per-column epilogue vectors, one private copy per epilogue warp (no cross-warp barrier needed)
   float *s_vec = reinterpret_cast<float *>(aux + 256);                 // [EPI_WARPS][3][EPI_COLS], 16-byte aligned
-  // output staging: [EPI_WARPS][32 rows x 32 bytes], 1024-byte aligned
+  // output staging: [EPI_WARPS][EPI_BUF_BYTES], 1024-byte aligned
   unsigned char *s_out = tiles + STAGES * STAGE_BYTES + AUX_BYTES(CAP_N);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -109,15 +115,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), 32 * EPI_WARPS * CTAS);    // epilogue threads of the whole pair
+      mbar_init(smem_u32(acc_empty + s), EPI_WARPS * CTAS);    // epilogue warps of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
-      mbar_init(smem_u32(fp_drained + s), 32 * EPI_WARPS * CTAS);
+      mbar_init(smem_u32(fp_drained + s), EPI_WARPS * CTAS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     prefetch_tmap(&tmap_a);
     prefetch_tmap(&tmap_b);
+    if (p.vec_out) prefetch_tmap(&tmap_out);
     if (HAS_FP) {
       prefetch_tmap(&tmap_fa);
       prefetch_tmap(&tmap_fb);
@@ -138,7 +145,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int unit = (int)blockIdx.x / CTAS, num_units = (int)gridDim.x / CTAS;    // a unit = CTA or CTA pair
   const int n_local = (p.num_tiles - unit + num_units - 1) / num_units;           // tiles of this unit
 
-  if (warp == 0) {
+  if (warp >= 4) {
+    // ================= epilogue (warps 4..11): gemm_epilogue.cuh =================
+    set_max_regs_up<REGS_EPILOGUE>();
+    EpilogueWarp<T, KIND, 0, CTAS, EPI_COLS(CAP_N), true> ew(p, &tmap_out, tmem_base, CAP_N, unit, num_units, rank, warp - 4, warp & 3, lane, s_vec,
+                                                       s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
+    ew.run(n_local);
+    if (p.dbg && warp == 4 && lane == 0) ew.write_counters((int)blockIdx.x);
+  } else if (set_max_regs_down<REGS_ISSUE>(); warp == 0) {
     // ================= TMA producer =================
     const bool elected = elect_one();
     int stage = 0;
@@ -223,12 +237,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         d[3] = (unsigned long long)n_local;
       }
     }
-  } else {
-    // ================= epilogue (warps 2..9): gemm_epilogue.cuh =================
-    EpilogueWarp<T, HAS_FP, CTAS, EPI_COLS(CAP_N)> ew(p, tmem_base, CAP_N, unit, num_units, rank, warp - 2, warp & 3, lane, s_vec,
-                                                      s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
-    ew.run(n_local);
-    if (p.dbg && warp == 2 && lane == 0) ew.write_counters((int)blockIdx.x);
   }
 
   // ---- teardown: every thread arrives here, also after an aborted wait
@@ -269,11 +277,11 @@ EncodeTiledFn get_encode_fn() {
 }  // namespace
 
 int make_tmap(CUtensorMap *map, const void *base, CUtensorMapDataType dt, int elem_bytes, int rows, int cols,
-              int box_rows, int box_row_bytes) {
+              int box_rows, int box_row_bytes, long long pitch) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return QUIK_ERR_CUDA;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
+  cuuint64_t strides[1] = {(cuuint64_t)(pitch > 0 ? pitch : cols) * elem_bytes};
   cuuint32_t box[2] = {(cuuint32_t)(box_row_bytes / elem_bytes), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   const CUtensorMapSwizzle sw = box_row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
@@ -346,7 +354,7 @@ int max_pairs(Kern kern, size_t smem) {
 
 // Units (CTAs, or CTA pairs) of one kernel instantiation that are resident at once on the current device.
 // The shared-memory opt-in and the occupancy answer belong to a device, so they are kept per device ordinal.
-template <typename T, int CAP_N, bool HAS_FP, int CTAS>
+template <typename T, int CAP_N, int KIND, int CTAS>
 int resident_units(int *out) {
   static std::mutex mu;
   static int cached[kMaxDevices];       // 0 = not asked yet, -1 = cannot launch
@@ -355,8 +363,11 @@ int resident_units(int *out) {
   if (dev < 0 || dev >= kMaxDevices) return QUIK_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lock(mu);
   if (cached[dev] == 0) {
-    auto kern = gemm_tcgen05_kernel<T, CAP_N, HAS_FP, CTAS>;
+    auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS>;
     constexpr size_t smem = smem_bytes(CAP_N, CTAS);
+    cudaFuncAttributes at;
+    QUIK_CUDA_TRY(cudaFuncGetAttributes(&at, kern));
+    if (at.numRegs < REGS_LAUNCH) return QUIK_ERR_UNSUPPORTED;      // the epilogue warps would wait for registers for ever
     QUIK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int n = CTAS == 1 ? num_sms() : max_pairs(kern, smem);
     cached[dev] = n > 0 ? n : -1;
@@ -365,18 +376,18 @@ int resident_units(int *out) {
   return QUIK_OK;
 }
 
-template <typename T, int CAP_N, bool HAS_FP, int CTAS>
+template <typename T, int CAP_N, int KIND, int CTAS>
 int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tfa, const CUtensorMap &tfb,
-             const GemmParams &p, cudaStream_t st) {
-  auto kern = gemm_tcgen05_kernel<T, CAP_N, HAS_FP, CTAS>;
+             const CUtensorMap &to, const GemmParams &p, cudaStream_t st) {
+  auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS>;
   constexpr size_t smem = smem_bytes(CAP_N, CTAS);
   int resident = 0;
-  const int rc = resident_units<T, CAP_N, HAS_FP, CTAS>(&resident);
+  const int rc = resident_units<T, CAP_N, KIND, CTAS>(&resident);
   if (rc != QUIK_OK) return rc;
   if (resident <= 0) return QUIK_ERR_UNSUPPORTED;
   const int units = p.num_tiles < resident ? p.num_tiles : resident;
   LaunchCfg lc(dim3(CTAS * units), dim3(NUM_THREADS), smem, st, CTAS);
-  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, kern, ta, tb, tfa, tfb, p));
+  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, kern, ta, tb, tfa, tfb, to, p));
   return check_launch("gemm_tcgen05_kernel");
 }
 
@@ -477,7 +488,6 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   p.num_tiles = m_tiles * ((N + block_n - 1) / block_n);
   p.idesc_int = make_idesc(2, 1, tile_m, block_n);                              // S32 accumulate, signed 8-bit operands
   p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, tile_m, block_n);   // F32 accumulate, F16 / BF16 operands
-  p.acc_shift = 0;
   p.l2_hint = g_l2_hint.load();
 
   CUtensorMap ta, tb, tfa, tfb;
@@ -492,22 +502,27 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
     tfa = ta;
     tfb = tb;
   }
-#define QUIK_LAUNCH_C(T, C)                                                                \
-  do {                                                                                     \
-    if (cap_n == 256) {                                                                    \
-      return has_fp ? launch_t<T, 256, true, C>(ta, tb, tfa, tfb, p, st)                   \
-                    : launch_t<T, 256, false, C>(ta, tb, tfa, tfb, p, st);                 \
-    }                                                                                      \
-    return has_fp ? launch_t<T, 128, true, C>(ta, tb, tfa, tfb, p, st)                     \
-                  : launch_t<T, 128, false, C>(ta, tb, tfa, tfb, p, st);                   \
+  // the result, where its rows allow bulk stores: boxes of 32 rows x 64 bytes
+  CUtensorMap to = ta;
+  if (p.vec_out) {
+    if (ep.mode == 0) rc = make_tmap(&to, ep.C, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, M, N, 32, 64);
+    else rc = make_tmap(&to, ep.out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, M, N, 32, 64, p.ldo);
+    if (rc != QUIK_OK) return rc;
+  }
+#define QUIK_LAUNCH_C(T, K, C) \
+  return cap_n == 256 ? launch_t<T, 256, K, C>(ta, tb, tfa, tfb, to, p, st) : launch_t<T, 128, K, C>(ta, tb, tfa, tfb, to, p, st)
+#define QUIK_LAUNCH(T, K)                  \
+  do {                                     \
+    if (ctas == 2) QUIK_LAUNCH_C(T, K, 2); \
+    QUIK_LAUNCH_C(T, K, 1);                \
   } while (0)
-#define QUIK_LAUNCH(T)                                                                     \
-  do {                                                                                     \
-    if (ctas == 2) QUIK_LAUNCH_C(T, 2);                                                    \
-    QUIK_LAUNCH_C(T, 1);                                                                   \
-  } while (0)
-  if (ep.dtype == QUIK_BF16) QUIK_LAUNCH(__nv_bfloat16);
-  QUIK_LAUNCH(__half);
+  if (ep.mode == 0) QUIK_LAUNCH(__half, 0);
+  if (ep.dtype == QUIK_BF16) {
+    if (has_fp) QUIK_LAUNCH(__nv_bfloat16, 2);
+    QUIK_LAUNCH(__nv_bfloat16, 1);
+  }
+  if (has_fp) QUIK_LAUNCH(__half, 2);
+  QUIK_LAUNCH(__half, 1);
 #undef QUIK_LAUNCH_C
 #undef QUIK_LAUNCH
 }

@@ -42,11 +42,12 @@ constexpr size_t ts_smem_bytes(int ctas) {
   return 1024 + (size_t)ts_num_stages(ctas) * ts_stage_bytes(ctas) + TS_AUX_BYTES + TS_EPI_WARPS * EPI_BUF_BYTES;
 }
 
-template <typename T, bool HAS_FP, int CTAS, bool A_PACKED>
+template <typename T, int KIND, int CTAS, bool A_PACKED>
 __global__ void __launch_bounds__(TS_THREADS, 1)
 gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const __grid_constant__ CUtensorMap tmap_fa, const __grid_constant__ CUtensorMap tmap_fb,
                        const GemmParams p) {
+  constexpr bool HAS_FP = KIND == 2;
   constexpr int STAGE_BYTES = ts_stage_bytes(CTAS);
   constexpr int STAGES = ts_num_stages(CTAS);
   constexpr int TILE_M = BLOCK_M * CTAS;
@@ -72,7 +73,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fp_drained + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   float *s_vec = reinterpret_cast<float *>(aux + 512);                 // [8][3][TS_HALF_CAP]
-  unsigned char *s_out = aux + TS_AUX_BYTES;                           // [8][32 x 32 bytes]
+  unsigned char *s_out = aux + TS_AUX_BYTES;                           // [8][EPI_BUF_BYTES]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -89,9 +90,9 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), 32 * TS_EPI_WARPS * CTAS);    // epilogue threads of the whole pair
+      mbar_init(smem_u32(acc_empty + s), TS_EPI_WARPS * CTAS);    // epilogue threads of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
-      mbar_init(smem_u32(fp_drained + s), 32 * TS_EPI_WARPS * CTAS);
+      mbar_init(smem_u32(fp_drained + s), TS_EPI_WARPS * CTAS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -257,7 +258,8 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
   } else {
     // ================= epilogue (warps 6..13): gemm_epilogue.cuh =================
-    EpilogueWarp<T, HAS_FP, CTAS, TS_HALF_CAP> ew(p, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec, s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
+    EpilogueWarp<T, KIND, A_PACKED ? 4 : 0, CTAS, TS_HALF_CAP, false> ew(p, nullptr, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec,
+                                                                   s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
     ew.run(n_local);
     if (p.dbg && warp == 6 && lane == 0) ew.write_counters((int)blockIdx.x);
   }
@@ -299,10 +301,10 @@ int ts_max_pairs(Kern kern, size_t smem) {
   return n;
 }
 
-template <typename T, bool HAS_FP, int CTAS, bool A_PACKED>
+template <typename T, int KIND, int CTAS, bool A_PACKED>
 int ts_launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tfa, const CUtensorMap &tfb,
                 const GemmParams &p, cudaStream_t st) {
-  auto kern = gemm_tcgen05_ts_kernel<T, HAS_FP, CTAS, A_PACKED>;
+  auto kern = gemm_tcgen05_ts_kernel<T, KIND, CTAS, A_PACKED>;
   constexpr size_t smem = ts_smem_bytes(CTAS);
   static std::mutex mu;
   static int cached[kMaxDevices];       // resident units per device: 0 = not asked yet, -1 = cannot launch
@@ -386,7 +388,6 @@ int launch_gemm_tcgen05_ts(const void *A, int a_packed, const int8_t *B, int M, 
   p.num_tiles = m_tiles * ((N + block_n - 1) / block_n);
   p.idesc_int = make_idesc(2, 1, tile_m, block_n);
   p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, tile_m, block_n);
-  p.acc_shift = a_packed ? 4 : 0;
   const int free_slots = (512 - 2 * block_n) / 32;
   p.a_slots = free_slots > TS_MAX_SLOTS ? TS_MAX_SLOTS : free_slots;
 
@@ -404,25 +405,22 @@ int launch_gemm_tcgen05_ts(const void *A, int a_packed, const int8_t *B, int M, 
     tfa = ta;
     tfb = tb;
   }
-#define QUIK_TS_P(T, F, C)                                                                        \
-  do {                                                                                            \
-    return a_packed ? ts_launch_t<T, F, C, true>(ta, tb, tfa, tfb, p, st)                         \
-                    : ts_launch_t<T, F, C, false>(ta, tb, tfa, tfb, p, st);                       \
+#define QUIK_TS_P(T, K, C)                                                \
+  return a_packed ? ts_launch_t<T, K, C, true>(ta, tb, tfa, tfb, p, st)   \
+                  : ts_launch_t<T, K, C, false>(ta, tb, tfa, tfb, p, st)
+#define QUIK_TS(T, K)                  \
+  do {                                 \
+    if (ctas == 2) QUIK_TS_P(T, K, 2); \
+    QUIK_TS_P(T, K, 1);                \
   } while (0)
-#define QUIK_TS_C(T, C)                                                                           \
-  do {                                                                                            \
-    if (has_fp) QUIK_TS_P(T, true, C);                                                            \
-    QUIK_TS_P(T, false, C);                                                                       \
-  } while (0)
-#define QUIK_TS(T)                                                                                \
-  do {                                                                                            \
-    if (ctas == 2) QUIK_TS_C(T, 2);                                                               \
-    QUIK_TS_C(T, 1);                                                                              \
-  } while (0)
-  if (ep.dtype == QUIK_BF16) QUIK_TS(__nv_bfloat16);
-  QUIK_TS(__half);
+  if (ep.mode == 0) QUIK_TS(__half, 0);
+  if (ep.dtype == QUIK_BF16) {
+    if (has_fp) QUIK_TS(__nv_bfloat16, 2);
+    QUIK_TS(__nv_bfloat16, 1);
+  }
+  if (has_fp) QUIK_TS(__half, 2);
+  QUIK_TS(__half, 1);
 #undef QUIK_TS_P
-#undef QUIK_TS_C
 #undef QUIK_TS
 }
 

@@ -13,7 +13,7 @@ constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;   // 2 s per device-
 // 2-D row-major tensor [rows, cols] of `elem_bytes` elements; box = box_row_bytes of a row x box_rows,
 // 128-byte swizzle when the box row is 128 bytes.
 int make_tmap(CUtensorMap *map, const void *base, CUtensorMapDataType dt, int elem_bytes, int rows, int cols,
-              int box_rows, int box_row_bytes = 128);
+              int box_rows, int box_row_bytes = 128, long long pitch = 0);
 // tcgen05 instruction descriptor: dense, K-major A and B.  c_format 1 = F32, 2 = S32; ab_format for
 // kind::i8: 1 = signed 8-bit, for kind::f16: 0 = F16, 1 = BF16.
 uint32_t make_idesc(int c_format, int ab_format, int m, int n);
@@ -82,6 +82,23 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
                                                unsigned int *status_word) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status_word));
 }
+// One box of shared memory to the tensor (coordinates beyond it are left out); the stores a thread has issued since its last
+// commit form a group.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// this thread's stores have read their shared memory / are complete
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// what this thread has written to shared memory is visible to bulk copies issued after this
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// registers of a warpgroup (four warps, all of which execute this): hands some back to the block, or takes them up again, waiting
+// until they are there.  The shares of a block's warpgroups may not exceed what it was launched with.
+template <int REGS> __device__ __forceinline__ void set_max_regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
+template <int REGS> __device__ __forceinline__ void set_max_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
+
 // true in exactly one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from oracle import kernel_path as kp
-from quik_b200 import _lib
+from quik_b200 import _lib, matmul
 from quik_b200.qlinear import MixedQLinear, SharedQuantizedInput
 from quik_b200.workloads import make_layer
 from tests.gpu_util import assert_device_clean, dev, rel_rms_err
@@ -87,6 +87,39 @@ def test_fused_layer_writes_only_its_columns(M, K, N, F, bits, tile, pair, engin
     border[row_pad:row_pad + M, col_pad:col_pad + N] = poison
     assert bool((border == poison).all()), "the layer wrote outside its [M, N] window"
     assert rel_rms_err(want.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+
+
+@pytest.mark.parametrize("F", [64, 0])
+@pytest.mark.parametrize("tile,pair", [(0, 0), (48, 1), (112, 2), (256, 2)])
+@pytest.mark.parametrize("N", [1, 9, 31, 250, 509])
+def test_rows_that_start_anywhere_in_a_sector(N, tile, pair, F):
+    """The tiled kernel's stores of rows without 16-byte alignment: windows that start at every column 0..15 of a slab whose row
+    pitch moves the start on by another odd amount per row, from a single column up to parts of several sectors.  Bits equal
+    those of the dense result, the rest of the slab is untouched, and so is an int32 product of N columns."""
+    M, K = 131, 224 + F
+    case = make_layer("t", M, K, N, 8, F=F, seed=N, device=dev(), clip=False)
+    try:
+        _lib.set_tile_n(tile)
+        _lib.set_cta_pair(pair)
+        want = case.module(case.x.unsqueeze(0))[0].clone()
+        for off in range(16):
+            slab = torch.full((M, N + 17 + (off & 2)), -1234.0, dtype=torch.float16, device=dev())
+            case.module.out_buffer = slab[:, off:off + N]
+            case.module(case.x.unsqueeze(0))
+            assert torch.equal(slab[:, off:off + N], want), off
+            slab[:, off:off + N] = -1234.0
+            assert bool((slab == -1234.0).all()), off
+        g = torch.Generator().manual_seed(N)
+        a = torch.randint(-128, 128, (M, 208), generator=g, dtype=torch.int8)
+        b = torch.randint(-128, 128, (N, 208), generator=g, dtype=torch.int8)
+        c = matmul.int8Matmul(a.to(dev()), b.to(dev()))
+        assert torch.equal(c.cpu().long(), a.long() @ b.long().t())
+    finally:
+        case.module.out_buffer = None
+        _lib.set_tile_n(0)
+        _lib.set_cta_pair(0)
+    assert rel_rms_err(want.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+    assert_device_clean()
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
