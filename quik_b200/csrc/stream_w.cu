@@ -44,6 +44,7 @@ constexpr int SW_A_COLS = 64;                      // 256 int8 codes per row = 6
 constexpr int SW_MAX_STAGES = 10;
 constexpr int SW_AUX_BYTES = 2048;                 // barriers, then the token scales
 constexpr int SW_SMEM_SM = 227 * 1024;
+constexpr int SW_BLOCKS_SAVED = 8;                 // that a second launch has to save (launch_stream_w)
 
 // Sizes that depend on the number of tokens (the MMA's N, a multiple of 16): shared-memory ring and tensor-memory plan.
 // Up to 64 tokens two CTAs may share an SM (256 tensor-memory columns and at most 113 KB each; the rule is in launch_stream_w),
@@ -517,6 +518,62 @@ int launch_t(const CUtensorMap &tw, const CUtensorMap &tx, const CUtensorMap &tf
   return check_launch("stream_w_kernel");
 }
 
+// Rows [first, first + count) of the layer (first a multiple of SW_ROWS), in one launch.
+int launch_rows(const void *q, const void *w, int bits, int M, int first, int count, int K_int, const Epilogue &ep, int per_sm, int splits,
+                cudaStream_t st) {
+  const int ntok = (M + 15) & ~15;                                                // the MMA's N
+  StreamParams p{};
+  p.M = M;
+  p.N = count;
+  const size_t at = (size_t)first;
+  const int w_row_bytes = bits == 4 ? K_int / 2 : K_int;
+  p.nk = (w_row_bytes + 127) / 128;
+  p.nf = ep.fp_a != nullptr && ep.F > 0 ? (ep.F + 63) / 64 : 0;
+  const int slabs = (count + SW_ROWS - 1) / SW_ROWS;
+  p.splits = splits;
+  const StreamPlan plan = plan_stream(bits, ntok, per_sm);
+  p.ntok = ntok;
+  p.stages = plan.stages;
+  p.stage_bytes = plan.stage_bytes;
+  p.x_bytes = plan.x_bytes;
+  p.a_slots = plan.a_slots;
+  p.d_int = plan.d_int;
+  p.d_fp = plan.d_fp;
+  p.tmem_cols = plan.tmem_cols;
+  p.idesc_int = make_idesc(2, 1, SW_ROWS, ntok);
+  p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, SW_ROWS, ntok);
+  p.meta = ep.meta;
+  auto row = [&](const void *v, size_t bytes) { return v ? static_cast<const unsigned char *>(v) + at * bytes : nullptr; };
+  p.scale_col = row(ep.scale_col, 2);
+  p.w_reduced = row(ep.w_reduced, 2);
+  p.bias = row(ep.bias, 2);
+  p.out = static_cast<unsigned char *>(ep.out) + at * 2;
+  p.ldo = ep.ldo;
+  p.shift_value = ep.shift_value;
+  p.dbg = get_debug_counters();
+  p.status = device_status_word();
+  if (p.status == nullptr) return QUIK_ERR_CUDA;
+
+  CUtensorMap tw, tx, tfw, tfx;
+  int rc;
+  if ((rc = make_tmap(&tw, row(w, w_row_bytes), CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, count, w_row_bytes, SW_ROWS)) != QUIK_OK) return rc;
+  if ((rc = make_tmap(&tx, q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K_int, ntok)) != QUIK_OK) return rc;
+  if (p.nf > 0) {
+    const CUtensorMapDataType fdt = ep.dtype == QUIK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    if ((rc = make_tmap(&tfw, row(ep.fp_b, 2 * (size_t)ep.F), fdt, 2, count, ep.F, SW_ROWS)) != QUIK_OK) return rc;
+    if ((rc = make_tmap(&tfx, ep.fp_a, fdt, 2, M, ep.F, ntok)) != QUIK_OK) return rc;
+  } else {
+    tfw = tw;
+    tfx = tx;
+  }
+  if (ep.dtype == QUIK_BF16)
+    return bits == 4 ? launch_t<__nv_bfloat16, 4>(tw, tx, tfw, tfx, p, slabs, plan.smem, st)
+                     : launch_t<__nv_bfloat16, 8>(tw, tx, tfw, tfx, p, slabs, plan.smem, st);
+  return bits == 4 ? launch_t<__half, 4>(tw, tx, tfw, tfx, p, slabs, plan.smem, st)
+                   : launch_t<__half, 8>(tw, tx, tfw, tfx, p, slabs, plan.smem, st);
+}
+
+
 }  // namespace
 
 // q: [M, K_int] int8 codes (one per byte); w: [N, K_int/2] packed int4 (bits == 4) or [N, K_int] int8.
@@ -530,24 +587,17 @@ int launch_stream_w(const void *q, const void *w, int bits, int M, int N, int K_
   if (has_fp && (ep.F % 8 != 0 || !aligned16(ep.fp_a) || !aligned16(ep.fp_b))) return QUIK_ERR_ALIGN;
   if (ep.meta == nullptr || ep.w_reduced == nullptr || ep.y != nullptr) return QUIK_ERR_UNSUPPORTED;
 
-  const int ntok = (M + 15) & ~15;                                                // the MMA's N
-  StreamParams p{};
-  p.M = M;
-  p.N = N;
-  const int w_row_bytes = bits == 4 ? K_int / 2 : K_int;
-  p.nk = (w_row_bytes + 127) / 128;
-  p.nf = has_fp ? (ep.F + 63) / 64 : 0;
+  const int ntok = (M + 15) & ~15, sms = num_sms();
+  const int nf = has_fp ? (ep.F + 63) / 64 : 0, total = ((bits == 4 ? K_int / 2 : K_int) + 127) / 128 + nf;
   const int slabs = (N + SW_ROWS - 1) / SW_ROWS;
   // Split K over a cluster while all CTAs still run at once, every CTA keeps at least two k-blocks and the outlier
   // blocks all fall to the first CTA.
-  const int total = p.nk + p.nf;
-  auto choose_splits = [&](int ctas_per_sm) {
+  auto choose_splits = [&](int ctas_per_sm, int of_slabs) {
     int s = 1;
-    while (s < 8 && total / (s * 2) >= (p.nf > 2 ? p.nf : 2) && slabs <= resident_clusters(ctas_per_sm, s * 2)) s *= 2;
+    while (s < 8 && total / (s * 2) >= (nf > 2 ? nf : 2) && of_slabs <= resident_clusters(ctas_per_sm, s * 2)) s *= 2;
     return s;
   };
-  int per_sm = 1;
-  p.splits = choose_splits(1);
+  int per_sm = 1, splits = choose_splits(1, slabs);
   if (ntok <= 64) {
     // Two CTAs per SM, each with half of the ring, or one?  More slabs than SMs: two (172 slabs of 4096 int4 columns, 48 tokens:
     // 19.3 against 27.6 us).  Otherwise two only where they allow a deeper split of a long K: each CTA starts and
@@ -556,51 +606,29 @@ int launch_stream_w(const void *q, const void *w, int bits, int M, int N, int K_
     // warps busier (40 slabs of 11008 columns 16.8 / 18.1 against 18.3 / 18.8 us, 120 slabs 26.1 / 27.4 against 29.9 /
     // 30.2); int8 blocks need no widening and gain only while most CTAs still have an SM for themselves (40 and 96
     // slabs of 11008 columns, 33 tokens: 17.1 against 19.7 and 29.6 against 31.3 us, 120 slabs: 33.3 against 32.1).
-    const int s2 = choose_splits(2), sms = num_sms();
-    if (slabs > sms || (s2 > p.splits && total / p.splits > 20 && (bits == 4 || 5 * slabs * s2 <= 7 * sms))) {
+    const int s2 = choose_splits(2, slabs);
+    if (slabs > sms || (s2 > splits && total / splits > 20 && (bits == 4 || 5 * slabs * s2 <= 7 * sms))) {
       per_sm = 2;
-      p.splits = s2;
+      splits = s2;
     }
   }
-  const StreamPlan plan = plan_stream(bits, ntok, per_sm);
-  p.ntok = ntok;
-  p.stages = plan.stages;
-  p.stage_bytes = plan.stage_bytes;
-  p.x_bytes = plan.x_bytes;
-  p.a_slots = plan.a_slots;
-  p.d_int = plan.d_int;
-  p.d_fp = plan.d_fp;
-  p.tmem_cols = plan.tmem_cols;
-  p.idesc_int = make_idesc(2, 1, SW_ROWS, ntok);
-  p.idesc_fp = make_idesc(1, ep.dtype == QUIK_BF16 ? 1 : 0, SW_ROWS, ntok);
-  p.meta = ep.meta;
-  p.scale_col = ep.scale_col;
-  p.w_reduced = ep.w_reduced;
-  p.bias = ep.bias;
-  p.out = ep.out;
-  p.ldo = ep.ldo > 0 ? ep.ldo : N;
-  p.shift_value = ep.shift_value;
-  p.dbg = get_debug_counters();
-  p.status = device_status_word();
-  if (p.status == nullptr) return QUIK_ERR_CUDA;
-
-  CUtensorMap tw, tx, tfw, tfx;
-  int rc;
-  if ((rc = make_tmap(&tw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, w_row_bytes, SW_ROWS)) != QUIK_OK) return rc;
-  if ((rc = make_tmap(&tx, q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K_int, ntok)) != QUIK_OK) return rc;
-  if (has_fp) {
-    const CUtensorMapDataType fdt = ep.dtype == QUIK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    if ((rc = make_tmap(&tfw, ep.fp_b, fdt, 2, N, ep.F, SW_ROWS)) != QUIK_OK) return rc;
-    if ((rc = make_tmap(&tfx, ep.fp_a, fdt, 2, M, ep.F, ntok)) != QUIK_OK) return rc;
-  } else {
-    tfw = tw;
-    tfx = tx;
+  Epilogue e = ep;
+  if (e.ldo <= 0) e.ldo = N;
+  // More slabs than run at once: the ones beyond the last full wave go to a launch of their own that splits K (its setup and first
+  // prefetch overlap the end of the first launch), where that takes at least eight blocks out of the chain.  A block is 0.55 us and
+  // the second launch costs about 4: 172 slabs of 4096 int4 columns, 96 tokens, 14 blocks saved: 30.5 -> 26.9 us; 197 slabs of 22752,
+  // 74 tokens, 46 saved: 112 -> 91; 217 slabs of 1536 columns, 4 saved: 18.2 -> 19.8.
+  const int wave = sms * per_sm, beyond = slabs > wave ? slabs % wave : 0;
+  if (beyond > 0) {
+    const int s = choose_splits(per_sm, beyond);
+    if (total - (total + s - 1) / s >= SW_BLOCKS_SAVED) {
+      const int first = (slabs - beyond) * SW_ROWS;
+      const int rc = launch_rows(q, w, bits, M, 0, first, K_int, e, per_sm, 1, st);
+      if (rc != QUIK_OK) return rc;
+      return launch_rows(q, w, bits, M, first, N - first, K_int, e, per_sm, s, st);
+    }
   }
-  if (ep.dtype == QUIK_BF16)
-    return bits == 4 ? launch_t<__nv_bfloat16, 4>(tw, tx, tfw, tfx, p, slabs, plan.smem, st)
-                     : launch_t<__nv_bfloat16, 8>(tw, tx, tfw, tfx, p, slabs, plan.smem, st);
-  return bits == 4 ? launch_t<__half, 4>(tw, tx, tfw, tfx, p, slabs, plan.smem, st)
-                   : launch_t<__half, 8>(tw, tx, tfw, tfx, p, slabs, plan.smem, st);
+  return launch_rows(q, w, bits, M, 0, N, K_int, e, per_sm, splits, st);
 }
 
 }  // namespace quik

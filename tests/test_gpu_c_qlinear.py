@@ -599,3 +599,22 @@ def test_streaming_engine_splits_and_short_sums(slabs, K, F, bits):
         assert torch.equal(case.module(case.x[:M].contiguous())[0], out)
         assert rel_rms_err(out.cpu(), ref[:M].cpu()) < 5e-3
     assert_device_clean()
+
+
+@pytest.mark.parametrize("M,slabs,K,F", [(80, 149, 2560, 64), (128, 149, 2560, 64), (65, 222, 5152, 0), (97, 300, 2560, 64),
+                                         (33, 297, 2560, 64), (17, 444, 5152, 0)])
+def test_streaming_engine_beyond_a_full_wave(M, slabs, K, F):
+    """More slabs of 128 rows than run at once: the last ones are a launch of their own that splits K.  One slab beyond a wave up to
+    half a wave, two CTAs per SM up to 64 tokens, with the last slab ragged, into a window of a wider matrix."""
+    N = 128 * slabs - 5
+    case = make_layer("t", M, K, N, 4, F=F, seed=M, device=dev(), clip=False)
+    out = case.module(case.x.unsqueeze(0))[0]
+    assert rel_rms_err(out.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+    slab = torch.full((M, N + 7), -1234.0, dtype=torch.float16, device=dev())
+    case.module.out_buffer = slab[:, 3:3 + N]
+    case.module(case.x.unsqueeze(0))
+    case.module.out_buffer = None
+    assert torch.equal(slab[:, 3:3 + N], out)
+    slab[:, 3:3 + N] = -1234.0
+    assert bool((slab == -1234.0).all())
+    assert_device_clean()
