@@ -93,7 +93,8 @@ def host():
             raise RuntimeError(f"quik_b200._host is missing or does not load ({e}): build it with "
                                "`python -m quik_b200.build`") from e
         mod.init(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
-            "quik_layer_quantize", "quik_mixed_linear_ld", "quik_strerror", "quik_last_cuda_error", "quik_config_get")))
+            "quik_layer_quantize", "quik_mixed_linear_ld", "quik_strerror", "quik_last_cuda_error", "quik_config_get",
+            "quik_rotary_inplace")))
         _host = mod
     return _host
 

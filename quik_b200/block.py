@@ -14,7 +14,7 @@ import math
 import torch
 import torch.nn.functional as F
 
-from ._lib import check, dtype_code, load, on_device, ptr, stream_of
+from ._lib import host
 from .qlinear import MixedQLinear, SharedQuantizedInput
 from .workloads import rtn_clip_scales
 
@@ -108,9 +108,7 @@ class QuikLlamaBlock(torch.nn.Module):
         """The same rotation in one pass, in place on the q and k projections [s, heads*head_dim] (they are this
         block's own fresh outputs); bit-identical to ``_rope``."""
         c, sn = self._angles(s, q.device, q.dtype)
-        with on_device(q):
-            check(load().quik_rotary_inplace(ptr(q), ptr(k), ptr(c), ptr(sn), dtype_code(q.dtype), s, self.heads,
-                                             self.kv_heads, self.head_dim, stream_of(q)), "rotary")
+        host().rotary(q, k, c, sn, s, self.heads, self.kv_heads, self.head_dim)
 
     _fused_groups = None
 
@@ -160,7 +158,8 @@ class QuikLlamaBlock(torch.nn.Module):
             q, k = self._rope(q, k)
         if self.kv_heads != self.heads:
             rep = self.heads // self.kv_heads
-            k, v = k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)
+            # every key / value head once per query head of its group (repeat_interleave, in half its time on the host)
+            k, v = (t.unsqueeze(2).expand(b, self.kv_heads, rep, s, self.head_dim).reshape(b, self.heads, s, self.head_dim) for t in (k, v))
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True, scale=1.0 / math.sqrt(self.head_dim))
         a = a.transpose(1, 2).reshape(b, s, self.hidden)
         x = x + lin("o_proj", a)

@@ -14,6 +14,7 @@
 
 #include <cstring>
 #include <string>
+#include <utility>
 
 #include "../../include/quik_b200.h"
 
@@ -25,7 +26,14 @@ struct Abi {
   decltype(&quik_config_get) config_get = nullptr;
   decltype(&quik_strerror) strerror_ = nullptr;
   decltype(&quik_last_cuda_error) last_cuda_error = nullptr;
+  decltype(&quik_rotary_inplace) rotary = nullptr;
 } abi;
+
+// attribute and buffer names of the module (interned once)
+struct Names {
+  PyObject *buffers, *int_weight, *int_indices, *fp_indices, *weights_scales, *reduced_w, *fp_weight, *bias, *int_features_num,
+      *out_features, *fp_features_num, *bits;
+} names;
 
 void check(int status, const char *what) {
   if (status == QUIK_OK) return;
@@ -182,9 +190,9 @@ at::Tensor launch_linear(const at::Tensor &x, const Codes &c, bool q_packed, con
 
 PyObject *py_init(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 5);
-  void *p[5];
-  for (int i = 0; i < 5; ++i) {
+  expect(n, 6);
+  void *p[6];
+  for (int i = 0; i < 6; ++i) {
     p[i] = PyLong_AsVoidPtr(a[i]);
     if (p[i] == nullptr) throw std::runtime_error("quik_b200._host.init: a library function is missing");
   }
@@ -193,6 +201,14 @@ PyObject *py_init(PyObject *, PyObject *const *a, Py_ssize_t n) {
   abi.strerror_ = reinterpret_cast<decltype(abi.strerror_)>(p[2]);
   abi.last_cuda_error = reinterpret_cast<decltype(abi.last_cuda_error)>(p[3]);
   abi.config_get = reinterpret_cast<decltype(abi.config_get)>(p[4]);
+  abi.rotary = reinterpret_cast<decltype(abi.rotary)>(p[5]);
+  const std::pair<PyObject **, const char *> all[] = {
+      {&names.buffers, "_buffers"}, {&names.int_weight, "int_weight"}, {&names.int_indices, "int_indices"},
+      {&names.fp_indices, "fp_indices"}, {&names.weights_scales, "weights_scales"}, {&names.reduced_w, "reduced_w"},
+      {&names.fp_weight, "fp_weight"}, {&names.bias, "bias"}, {&names.int_features_num, "int_features_num"},
+      {&names.out_features, "out_features"}, {&names.fp_features_num, "fp_features_num"}, {&names.bits, "bits"}};
+  for (auto &a : all)
+    if ((*a.first = PyUnicode_InternFromString(a.second)) == nullptr) return nullptr;
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -259,11 +275,29 @@ PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids, seen):
-// quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  The ids are settled (see
-// quik_layer_quantize).  w: the weights in storage
-// format; w8: 4-bit weights one code per byte; None is returned, and nothing launched, where the settings ask for them and
-// they were not given.
+// Quantizer and fused launch, the quantized input in a workspace that lives as long as the call.  The ids are settled (see
+// quik_layer_quantize).  w: the weights in storage format; w8: 4-bit weights one code per byte; an undefined tensor is returned,
+// and nothing launched, where the settings ask for them and they were not given.
+at::Tensor run_layer(const at::Tensor &given, const at::Tensor &out, const Layer &l, const at::Tensor &w, const at::Tensor &w8,
+                     const at::Tensor &ids, const at::Tensor &fp_ids, char *seen) {
+  settle_weights(given, w, l.fp_w, seen);
+  py::gil_scoped_release nogil;
+  const at::Tensor x = given.dim() == 3 ? given.select(0, 0) : given;      // the first matrix of a batch, as ever
+  const char *op = check_quantize(0, x, at::Tensor(), ids, fp_ids, l.bits);
+  const int64_t m = x.size(0);
+  const Layouts lay = operand_layouts(l.bits, l.k_int, m);
+  const bool needs_w8 = l.bits == 4 && !lay.w_packed;
+  if (needs_w8 && !w8.defined()) return at::Tensor();
+  const c10::cuda::OptionalCUDAGuard guard(x.device());
+  const int64_t b_q = align256(m * ids.numel()), b_meta = align256(m * 4);
+  const at::Tensor ws = at::empty({b_q + b_meta + m * fp_ids.numel() * 2}, x.options().dtype(at::kByte));
+  unsigned char *base = static_cast<unsigned char *>(ptr(ws));
+  const Codes c{base, base + b_q, base + b_q + b_meta};
+  launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !lay.q_packed, true, c);
+  return launch_linear(x, c, lay.q_packed, ptr(needs_w8 ? w8 : w), lay.w_packed, l, out);
+}
+
+// (x, out | None, scales, reduced, fp_w | None, bias | None, k_int, n, f, bits, w, w8 | None, int_ids, fp_ids, seen): run_layer
 PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 15);
@@ -271,27 +305,191 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
                    ids = tensor_arg(a[12]), fp_ids = tensor_arg(a[13]);
   Layer l;
   if (!layer_args(a + 2, &l)) return nullptr;
-  settle_weights(given, w, l.fp_w, seen_arg(a[14]));
+  at::Tensor result = run_layer(given, out, l, w, w8, ids, fp_ids, seen_arg(a[14]));
+  if (!result.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// ---- calls by module and plan -----------------------------------------------------------------------------------------------
+// A plan is the tuple (int_ids, fp_ids, w8 | None, key) of a module's derived operands; the key says which buffers, by address and
+// version, they were derived from.  The module's buffers and sizes are read on every call; where they are not those of the
+// plan, or something is missing, a call returns None having launched nothing, and the module's own path derives them anew.  Reading
+// attributes, comparing keys and collecting arguments in Python was 6 us of the 15 us of a call for one token.
+constexpr Py_ssize_t kKeyBytes = 6 * sizeof(int64_t);
+bool plan_key(const at::Tensor &int_ids, const at::Tensor &fp_ids, const at::Tensor &w, int64_t *key) {
+  const at::Tensor *const t[3] = {&int_ids, &fp_ids, &w};
+  for (int i = 0; i < 3; ++i) {
+    if (t[i]->is_inference()) return false;      // counts no versions
+    key[2 * i] = (int64_t)(intptr_t)ptr(*t[i]);
+    key[2 * i + 1] = (int64_t)t[i]->_version();
+  }
+  return true;
+}
+struct Planned {
+  Layer l;
+  at::Tensor w, w8, ids, fp_ids;
+};
+// 1: read, 0: not the plan's module any more, -1: Python error
+int read_planned(PyObject *module, PyObject *plan, Planned *r) {
+  if (!PyTuple_Check(plan) || PyTuple_GET_SIZE(plan) != 4 || !PyBytes_Check(PyTuple_GET_ITEM(plan, 3)) ||
+      PyBytes_GET_SIZE(PyTuple_GET_ITEM(plan, 3)) != kKeyBytes)
+    return 0;
+  PyObject *buffers = PyObject_GetAttr(module, names.buffers);
+  if (!buffers) return -1;
+  bool have = PyDict_Check(buffers);
+  auto buffer = [&](PyObject *name, at::Tensor *t, bool may_be_none) {
+    PyObject *o = have ? PyDict_GetItemWithError(buffers, name) : nullptr;
+    if (o && THPVariable_Check(o)) *t = THPVariable_Unpack(o);
+    else if (!(o == Py_None && may_be_none)) have = false;
+  };
+  auto size = [&](PyObject *name) -> int64_t {
+    if (!have) return 0;
+    PyObject *o = PyObject_GetAttr(module, name);
+    const int64_t v = o ? PyLong_AsLongLong(o) : -1;
+    Py_XDECREF(o);
+    if (PyErr_Occurred()) have = false;
+    return v;
+  };
+  at::Tensor ids64, fp64;
+  buffer(names.int_weight, &r->w, false);
+  buffer(names.int_indices, &ids64, false);
+  buffer(names.fp_indices, &fp64, false);
+  buffer(names.weights_scales, &r->l.scales, false);
+  buffer(names.reduced_w, &r->l.reduced, false);
+  buffer(names.bias, &r->l.bias, true);
+  r->l.k_int = size(names.int_features_num);
+  r->l.n = size(names.out_features);
+  r->l.f = size(names.fp_features_num);
+  r->l.bits = (int)size(names.bits);
+  if (have && r->l.f > 0) buffer(names.fp_weight, &r->l.fp_w, false);
+  Py_DECREF(buffers);
+  if (PyErr_Occurred()) return -1;
+  int64_t key[6];
+  if (!have || r->l.k_int <= 0 || !plan_key(ids64, fp64, r->w, key) ||
+      std::memcmp(key, PyBytes_AS_STRING(PyTuple_GET_ITEM(plan, 3)), kKeyBytes) != 0)
+    return 0;
+  r->ids = tensor_arg(PyTuple_GET_ITEM(plan, 0));
+  r->fp_ids = tensor_arg(PyTuple_GET_ITEM(plan, 1));
+  r->w8 = optional_arg(PyTuple_GET_ITEM(plan, 2));
+  return 1;
+}
+// the device of x becomes the current one, as the module's forward has it
+void make_current(const at::Tensor &x) {
+  if (c10::cuda::current_device() != x.device().index()) c10::cuda::set_device(x.device().index());
+}
+
+// (int_indices, fp_indices, int_weight) -> key, or None where they count no versions
+PyObject *py_plan_key(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 3);
+  int64_t key[6];
+  if (!plan_key(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), key)) Py_RETURN_NONE;
+  return PyBytes_FromStringAndSize(reinterpret_cast<const char *>(key), kKeyBytes);
+  END_HANDLE_TH_ERRORS
+}
+
+// (module, plan, seen, x) -> output | None
+PyObject *py_forward(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 4);
+  Planned r;
+  const int ok = read_planned(a[0], a[1], &r);
+  if (ok < 0) return nullptr;
+  if (ok == 0 || !THPVariable_Check(a[3])) Py_RETURN_NONE;
+  const at::Tensor x = tensor_arg(a[3]);
+  if (!x.is_cuda()) Py_RETURN_NONE;
+  make_current(x);
+  at::Tensor result = run_layer(x, at::Tensor(), r.l, r.w, r.w8, r.ids, r.fp_ids, seen_arg(a[2]));
+  if (!result.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// (module, plan, producer, x, aux | None, eps) -> (codes, meta, fp_x, one code per byte) | None; x [1, M, K] or [M, K]
+PyObject *py_quantize_for(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 6);
+  Planned r;
+  const int ok = read_planned(a[0], a[1], &r);
+  if (ok < 0) return nullptr;
+  const int producer = (int)PyLong_AsLong(a[2]);
+  const double eps = PyFloat_AsDouble(a[5]);
+  if (PyErr_Occurred()) return nullptr;
+  if (ok == 0 || producer < 0 || producer > 2 || !THPVariable_Check(a[3])) Py_RETURN_NONE;
+  at::Tensor x = tensor_arg(a[3]), aux = optional_arg(a[4]);
+  if (!x.is_cuda()) Py_RETURN_NONE;
+  if (producer == 0) make_current(x);
+  if (producer && !aux.defined()) throw std::runtime_error("expected a tensor");
+  at::Tensor q, meta, fp_x;
+  bool wide;
+  {
+    py::gil_scoped_release nogil;
+    if (x.dim() == 3) x = x.select(0, 0);
+    if (producer) x = x.contiguous();
+    if (producer == 2) aux = (aux.dim() == 3 ? aux.select(0, 0) : aux).contiguous();
+    const char *op = check_quantize(producer, x, aux, r.ids, r.fp_ids, r.l.bits);
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    const int64_t rows = x.size(0), num_int = r.ids.numel();
+    wide = !operand_layouts(r.l.bits, r.l.k_int, rows).q_packed;
+    q = r.l.bits == 4 && !wide ? at::empty({rows, num_int / 2}, x.options().dtype(at::kByte))
+                               : at::empty({rows, num_int}, x.options().dtype(at::kChar));
+    meta = at::empty({2 * rows}, x.options());
+    fp_x = at::empty({rows, r.fp_ids.numel()}, x.options());
+    launch_quantize(op, producer, x, aux, eps, r.ids, r.fp_ids, r.l.bits, wide, true, Codes{ptr(q), ptr(meta), ptr(fp_x)});
+  }
+  PyObject *t = PyTuple_New(4);
+  if (!t) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(q)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(meta)));
+  PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(std::move(fp_x)));
+  PyTuple_SET_ITEM(t, 3, PyBool_FromLong(wide));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
+// (module, plan, seen, x, codes, meta, fp_x, one code per byte) -> output | None: the fused launch on a quantized input
+PyObject *py_forward_quantized(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 8);
+  Planned r;
+  const int ok = read_planned(a[0], a[1], &r);
+  if (ok < 0) return nullptr;
+  if (ok == 0) Py_RETURN_NONE;
+  for (int i = 3; i < 7; ++i)
+    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
+  const bool wide = PyObject_IsTrue(a[7]) == 1;
+  const at::Tensor given = tensor_arg(a[3]), q = tensor_arg(a[4]), meta = tensor_arg(a[5]), fp_x = tensor_arg(a[6]);
+  if (!given.is_cuda() || given.dim() < 1) Py_RETURN_NONE;
+  const at::Tensor x = given.dim() == 3 ? given.select(0, 0) : given;
+  const Layouts lay = operand_layouts(r.l.bits, r.l.k_int, x.size(0));
+  const bool needs_w8 = r.l.bits == 4 && !lay.w_packed;
+  if ((r.l.bits == 4 && wide == lay.q_packed) || (needs_w8 && !r.w8.defined())) Py_RETURN_NONE;
+  make_current(x);
+  settle_weights(x, needs_w8 ? r.w8 : r.w, r.l.fp_w, seen_arg(a[2]));
   at::Tensor result;
   {
     py::gil_scoped_release nogil;
-    const at::Tensor x = given.dim() == 3 ? given.select(0, 0) : given;      // the first matrix of a batch, as ever
-    const char *op = check_quantize(0, x, at::Tensor(), ids, fp_ids, l.bits);
-    const int64_t m = x.size(0);
-    const Layouts lay = operand_layouts(l.bits, l.k_int, m);
-    const bool needs_w8 = l.bits == 4 && !lay.w_packed;
-    if (!needs_w8 || w8.defined()) {
-      const c10::cuda::OptionalCUDAGuard guard(x.device());
-      const int64_t b_q = align256(m * ids.numel()), b_meta = align256(m * 4);
-      const at::Tensor ws = at::empty({b_q + b_meta + m * fp_ids.numel() * 2}, x.options().dtype(at::kByte));
-      unsigned char *base = static_cast<unsigned char *>(ptr(ws));
-      const Codes c{base, base + b_q, base + b_q + b_meta};
-      launch_quantize(op, 0, x, at::Tensor(), 0.0, ids, fp_ids, l.bits, !lay.q_packed, true, c);
-      result = launch_linear(x, c, lay.q_packed, ptr(needs_w8 ? w8 : w), lay.w_packed, l, out);
-    }
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    result = launch_linear(x, Codes{ptr(q), ptr(meta), ptr(fp_x)}, lay.q_packed, ptr(needs_w8 ? r.w8 : r.w), lay.w_packed, r.l, at::Tensor());
   }
-  if (!result.defined()) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// (q, k, cos, sin, tokens, q_heads, k_heads, head_dim): rotary embedding in place
+PyObject *py_rotary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 8);
+  const at::Tensor q = tensor_arg(a[0]), k = tensor_arg(a[1]), c = tensor_arg(a[2]), s = tensor_arg(a[3]);
+  int v[4];
+  for (int i = 0; i < 4; ++i) v[i] = (int)PyLong_AsLong(a[4 + i]);
+  if (PyErr_Occurred()) return nullptr;
+  const c10::cuda::OptionalCUDAGuard guard(q.device());
+  check(abi.rotary(ptr(q), ptr(k), ptr(c), ptr(s), dtype_code(q.scalar_type()), v[0], v[1], v[2], v[3],
+                   c10::cuda::getCurrentCUDAStream(q.device().index()).stream()),
+        "rotary");
+  Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -328,6 +526,13 @@ PyMethodDef methods[] = {
      "operand layouts for a token count"},
     {"weights_changed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_weights_changed)), METH_FASTCALL,
      "weights against a record"},
+    {"plan_key", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_plan_key)), METH_FASTCALL, "key of a plan"},
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_forward)), METH_FASTCALL, "a module's forward by its plan"},
+    {"quantize_for", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize_for)), METH_FASTCALL,
+     "activation quantizer for a module by its plan"},
+    {"forward_quantized", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_forward_quantized)), METH_FASTCALL,
+     "fused launch of a module by its plan"},
+    {"rotary", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_rotary)), METH_FASTCALL, "rotary embedding in place"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of the layer", -1, methods};
 

@@ -75,6 +75,8 @@ class MixedQLinear(torch.nn.Module):
     out_buffer = None
     # weights of the last call for few tokens (see _host.weights_changed); every layer has its own
     _seen = bytearray(32)
+    # derived operands for the native host path (see _make_plan); every layer has its own
+    _plan = None
 
     def __init__(self, in_features, out_features, shared_input=None,
                  fp_features_num=0, symm=False, bits=4, dtype=torch.float16):
@@ -170,6 +172,34 @@ class MixedQLinear(torch.nn.Module):
         i16, f16 = self._idx16()
         return _lib.host().quantize(producer, x, aux, eps, i16, f16, self.bits, wide, True)
 
+    def _make_plan(self):
+        """What the native host path needs of this layer beside its buffers: 16-bit column ids, weight codes one per byte where
+        they have been made, and the key of the buffers that these come from.  It reads the buffers itself on every call and
+        declines where the key is another: the layer's own path then runs, and ends here again."""
+        self._plan = None
+        b = self._buffers
+        w, sources = b.get("int_weight"), (b.get("int_indices"), b.get("fp_indices"), b.get("int_weight"))
+        if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None for t in sources):
+            return
+        key = _lib.host().plan_key(*sources)
+        if key is None:
+            return
+        i16, f16 = self._idx16()
+        w8 = self._cache.get("w8")
+        current = w8 is not None and w8[0] == (w.data_ptr(), w._version, w.get_device())
+        self._plan = (i16, f16, w8[1] if current else None, key)
+
+    def _quantize_by_plan(self, producer, x, aux, eps):
+        """Fills the group's shared input from the native host path; False where that declines."""
+        plan, shared_input = self._plan, self.shared_input
+        if plan is None or shared_input is None:
+            return False
+        filled = _lib.host().quantize_for(self, plan, producer, x, aux, eps)
+        if filled is None:
+            return False
+        shared_input.qint_x, shared_input.meta, shared_input.fp_x, shared_input.wide = filled
+        return True
+
     def _fill_shared(self, quantized, wide):
         shared_input = self.shared_input
         if shared_input is None:
@@ -181,12 +211,16 @@ class MixedQLinear(torch.nn.Module):
         """Quantizes RMSNorm(x) * norm_weight straight into this layer's shared input (one pass over x, the normalised
         activations never go to HBM).  The following forward calls of the group's members find the codes and skip their
         own quantizer; pass them any tensor of x's shape, dtype and device (it is not read)."""
+        if self._quantize_by_plan(1, x, norm_weight, eps):
+            return
         x2 = x[0] if x.dim() == 3 else x
         q_packed, _ = self._operand_layouts(x2.shape[0])
         self._fill_shared(self._quantize(1, x2.contiguous(), norm_weight, eps, not q_packed), not q_packed)
 
     def quantize_silu_mul(self, gate, up):
         """Quantizes SiLU(gate) * up straight into this layer's shared input (see :meth:`quantize_rmsnorm`)."""
+        if self._quantize_by_plan(2, gate, up, 0.0):
+            return
         g2 = gate[0] if gate.dim() == 3 else gate
         u2 = up[0] if up.dim() == 3 else up
         q_packed, _ = self._operand_layouts(g2.shape[0])
@@ -194,6 +228,22 @@ class MixedQLinear(torch.nn.Module):
 
     # ------------------------------------------------------------------ forward
     def forward(self, x):
+        plan = self._plan
+        if plan is not None and self.fused and not self.symmetric and MixedQLinear.launch_hook is None and self.out_buffer is None:
+            shared_input = self.shared_input
+            if shared_input is None:
+                out = _lib.host().forward(self, plan, self._seen, x)
+                if out is not None:
+                    return out
+            elif shared_input.qint_x is not None or self._quantize_by_plan(0, x, None, 0.0):
+                out = _lib.host().forward_quantized(self, plan, self._seen, x, shared_input.qint_x, shared_input.meta,
+                                                    shared_input.fp_x, shared_input.wide)
+                if out is not None:
+                    shared_input.finish()
+                    return out
+        return self._forward_checked(x)
+
+    def _forward_checked(self, x):
         if self.int_features_num <= 0:
             return torch.nn.functional.linear(x, self.fp_weight, self.bias)
         if torch.cuda.current_device() != x.device.index:
@@ -229,6 +279,7 @@ class MixedQLinear(torch.nn.Module):
         if hook is not None:
             hook(self, False)
         shared_input.finish()
+        self._make_plan()
         return out
 
     def _out_buffer_for(self, x, M):
@@ -259,6 +310,7 @@ class MixedQLinear(torch.nn.Module):
         res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids, self._seen)
         if res is None:          # a setting that another thread has changed since asks for weight codes one per byte
             res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids, self._seen)
+        self._make_plan()
         return res
 
     def _forward_unfused(self, x, shared_input):

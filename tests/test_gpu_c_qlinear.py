@@ -1,4 +1,6 @@
 """GPU parity: MixedQLinear.forward (fused, unfused, shared input, small-M, bf16) vs the CPU oracle."""
+import copy
+
 import pytest
 import torch
 
@@ -617,4 +619,41 @@ def test_streaming_engine_beyond_a_full_wave(M, slabs, K, F):
     assert torch.equal(slab[:, 3:3 + N], out)
     slab[:, 3:3 + N] = -1234.0
     assert bool((slab == -1234.0).all())
+    assert_device_clean()
+
+
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("M,bits,F", [(5, 4, 64), (40, 4, 64), (200, 4, 64), (200, 8, 0)])
+def test_native_path_follows_the_buffers(M, bits, F, shared):
+    """The native host path works from operands derived from the layer's buffers: after each change of a buffer, in place or by
+    another tensor, a call gives the bits of the path that derives them anew, and so does a copy of the layer."""
+    case = make_layer("t", M, 1024 + F, 264, bits, F=F, seed=M, device=dev(), clip=False)
+    layer, x = case.module, case.x.unsqueeze(0)
+    layer.shared_input = SharedQuantizedInput(1) if shared else None
+
+    def check():
+        want = layer._forward_checked(x)
+        assert layer._plan is not None
+        got = layer(x)
+        assert torch.equal(got, want)
+        return got
+
+    first = check()
+    assert torch.equal(copy.deepcopy(layer)(x), first)
+    with torch.no_grad():
+        ids = layer.int_indices.clone()
+        layer.int_indices[0], layer.int_indices[1] = ids[1], ids[0]                    # in place
+        got = layer(x)
+        assert not torch.equal(got, first) and torch.equal(got, layer._forward_checked(x))
+        layer.int_indices = ids                                                       # another tensor
+        assert torch.equal(layer(x), first)
+        check()
+        layer.int_weight.copy_(layer.int_weight.flip(0))
+        got = layer(x)
+        assert torch.equal(got, layer._forward_checked(x)) and not torch.equal(got, first)
+        layer.weights_scales = layer.weights_scales * 2
+        layer.bias = None
+        check()
+    with pytest.raises(Exception):
+        layer(x.cpu())
     assert_device_clean()
