@@ -179,6 +179,18 @@ __device__ __forceinline__ float warp_min(float v) {
   return v;
 }
 
+// max / min over the warp, NaN left out
+__device__ __forceinline__ float redux_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float redux_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // ---- launchers implemented in the individual .cu files ---------------------------------------
 int launch_asym_quantize(const void *src, int dtype, int rows, int cols, const int64_t *int_idx, int num_int,
                          const int64_t *fp_idx, int num_fp, int bits, void *dst, void *meta, void *fp_x, cudaStream_t st);

@@ -41,50 +41,48 @@ __device__ __forceinline__ int quantize_code(T x, T zero, T scale) {
 //   * clamping the quotient to [0, 2^b - 1] before rounding equals clamping after (the bounds are
 //     integers and rounding is monotone; NaN turns into 0 either way);
 //   * adding 1024 in fp16 leaves round-to-nearest-even(q) in the low mantissa bits (ulp is 1 there).
+// (Packed max / min for bfloat16 too, signed codes out of the addition, one-instruction reductions: [2048, 4096] fp16 9.8 -> 8.4 us,
+// bf16 11.1 -> 9.4; [4096, 28672] 8 bits 110 -> 102; 16 rows of 4096 2.1 -> 1.9; RMSNorm of [2048, 4096] 15.1 -> 13.7.)
 __device__ __forceinline__ uint32_t pack_halves(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x5410); }
 
-template <int BITS>
+// A pair's codes end in the low bytes of the two halves, whatever lies above them: unsigned, or (SIGNED) less 2^(b-1) as signed
+// bytes.  Adding 1024 + an even n leaves n + code in the low mantissa bits; n = 128 (8 bits) or 248 (4 bits) makes that the signed
+// code modulo 256.
+template <int BITS, bool SIGNED>
 __device__ __forceinline__ uint32_t codes_of_pair(uint32_t pair, __half2 zero2, float rcp_scale) {
   const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&pair), zero2);
   const float2 f = __half22float2(d);
   __half2 q = __floats2half2_rn(f.x * rcp_scale, f.y * rcp_scale);
   q = __hmin2(__hmax2(q, __float2half2_rn(0.f)), __float2half2_rn((float)((1 << BITS) - 1)));
-  q = __hadd2(q, __float2half2_rn(1024.f));
-  return *reinterpret_cast<const uint32_t *>(&q) & 0x00FF00FFu;      // code_lo | code_hi << 16, both unsigned
+  q = __hadd2(q, __float2half2_rn(!SIGNED ? 1024.f : (BITS == 8 ? 1152.f : 1272.f)));
+  return *reinterpret_cast<const uint32_t *>(&q);
 }
 
 // bfloat16: the same product and clamp, rounded to an integer by adding 2^23 in fp32 (quotients of 8-bit significands keep an
 // even larger distance from a rounding boundary; all 2^14 pairs are checked in the same test).
-template <int BITS>
+template <int BITS, bool SIGNED>
 __device__ __forceinline__ uint32_t codes_of_pair(uint32_t pair, __nv_bfloat162 zero2, float rcp_scale) {
   const float2 f = __bfloat1622float2(__hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&pair), zero2));
-  const float2 q = __bfloat1622float2(__floats2bfloat162_rn(f.x * rcp_scale, f.y * rcp_scale));
-  constexpr float kMaxQ = (float)((1 << BITS) - 1);
-  const uint32_t a = __float_as_uint(fminf(fmaxf(q.x, 0.f), kMaxQ) + 8388608.f);
-  const uint32_t b = __float_as_uint(fminf(fmaxf(q.y, 0.f), kMaxQ) + 8388608.f);
-  return (a & 0xFFu) | ((b & 0xFFu) << 16);
+  __nv_bfloat162 c = __floats2bfloat162_rn(f.x * rcp_scale, f.y * rcp_scale);
+  c = __hmin2(__hmax2(c, __float2bfloat162_rn(0.f)), __float2bfloat162_rn((float)((1 << BITS) - 1)));
+  const float2 q = __bfloat1622float2(c);
+  constexpr float kMagic = 8388608.f + (!SIGNED ? 0.f : (BITS == 8 ? 128.f : 248.f));
+  return __byte_perm(__float_as_uint(q.x + kMagic), __float_as_uint(q.y + kMagic), 0x5410);
 }
 
-// Four pair words (8 unsigned codes) -> output bytes.  PACKED: 8 nibbles in one word (code - 8 == code ^ 8
-// on a nibble).  Otherwise one signed byte per code in two words: code - 128 == code ^ 0x80 (8 bits), and
-// code - 8 through a borrow-free byte-wise subtraction (4 bits, one code per byte).
-template <int BITS, bool PACKED>
+// Four pair words (8 codes) -> output bytes.  PACKED: unsigned codes, 8 nibbles in one word (code - 8 == code ^ 8 on a nibble).
+// Otherwise signed codes, one byte each in two words.
+template <bool PACKED>
 __device__ __forceinline__ void emit_codes(const uint32_t (&c)[4], uint32_t &w0, uint32_t &w1) {
   if (PACKED) {
     uint32_t w = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w |= ((c[j] | (c[j] >> 12)) & 0xFFu) << (8 * j);
+    for (int j = 0; j < 4; ++j) w |= ((c[j] & 0xFu) | (c[j] >> 12 & 0xF0u)) << (8 * j);
     w0 = w ^ 0x88888888u;
     w1 = 0;
   } else {
-    const uint32_t a = __byte_perm(c[0], c[1], 0x6420), b = __byte_perm(c[2], c[3], 0x6420);
-    if (BITS == 8) {
-      w0 = a ^ 0x80808080u;
-      w1 = b ^ 0x80808080u;
-    } else {
-      w0 = ((a | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
-      w1 = ((b | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
-    }
+    w0 = __byte_perm(c[0], c[1], 0x6420);
+    w1 = __byte_perm(c[2], c[3], 0x6420);
   }
 }
 
@@ -266,29 +264,18 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
 
   // ---- pass 1: gather (kept in registers) and max / min
   uint32_t pr[NC][4];
-  float mx = -INFINITY, mn = INFINITY;
+  using T2 = typename Traits<T>::T2;
+  T2 mx2 = {Traits<T>::from_float(-INFINITY), Traits<T>::from_float(-INFINITY)};
+  T2 mn2 = {Traits<T>::from_float(INFINITY), Traits<T>::from_float(INFINITY)};
   auto gather = [&](const uint32_t (&w)[4], uint32_t (&p)[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) p[j] = pack_halves(row16[w[j] & 0xffffu], row16[w[j] >> 16]);
   };
   auto minmax = [&](const uint32_t (&p)[4]) {
-    if (Traits<T>::kIsHalf) {
-      __half2 mx2 = __float2half2_rn(-INFINITY), mn2 = __float2half2_rn(INFINITY);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        mx2 = __hmax2(mx2, *reinterpret_cast<const __half2 *>(&p[j]));
-        mn2 = __hmin2(mn2, *reinterpret_cast<const __half2 *>(&p[j]));
-      }
-      mx = fmaxf(mx, fmaxf(__low2float(mx2), __high2float(mx2)));
-      mn = fminf(mn, fminf(__low2float(mn2), __high2float(mn2)));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const T *e = reinterpret_cast<const T *>(&p[j]);
-        const float a = Traits<T>::to_float(e[0]), b = Traits<T>::to_float(e[1]);
-        mx = fmaxf(mx, fmaxf(a, b));
-        mn = fminf(mn, fminf(a, b));
-      }
+    for (int j = 0; j < 4; ++j) {
+      mx2 = __hmax2(mx2, *reinterpret_cast<const T2 *>(&p[j]));
+      mn2 = __hmin2(mn2, *reinterpret_cast<const T2 *>(&p[j]));
     }
   };
 #pragma unroll
@@ -305,18 +292,16 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
     gather(w, p);
     minmax(p);
   }
-  mx = warp_max(mx);
-  mn = warp_min(mn);
+  // over the warp, then over the warps: one reduction instruction each
+  float mx = redux_max(fmaxf(Traits<T>::to_float(mx2.x), Traits<T>::to_float(mx2.y)));
+  float mn = redux_min(fminf(Traits<T>::to_float(mn2.x), Traits<T>::to_float(mn2.y)));
   if (lane == 0) {
     s_red[0][warp] = mx;
     s_red[1][warp] = mn;
   }
   __syncthreads();
-#pragma unroll
-  for (int w = 0; w < NTHR / 32; ++w) {
-    mx = fmaxf(mx, s_red[0][w]);
-    mn = fminf(mn, s_red[1][w]);
-  }
+  mx = redux_max(s_red[0][lane % (NTHR / 32)]);
+  mn = redux_min(s_red[1][lane % (NTHR / 32)]);
   const T scale = Traits<T>::from_float(fmaxf((mx - mn) / (float)((1 << BITS) - 1), 1e-6f));
   const T zero = Traits<T>::from_float(mn);           // exact: mn is a value of type T
   if (tid == 0) {
@@ -327,12 +312,12 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
   // ---- pass 2: quantize + pack
   uint8_t *drow = dst + (size_t)r * (kPacked ? (size_t)(num_int >> 1) : (size_t)num_int);
   const float rcp_scale = __frcp_rn(Traits<T>::to_float(scale));
-  const typename Traits<T>::T2 zero2 = {zero, zero};
+  const T2 zero2 = {zero, zero};
   auto emit = [&](int c, const uint32_t (&p)[4]) {
     uint32_t w0, w1, codes[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) codes[j] = codes_of_pair<BITS>(p[j], zero2, rcp_scale);
-    emit_codes<BITS, kPacked>(codes, w0, w1);
+    for (int j = 0; j < 4; ++j) codes[j] = codes_of_pair<BITS, !kPacked>(p[j], zero2, rcp_scale);
+    emit_codes<kPacked>(codes, w0, w1);
     if (kPacked) {
       if (vec_store) {
         *reinterpret_cast<uint32_t *>(drow + (size_t)c * 4) = w0;

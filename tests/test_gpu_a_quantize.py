@@ -58,6 +58,42 @@ def test_asym_quantize_matches_oracle(dtype, bits, M, K, F, order):
     assert_device_clean()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits,wide", [(4, False), (4, True), (8, True)])
+@pytest.mark.parametrize("rows,K,F,order", [(7, 264, 8, "ascending"), (300, 264, 8, "shuffled"), (160, 4096, 256, "ascending")])
+def test_rows_at_the_ends_of_the_range(dtype, bits, wide, rows, K, F, order):
+    """Constant rows, ranges below the smallest scale, the type's extremes, zeros of both signs: codes and meta as the oracle has them.
+    NaN takes the lowest code and leaves the row's range alone; in a row with an infinity the scale is infinite and every code
+    the lowest."""
+    import quik
+    from quik_b200.qlinear import _to_u16
+    ints, fp = make_indices(K, F, order)
+    x = outlier_x(rows, K, fp, dtype)
+    big = torch.finfo(dtype).max
+    x[0] = 3.25
+    x[1] = x[1] * 1e-6
+    x[2] = 0.0
+    x[2, ::3] = -0.0
+    x[3, ints[0]], x[3, ints[-1]] = big / 4, -big / 4
+    x[4] = (x[4] > 0).to(dtype) * 2.0 ** -14
+    q_ref, meta_ref, _ = kp.asym_quantize(x, ints, fp, bits)
+    want, low = _codes(q_ref, bits), -(1 << (bits - 1))
+    y = x.clone()
+    y[5, ints[::7]] = float("nan")
+    zero5 = y[5, ints][~y[5, ints].isnan()].min()
+    y[6, ints[3]] = float("inf")
+    q, meta, fp_x = quik.asymmetric.quantize_u16(y.to(dev()), _to_u16(ints.to(dev())), _to_u16(fp.to(dev())), bits, wide)
+    got, meta = _codes(q, bits, wide), meta.cpu()
+    plain = [r for r in range(rows) if r not in (5, 6)]
+    assert torch.equal(meta.view(-1, 2)[plain], meta_ref.view(-1, 2)[plain])
+    diff = (got[plain] - want[plain]).abs()
+    assert diff.max().item() <= 1 and (diff != 0).float().mean().item() <= CODE_MISMATCH_FRACTION
+    assert meta.view(-1, 2)[5, 1] == zero5 and bool((got[5, ::7] == low).all()) and got[5].max().item() == low + (1 << bits) - 1
+    assert meta.view(-1, 2)[6, 0].item() == float("inf") and bool((got[6] == low).all())
+    assert torch.equal(fp_x.cpu(), x[:, fp])
+    assert_device_clean()
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 def test_reference_test_quantize(bits):
     """test/python/test_quant.py:24-39: quantize == find_meta + quantizeOld on gathered columns."""
