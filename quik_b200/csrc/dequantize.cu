@@ -14,25 +14,25 @@ __device__ __forceinline__ float dequant_value(int acc, float srow, float zrow, 
   return __fadd_rn(xe, __fadd_rn(sh, y));
 }
 
-template <typename T, int VEC>
-__global__ void asym_dequantize_kernel(const int32_t *__restrict__ x, const T *__restrict__ meta,
-                                       const T *__restrict__ scale_col, const T *__restrict__ wred,
-                                       const T *__restrict__ y, T *__restrict__ out, int rows,
-                                       int cols, float shift) {
-  const int cvec = cols / VEC;
-  const size_t total = (size_t)rows * cvec;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (size_t)gridDim.x * blockDim.x) {
+// Rows by 32-bit division wherever the matrix allows (a 64-bit one costs more than the eight values it is for), and a dependent
+// launch: what the kernel reads comes after its wait, by ordinary loads of pointers that are not declared constant.
+template <typename T, int VEC, typename Index>
+__global__ void asym_dequantize_kernel(const int32_t *x, const T *meta, const T *scale_col, const T *wred, const T *y, T *__restrict__ out,
+                                       Index total, int cols, float shift) {
+  const unsigned cvec = (unsigned)cols / VEC;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
     const int r = (int)(i / cvec), c0 = (int)(i % cvec) * VEC;
     const float srow = Traits<T>::to_float(meta[2 * (size_t)r]);
     const float zrow = Traits<T>::to_float(meta[2 * (size_t)r + 1]);
     const size_t off = (size_t)r * cols + c0;
     if (VEC == 8) {
-      const int4 a0 = __ldg(reinterpret_cast<const int4 *>(x + off));
-      const int4 a1 = __ldg(reinterpret_cast<const int4 *>(x + off) + 1);
-      const uint4 yv = __ldg(reinterpret_cast<const uint4 *>(y + off));
-      const uint4 sv = __ldg(reinterpret_cast<const uint4 *>(scale_col + c0));
-      const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(wred + c0));
+      const int4 a0 = reinterpret_cast<const int4 *>(x + off)[0];
+      const int4 a1 = reinterpret_cast<const int4 *>(x + off)[1];
+      const uint4 yv = *reinterpret_cast<const uint4 *>(y + off);
+      const uint4 sv = *reinterpret_cast<const uint4 *>(scale_col + c0);
+      const uint4 wv = *reinterpret_cast<const uint4 *>(wred + c0);
       const int acc[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
       const T *ye = reinterpret_cast<const T *>(&yv);
       const T *se = reinterpret_cast<const T *>(&sv);
@@ -72,15 +72,18 @@ __global__ void sym_dequantize_kernel(const X *__restrict__ x, const __half *__r
   }
 }
 
-// packed int4 -> int8, 16 bytes in / 32 bytes out per thread step (include/int4.h:78-98 order:
-// low nibble first).
-__global__ void unpack_int4_kernel(const uint8_t *__restrict__ src, int8_t *__restrict__ dst,
-                                   size_t nbytes, int vec) {
+// Packed int4 -> int8, 16 bytes in / 32 bytes out per thread step (include/int4.h:78-98 order: low nibble first); one or two
+// matrices per launch.
+struct Unpack {
+  const uint8_t *src;
+  int8_t *dst;
+  size_t nbytes;
+};
+__device__ __forceinline__ void unpack_matrix(const Unpack &m, size_t first, size_t step, int vec) {
   if (vec) {
-    const size_t nvec = nbytes >> 4;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-         i += (size_t)gridDim.x * blockDim.x) {
-      const uint4 p = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+    const size_t nvec = m.nbytes >> 4;
+    for (size_t i = first; i < nvec; i += step) {
+      const uint4 p = reinterpret_cast<const uint4 *>(m.src)[i];
       const uint32_t w[4] = {p.x, p.y, p.z, p.w};
       uint32_t o[8];
 #pragma unroll
@@ -93,18 +96,26 @@ __global__ void unpack_int4_kernel(const uint8_t *__restrict__ src, int8_t *__re
         o[2 * j] = __byte_perm(slo, shi, 0x5140);
         o[2 * j + 1] = __byte_perm(slo, shi, 0x7362);
       }
-      uint4 *d = reinterpret_cast<uint4 *>(dst) + 2 * i;
+      uint4 *d = reinterpret_cast<uint4 *>(m.dst) + 2 * i;
       d[0] = make_uint4(o[0], o[1], o[2], o[3]);
       d[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
   } else {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nbytes;
-         i += (size_t)gridDim.x * blockDim.x) {
-      const int b = src[i];
-      dst[2 * i] = (int8_t)(((b & 0xF) ^ 8) - 8);
-      dst[2 * i + 1] = (int8_t)((((b >> 4) & 0xF) ^ 8) - 8);
+    for (size_t i = first; i < m.nbytes; i += step) {
+      const int b = m.src[i];
+      m.dst[2 * i] = (int8_t)(((b & 0xF) ^ 8) - 8);
+      m.dst[2 * i + 1] = (int8_t)((((b >> 4) & 0xF) ^ 8) - 8);
     }
   }
+}
+// The int4 product widens both operands before it starts: one launch for the two, which the product's own setup overlaps (two
+// ordinary launches before).
+__global__ void unpack_int4_kernel(const Unpack a, const Unpack b, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  unpack_matrix(a, first, step, vec & 1);
+  unpack_matrix(b, first, step, vec >> 1);
 }
 
 inline int ew_grid(size_t total, int threads) {
@@ -124,14 +135,22 @@ int launch_asym_dequantize(const int32_t *x, const void *meta, const void *scale
                    aligned16(scale_col) && aligned16(w_reduced);
   const int threads = 256;
   const int grid = ew_grid((size_t)rows * (vec ? cols / 8 : cols), threads);
-#define QUIK_DQ(T, V)                                                                              \
-  asym_dequantize_kernel<T, V><<<grid, threads, 0, st>>>(                                          \
-      x, static_cast<const T *>(meta), static_cast<const T *>(scale_col),                          \
-      static_cast<const T *>(w_reduced), static_cast<const T *>(y), static_cast<T *>(out), rows,   \
-      cols, shift)
+  const size_t total = (size_t)rows * (vec ? cols / 8 : cols);
+  const bool small = total < ((size_t)1 << 31);
+  LaunchCfg lc(dim3(grid), dim3(threads), 0, st);
+#define QUIK_DQ_I(T, V, I)                                                                                                     \
+  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, asym_dequantize_kernel<T, V, I>, x, static_cast<const T *>(meta),                  \
+                                   static_cast<const T *>(scale_col), static_cast<const T *>(w_reduced),                       \
+                                   static_cast<const T *>(y), static_cast<T *>(out), (I)total, cols, shift))
+#define QUIK_DQ(T, V)                              \
+  do {                                             \
+    if (small) QUIK_DQ_I(T, V, unsigned);          \
+    else QUIK_DQ_I(T, V, unsigned long long);      \
+  } while (0)
   if (dtype == QUIK_F16) { if (vec) QUIK_DQ(__half, 8); else QUIK_DQ(__half, 1); }
   else { if (vec) QUIK_DQ(__nv_bfloat16, 8); else QUIK_DQ(__nv_bfloat16, 1); }
 #undef QUIK_DQ
+#undef QUIK_DQ_I
   return check_launch("asym_dequantize_kernel");
 }
 
@@ -149,11 +168,17 @@ int launch_sym_dequantize(const void *x, int x_bits, const void *scale_row, cons
 }
 
 int launch_unpack_int4(const uint8_t *src, int8_t *dst, int rows, int cols, cudaStream_t st) {
-  const size_t nbytes = (size_t)rows * (cols / 2);
-  if (nbytes == 0) return QUIK_OK;
-  const int vec = (nbytes % 16 == 0) && aligned16(src) && aligned16(dst);
-  const int threads = 256, grid = ew_grid(vec ? nbytes / 16 : nbytes, threads);
-  unpack_int4_kernel<<<grid, threads, 0, st>>>(src, dst, nbytes, vec);
+  return launch_unpack_int4_pair(src, dst, rows, nullptr, nullptr, 0, cols, st);
+}
+
+int launch_unpack_int4_pair(const uint8_t *a, int8_t *a8, int rows_a, const uint8_t *b, int8_t *b8, int rows_b, int cols, cudaStream_t st) {
+  const Unpack ua{a, a8, (size_t)rows_a * (cols / 2)}, ub{b, b8, (size_t)rows_b * (cols / 2)};
+  if (ua.nbytes + ub.nbytes == 0) return QUIK_OK;
+  auto vec = [](const Unpack &m) { return (m.nbytes % 16 == 0) && aligned16(m.src) && aligned16(m.dst); };
+  const size_t steps_a = vec(ua) ? ua.nbytes / 16 : ua.nbytes, steps_b = vec(ub) ? ub.nbytes / 16 : ub.nbytes;
+  const int threads = 256;
+  LaunchCfg lc(dim3(ew_grid(steps_a > steps_b ? steps_a : steps_b, threads)), dim3(threads), 0, st);
+  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, unpack_int4_kernel, ua, ub, (int)vec(ua) | (int)vec(ub) << 1));
   return check_launch("unpack_int4_kernel");
 }
 

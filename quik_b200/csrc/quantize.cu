@@ -158,6 +158,12 @@ asym_quantize_row_kernel(const T *__restrict__ src, const IdxT *__restrict__ int
     if (vec_ids) {
       const uint4 v = ld_ids8(int_idx + 8 * (size_t)c);
       w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else if (sizeof(IdxT) == 8 && c * 8 + 8 <= num_int && (reinterpret_cast<uintptr_t>(int_idx) & 15u) == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {        // two 64-bit ids, of which the low words count
+        const uint4 v = ld_ids8(int_idx + 8 * (size_t)c + 2 * j);
+        w[j] = (v.x & 0xffffu) | (v.z << 16);
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
