@@ -144,9 +144,9 @@ int quik_device_status(int clear) { return device_status_read(clear); }
 
 int quik_gemm_plan(int M, int N, int K_int, int F, int *ctas, int *block_n) {
   if (M <= 0 || N <= 0 || K_int <= 0 || F < 0 || !ctas || !block_n) return QUIK_ERR_SHAPE;
-  const int kblocks = (K_int + 127) / 128 + (F + 63) / 64;
-  if (g_engine.load() == QUIK_ENGINE_TCGEN05_TS) choose_tile_ts(M, N, kblocks, ctas, block_n);
-  else choose_tile(M, N, kblocks, ctas, block_n);
+  const int int_kb = (K_int + 127) / 128, fp_kb = (F + 63) / 64;
+  if (g_engine.load() == QUIK_ENGINE_TCGEN05_TS) choose_tile_ts(M, N, int_kb + fp_kb, ctas, block_n);
+  else choose_tile(M, N, int_kb, fp_kb, ctas, block_n);
   return QUIK_OK;
 }
 

@@ -115,8 +115,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // ---- device status word (bounded waits report here); lives in gemm_tcgen05.cu ---------------
 int device_status_read(int clear);   // synchronises the device
-// tile shape the tcgen05 GEMM uses for an M x N problem of `kblocks` 128-byte k-blocks: CTAs per tile (1, 2) and width
-void choose_tile(int M, int N, int kblocks, int *ctas_out, int *bn_out);
+// tile shape the tcgen05 GEMM uses for an M x N problem of 128-byte k-blocks (integer and outlier ones): CTAs per tile (1, 2) and width
+void choose_tile(int M, int N, int int_kb, int fp_kb, int *ctas_out, int *bn_out);
 void set_tile_n(int n);               // 0 = by shape, else a multiple of 16 in [32, 256]
 int get_tile_n();
 void set_cta_pair(int mode);           // 0 = by shape, 1 = never, 2 = always

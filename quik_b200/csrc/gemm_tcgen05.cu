@@ -393,26 +393,25 @@ int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tf
 
 // ---- tile shape per problem -------------------------------------------------------------------
 // A launch is a number of waves of equally sized tiles over the resident units (CTAs or CTA pairs).  The time of a tile depends
-// little on its width: a k-block of a pair moves 16 KB of A and 64 * block_n bytes of B per CTA from L2 (a sweep over 30 problems
-// of 160 to 2048 tokens fits 179 + 0.50 * block_n ns, single CTAs 215 + 0.67 * block_n, 15 to 18 TB/s over the chip), so per k-block
-// a tile costs about kBlockClk + kColClk * block_n cycles.  A narrower tile is therefore almost as expensive as the
-// widest one and only pays where it saves a whole wave; among widths with the same number of waves the narrowest wins by a
-// little.  In that sweep the choice was within 2 % of the best width for all but three problems (10 % for 160 tokens through
-// 4096 x 4096).
-constexpr double kBlockClk = 366.0;
-constexpr double kColClk = 0.45;
-constexpr double kTileFixedClk = 1500.0;
-
-double tile_cost(int M, int N, int kblocks, int ctas, int bn, int units) {
+// little on its width: a k-block of a pair moves 16 KB of A and 64 * block_n bytes of B per CTA from L2, 15 to 18 TB/s over the chip,
+// which takes about 179 + 0.50 * block_n ns (single CTAs 200 + 0.70 * block_n); but its epilogue takes 2000 + 20 * block_n ns (six
+// tenths of that without an outlier product; a fifth more in pairs, whose regions are free when both CTAs are done), and with few
+// k-blocks that is the longer one.  Pairs also start and end 900 ns later.  So a narrower tile only pays where it saves a wave or where epilogues bound the launch; among
+// equals the widest is taken, and pairs before singles.  Fitted to all widths of 24 problems of 200 to 4096 tokens, 896 to 18208 integer
+// columns, and to the choices of earlier constants on 60 more: the choice costs 0.5 % more than the best width on average (one rule for
+// singles and pairs and no epilogue: 2.9 %; 333 tokens through 11008 x 4096 33.5 us, now 29.1, 777 through 4096 x 6912 32.1, now 27.1).
+double tile_cost(int M, int N, int kblocks, bool outliers, int ctas, int bn, int units) {
   const int tile_m = BLOCK_M * ctas;
   const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);
   const long long waves = (tiles + units - 1) / units;
-  return (double)waves * (kblocks * (kBlockClk + kColClk * bn) + kTileFixedClk);
+  const double products = kblocks * (ctas == 2 ? 179.0 + 0.50 * bn : 200.0 + 0.70 * bn) + 800.0;
+  const double epilogue = (2000.0 + 20.0 * bn) * (outliers ? 1.0 : 0.6) * (ctas == 2 ? 1.2 : 1.0);
+  return (double)waves * (products > epilogue ? products : epilogue) + (ctas == 2 ? 900.0 : 0.0);
 }
 
 }  // namespace
 
-void choose_tile(int M, int N, int kblocks, int *ctas_out, int *bn_out) {
+void choose_tile(int M, int N, int int_kb, int fp_kb, int *ctas_out, int *bn_out) {
   const int forced_n = g_tile_n.load(), pair_mode = g_cta_pair.load();
   const int sms = num_sms();
   const int n16 = (N + 15) & ~15;
@@ -430,7 +429,7 @@ void choose_tile(int M, int N, int kblocks, int *ctas_out, int *bn_out) {
         cand = forced_n;
       }
       if (cand > n16) cand = n16 < 32 ? 32 : n16;   // a tile wider than the matrix only wastes columns
-      const double c = tile_cost(M, N, kblocks, ctas, cand, units);
+      const double c = tile_cost(M, N, int_kb + fp_kb, fp_kb > 0, ctas, cand, units);
       if (!have || c < best) {
         have = true;
         best = c;
@@ -475,7 +474,7 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   p.int_kb = (K + STAGE_K_BYTES - 1) / STAGE_K_BYTES;
   p.fp_kb = has_fp ? (ep.F + 63) / 64 : 0;
   int ctas = 1, block_n = 128;
-  choose_tile(M, N, p.int_kb + p.fp_kb, &ctas, &block_n);
+  choose_tile(M, N, p.int_kb, p.fp_kb, &ctas, &block_n);
   const int tile_m = BLOCK_M * ctas;
   const int m_tiles = (M + tile_m - 1) / tile_m;
   const int cap_n = block_n <= 128 ? 128 : 256;
