@@ -267,6 +267,7 @@ struct EpilogueWarp {
       if (lane == 0 && o.rows > 0) tma_store_2d(out_map, smem_u32(s_stage), t.n0 + (KIND == 0 ? 8 : 16) * (c - 1), t.m0);
     }
   }
+  // Comes before whatever writes the staging buffer anew: it has been read out, by the warp's lanes and by its bulk stores.
   __device__ __forceinline__ void reuse_stage() const {
     if (lane == 0) tma_store_wait_read();
     __syncwarp();
@@ -353,8 +354,9 @@ struct EpilogueWarp {
         w[4 * jj] = v.x; w[4 * jj + 1] = v.y; w[4 * jj + 2] = v.z; w[4 * jj + 3] = v.w;
       }
     } else {
-      // half a warp fetches the 16 columns of a row (32 contiguous bytes); the staging buffer turns them
-      __syncwarp();
+      // half a warp fetches the 16 columns of a row (32 contiguous bytes); the staging buffer turns them.  A bulk store of the
+      // tile before may still be reading it.
+      reuse_stage();
       const int cc = lane & 15;
 #pragma unroll 4
       for (int k = 0; k < 16; ++k) {

@@ -1,4 +1,6 @@
 """GPU parity: exact int32 GEMMs (both engines) and the fused GEMM+dequantize ops."""
+import functools
+
 import pytest
 import torch
 
@@ -166,3 +168,49 @@ def test_fused_dequantize_ops(engine, bits, M, N, K):
     ref16s = kp.sym_fused_dequantize_fp16(acc, sr, sc, y)
     ulp = torch.maximum(torch.maximum(t1, y.float().abs()), ref16s.float().abs()) * 2 ** -10
     assert ((out_s.float() - ref16s.float()).abs() <= 3 * ulp).all()
+
+
+@functools.lru_cache(maxsize=1)
+def _addend_case(N):
+    M, K, sv = 2000, 256, 0.4376
+    a, b, sr, sc, zr, wr, y = _fused_inputs(8, M, N, K, seed=N)
+    acc = kp.int8_matmul(a, b)
+    zero = torch.zeros_like(sr).float()
+    asym = kp.dequantize_fma(acc, sr.float(), zr.float(), sc.float(), wr.float(), y.float(), sv).half()
+    sym = kp.dequantize_fma(acc, sr.float(), zero, sc.float(), torch.zeros_like(sc).float(), y.float(), 0.0).half()
+    return (a, b, sr, sc, zr, wr, y), sv, asym, sym
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("N", [5000, 5001, 5008])
+@pytest.mark.parametrize("eng,tile,pair", [(_lib.ENGINE_AUTO, 0, 0), (_lib.ENGINE_TCGEN05, 32, 1), (_lib.ENGINE_TCGEN05, 256, 1),
+                                           (_lib.ENGINE_TCGEN05, 256, 2), (_lib.ENGINE_TCGEN05_TS, 0, 0)])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_addend_of_every_tile_of_a_cta(bits, eng, tile, pair, N, offset):
+    """A CTA's later tiles fetch their addend while stores of the tile before are under way; at a width of 8 modulo 16 and for an
+    addend off a 16-byte boundary both pass through the same staging buffer.  Three to sixteen tiles per CTA, calls in close
+    succession, asymmetric and symmetric, against the fp32 formula."""
+    import quik
+    (a, b, sr, sc, zr, wr, y), sv, want, want_s = _addend_case(N)
+    d = dev()
+    qa, qb = (kp.pack_to_i4(a), kp.pack_to_i4(b)) if bits == 4 else (a, b)
+    qa, qb, sr, sc, zr, wr = (t.to(d) for t in (qa, qb, sr, sc, zr, wr))
+    slab = torch.empty(offset + y.numel(), dtype=y.dtype, device=d)
+    yd = slab[offset:].view(y.shape)
+    yd.copy_(y)
+    asym = quik.asymmetric.int4FusedDequantize if bits == 4 else quik.asymmetric.int8FusedDequantize
+    sym = quik.symmetric.int4FusedDequantize if bits == 4 else quik.symmetric.int8FusedDequantize
+    try:
+        _lib.set_engine(eng)
+        _lib.set_tile_n(tile)
+        _lib.set_cta_pair(pair)
+        got = [asym(qa, qb, sr, sc, sv, zr, wr, yd) for _ in range(4)]
+        got_s = sym(qa, qb, sr, sc, yd)
+    finally:
+        _lib.set_engine(_lib.ENGINE_AUTO)
+        _lib.set_tile_n(0)
+        _lib.set_cta_pair(0)
+    _assert_same_rounding(got[0].cpu(), want)
+    assert all(torch.equal(g, got[0]) for g in got[1:])
+    _assert_same_rounding(got_s.cpu(), want_s)
+    assert_device_clean()
