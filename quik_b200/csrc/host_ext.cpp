@@ -13,8 +13,10 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstring>
+#include <memory>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "../../include/quik_b200.h"
 
@@ -312,29 +314,42 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- calls by module and plan -----------------------------------------------------------------------------------------------
-// A plan is the tuple (int_ids, fp_ids, w8 | None, key) of a module's derived operands; the key says which buffers, by address and
-// version, they were derived from.  The module's buffers and sizes are read on every call; where they are not those of the
-// plan, or something is missing, a call returns None having launched nothing, and the module's own path derives them anew.  Reading
-// attributes, comparing keys and collecting arguments in Python was 6 us of the 15 us of a call for one token.
-constexpr Py_ssize_t kKeyBytes = 6 * sizeof(int64_t);
-bool plan_key(const at::Tensor &int_ids, const at::Tensor &fp_ids, const at::Tensor &w, int64_t *key) {
-  const at::Tensor *const t[3] = {&int_ids, &fp_ids, &w};
-  for (int i = 0; i < 3; ++i) {
-    if (t[i]->is_inference()) return false;      // counts no versions
-    key[2 * i] = (int64_t)(intptr_t)ptr(*t[i]);
-    key[2 * i + 1] = (int64_t)t[i]->_version();
+// A plan is the tuple (int_ids, fp_ids, w8 | None, sources) of a module's derived operands; the sources say which buffers they were
+// derived from.  The module's buffers and sizes are read on every call; where they are not those of the plan, or something is
+// missing, a call returns None having launched nothing, and the module's own path derives them anew.  Reading attributes, comparing
+// keys and collecting arguments in Python was 6 us of the 15 us of a call for one token.
+
+// A tensor that something was derived from, at one version of its contents.  Address and version alone do not name it: the allocator
+// gives the memory of a tensor that was freed to the next of its size, whose version starts at zero too.  The weak handles keep
+// no device memory, but they keep the addresses of the tensor and of its storage object from being given out again.
+struct Source {
+  c10::weak_intrusive_ptr<at::TensorImpl, at::UndefinedTensorImpl> tensor;
+  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+  const void *data;
+  int64_t version;
+  explicit Source(const at::Tensor &t)
+      : tensor(t.getIntrusivePtr()), storage(t.storage().getWeakStorageImpl()), data(ptr(t)), version((int64_t)t._version()) {}
+  bool same(const at::Tensor &t) const {
+    return t.unsafeGetTensorImpl() == tensor._unsafe_get_target() && t.storage().unsafeGetStorageImpl() == storage._unsafe_get_target() &&
+           ptr(t) == data && !t.is_inference() && (int64_t)t._version() == version;
   }
-  return true;
+};
+using Sources = std::vector<Source>;
+constexpr const char *kSourcesName = "quik_b200.sources";
+// of the capsule that py_sources made, else nullptr
+const Sources *sources_arg(PyObject *o) {
+  return PyCapsule_IsValid(o, kSourcesName) ? static_cast<const Sources *>(PyCapsule_GetPointer(o, kSourcesName)) : nullptr;
 }
+
 struct Planned {
   Layer l;
   at::Tensor w, w8, ids, fp_ids;
 };
 // 1: read, 0: not the plan's module any more, -1: Python error
 int read_planned(PyObject *module, PyObject *plan, Planned *r) {
-  if (!PyTuple_Check(plan) || PyTuple_GET_SIZE(plan) != 4 || !PyBytes_Check(PyTuple_GET_ITEM(plan, 3)) ||
-      PyBytes_GET_SIZE(PyTuple_GET_ITEM(plan, 3)) != kKeyBytes)
-    return 0;
+  if (!PyTuple_Check(plan) || PyTuple_GET_SIZE(plan) != 4) return 0;
+  const Sources *sources = sources_arg(PyTuple_GET_ITEM(plan, 3));
+  if (!sources || sources->size() != 3) return 0;
   PyObject *buffers = PyObject_GetAttr(module, names.buffers);
   if (!buffers) return -1;
   bool have = PyDict_Check(buffers);
@@ -365,10 +380,7 @@ int read_planned(PyObject *module, PyObject *plan, Planned *r) {
   if (have && r->l.f > 0) buffer(names.fp_weight, &r->l.fp_w, false);
   Py_DECREF(buffers);
   if (PyErr_Occurred()) return -1;
-  int64_t key[6];
-  if (!have || r->l.k_int <= 0 || !plan_key(ids64, fp64, r->w, key) ||
-      std::memcmp(key, PyBytes_AS_STRING(PyTuple_GET_ITEM(plan, 3)), kKeyBytes) != 0)
-    return 0;
+  if (!have || r->l.k_int <= 0 || !(*sources)[0].same(ids64) || !(*sources)[1].same(fp64) || !(*sources)[2].same(r->w)) return 0;
   r->ids = tensor_arg(PyTuple_GET_ITEM(plan, 0));
   r->fp_ids = tensor_arg(PyTuple_GET_ITEM(plan, 1));
   r->w8 = optional_arg(PyTuple_GET_ITEM(plan, 2));
@@ -379,13 +391,26 @@ void make_current(const at::Tensor &x) {
   if (c10::cuda::current_device() != x.device().index()) c10::cuda::set_device(x.device().index());
 }
 
-// (int_indices, fp_indices, int_weight) -> key, or None where they count no versions
-PyObject *py_plan_key(PyObject *, PyObject *const *a, Py_ssize_t n) {
+// (tensor, ...) -> sources: the tensors and the versions of their contents; RuntimeError where one counts no versions
+PyObject *py_sources(PyObject *, PyObject *const *a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 3);
-  int64_t key[6];
-  if (!plan_key(tensor_arg(a[0]), tensor_arg(a[1]), tensor_arg(a[2]), key)) Py_RETURN_NONE;
-  return PyBytes_FromStringAndSize(reinterpret_cast<const char *>(key), kKeyBytes);
+  auto made = std::make_unique<Sources>();
+  made->reserve(n);
+  for (Py_ssize_t i = 0; i < n; ++i) made->emplace_back(tensor_arg(a[i]));
+  PyObject *o = PyCapsule_New(made.get(), kSourcesName, [](PyObject *c) { delete const_cast<Sources *>(sources_arg(c)); });
+  if (o) made.release();
+  return o;
+  END_HANDLE_TH_ERRORS
+}
+
+// (sources, tensor, ...) -> whether these are the tensors that the sources were made of, unchanged
+PyObject *py_same_sources(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n < 1) expect(n, 1);
+  const Sources *sources = sources_arg(a[0]);
+  bool same = sources && (Py_ssize_t)sources->size() == n - 1;
+  for (Py_ssize_t i = 1; same && i < n; ++i) same = (*sources)[i - 1].same(tensor_arg(a[i]));
+  return PyBool_FromLong(same);
   END_HANDLE_TH_ERRORS
 }
 
@@ -526,7 +551,9 @@ PyMethodDef methods[] = {
      "operand layouts for a token count"},
     {"weights_changed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_weights_changed)), METH_FASTCALL,
      "weights against a record"},
-    {"plan_key", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_plan_key)), METH_FASTCALL, "key of a plan"},
+    {"sources", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sources)), METH_FASTCALL, "tensors at their versions"},
+    {"same_sources", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_same_sources)), METH_FASTCALL,
+     "tensors against sources"},
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_forward)), METH_FASTCALL, "a module's forward by its plan"},
     {"quantize_for", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_quantize_for)), METH_FASTCALL,
      "activation quantizer for a module by its plan"},

@@ -136,12 +136,19 @@ class MixedQLinear(torch.nn.Module):
 
     # ------------------------------------------------------------------ derived, lazily built operands
     def _cached(self, name, src: Tensor, make):
-        key = (src.data_ptr(), src._version, src.get_device())
+        """make(src), kept as long as ``src`` is the same tensor at the same version (not only at the same address)."""
         ent = self._cache.get(name)
-        if ent is None or ent[0] != key:
-            ent = (key, make(src))
+        if ent is None or not _lib.host().same_sources(ent[0], src):
+            ent = (_lib.host().sources(src), make(src))
             self._cache[name] = ent
         return ent[1]
+
+    def __getstate__(self):
+        # what was derived from this object's buffers stays here: a copy, or the object read back from a file, derives its own
+        state = self.__dict__.copy()
+        state.pop("_plan", None)
+        state.update(_cache={}, _seen=bytearray(32))
+        return state
 
     def _idx16(self):
         k = self.in_features
@@ -174,20 +181,18 @@ class MixedQLinear(torch.nn.Module):
 
     def _make_plan(self):
         """What the native host path needs of this layer beside its buffers: 16-bit column ids, weight codes one per byte where
-        they have been made, and the key of the buffers that these come from.  It reads the buffers itself on every call and
-        declines where the key is another: the layer's own path then runs, and ends here again."""
+        they have been made, and the buffers that these come from.  It reads the buffers itself on every call and declines where
+        they are others: the layer's own path then runs, and ends here again."""
         self._plan = None
         b = self._buffers
         w, sources = b.get("int_weight"), (b.get("int_indices"), b.get("fp_indices"), b.get("int_weight"))
-        if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None for t in sources):
+        if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None or t.is_inference() for t in sources):
             return
-        key = _lib.host().plan_key(*sources)
-        if key is None:
-            return
+        host = _lib.host()
+        key = host.sources(*sources)
         i16, f16 = self._idx16()
         w8 = self._cache.get("w8")
-        current = w8 is not None and w8[0] == (w.data_ptr(), w._version, w.get_device())
-        self._plan = (i16, f16, w8[1] if current else None, key)
+        self._plan = (i16, f16, w8[1] if w8 is not None and host.same_sources(w8[0], w) else None, key)
 
     def _quantize_by_plan(self, producer, x, aux, eps):
         """Fills the group's shared input from the native host path; False where that declines."""

@@ -657,3 +657,28 @@ def test_native_path_follows_the_buffers(M, bits, F, shared):
     with pytest.raises(Exception):
         layer(x.cpu())
     assert_device_clean()
+
+
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("M,bits", [(5, 4), (200, 4), (200, 8)])
+def test_buffers_replaced_at_the_same_address(M, bits, shared):
+    """A buffer that is replaced by another tensor at the same address and version (memory that the allocator gives out again): the
+    next call uses the new one's contents."""
+    case = make_layer("t", M, 1024 + 64, 264, bits, F=64, seed=M, device=dev(), clip=False)
+    layer, x = case.module, case.x.unsqueeze(0)
+    layer.shared_input = SharedQuantizedInput(1) if shared else None
+    for name in ("int_weight", "int_indices", "fp_indices"):
+        old = getattr(layer, name).clone()
+        memory = old.clone()
+        setattr(layer, name, memory.data)                     # .data: another tensor over the memory, at version 0
+        layer(x)
+        first = layer(x)
+        at = getattr(layer, name).data_ptr(), getattr(layer, name)._version
+        memory.copy_(old.flip(0))
+        setattr(layer, name, memory.data)
+        assert (getattr(layer, name).data_ptr(), getattr(layer, name)._version) == at
+        got = layer(x)
+        assert torch.equal(got, copy.deepcopy(layer)(x)) and not torch.equal(got, first)
+        setattr(layer, name, old)
+        assert torch.equal(layer(x), first)
+    assert_device_clean()

@@ -214,6 +214,55 @@ def test_changed_weights_are_noticed():
         _lib.host().weights_changed(bytearray(8), layer.fp_weight, None)
 
 
+def _tensor_over(array):
+    """A tensor over the memory of ``array``: a new one at each call, at the same address and version."""
+    return torch.from_numpy(array)
+
+
+def test_derived_operands_follow_a_tensor_at_a_reused_address():
+    """A buffer that is replaced by another tensor may find it at the same address, at the same version: the allocator gives out
+    the memory that was freed.  Operands derived from the first one are not taken for the second one's."""
+    layer = qlinear.MixedQLinear(96, 8, fp_features_num=32, bits=4)
+    ids, fp_ids = np.arange(64), np.arange(64, 96)
+    layer.int_indices, layer.fp_indices = _tensor_over(ids), _tensor_over(fp_ids)
+    first = layer._idx16()
+    assert all(a is b for a, b in zip(layer._idx16(), first))                 # kept while nothing changes
+    at = layer.int_indices.data_ptr(), layer.int_indices._version
+    ids[:] = ids[::-1].copy()
+    layer.int_indices = _tensor_over(ids)
+    assert (layer.int_indices.data_ptr(), layer.int_indices._version) == at
+    i16, f16 = layer._idx16()
+    assert i16.tolist() == list(range(63, -1, -1)) and f16 is first[1]
+    layer.fp_indices.copy_(layer.fp_indices.flip(0))                          # the same tensor at another version
+    assert layer._idx16()[1].tolist() == list(range(95, 63, -1))
+    layer.int_indices.data = _tensor_over(np.arange(64))                      # the same tensor with other storage
+    assert layer._idx16()[0].tolist() == list(range(64))
+    memory = np.zeros((8, 32), dtype=np.uint8)
+    for value in (0, 1):
+        memory[:] = value
+        layer.int_weight = _tensor_over(memory)
+        assert bool((layer._cached("w8", layer.int_weight, torch.clone) == value).all())
+
+
+def test_a_copy_of_a_layer_derives_its_own_operands():
+    """Copies and layers read back from a file start without the derived operands of the original, and one that still has them (or
+    a record of them in an earlier form) derives them anew."""
+    import copy
+    import pickle
+    layer = qlinear.MixedQLinear(96, 8, fp_features_num=32, bits=4)
+    layer.int_indices.copy_(torch.arange(64))
+    layer.fp_indices.copy_(torch.arange(64, 96))
+    i16, f16 = layer._idx16()
+    for other in (copy.deepcopy(layer), copy.copy(layer), pickle.loads(pickle.dumps(layer))):
+        assert not other._cache and other._plan is None and other._seen is not layer._seen
+        assert torch.equal(other._idx16()[0], i16) and torch.equal(other._idx16()[1], f16)
+        assert other._idx16()[0] is not i16
+    assert layer._idx16()[0] is i16
+    key = (layer.int_indices.data_ptr(), layer.int_indices._version, layer.int_indices.get_device())
+    layer._cache["int16"] = (key, torch.zeros(64, dtype=torch.int16))
+    assert torch.equal(layer._idx16()[0], i16)
+
+
 def test_operand_layouts_by_engine():
     """One rule picks the operand layouts, for a layer's single native call and for members of a shared input alike."""
     from quik_b200 import _lib
