@@ -314,8 +314,8 @@ PyObject *py_layer(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- calls by module and plan -----------------------------------------------------------------------------------------------
-// A plan is the tuple (int_ids, fp_ids, w8 | None, sources) of a module's derived operands; the sources say which buffers they were
-// derived from.  The module's buffers and sizes are read on every call; where they are not those of the plan, or something is
+// A plan is the tuple (int_ids | None, fp_ids | None, w8 | None, sources) of a module's derived operands, where it has derived them; the
+// sources say which buffers they were derived from.  The module's buffers and sizes are read on every call; where they are not those of the plan, or something is
 // missing, a call returns None having launched nothing, and the module's own path derives them anew.  Reading attributes, comparing
 // keys and collecting arguments in Python was 6 us of the 15 us of a call for one token.
 
@@ -381,8 +381,8 @@ int read_planned(PyObject *module, PyObject *plan, Planned *r) {
   Py_DECREF(buffers);
   if (PyErr_Occurred()) return -1;
   if (!have || r->l.k_int <= 0 || !(*sources)[0].same(ids64) || !(*sources)[1].same(fp64) || !(*sources)[2].same(r->w)) return 0;
-  r->ids = tensor_arg(PyTuple_GET_ITEM(plan, 0));
-  r->fp_ids = tensor_arg(PyTuple_GET_ITEM(plan, 1));
+  r->ids = optional_arg(PyTuple_GET_ITEM(plan, 0));
+  r->fp_ids = optional_arg(PyTuple_GET_ITEM(plan, 1));
   r->w8 = optional_arg(PyTuple_GET_ITEM(plan, 2));
   return 1;
 }
@@ -421,7 +421,7 @@ PyObject *py_forward(PyObject *, PyObject *const *a, Py_ssize_t n) {
   Planned r;
   const int ok = read_planned(a[0], a[1], &r);
   if (ok < 0) return nullptr;
-  if (ok == 0 || !THPVariable_Check(a[3])) Py_RETURN_NONE;
+  if (ok == 0 || !r.ids.defined() || !r.fp_ids.defined() || !THPVariable_Check(a[3])) Py_RETURN_NONE;
   const at::Tensor x = tensor_arg(a[3]);
   if (!x.is_cuda()) Py_RETURN_NONE;
   make_current(x);
@@ -441,7 +441,7 @@ PyObject *py_quantize_for(PyObject *, PyObject *const *a, Py_ssize_t n) {
   const int producer = (int)PyLong_AsLong(a[2]);
   const double eps = PyFloat_AsDouble(a[5]);
   if (PyErr_Occurred()) return nullptr;
-  if (ok == 0 || producer < 0 || producer > 2 || !THPVariable_Check(a[3])) Py_RETURN_NONE;
+  if (ok == 0 || !r.ids.defined() || !r.fp_ids.defined() || producer < 0 || producer > 2 || !THPVariable_Check(a[3])) Py_RETURN_NONE;
   at::Tensor x = tensor_arg(a[3]), aux = optional_arg(a[4]);
   if (!x.is_cuda()) Py_RETURN_NONE;
   if (producer == 0) make_current(x);

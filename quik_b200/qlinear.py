@@ -177,22 +177,27 @@ class MixedQLinear(torch.nn.Module):
         """(codes, meta, outliers) of producer(x) with this layer's columns; its ids are settled: ``_to_u16`` made them on the
         host and copied them synchronously."""
         i16, f16 = self._idx16()
+        if self._plan is not None and (self._plan[0] is None or self._plan[1] is None):
+            self._plan = None            # made before the ids were: the layer's next launch makes it again
         return _lib.host().quantize(producer, x, aux, eps, i16, f16, self.bits, wide, True)
 
     def _make_plan(self):
-        """What the native host path needs of this layer beside its buffers: 16-bit column ids, weight codes one per byte where
-        they have been made, and the buffers that these come from.  It reads the buffers itself on every call and declines where
-        they are others: the layer's own path then runs, and ends here again."""
+        """What the native host path needs of this layer beside its buffers: 16-bit column ids and weight codes one per byte, each
+        where this layer has derived them, and the buffers that these come from.  It reads the buffers itself on every call
+        and declines where they are others or something is missing: the layer's own path then runs, and ends here again.  Nothing
+        is derived here: a member of a group whose input another member quantizes needs no ids, and may not even have any."""
         self._plan = None
         b = self._buffers
-        w, sources = b.get("int_weight"), (b.get("int_indices"), b.get("fp_indices"), b.get("int_weight"))
+        sources = b.get("int_indices"), b.get("fp_indices"), b.get("int_weight")
         if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None or t.is_inference() for t in sources):
             return
         host = _lib.host()
         key = host.sources(*sources)
-        i16, f16 = self._idx16()
-        w8 = self._cache.get("w8")
-        self._plan = (i16, f16, w8[1] if w8 is not None and host.same_sources(w8[0], w) else None, key)
+
+        def derived(name, src):
+            ent = self._cache.get(name)
+            return ent[1] if ent is not None and host.same_sources(ent[0], src) else None
+        self._plan = (*map(derived, ("int16", "fp16", "w8"), sources), key)
 
     def _quantize_by_plan(self, producer, x, aux, eps):
         """Fills the group's shared input from the native host path; False where that declines."""

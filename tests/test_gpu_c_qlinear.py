@@ -682,3 +682,43 @@ def test_buffers_replaced_at_the_same_address(M, bits, shared):
         setattr(layer, name, old)
         assert torch.equal(layer(x), first)
     assert_device_clean()
+
+
+@pytest.mark.parametrize("M,bits", [(5, 4), (40, 4), (200, 4), (200, 8)])
+def test_members_that_never_quantize_need_no_ids(M, bits):
+    """A group of three on one quantized input: only the member that quantizes derives column ids; the others may have none, at the
+    first call and at later ones.  One that quantizes later derives its own then, and its next calls take the native path too."""
+    case = make_layer("t", M, 1024 + 64, 264, bits, F=64, seed=M, device=dev(), clip=False)
+    x = case.x.unsqueeze(0)
+    want = case.module(x)
+    shared = SharedQuantizedInput(3)
+    a, b, c = (copy.deepcopy(case.module) for _ in range(3))
+    for m in (a, b, c):
+        m.shared_input = shared
+    ids, fp_ids = b.int_indices.clone(), b.fp_indices.clone()
+    for m in (b, c):
+        m.int_indices.zero_()
+        m.fp_indices.zero_()
+    for _ in range(3):
+        for m in (a, b, c):
+            assert torch.equal(m(x), want)
+            assert m._plan is not None and (m._plan[0] is None) == (m is not a) and ("int16" in m._cache) == (m is a)
+    with pytest.raises(RuntimeError, match="exactly once"):
+        b(x)
+    assert shared.qint_x is None and shared.cur_group_elem == 0
+    b.int_indices.copy_(ids)
+    b.fp_indices.copy_(fp_ids)
+    for _ in range(2):
+        for m in (b, c, a):
+            assert torch.equal(m(x), want)
+    assert b._plan[0] is not None and c._plan[0] is None
+    norm = torch.ones(x.shape[-1], dtype=x.dtype, device=x.device)
+    c.int_indices.copy_(ids)
+    c.fp_indices.copy_(fp_ids)
+    got = []
+    for _ in range(3):
+        c.quantize_rmsnorm(x, norm, 1e-5)
+        got.append([m(x) for m in (c, a, b)])
+    assert c._plan[0] is not None
+    assert all(torch.equal(t, got[0][0]) for outs in got for t in outs) and not torch.equal(got[0][0], want)
+    assert_device_clean()
