@@ -349,7 +349,7 @@ struct Planned {
 int read_planned(PyObject *module, PyObject *plan, Planned *r) {
   if (!PyTuple_Check(plan) || PyTuple_GET_SIZE(plan) != 4) return 0;
   const Sources *sources = sources_arg(PyTuple_GET_ITEM(plan, 3));
-  if (!sources || sources->size() != 3) return 0;
+  if (!sources || sources->size() < 3) return 0;
   PyObject *buffers = PyObject_GetAttr(module, names.buffers);
   if (!buffers) return -1;
   bool have = PyDict_Check(buffers);
@@ -380,7 +380,9 @@ int read_planned(PyObject *module, PyObject *plan, Planned *r) {
   if (have && r->l.f > 0) buffer(names.fp_weight, &r->l.fp_w, false);
   Py_DECREF(buffers);
   if (PyErr_Occurred()) return -1;
-  if (!have || r->l.k_int <= 0 || !(*sources)[0].same(ids64) || !(*sources)[1].same(fp64) || !(*sources)[2].same(r->w)) return 0;
+  if (!have || r->l.k_int <= 0 || !(*sources)[0].same(ids64) || !(*sources)[1].same(fp64) || !(*sources)[2].same(r->w) ||
+      sources->size() != (r->l.f > 0 ? 4u : 3u) || (r->l.f > 0 && !(*sources)[3].same(r->l.fp_w)))
+    return 0;
   r->ids = optional_arg(PyTuple_GET_ITEM(plan, 0));
   r->fp_ids = optional_arg(PyTuple_GET_ITEM(plan, 1));
   r->w8 = optional_arg(PyTuple_GET_ITEM(plan, 2));

@@ -73,7 +73,7 @@ class MixedQLinear(torch.nn.Module):
     # optional caller-owned output buffer [M, out_features] (e.g. symmetric memory of a tensor-parallel
     # group); used by the fused path when its shape, dtype and device match
     out_buffer = None
-    # weights of the last call for few tokens (see _host.weights_changed); every layer has its own
+    # weights of the last call for few tokens (see _weights_record); every layer has its own
     _seen = bytearray(32)
     # derived operands for the native host path (see _make_plan); every layer has its own
     _plan = None
@@ -188,7 +188,7 @@ class MixedQLinear(torch.nn.Module):
         is derived here: a member of a group whose input another member quantizes needs no ids, and may not even have any."""
         self._plan = None
         b = self._buffers
-        sources = b.get("int_indices"), b.get("fp_indices"), b.get("int_weight")
+        sources = b.get("int_indices"), b.get("fp_indices"), b.get("int_weight"), *([b.get("fp_weight")] if self.fp_features_num > 0 else [])
         if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None or t.is_inference() for t in sources):
             return
         host = _lib.host()
@@ -198,6 +198,15 @@ class MixedQLinear(torch.nn.Module):
             ent = self._cache.get(name)
             return ent[1] if ent is not None and host.same_sources(ent[0], src) else None
         self._plan = (*map(derived, ("int16", "fp16", "w8"), sources), key)
+
+    def _weights_record(self):
+        """The record of the weights of this layer's last call for few tokens, emptied where they are other tensors since: the record
+        itself knows them by address and version only.  (The native path checks by its plan that they are the same.)"""
+        host, weights = _lib.host(), [self.int_weight, *([self.fp_weight] if self.fp_features_num > 0 else [])]
+        if not any(t.is_inference() for t in weights) and not host.same_sources(self._cache.get("weights"), *weights):
+            self._seen[:] = bytes(32)
+            self._cache["weights"] = host.sources(*weights)
+        return self._seen
 
     def _quantize_by_plan(self, producer, x, aux, eps):
         """Fills the group's shared input from the native host path; False where that declines."""
@@ -285,7 +294,7 @@ class MixedQLinear(torch.nn.Module):
         if hook is not None:
             hook(self, True)
         out = _lib.host().linear(x, self._out_buffer_for(x, M), *self._constants(), w, w_packed, shared_input.qint_x, q_packed,
-                                 shared_input.meta, shared_input.fp_x, self._seen)
+                                 shared_input.meta, shared_input.fp_x, self._weights_record())
         if hook is not None:
             hook(self, False)
         shared_input.finish()
@@ -317,7 +326,7 @@ class MixedQLinear(torch.nn.Module):
         M = x.shape[-2] if x.dim() > 1 else 0
         wide = self._weight_codes_int8() if self.bits == 4 and not self._operand_layouts(M)[1] else None
         out = self._out_buffer_for(x, M)
-        res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids, self._seen)
+        res = _lib.host().layer(x, out, *self._constants(), w, wide, ids, fp_ids, self._weights_record())
         if res is None:          # a setting that another thread has changed since asks for weight codes one per byte
             res = _lib.host().layer(x, out, *self._constants(), w, self._weight_codes_int8(), ids, fp_ids, self._seen)
         self._make_plan()

@@ -722,3 +722,31 @@ def test_members_that_never_quantize_need_no_ids(M, bits):
     assert c._plan[0] is not None
     assert all(torch.equal(t, got[0][0]) for outs in got for t in outs) and not torch.equal(got[0][0], want)
     assert_device_clean()
+
+
+@pytest.mark.parametrize("F", [0, 64])
+def test_quantized_weights_at_a_reused_address_are_waited_for(F):
+    """Few tokens through the ring engine, which loads its weights before it waits for the stream: weights that the quantizer (which
+    lets later launches start early) has just written, in a tensor at the address and version of the last ones."""
+    M, K, N = 16, 4096 + F, 8192
+    case = make_layer("t", M, K, N, 8, F=F, seed=F, device=dev(), clip=False)
+    layer, x = case.module, case.x.unsqueeze(0)
+    memory = layer.int_weight.clone()
+    g = torch.Generator().manual_seed(7)
+    sources = [torch.randn(N, K - F, generator=g).half().to(dev()) for _ in range(2)]
+    all_ids, meta = torch.arange(K - F, device=dev()), torch.empty(2 * N, dtype=torch.float16, device=dev())
+
+    def write(i):
+        _lib.check(_lib.load().quik_asym_quantize(_lib.ptr(sources[i]), 0, N, K - F, _lib.ptr(all_ids), K - F, None, 0, 8,
+                                                  _lib.ptr(memory), _lib.ptr(meta), None, _lib.stream_of(memory)), "quantize")
+        layer.int_weight = memory.data
+    want = []
+    for i in (0, 1):
+        write(i)
+        torch.cuda.synchronize()
+        want.append(layer(x).clone())
+    assert not torch.equal(*want)
+    for rep in range(20):
+        write(rep & 1)
+        assert torch.equal(layer(x), want[rep & 1]), rep
+    assert_device_clean()

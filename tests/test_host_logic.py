@@ -244,6 +244,25 @@ def test_derived_operands_follow_a_tensor_at_a_reused_address():
         assert bool((layer._cached("w8", layer.int_weight, torch.clone) == value).all())
 
 
+def test_changed_weights_are_noticed_at_a_reused_address():
+    """The same for weights that are replaced by other tensors at the address and version of the old ones."""
+    from quik_b200 import _lib
+    layer = qlinear.MixedQLinear(96, 8, fp_features_num=32, bits=8)
+    codes, values = np.zeros((8, 64), dtype=np.int8), np.zeros((8, 32), dtype=np.float16)
+
+    def changed():
+        return _lib.host().weights_changed(layer._weights_record(), layer.int_weight, layer.fp_weight)
+    layer.int_weight, layer.fp_weight = _tensor_over(codes), _tensor_over(values)
+    assert changed() and not changed()
+    layer.int_weight = _tensor_over(codes)
+    assert changed() and not changed()
+    layer.fp_weight = _tensor_over(values)
+    assert changed() and not changed()
+    with torch.inference_mode():
+        layer.fp_weight = layer.fp_weight.clone()
+    assert changed() and changed()
+
+
 def test_a_copy_of_a_layer_derives_its_own_operands():
     """Copies and layers read back from a file start without the derived operands of the original, and one that still has them (or
     a record of them in an earlier form) derives them anew."""
