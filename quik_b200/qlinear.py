@@ -75,8 +75,6 @@ class MixedQLinear(torch.nn.Module):
     out_buffer = None
     # weights of the last call for few tokens (see _weights_record); every layer has its own
     _seen = bytearray(32)
-    # derived operands for the native host path (see _make_plan); every layer has its own
-    _plan = None
 
     def __init__(self, in_features, out_features, shared_input=None,
                  fp_features_num=0, symm=False, bits=4, dtype=torch.float16):
@@ -146,7 +144,6 @@ class MixedQLinear(torch.nn.Module):
     def __getstate__(self):
         # what was derived from this object's buffers stays here: a copy, or the object read back from a file, derives its own
         state = self.__dict__.copy()
-        state.pop("_plan", None)
         state.update(_cache={}, _seen=bytearray(32))
         return state
 
@@ -177,19 +174,29 @@ class MixedQLinear(torch.nn.Module):
         """(codes, meta, outliers) of producer(x) with this layer's columns; its ids are settled: ``_to_u16`` made them on the
         host and copied them synchronously."""
         i16, f16 = self._idx16()
-        if self._plan is not None and (self._plan[0] is None or self._plan[1] is None):
-            self._plan = None            # made before the ids were: the layer's next launch makes it again
+        plan = self._plan
+        if plan is not None and (plan[0] is None or plan[1] is None):
+            del self._cache["plan"]      # made before the ids were: the layer's next launch makes it again
         return _lib.host().quantize(producer, x, aux, eps, i16, f16, self.bits, wide, True)
+
+    @property
+    def _plan(self):
+        """Derived operands for the native host path (see _make_plan), part of the layer's cache and dropped with it."""
+        return self._cache.get("plan")
 
     def _make_plan(self):
         """What the native host path needs of this layer beside its buffers: 16-bit column ids and weight codes one per byte, each
         where this layer has derived them, and the buffers that these come from.  It reads the buffers itself on every call
         and declines where they are others or something is missing: the layer's own path then runs, and ends here again.  Nothing
-        is derived here: a member of a group whose input another member quantizes needs no ids, and may not even have any."""
-        self._plan = None
+        is derived here: a member of a group whose input another member quantizes needs no ids, and may not even have any.  No plan
+        where none could serve: the path is not taken, or what it reads is not a buffer of the layer."""
+        self._cache.pop("plan", None)
+        if self.out_buffer is not None or MixedQLinear.launch_hook is not None:
+            return
         b = self._buffers
-        sources = b.get("int_indices"), b.get("fp_indices"), b.get("int_weight"), *([b.get("fp_weight")] if self.fp_features_num > 0 else [])
-        if self.out_buffer is not None or MixedQLinear.launch_hook is not None or any(t is None or t.is_inference() for t in sources):
+        sources = [b.get(n) for n in ("int_indices", "fp_indices", "int_weight", "fp_weight")[:4 if self.fp_features_num > 0 else 3]]
+        if "bias" not in b or b.get("weights_scales") is None or b.get("reduced_w") is None \
+                or any(t is None or t.is_inference() for t in sources):
             return
         host = _lib.host()
         key = host.sources(*sources)
@@ -197,7 +204,7 @@ class MixedQLinear(torch.nn.Module):
         def derived(name, src):
             ent = self._cache.get(name)
             return ent[1] if ent is not None and host.same_sources(ent[0], src) else None
-        self._plan = (*map(derived, ("int16", "fp16", "w8"), sources), key)
+        self._cache["plan"] = (*map(derived, ("int16", "fp16", "w8"), sources), key)
 
     def _weights_record(self):
         """The record of the weights of this layer's last call for few tokens, emptied where they are other tensors since: the record
@@ -247,7 +254,7 @@ class MixedQLinear(torch.nn.Module):
 
     # ------------------------------------------------------------------ forward
     def forward(self, x):
-        plan = self._plan
+        plan = self._cache.get("plan")
         if plan is not None and self.fused and not self.symmetric and MixedQLinear.launch_hook is None and self.out_buffer is None:
             shared_input = self.shared_input
             if shared_input is None:

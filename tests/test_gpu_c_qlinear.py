@@ -1,5 +1,6 @@
 """GPU parity: MixedQLinear.forward (fused, unfused, shared input, small-M, bf16) vs the CPU oracle."""
 import copy
+import weakref
 
 import pytest
 import torch
@@ -749,4 +750,30 @@ def test_quantized_weights_at_a_reused_address_are_waited_for(F):
     for rep in range(20):
         write(rep & 1)
         assert torch.equal(layer(x), want[rep & 1]), rep
+    assert_device_clean()
+
+
+def test_plans_only_where_they_can_serve():
+    """A plan goes with the layer's cache, and there is none for calls that the native path declines: a bias or weights that are no
+    buffers, an output buffer of the caller.  Outputs are the same either way."""
+    case = make_layer("t", 200, 1024 + 64, 264, 4, F=64, seed=3, device=dev(), clip=False)
+    layer, x = case.module, case.x.unsqueeze(0)
+    layer.bias = None
+    want = layer(x)
+    w8 = weakref.ref(layer._plan[2])
+    layer._cache.clear()
+    assert layer._plan is None and w8() is None
+    assert torch.equal(layer(x), want) and layer._plan is not None
+    layer.out_buffer = torch.empty_like(want[0])
+    assert torch.equal(layer(x), want) and layer._plan is None
+    layer.out_buffer = None
+    assert torch.equal(layer(x), want) and layer._plan is not None
+    for name in ("bias", "fp_weight", "reduced_w"):
+        value = layer._buffers.pop(name)
+        object.__setattr__(layer, name, value)
+        for _ in range(2):
+            assert torch.equal(layer(x), want) and layer._plan is None
+        object.__delattr__(layer, name)
+        layer.register_buffer(name, value)
+        assert torch.equal(layer(x), want) and layer._plan is not None
     assert_device_clean()
