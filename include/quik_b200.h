@@ -63,7 +63,8 @@ extern "C" {
  * it waits for the predecessor's completion before its first global load or store, so results are those of
  * plain stream order.  Two exceptions read constants before that wait: the ring streaming engine the weights (see
  * QUIK_CFG_STREAM_PRELOAD), and quik_layer_quantize the column ids where its caller states that they are settled.
- * 0 launches in plain stream order. */
+ * quik_asym_dequantize, quik_unpack_int4 and quik_rotary_inplace may start early too, but nothing starts before they are
+ * complete: to the launches after them they are ordinary kernels.  0 launches in plain stream order. */
 #define QUIK_CFG_PDL           5
 /* Accepted (1 or 2) for callers that set it and without effect: one warp issues every product of the tcgen05 engine, which
  * keeps the tensor pipe busy (512 to 545 cycles per 256 x 256 x 128 block of a CTA pair, 512 being the pipe's own time). */
@@ -75,8 +76,9 @@ extern "C" {
  * not wait for the kernel that produces the token codes.  1 (default): the weight tiles (w, fp_w) of the first ring fill are
  * loaded before that wait, the token tiles of the same stages after it (measured 56.8 against 58.1 us for the four
  * Llama-2-7B layers at 16 tokens).  The weights must therefore be settled: complete on the device when the call is made
- * (a captured launch: when its graph is launched), or followed on the stream by an ordinary kernel or copy, one without
- * programmatic dependence, before this library's launches.  0: only an L2 prefetch of the first tiles precedes the wait,
+ * (a captured launch: when its graph is launched), or written or followed on the stream by an ordinary kernel or copy, one
+ * that lets nothing start before it is complete, before this library's launches (of its own: any but the quantizers with column
+ * ids, the integer products, quik_fused_dequantize and quik_mixed_linear).  0: only an L2 prefetch of the first tiles precedes the wait,
  * the weights may be written by any earlier work of the stream; 2: like 1 plus an L2 prefetch of the later tiles
  * (measured slower: 60.7 us). */
 #define QUIK_CFG_STREAM_PRELOAD 8

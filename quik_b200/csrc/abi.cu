@@ -312,7 +312,7 @@ static int run_int4_gemm(const uint8_t *A, const uint8_t *B, int M, int N, int K
   int8_t *b8 = a8 + align256((size_t)M * K);
   const int engine = g_engine.load();
   const bool on_chip = engine == QUIK_ENGINE_TCGEN05_TS && aligned16(A);
-  const int rc = on_chip ? launch_unpack_int4(B, b8, N, K, st) : launch_unpack_int4_pair(B, b8, N, A, a8, M, K, st);
+  const int rc = launch_unpack_int4_operands(B, b8, N, on_chip ? nullptr : A, a8, on_chip ? 0 : M, K, st);
   if (rc != QUIK_OK) return rc;
   if (on_chip) return launch_gemm_tcgen05_ts(A, 1, b8, M, N, K, ep, st);
   return run_int8_gemm(a8, b8, M, N, K, ep, st);

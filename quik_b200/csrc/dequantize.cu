@@ -15,12 +15,12 @@ __device__ __forceinline__ float dequant_value(int acc, float srow, float zrow, 
 }
 
 // Rows by 32-bit division wherever the matrix allows (a 64-bit one costs more than the eight values it is for), and a dependent
-// launch: what the kernel reads comes after its wait, by ordinary loads of pointers that are not declared constant.
+// launch: what the kernel reads comes after its wait, by ordinary loads of pointers that are not declared constant.  Launches after
+// it start when it is complete: its result may be a layer's outlier weights, which the ring streaming engine loads before its wait.
 template <typename T, int VEC, typename Index>
 __global__ void asym_dequantize_kernel(const int32_t *x, const T *meta, const T *scale_col, const T *wred, const T *y, T *__restrict__ out,
                                        Index total, int cols, float shift) {
   const unsigned cvec = (unsigned)cols / VEC;
-  pdl_launch_dependents();
   pdl_wait();
   for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (Index)gridDim.x * blockDim.x) {
     const int r = (int)(i / cvec), c0 = (int)(i % cvec) * VEC;
@@ -109,9 +109,11 @@ __device__ __forceinline__ void unpack_matrix(const Unpack &m, size_t first, siz
   }
 }
 // The int4 product widens both operands before it starts: one launch for the two, which the product's own setup overlaps (two
-// ordinary launches before).
+// ordinary launches before).  RELEASE: the product may start early.  Not where the caller has a matrix widened: it may be a layer's
+// weights, which the ring streaming engine loads before its wait.
+template <bool RELEASE>
 __global__ void unpack_int4_kernel(const Unpack a, const Unpack b, int vec) {
-  pdl_launch_dependents();
+  if (RELEASE) pdl_launch_dependents();
   pdl_wait();
   const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
   unpack_matrix(a, first, step, vec & 1);
@@ -167,19 +169,23 @@ int launch_sym_dequantize(const void *x, int x_bits, const void *scale_row, cons
   return check_launch("sym_dequantize_kernel");
 }
 
-int launch_unpack_int4(const uint8_t *src, int8_t *dst, int rows, int cols, cudaStream_t st) {
-  return launch_unpack_int4_pair(src, dst, rows, nullptr, nullptr, 0, cols, st);
-}
-
-int launch_unpack_int4_pair(const uint8_t *a, int8_t *a8, int rows_a, const uint8_t *b, int8_t *b8, int rows_b, int cols, cudaStream_t st) {
-  const Unpack ua{a, a8, (size_t)rows_a * (cols / 2)}, ub{b, b8, (size_t)rows_b * (cols / 2)};
+template <bool RELEASE>
+static int launch_unpack(const Unpack &ua, const Unpack &ub, cudaStream_t st) {
   if (ua.nbytes + ub.nbytes == 0) return QUIK_OK;
   auto vec = [](const Unpack &m) { return (m.nbytes % 16 == 0) && aligned16(m.src) && aligned16(m.dst); };
   const size_t steps_a = vec(ua) ? ua.nbytes / 16 : ua.nbytes, steps_b = vec(ub) ? ub.nbytes / 16 : ub.nbytes;
   const int threads = 256;
   LaunchCfg lc(dim3(ew_grid(steps_a > steps_b ? steps_a : steps_b, threads)), dim3(threads), 0, st);
-  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, unpack_int4_kernel, ua, ub, (int)vec(ua) | (int)vec(ub) << 1));
+  QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, unpack_int4_kernel<RELEASE>, ua, ub, (int)vec(ua) | (int)vec(ub) << 1));
   return check_launch("unpack_int4_kernel");
+}
+
+int launch_unpack_int4(const uint8_t *src, int8_t *dst, int rows, int cols, cudaStream_t st) {
+  return launch_unpack<false>(Unpack{src, dst, (size_t)rows * (cols / 2)}, Unpack{nullptr, nullptr, 0}, st);
+}
+
+int launch_unpack_int4_operands(const uint8_t *a, int8_t *a8, int rows_a, const uint8_t *b, int8_t *b8, int rows_b, int cols, cudaStream_t st) {
+  return launch_unpack<true>(Unpack{a, a8, (size_t)rows_a * (cols / 2)}, Unpack{b, b8, (size_t)rows_b * (cols / 2)}, st);
 }
 
 }  // namespace quik

@@ -15,8 +15,7 @@ template <typename T>
 __global__ void rotary_kernel(T *q, T *k, const T *cos_t, const T *sin_t, int tokens, int q_heads, int k_heads, int head_dim) {
   const int half = head_dim / 2;
   const unsigned vec_per_head = (unsigned)half / 8, pieces = (unsigned)(q_heads + k_heads) * vec_per_head;
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();      // (launches after this one start when it is complete)
   for (int t = blockIdx.x; t < tokens; t += gridDim.x) {
     for (unsigned i = threadIdx.x; i < pieces; i += blockDim.x) {
       const int h = (int)(i / vec_per_head), v = (int)(i - (unsigned)h * vec_per_head);

@@ -777,3 +777,48 @@ def test_plans_only_where_they_can_serve():
         layer.register_buffer(name, value)
         assert torch.equal(layer(x), want) and layer._plan is not None
     assert_device_clean()
+
+
+@pytest.mark.parametrize("writer", ["unpack", "dequantize", "rotary"])
+def test_operators_before_a_launch_settle_its_weights(writer):
+    """The ring engine loads its weights before it waits for the stream.  Weights that the widening, dequantize or rotary operator has
+    just written are used as written: nothing starts before those operators are complete (calls of the C interface, which has no
+    record of weights)."""
+    M, F, N = 16, 64, 8192
+    K = 4096 + F
+    case = make_layer("t", M, K, N, 8, F=F, seed=5, device=dev(), clip=False)
+    layer, lib = case.module, _lib.load()
+    i16, f16 = layer._idx16()
+    w, fw, p, st = layer.int_weight.clone(), layer.fp_weight.clone(), _lib.ptr, _lib.stream_of(case.x)
+    q, meta = torch.empty(M, K - F, dtype=torch.int8, device=dev()), torch.empty(2 * M, dtype=torch.float16, device=dev())
+    fp_x, out = torch.empty(M, F, dtype=torch.float16, device=dev()), torch.empty(M, N, dtype=torch.float16, device=dev())
+    packed = [torch.randint(0, 256, (N, (K - F) // 2), dtype=torch.uint8, device=dev()) for _ in range(2)]
+    acc = [torch.randint(-99, 99, (N, F), dtype=torch.int32, device=dev()) for _ in range(2)]
+    ones, zeros = torch.ones(2 * N, dtype=torch.float16, device=dev()), torch.zeros(N * F, dtype=torch.float16, device=dev())
+    quarter = [torch.tensor(v, dtype=torch.float16, device=dev()).expand(N, F // 2).contiguous() for v in (0.0, 1.0)]
+
+    def write(i):
+        if writer == "unpack":
+            rc = lib.quik_unpack_int4(p(packed[i]), p(w), N, K - F, st)
+        elif writer == "dequantize":
+            rc = lib.quik_asym_dequantize(p(acc[i]), p(ones), p(ones), p(zeros), p(zeros), p(fw), 0, N, F, 8, st)
+        else:                                             # a quarter turn of every pair of columns
+            rc = lib.quik_rotary_inplace(p(fw), None, p(quarter[0]), p(quarter[1]), 0, N, 1, 0, F, st)
+        _lib.check(rc, writer)
+
+    def launch():
+        _lib.check(lib.quik_layer_quantize(0, p(case.x), None, 0.0, 0, M, K, p(i16), K - F, p(f16), F, 8, 1, 1, p(q), p(meta), p(fp_x), st),
+                   "quantize")
+        _lib.check(lib.quik_mixed_linear(p(q), 0, p(w), 0, p(meta), p(layer.weights_scales), p(layer.reduced_w), p(fp_x), p(fw), None,
+                                         p(out), 0, M, N, K - F, F, 8, st), "linear")
+        return out.clone()
+    want = []
+    for i in range(4):                                    # (four quarter turns come back to the start)
+        write(i & 1)
+        torch.cuda.synchronize()
+        want.append(launch())
+    assert not torch.equal(want[0], want[1])
+    for rep in range(40):
+        write(rep & 1)
+        assert torch.equal(launch(), want[rep % 4]), rep
+    assert_device_clean()
