@@ -44,7 +44,6 @@ constexpr int SW_A_COLS = 64;                      // 256 int8 codes per row = 6
 constexpr int SW_MAX_STAGES = 10;
 constexpr int SW_AUX_BYTES = 2048;                 // barriers, then the token scales
 constexpr int SW_SMEM_SM = 227 * 1024;
-constexpr int SW_BLOCKS_SAVED = 8;                 // that a second launch has to save (launch_stream_w)
 
 // Sizes that depend on the number of tokens (the MMA's N, a multiple of 16): shared-memory ring and tensor-memory plan.
 // Up to 64 tokens two CTAs may share an SM (256 tensor-memory columns and at most 113 KB each; the rule is in launch_stream_w),
@@ -614,14 +613,24 @@ int launch_stream_w(const void *q, const void *w, int bits, int M, int N, int K_
   }
   Epilogue e = ep;
   if (e.ldo <= 0) e.ldo = N;
-  // More slabs than run at once: the ones beyond the last full wave go to a launch of their own that splits K (its setup and first
-  // prefetch overlap the end of the first launch), where that takes at least eight blocks out of the chain.  A block is 0.55 us and
-  // the second launch costs about 4: 172 slabs of 4096 int4 columns, 96 tokens, 14 blocks saved: 30.5 -> 26.9 us; 197 slabs of 22752,
-  // 74 tokens, 46 saved: 112 -> 91; 217 slabs of 1536 columns, 4 saved: 18.2 -> 19.8.
+  // More slabs than run at once: the ones beyond the last full wave may go to a launch of their own that splits K (its setup and
+  // first prefetch overlap the end of the first launch, its loads come after).  It costs about 4 us and takes integer blocks out of the
+  // chain.  With one CTA per SM a block of the last wave is 0.5 us (int8: 0.25), however many slabs are left: at least 8
+  // (int8: 16) blocks have to go.  Two CTAs per SM share the weight stream: few slabs leave SMs with one CTA, whose blocks then
+  // come faster, and many fill the SMs anyway, so only up to a quarter of a wave, and for about twice the blocks.  From three full
+  // waves on CTAs do not end together any more, the last slabs start as SMs come free: twice the blocks again.
+  // One launch against two, us: 80 tokens, slabs beyond 148, columns (blocks saved): int4 37, 2048 (4) 24.0 / 24.7; 60, 4096 (8)
+  // 34.2 / 33.0; 18, 8192 (24) 51.5 / 42.3; 74, 16384 (32) 91.2 / 77.7; int8 37, 2048 (8) 25.5 / 25.6; 18, 4096 (24) 35.8 / 33.1.
+  // 20 tokens, beyond 296: int4 36, 4096 (12) 34.9 / 36.1; 36, 8192 (24) 55.9 / 53.7; 74, 16384 (32) 98.5 / 90.5; 120, 8192 (16)
+  // 57.3 / 60.2; int8 74, 4096 (16) 46.8 / 48.1; 36, 11008 (64) 99.0 / 89.0; 148, 11008 (43) 109 / 113.  (A line at 8 blocks for all, as
+  // it was before, took 5 us too long in places.  Of 700 drawn layers with up to half a wave beyond full ones, not those that the
+  // lines were drawn by, 308 now get two launches, one of them wrongly by more than 1 %: 1.6 %.)
   const int wave = sms * per_sm, beyond = slabs > wave ? slabs % wave : 0;
-  if (beyond > 0) {
-    const int s = choose_splits(per_sm, beyond);
-    if (total - (total + s - 1) / s >= SW_BLOCKS_SAVED) {
+  if (beyond > 0 && (per_sm == 1 || 4 * beyond <= wave)) {
+    const int s = choose_splits(per_sm, beyond), nk = total - nf;
+    int least = per_sm == 1 ? (bits == 4 ? 8 : 16) : (bits == 4 ? 20 : 32);
+    if (slabs >= 3 * wave) least *= 2;
+    if (nk - (nk + s - 1) / s >= least) {
       const int first = (slabs - beyond) * SW_ROWS;
       const int rc = launch_rows(q, w, bits, M, 0, first, K_int, e, per_sm, 1, st);
       if (rc != QUIK_OK) return rc;

@@ -822,3 +822,45 @@ def test_operators_before_a_launch_settle_its_weights(writer):
         write(rep & 1)
         assert torch.equal(launch(), want[rep % 4]), rep
     assert_device_clean()
+
+
+@pytest.mark.parametrize("M,slabs,K_int,F,bits,split", [
+    (80, 149, 4096, 0, 4, 8), (80, 222, 4096, 64, 4, 2), (80, 222, 3840, 64, 4, 0), (80, 223, 8192, 0, 4, 0), (80, 149, 2048, 64, 4, 0),
+    (128, 178, 2816, 64, 8, 4), (128, 178, 2688, 64, 8, 0), (80, 445, 4864, 0, 4, 8), (80, 445, 4608, 0, 4, 0),
+    (40, 370, 10240, 0, 4, 2), (40, 370, 9984, 0, 4, 0), (40, 371, 10240, 0, 4, 0), (64, 300, 6144, 64, 4, 8), (64, 300, 4608, 64, 4, 0),
+    (20, 370, 8192, 0, 8, 2), (20, 370, 8064, 0, 8, 0)])
+def test_streaming_engine_second_launch_is_chosen_by_what_it_saves(M, slabs, K_int, F, bits, split):
+    """Slabs beyond full waves split K in a launch of their own where that takes enough blocks out of the chain, up to a quarter of a
+    wave with two CTAs per SM, and for more blocks from three full waves on; both sides of each line.  The first CTA of the last launch counts its blocks: all of the layer's (split 0),
+    or its share.  The outputs are those of the tiled engine."""
+    N, d = 128 * slabs - 3, dev()
+    layer = MixedQLinear(K_int + F, 8, fp_features_num=F, bits=bits).to(d)
+    g = torch.Generator(device=d).manual_seed(slabs)
+    layer.out_features = N
+    if bits == 4:
+        layer.int_weight = torch.randint(0, 256, (N, K_int // 2), dtype=torch.uint8, device=d, generator=g)
+    else:
+        layer.int_weight = torch.randint(-128, 128, (N, K_int), dtype=torch.int8, device=d, generator=g)
+    layer.weights_scales = 0.01 + 0.01 * torch.rand(N, 1, device=d, generator=g).half()
+    layer.reduced_w = torch.randn(1, N, device=d, generator=g).half()
+    layer.bias = torch.randn(N, device=d, generator=g).half()
+    layer.int_indices, layer.fp_indices = torch.arange(K_int, device=d), torch.arange(K_int, K_int + F, device=d)
+    if F:
+        layer.fp_weight = torch.randn(N, F, device=d, generator=g).half()
+    x = torch.randn(1, M, K_int + F, device=d, generator=g).half()
+    counters = torch.zeros(16 * 1024, dtype=torch.int64, device=d)
+    try:
+        _lib.check(_lib.load().quik_debug_counters(counters.data_ptr()), "quik_debug_counters")
+        out = layer(x)
+        torch.cuda.synchronize()
+    finally:
+        _lib.load().quik_debug_counters(None)
+    total = K_int * bits // 1024 + F // 64
+    assert int(counters[3]) == (total // split if split else total)
+    try:
+        _lib.set_small_m(_lib.SMALL_M_OFF)
+        want = layer(x)
+    finally:
+        _lib.set_small_m(True)
+    assert rel_rms_err(out.cpu(), want.cpu()) < 5e-3
+    assert_device_clean()
