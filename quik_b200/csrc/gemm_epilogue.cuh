@@ -276,8 +276,7 @@ struct EpilogueWarp {
   // The same for rows without 16-byte alignment (an odd N): every row starts somewhere inside a 32-byte sector.  Its bytes pass
   // through a ring of two sectors per row in shared memory at the place that they have in memory, modulo 64; when piece c is in,
   // sector c of the row is complete and leaves as two 16-byte stores, and only the first and the last sector of the part are
-  // written in pieces.  (Element by element, 32 bytes of a row at a time, 3111 tokens through 1024 x 25036 took 226 us, now 192;
-  // 25040 columns took 164, now, by bulk stores, 151.)
+  // written in pieces.  (Element by element, 32 bytes of a row at a time, 3111 tokens through 1024 x 25036 took 194 us, now 160.)
   struct Sectors {
     int word;                // of the lane's own row: word of its sector that the part starts in,
     uint32_t turn;           // bits that the pieces are shifted by to words of memory,
@@ -323,21 +322,46 @@ struct EpilogueWarp {
   }
   template <int ELEM>
   __device__ __forceinline__ void edge_sector(const Rows &o, const Sectors &x, int c) const {
-#pragma unroll 1
+#pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int rr = 16 * k + (lane >> 1), off = (k ? x.off[1] : x.off[0]) + 32 * c;      // of the 16 bytes in the row
-      const unsigned char *from = s_stage + rr * EPI_RING_PITCH + 32 * (c & 1) + 16 * (lane & 1);
-      unsigned char *to = (k ? x.to[1] : x.to[0]) + 32 * c;
-      if (rr >= o.rows || off >= o.bytes || off <= -16) continue;
-      if (off >= 0 && off + 16 <= o.bytes) {
-        *reinterpret_cast<uint4 *>(to) = *reinterpret_cast<const uint4 *>(from);
+      const int rr = 16 * k + (lane >> 1), off = x.off[k] + 32 * c;      // of the 16 bytes in the row
+      const uint4 v = *reinterpret_cast<const uint4 *>(s_stage + rr * EPI_RING_PITCH + 32 * (c & 1) + 16 * (lane & 1));
+      unsigned char *to = x.to[k] + 32 * c;
+      const int first = -off, end = rr < o.rows ? o.bytes - off : 0;     // of the 16 bytes, those of the row
+      if (first <= 0 && end >= 16) {
+        *reinterpret_cast<uint4 *>(to) = v;
       } else {
-#pragma unroll 1
-        for (int b = max(0, -off); b < min(16, o.bytes - off); b += ELEM) {
-          if (ELEM == 2) *reinterpret_cast<uint16_t *>(to + b) = *reinterpret_cast<const uint16_t *>(from + b);
-          else *reinterpret_cast<uint32_t *>(to + b) = *reinterpret_cast<const uint32_t *>(from + b);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int b = 0; b < 16; b += ELEM) {
+          if (b < first || b >= end) continue;
+          if (ELEM == 2) *reinterpret_cast<uint16_t *>(to + b) = (uint16_t)(w[b / 4] >> (8 * (b & 2)));
+          else *reinterpret_cast<uint32_t *>(to + b) = w[b / 4];
         }
       }
+    }
+  }
+
+  // The same element by element, still 32 contiguous bytes of a row at a time: for parts of up to 64 columns (tiles of up to 128), of
+  // whose few sectors most are first or last ones.  (By sectors, and element by element: 136 tokens through 2368 x 4287, 64
+  // columns to a tile, 16.7 us, now 14.9; 430 through 1280 x 2109 13.6, now 11.9.  In tiles of 160 the two are equal, beyond that whole
+  // sectors gain.)
+  template <int ELEM>
+  __device__ __forceinline__ void store_elements(const Rows &o, int c, uint4 p0, uint4 p1) const {
+    __syncwarp();                            // the buffer has been read out
+    const int flip = (lane >> 2) & 1;
+    *reinterpret_cast<uint4 *>(s_stage + lane * 32 + 16 * flip) = p0;
+    *reinterpret_cast<uint4 *>(s_stage + lane * 32 + 16 * (flip ^ 1)) = p1;
+    __syncwarp();
+    constexpr int PER_ROW = 32 / ELEM, ROWS = 32 / PER_ROW;
+    const int off = (lane % PER_ROW) * ELEM;
+#pragma unroll 4
+    for (int k = 0; k < 32 / ROWS; ++k) {
+      const int rr = ROWS * k + lane / PER_ROW;
+      const unsigned char *from = s_stage + rr * 32 + 16 * ((off >> 4) ^ ((rr >> 2) & 1)) + (off & 15);
+      if (32 * c + off >= o.bytes || rr >= o.rows) continue;
+      if (ELEM == 2) *reinterpret_cast<uint16_t *>(o.row(rr) + 32 * c + off) = *reinterpret_cast<const uint16_t *>(from);
+      else *reinterpret_cast<uint32_t *>(o.row(rr) + 32 * c + off) = *reinterpret_cast<const uint32_t *>(from);
     }
   }
 
@@ -376,8 +400,8 @@ struct EpilogueWarp {
   }
 
   // `keep`: the kept outlier product, or room for the addend y of a tile without one
-  // STORES: SECTORS for any rows, ROWS for rows of 16-byte alignment, BULK for those where there is a map of the result
-  enum Stores { SECTORS, ROWS, BULK };
+  // STORES: SECTORS and ELEMENTS for any rows, ROWS for rows of 16-byte alignment, BULK for those where there is a map of the result
+  enum Stores { SECTORS, ELEMENTS, ROWS, BULK };
   template <int STORES>
   __device__ __forceinline__ void finish(int j, uint32_t (&keep)[COLS / 2], const Rows &o) {
     const Part t = part(j);
@@ -400,6 +424,7 @@ struct EpilogueWarp {
         auto piece = [&](int n, int odd, uint4 p0, uint4 p1) {      // odd: n & 1, known when this is compiled
           if (STORES == ROWS || (STORES == BULK && KIND != 0 && !odd && 32 * (n + 1) >= o.bytes)) store_aligned(o, n, p0, p1);
           else if (STORES == BULK) store_bulk(t, o, n, odd, p0, p1);
+          else if (STORES == ELEMENTS) store_elements<KIND == 0 ? 4 : 2>(o, n, p0, p1);
           else store_sector<KIND == 0 ? 4 : 2>(o, x, n, odd, 32 * (n + 1) >= o.bytes, p0, p1);
         };
         if (KIND == 0) {
@@ -445,7 +470,8 @@ struct EpilogueWarp {
   // all tiles of this CTA (the two forms of the stores share no code: held together they take 60 registers more)
   __device__ __forceinline__ void run(int n_local) {
     if (!p.vec_out) {
-      run_tiles<SECTORS>(n_local);
+      if (p.split_n <= 64) run_tiles<ELEMENTS>(n_local);
+      else run_tiles<SECTORS>(n_local);
     } else if (BULK_STORES) {
       run_tiles<BULK>(n_local);
       if (lane == 0) tma_store_wait_all();

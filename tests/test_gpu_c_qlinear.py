@@ -125,6 +125,40 @@ def test_rows_that_start_anywhere_in_a_sector(N, tile, pair, F):
     assert_device_clean()
 
 
+@pytest.mark.parametrize("F", [64, 0])
+@pytest.mark.parametrize("tile", [32, 128, 144, 224])
+@pytest.mark.parametrize("N", [3, 130, 257, 1021])
+def test_rows_without_alignment_by_tile_width(N, tile, F):
+    """Either side of the tile width up to which rows without 16-byte alignment are stored element by element, beyond it by sectors:
+    the outputs are those of the other side, and only the layer's columns are written; an int32 product too."""
+    M, K = 131, 224 + F
+    case = make_layer("t", M, K, N, 8, F=F, seed=N, device=dev(), clip=False)
+    g = torch.Generator().manual_seed(N)
+    a = torch.randint(-128, 128, (M, 208), generator=g, dtype=torch.int8)
+    b = torch.randint(-128, 128, (N, 208), generator=g, dtype=torch.int8)
+    try:
+        _lib.set_tile_n(80)
+        want = case.module(case.x.unsqueeze(0))[0].clone()
+        _lib.set_tile_n(tile)
+        for pair in (1, 2):
+            _lib.set_cta_pair(pair)
+            for off in (0, 1, 6, 15):
+                slab = torch.full((M, N + 16 + (off & 1)), -1234.0, dtype=torch.float16, device=dev())
+                case.module.out_buffer = slab[:, off:off + N]
+                case.module(case.x.unsqueeze(0))
+                assert torch.equal(slab[:, off:off + N], want), off
+                slab[:, off:off + N] = -1234.0
+                assert bool((slab == -1234.0).all()), off
+            c = matmul.int8Matmul(a.to(dev()), b.to(dev()))
+            assert torch.equal(c.cpu().long(), a.long() @ b.long().t())
+    finally:
+        case.module.out_buffer = None
+        _lib.set_tile_n(0)
+        _lib.set_cta_pair(0)
+    assert rel_rms_err(want.cpu(), _oracle_out(case, round_y=False)) < TOL_RMS
+    assert_device_clean()
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("M,K,N,F,bits", [
     (16, 256, 128, 0, 4), (16, 1280, 128, 256, 8), (1, 4352, 512, 256, 4), (16, 4352, 264, 256, 4), (7, 11264, 256, 256, 8),
