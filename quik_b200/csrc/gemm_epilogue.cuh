@@ -83,12 +83,14 @@ __device__ __forceinline__ uint64_t *region_barrier(int j, bool fp, uint64_t *ac
 
 // One epilogue warp.  Warp (sub, group) owns rows [32*sub, 32*sub+32) of the CTA's 128 rows of the tile and the
 // columns [cb, cb + cn), COLS at most, of it (group g: the g-th split_n columns).  It walks them 16 at a time.
-// KIND: 0 the int32 product as it is, 1 dequantize, 2 dequantize with an outlier product.  SHIFT: the integer accumulator holds the
+// KIND: 0 the int32 product as it is, 1 dequantize, 2 dequantize with an outlier product, 3 dequantize with an addend y.  SHIFT: the integer accumulator holds the
 // product times 2^SHIFT (operands widened on chip).
 // BULK_STORES: there is a map of the result for bulk stores.
+// (The addend has a kind of its own: its loads, eight times in the code, are fetched, or jumped over, by launches that have none.  As a
+// branch of kind 1 they cost layers without outliers 180 tokens x 2496 -> 12544 16.9 us, now 15.2; 402 x 3584 -> 4864 18.1, now 16.7.)
 template <typename T, int KIND, int SHIFT, int CTAS, int COLS, bool BULK_STORES>
 struct EpilogueWarp {
-  static constexpr bool HAS_FP = KIND == 2;
+  static constexpr bool HAS_FP = KIND == 2, HAS_Y = KIND == 3;
   static constexpr int CHUNKS = COLS / 16;
   static constexpr int LANE_COLS = COLS / 32;         // columns whose vectors a lane fetches
   const GemmParams &p;
@@ -276,7 +278,7 @@ struct EpilogueWarp {
   // The same for rows without 16-byte alignment (an odd N): every row starts somewhere inside a 32-byte sector.  Its bytes pass
   // through a ring of two sectors per row in shared memory at the place that they have in memory, modulo 64; when piece c is in,
   // sector c of the row is complete and leaves as two 16-byte stores, and only the first and the last sector of the part are
-  // written in pieces.  (Element by element, 32 bytes of a row at a time, 3111 tokens through 1024 x 25036 took 194 us, now 160.)
+  // written in pieces.  (Element by element, 32 bytes of a row at a time, 3111 tokens through 1024 x 25036 took 194 us, now 133.)
   struct Sectors {
     int word;                // of the lane's own row: word of its sector that the part starts in,
     uint32_t turn;           // bits that the pieces are shifted by to words of memory,
@@ -453,7 +455,7 @@ struct EpilogueWarp {
               a = Traits<T>::unpack(keep[8 * h + i / 2], i & 1);
             } else {
               a = s_bias[16 * c + i];
-              if (p.y != nullptr) a += Traits<T>::unpack(keep[8 * h + i / 2], i & 1);
+              if (HAS_Y) a += Traits<T>::unpack(keep[8 * h + i / 2], i & 1);
             }
             // out = acc * (s_row * s_col) + ((zero + shift * s_row) * w_red + addend), fused multiply-adds
             f[q] = fmaf((float)((int)v[i] >> SHIFT), srow * sc[q], fmaf(zs, wr[q], a));
@@ -463,7 +465,7 @@ struct EpilogueWarp {
         }
         piece(c, h, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
       }
-      if (HAS_FP || (KIND == 1 && p.y != nullptr)) rotate(keep);
+      if (HAS_FP || HAS_Y) rotate(keep);
     }
   }
 
@@ -489,7 +491,7 @@ struct EpilogueWarp {
       if (HAS_FP) drain(j, keep);
       if (!ok) break;
       const Part t = part(j);
-      if (KIND == 1 && p.y != nullptr) {
+      if (HAS_Y) {
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c)
           if (16 * c < t.lim) load_y(t, c, keep + 8 * c);

@@ -468,6 +468,7 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   if (K % 16 != 0 || K <= 0) return QUIK_ERR_SHAPE;
   if (!aligned16(A) || !aligned16(B)) return QUIK_ERR_ALIGN;
   const bool has_fp = ep.mode == 1 && ep.fp_a != nullptr && ep.F > 0;
+  if (ep.y != nullptr && (has_fp || ep.dtype != QUIK_F16)) return QUIK_ERR_UNSUPPORTED;      // no operator asks for it
   if (has_fp && (ep.F % 8 != 0 || !aligned16(ep.fp_a) || !aligned16(ep.fp_b))) return QUIK_ERR_ALIGN;
 
   GemmParams p{};
@@ -521,6 +522,7 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
     QUIK_LAUNCH(__nv_bfloat16, 1);
   }
   if (has_fp) QUIK_LAUNCH(__half, 2);
+  if (ep.y) QUIK_LAUNCH(__half, 3);
   QUIK_LAUNCH(__half, 1);
 #undef QUIK_LAUNCH_C
 #undef QUIK_LAUNCH

@@ -371,6 +371,7 @@ int launch_gemm_tcgen05_ts(const void *A, int a_packed, const int8_t *B, int M, 
   if (K <= 0 || K % (a_packed ? 32 : 16) != 0) return QUIK_ERR_SHAPE;
   if (!aligned16(A) || !aligned16(B)) return QUIK_ERR_ALIGN;
   const bool has_fp = ep.mode == 1 && ep.fp_a != nullptr && ep.F > 0;
+  if (ep.y != nullptr && (has_fp || ep.dtype != QUIK_F16)) return QUIK_ERR_UNSUPPORTED;      // no operator asks for it
   if (has_fp && (ep.F % 8 != 0 || !aligned16(ep.fp_a) || !aligned16(ep.fp_b))) return QUIK_ERR_ALIGN;
 
   GemmParams p{};
@@ -419,6 +420,7 @@ int launch_gemm_tcgen05_ts(const void *A, int a_packed, const int8_t *B, int M, 
     QUIK_TS(__nv_bfloat16, 1);
   }
   if (has_fp) QUIK_TS(__half, 2);
+  if (ep.y) QUIK_TS(__half, 3);
   QUIK_TS(__half, 1);
 #undef QUIK_TS_P
 #undef QUIK_TS
