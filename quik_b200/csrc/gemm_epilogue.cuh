@@ -101,7 +101,7 @@ struct EpilogueWarp {
   int lane, sub;
   int cb, cn;
   float *s_scol, *s_wred, *s_bias;   // [COLS] each, private to this warp
-  unsigned char *s_stage;            // 32 x 32 bytes, private to this warp
+  unsigned char *s_stage;            // EPI_BUF_BYTES, private to this warp: 32 rows x 32 bytes, a box of 32 x 64, or 32 rings of 64
   uint64_t *acc_full, *acc_empty, *fp_full, *fp_drained;
   volatile int *abort_flag;
   float srow = 0.f, zs = 0.f;        // of this lane's row: scale, zero + shift * scale
@@ -193,8 +193,8 @@ struct EpilogueWarp {
 
   // The kept words move on by two chunks, so that loops over the chunks need not be unrolled to name them.  Code is fetched from
   // L2, or from memory where weights have streamed through L2 since the last launch, and most launches have one or two tiles per
-  // CTA: unrolled eight times, the epilogue's code took longer to arrive than to run (the four layers of Llama-2-7B at 333 tokens: 148.5
-  // us, in loops 136.9).
+  // CTA: unrolled eight times, the epilogue's code took longer to arrive than to run (the four layers of Llama-2-7B at 333 tokens: 147.5
+  // us, in loops 134.2).
   __device__ __forceinline__ static void rotate(uint32_t (&keep)[COLS / 2]) {
 #pragma unroll
     for (int i = 0; i < COLS / 2 - 16; ++i) keep[i] = keep[i + 16];
@@ -527,9 +527,6 @@ struct EpilogueWarp {
 };
 
 // ---- host helpers shared by the launchers -----------------------------------------------------
-struct TileGeometry {
-  int ctas, block_n;
-};
 // fills the shape-independent fields of GemmParams from the epilogue description
 inline void fill_epilogue_params(GemmParams &p, const Epilogue &ep, int M, int N) {
   p.M = M;

@@ -398,8 +398,10 @@ int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tf
 // tenths of that without an outlier product; a fifth more in pairs, whose regions are free when both CTAs are done), and with few
 // k-blocks that is the longer one.  Pairs also start and end 900 ns later.  So a narrower tile only pays where it saves a wave or where epilogues bound the launch; among
 // equals the widest is taken, and pairs before singles.  Fitted to all widths of 24 problems of 200 to 4096 tokens, 896 to 18208 integer
-// columns, and to the choices of earlier constants on 60 more: the choice costs 0.5 % more than the best width on average (one rule for
-// singles and pairs and no epilogue: 2.9 %; 333 tokens through 11008 x 4096 33.5 us, now 29.1, 777 through 4096 x 6912 32.1, now 27.1).
+// columns.  On 1686 drawn problems of 129 to 4096 tokens, the two narrowest widths of each number of waves timed for singles and
+// pairs, the choice costs 0.9 % more than the best of them on average, 11 % at worst (one rule for singles and pairs and no epilogue:
+// 3.4 and 23 %; constants refitted to 3985 others: 0.9).  Problems of one wave of 32-column tiles are where it errs most often, to
+// either side by up to 5 %.  333 tokens through 11008 x 4096 33.5 us, now 29.1, 777 through 4096 x 6912 32.1, now 27.1.
 double tile_cost(int M, int N, int kblocks, bool outliers, int ctas, int bn, int units) {
   const int tile_m = BLOCK_M * ctas;
   const long long tiles = (long long)((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);

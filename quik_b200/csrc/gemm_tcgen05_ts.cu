@@ -90,7 +90,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(acc_full + s), 1);
-      mbar_init(smem_u32(acc_empty + s), TS_EPI_WARPS * CTAS);    // epilogue threads of the whole pair
+      mbar_init(smem_u32(acc_empty + s), TS_EPI_WARPS * CTAS);    // epilogue warps of the whole pair
       mbar_init(smem_u32(fp_full + s), 1);
       mbar_init(smem_u32(fp_drained + s), TS_EPI_WARPS * CTAS);
     }
