@@ -85,10 +85,13 @@ __device__ __forceinline__ uint64_t *region_barrier(int j, bool fp, uint64_t *ac
 // columns [cb, cb + cn), COLS at most, of it (group g: the g-th split_n columns).  It walks them 16 at a time.
 // KIND: 0 the int32 product as it is, 1 dequantize, 2 dequantize with an outlier product, 3 dequantize with an addend y.  SHIFT: the integer accumulator holds the
 // product times 2^SHIFT (operands widened on chip).
-// BULK_STORES: there is a map of the result for bulk stores.
+// ROWS_ARE: of what alignment the result's rows are; ALIGNED: 16 bytes, and there is a map of the result for bulk stores.  (Known when
+// the kernel is compiled, as is the tile's capacity, by which unaligned rows are stored: over 1132 drawn layers 1.3 % faster than all
+// forms of the stores in one kernel; 741 tokens through 5152 x 3333 28.2 us, now 27.6.)
 // (The addend has a kind of its own: its loads, eight times in the code, are fetched, or jumped over, by launches that have none.  As a
 // branch of kind 1 they cost layers without outliers 180 tokens x 2496 -> 12544 16.9 us, now 15.2; 402 x 3584 -> 4864 18.1, now 16.7.)
-template <typename T, int KIND, int SHIFT, int CTAS, int COLS, bool BULK_STORES>
+enum RowAlignment { ANY, ALIGNED, UNALIGNED };
+template <typename T, int KIND, int SHIFT, int CTAS, int COLS, int ROWS_ARE>
 struct EpilogueWarp {
   static constexpr bool HAS_FP = KIND == 2, HAS_Y = KIND == 3;
   static constexpr int CHUNKS = COLS / 16;
@@ -344,8 +347,8 @@ struct EpilogueWarp {
     }
   }
 
-  // The same element by element, still 32 contiguous bytes of a row at a time: for parts of up to 64 columns (tiles of up to 128), of
-  // whose few sectors most are first or last ones.  (By sectors, and element by element: 136 tokens through 2368 x 4287, 64
+  // The same element by element, still 32 contiguous bytes of a row at a time: for parts of up to 64 columns (COLS: tiles of up to
+  // 128), of whose few sectors most are first or last ones.  (By sectors, and element by element: 136 tokens through 2368 x 4287, 64
   // columns to a tile, 16.7 us, now 14.9; 430 through 1280 x 2109 13.6, now 11.9.  In tiles of 160 the two are equal, beyond that whole
   // sectors gain.)
   template <int ELEM>
@@ -469,16 +472,15 @@ struct EpilogueWarp {
     }
   }
 
-  // all tiles of this CTA (the two forms of the stores share no code: held together they take 60 registers more)
+  // all tiles of this CTA
   __device__ __forceinline__ void run(int n_local) {
-    if (!p.vec_out) {
-      if (p.split_n <= 64) run_tiles<ELEMENTS>(n_local);
-      else run_tiles<SECTORS>(n_local);
-    } else if (BULK_STORES) {
+    if (ROWS_ARE == ALIGNED) {
       run_tiles<BULK>(n_local);
       if (lane == 0) tma_store_wait_all();
-    } else {
+    } else if (ROWS_ARE == ANY && p.vec_out) {
       run_tiles<ROWS>(n_local);
+    } else {
+      run_tiles<COLS <= 64 ? ELEMENTS : SECTORS>(n_local);
     }
   }
   template <int STORES>

@@ -72,8 +72,8 @@ constexpr int num_stages(int cap_n, int ctas) {
 // loads its own 128 rows of A and only its half of the B rows, so a CTA moves a third less operand
 // data per multiply-accumulate than alone.  The leader (cluster rank 0) issues the MMAs for the pair
 // and owns the barriers that count loads and region releases; commits reach both CTAs.
-// KIND: what becomes of the integer product, see EpilogueWarp.
-template <typename T, int CAP_N, int KIND, int CTAS>
+// KIND, ROWS_ARE: what becomes of the integer product and how it is stored, see EpilogueWarp.
+template <typename T, int CAP_N, int KIND, int CTAS, int ROWS_ARE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_fa, const __grid_constant__ CUtensorMap tmap_fb,
@@ -124,7 +124,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     prefetch_tmap(&tmap_a);
     prefetch_tmap(&tmap_b);
-    if (p.vec_out) prefetch_tmap(&tmap_out);
+    if (ROWS_ARE == ALIGNED) prefetch_tmap(&tmap_out);
     if (HAS_FP) {
       prefetch_tmap(&tmap_fa);
       prefetch_tmap(&tmap_fb);
@@ -148,7 +148,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp >= 4) {
     // ================= epilogue (warps 4..11): gemm_epilogue.cuh =================
     set_max_regs_up<REGS_EPILOGUE>();
-    EpilogueWarp<T, KIND, 0, CTAS, EPI_COLS(CAP_N), true> ew(p, &tmap_out, tmem_base, CAP_N, unit, num_units, rank, warp - 4, warp & 3, lane, s_vec,
+    EpilogueWarp<T, KIND, 0, CTAS, EPI_COLS(CAP_N), ROWS_ARE> ew(p, &tmap_out, tmem_base, CAP_N, unit, num_units, rank, warp - 4, warp & 3, lane, s_vec,
                                                        s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
     ew.run(n_local);
     if (p.dbg && warp == 4 && lane == 0) ew.write_counters((int)blockIdx.x);
@@ -354,7 +354,7 @@ int max_pairs(Kern kern, size_t smem) {
 
 // Units (CTAs, or CTA pairs) of one kernel instantiation that are resident at once on the current device.
 // The shared-memory opt-in and the occupancy answer belong to a device, so they are kept per device ordinal.
-template <typename T, int CAP_N, int KIND, int CTAS>
+template <typename T, int CAP_N, int KIND, int CTAS, int ROWS_ARE>
 int resident_units(int *out) {
   static std::mutex mu;
   static int cached[kMaxDevices];       // 0 = not asked yet, -1 = cannot launch
@@ -363,7 +363,7 @@ int resident_units(int *out) {
   if (dev < 0 || dev >= kMaxDevices) return QUIK_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lock(mu);
   if (cached[dev] == 0) {
-    auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS>;
+    auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS, ROWS_ARE>;
     constexpr size_t smem = smem_bytes(CAP_N, CTAS);
     cudaFuncAttributes at;
     QUIK_CUDA_TRY(cudaFuncGetAttributes(&at, kern));
@@ -376,13 +376,13 @@ int resident_units(int *out) {
   return QUIK_OK;
 }
 
-template <typename T, int CAP_N, int KIND, int CTAS>
+template <typename T, int CAP_N, int KIND, int CTAS, int ROWS_ARE>
 int launch_t(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tfa, const CUtensorMap &tfb,
              const CUtensorMap &to, const GemmParams &p, cudaStream_t st) {
-  auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS>;
+  auto kern = gemm_tcgen05_kernel<T, CAP_N, KIND, CTAS, ROWS_ARE>;
   constexpr size_t smem = smem_bytes(CAP_N, CTAS);
   int resident = 0;
-  const int rc = resident_units<T, CAP_N, KIND, CTAS>(&resident);
+  const int rc = resident_units<T, CAP_N, KIND, CTAS, ROWS_ARE>(&resident);
   if (rc != QUIK_OK) return rc;
   if (resident <= 0) return QUIK_ERR_UNSUPPORTED;
   const int units = p.num_tiles < resident ? p.num_tiles : resident;
@@ -511,8 +511,13 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
     else rc = make_tmap(&to, ep.out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, M, N, 32, 64, p.ldo);
     if (rc != QUIK_OK) return rc;
   }
-#define QUIK_LAUNCH_C(T, K, C) \
-  return cap_n == 256 ? launch_t<T, 256, K, C>(ta, tb, tfa, tfb, to, p, st) : launch_t<T, 128, K, C>(ta, tb, tfa, tfb, to, p, st)
+#define QUIK_LAUNCH_R(T, K, C, R) \
+  return cap_n == 256 ? launch_t<T, 256, K, C, R>(ta, tb, tfa, tfb, to, p, st) : launch_t<T, 128, K, C, R>(ta, tb, tfa, tfb, to, p, st)
+#define QUIK_LAUNCH_C(T, K, C)                      \
+  do {                                              \
+    if (p.vec_out) QUIK_LAUNCH_R(T, K, C, ALIGNED); \
+    QUIK_LAUNCH_R(T, K, C, UNALIGNED);              \
+  } while (0)
 #define QUIK_LAUNCH(T, K)                  \
   do {                                     \
     if (ctas == 2) QUIK_LAUNCH_C(T, K, 2); \
@@ -526,6 +531,7 @@ int launch_gemm_tcgen05(const int8_t *A, const int8_t *B, int M, int N, int K, c
   if (has_fp) QUIK_LAUNCH(__half, 2);
   if (ep.y) QUIK_LAUNCH(__half, 3);
   QUIK_LAUNCH(__half, 1);
+#undef QUIK_LAUNCH_R
 #undef QUIK_LAUNCH_C
 #undef QUIK_LAUNCH
 }

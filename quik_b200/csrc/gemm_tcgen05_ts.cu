@@ -258,7 +258,7 @@ gemm_tcgen05_ts_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
   } else {
     // ================= epilogue (warps 6..13): gemm_epilogue.cuh =================
-    EpilogueWarp<T, KIND, A_PACKED ? 4 : 0, CTAS, TS_HALF_CAP, false> ew(p, nullptr, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec,
+    EpilogueWarp<T, KIND, A_PACKED ? 4 : 0, CTAS, TS_HALF_CAP, ANY> ew(p, nullptr, tmem_base, bn, unit, num_units, rank, warp - 6, warp & 3, lane, s_vec,
                                                                    s_out, acc_full, acc_empty, fp_full, fp_drained, abort_flag);
     ew.run(n_local);
     if (p.dbg && warp == 6 && lane == 0) ew.write_counters((int)blockIdx.x);
