@@ -533,7 +533,7 @@ def measure_workload(args, wl, peaks, i8peaks, rank, world, dev, sync_all, sampl
                              "shape": f"{c.K}->{c.N} int{c.bits}"}
     tensor_bound = M > 128
     achieved = gemm_ops / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else 0.0
-    peak, peak_src = i8peaks["sustained"]
+    peak, peak_src = i8peaks["burst"]
     traffic = None
     if world == 1:
         t = [NCU_TRAFFIC_BYTES.get((M, c.K, c.N)) for c in wl.cases]
@@ -551,9 +551,10 @@ def measure_workload(args, wl, peaks, i8peaks, rank, world, dev, sync_all, sampl
                     "traffic_source": traffic_source,
                     "algorithmic_bytes_per_launch": kernel_alg_bytes,
                     "kernel": "gemm_tcgen05_kernel (fused int8 GEMM + fp16 outlier GEMM + dequantize)",
-                    "peak_source": f"sustained figure (the launches are timed inside a long region): {peak_src}; "
-                                   f"nominal dense int8 is 4500",
+                    "peak_source": f"burst figure: {peak_src}; nominal dense int8 is 4500 (twice the sustained bf16 rate is no "
+                                   f"bound: int8 products draw less power, and the launches read above it)",
                     "frac_of_burst_peak": achieved / i8peaks["burst"][0],
+                    "frac_of_sustained_proxy": achieved / i8peaks["sustained"][0],
                     "frac_of_nominal_4500": achieved / 4500.0,
                     "per_layer": per_layer,
                     "timing": f"CUDA events around each launch of the kernel over {eager_steps} eagerly launched steps "
