@@ -176,7 +176,7 @@ class MixedQLinear(torch.nn.Module):
         i16, f16 = self._idx16()
         plan = self._plan
         if plan is not None and (plan[0] is None or plan[1] is None):
-            del self._cache["plan"]      # made before the ids were: the layer's next launch makes it again
+            self._cache.pop("plan", None)      # made before the ids were: the layer's next launch makes it again
         return _lib.host().quantize(producer, x, aux, eps, i16, f16, self.bits, wide, True)
 
     @property
