@@ -14,7 +14,7 @@ __device__ __forceinline__ float dequant_value(int acc, float srow, float zrow, 
   return __fadd_rn(xe, __fadd_rn(sh, y));
 }
 
-// Rows by 32-bit division wherever the matrix allows (a 64-bit one costs more than the eight values it is for), and a dependent
+// Rows by 32-bit division wherever the matrix allows (a 64-bit one costs more than the eight values it is for).  It may be a dependent
 // launch: what the kernel reads comes after its wait, by ordinary loads of pointers that are not declared constant.  Launches after
 // it start when it is complete: its result may be a layer's outlier weights, which the ring streaming engine loads before its wait.
 template <typename T, int VEC, typename Index>
@@ -140,6 +140,11 @@ int launch_asym_dequantize(const int32_t *x, const void *meta, const void *scale
   const size_t total = (size_t)rows * (vec ? cols / 8 : cols);
   const bool small = total < ((size_t)1 << 31);
   LaunchCfg lc(dim3(grid), dim3(threads), 0, st);
+  // A dependent launch for small matrices only.  Its blocks take the SMs as the product's blocks leave them and wait there, and from some size
+  // on that costs more than the early start gives.  Product and this, us, dependent and ordinary launch: int32 result of 73 MB 68.6 / 56.8,
+  // 144 MB 168 / 145, 187 MB 177 / 140; quantizer, int4 product and this over drawn sizes, speed of the ordinary launch against the
+  // dependent one: below 4 MB 0.992, to 16 MB 0.993, to 40 MB 1.002, beyond 1.02.
+  if ((size_t)rows * cols * 4 > ((size_t)16 << 20)) lc.cfg.numAttrs = 0;
 #define QUIK_DQ_I(T, V, I)                                                                                                     \
   QUIK_CUDA_TRY(cudaLaunchKernelEx(&lc.cfg, asym_dequantize_kernel<T, V, I>, x, static_cast<const T *>(meta),                  \
                                    static_cast<const T *>(scale_col), static_cast<const T *>(w_reduced),                       \
